@@ -105,15 +105,108 @@ __device__ __forceinline__ d3 jl_inv_t(d3 p, d3 v) {
     return (v + c1 * .5) + c2 * A;
 }
 
+// ---- FP64 arithmetic for a narrow FP64 pipe -----------------------------------------------
+// GB300 issues one FP64 warp instruction per 19 cycles and SM (measured: 64 cycles on each of
+// the four sub-partitions alone, adds, multiplies, compares and conversions alike), while the
+// integer and FP32 pipes idle beside it.  So comparisons, sign changes, halvings and
+// conversions are done on the bit patterns, and square roots start from the FP32 estimate.
+
+// v > 0 (false for NaN, as the comparison).
+__device__ __forceinline__ bool positive(double v) {
+    return (unsigned long long)(__double_as_longlong(v) - 1) < 0x7ff0000000000000ULL;
+}
+// a < b for non-negative a and b (false where a is NaN).
+__device__ __forceinline__ bool less_bits(double a, double b) { return __double_as_longlong(a) < __double_as_longlong(b); }
+__device__ __forceinline__ bool negative_sign(double v) { return __double2hiint(v) < 0; }
+// v with the sign bit of s xored in.
+__device__ __forceinline__ double xor_sign(double v, double s) {
+    return __hiloint2double(__double2hiint(v) ^ (__double2hiint(s) & int(0x80000000u)), __double2loint(v));
+}
+// v / 2 for a normal v above the smallest exponent.
+__device__ __forceinline__ double half_of(double v) {
+    return __hiloint2double(__double2hiint(v) - 0x00100000, __double2loint(v));
+}
+// |v - 1| < 2^-20: a squared norm whose square root is 1 + (v - 1) / 2 to FP64 precision when
+// it differs from one by rounding only.
+__device__ __forceinline__ bool near_one(double v) {
+    return unsigned(__double2hiint(v)) - 0x3feffffeu < 4u;
+}
+// a in [2^-111, 2^98): its FP32 estimate below neither overflows nor loses bits.
+__device__ __forceinline__ bool rsqrt_range(double a) {
+    return unsigned(__double2hiint(a)) - 0x39000000u < 0x0d100000u;
+}
+// 1 / sqrt(a), a in rsqrt_range: the FP32 estimate y0 of the truncated a (relative error below
+// 2^-21), then one third-order step y = y0 (1 + e / 2 + 3 e^2 / 8), e = 1 - a y0^2 (the binomial
+// series of (1 - e)^(-1/2); what is left is of order e^3 < 2^-60).  Five FP64 instructions.
+__device__ __forceinline__ double rsqrt_est(double a) {
+    const float f = __int_as_float(int(__funnelshift_l(__double2loint(a), __double2hiint(a) - 0x38000000, 3)));
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(f));
+    const int b = __float_as_int(y);
+    const double y0 = __hiloint2double((b >> 3) + 0x38000000, b << 29);
+    const double e = fma(-(a * y0), y0, 1.0);
+    return fma(y0 * e, fma(.375, e, .5), y0);
+}
+// sqrt(a) from y = rsqrt_est(a): a y corrected by its residual (P. Markstein, IBM J. Res. Dev.
+// 34 (1990) 111), correctly rounded but for rare cases.
+__device__ __forceinline__ double sqrt_from(double a, double y) {
+    const double g = a * y;
+    return fma(fma(-g, g, a), half_of(y), g);
+}
+__device__ __forceinline__ double rsqrt_any(double a) { return rsqrt_range(a) ? rsqrt_est(a) : rsqrt(a); }
+
+// Conversions on the bit patterns; values outside FP32's normal range (zero among them, which
+// stays cheap) take the instruction.
+enum class RoundTo { kNearest, kDown, kUp };
+template <RoundTo M>
+__device__ __forceinline__ float to_float(double v) {
+    const int hi = __double2hiint(v), lo = __double2loint(v);
+    const unsigned mag = unsigned(hi) & 0x7fffffffu;
+    if (mag - 0x38100000u >= 0x0fe00000u) {  // not in [2^-126, 2^128)
+        if ((mag | unsigned(lo)) == 0) return __int_as_float(hi);
+        return M == RoundTo::kNearest ? __double2float_rn(v) : M == RoundTo::kDown ? __double2float_rd(v) : __double2float_ru(v);
+    }
+    unsigned t = __funnelshift_l(unsigned(lo), mag - 0x38000000u, 3);
+    const unsigned rest = unsigned(lo) & 0x1fffffffu;
+    if (M == RoundTo::kNearest) t += rest + (t & 1u) > 0x10000000u;
+    else t += rest != 0 && (hi < 0) == (M == RoundTo::kDown);
+    return __int_as_float(int(t | (unsigned(hi) & 0x80000000u)));
+}
+__device__ __forceinline__ double to_double(float v) {
+    const unsigned b = unsigned(__float_as_int(v)), mag = b & 0x7fffffffu;
+    if (mag - 0x00800000u >= 0x7f000000u) return mag == 0 ? __hiloint2double(int(b), 0) : double(v);
+    return __hiloint2double(int((b & 0x80000000u) | ((mag >> 3) + 0x38000000u)), int(b << 29));
+}
+
+// exp of the rotation vector v as a unit quaternion, for |v| <= 1 (v2 = |v|^2): cos(a / 2) and
+// sin(a / 2) / a as polynomials in a^2 (Chebyshev interpolation on [0, 1], errors 6e-18 and
+// 9e-19), so that neither a square root nor a division nor a sine is taken.
+__device__ __forceinline__ q4 exp_map_small(d3 v, double v2) {
+    double c = 0x1.1d8d32755f8fbp-41, s = 0x1.5fac6e0083f22p-46;
+    c = fma(c, v2, -0x1.27e40964b47d4p-32); s = fma(s, v2, -0x1.ae63543245d1fp-37);
+    c = fma(c, v2, 0x1.a01a00fb1bc6fp-24); s = fma(s, v2, 0x1.71de39fd64b1fp-28);
+    c = fma(c, v2, -0x1.6c16c16bdd04ep-16); s = fma(s, v2, -0x1.a01a019ffb337p-20);
+    c = fma(c, v2, 0x1.5555555555421p-9); s = fma(s, v2, 0x1.11111111110bfp-12);
+    c = fma(c, v2, -0x1.fffffffffffffp-4); s = fma(s, v2, -0x1.5555555555555p-6);
+    c = fma(c, v2, 0x1p+0); s = fma(s, v2, 0x1p-1);
+    return {c, v.x * s, v.y * s, v.z * s};
+}
+// Unit quaternion of q when |q| differs from one by rounding only, else qnorm.
+__device__ __forceinline__ q4 qnorm_near(q4 q) {
+    const double n2 = q.w * q.w + q.x * q.x + q.y * q.y + q.z * q.z;
+    if (!near_one(n2)) return qnorm(q);
+    const double r = fma(-.5, n2, 1.5);
+    return {q.w * r, q.x * r, q.y * r, q.z * r};
+}
+
 // Rotation matrix of a unit quaternion, rows as 32-byte records (x, y, z, pad).
 struct m3 { d3 r0, r1, r2; };
 __device__ __forceinline__ m3 quat_matrix(q4 q) {
-    const double xx = q.x * q.x, yy = q.y * q.y, zz = q.z * q.z;
-    const double xy = q.x * q.y, xz = q.x * q.z, yz = q.y * q.z;
-    const double wx = q.w * q.x, wy = q.w * q.y, wz = q.w * q.z;
-    return m3{d3{1 - 2 * (yy + zz), 2 * (xy - wz), 2 * (xz + wy)},
-              d3{2 * (xy + wz), 1 - 2 * (xx + zz), 2 * (yz - wx)},
-              d3{2 * (xz - wy), 2 * (yz + wx), 1 - 2 * (xx + yy)}};
+    const double x2 = 2 * q.x, y2 = 2 * q.y, z2 = 2 * q.z;
+    const double wx = q.w * x2, wy = q.w * y2, wz = q.w * z2;
+    return m3{d3{fma(-q.y, y2, fma(-q.z, z2, 1.0)), fma(q.x, y2, -wz), fma(q.x, z2, wy)},
+              d3{fma(q.x, y2, wz), fma(-q.x, x2, fma(-q.z, z2, 1.0)), fma(q.y, z2, -wx)},
+              d3{fma(q.x, z2, -wy), fma(q.y, z2, wx), fma(-q.x, x2, fma(-q.y, y2, 1.0))}};
 }
 __device__ __forceinline__ d3 mrot(const m3& m, d3 v) { return d3{dot(m.r0, v), dot(m.r1, v), dot(m.r2, v)}; }
 __device__ __forceinline__ d3 mrot_t(const m3& m, d3 v) {
@@ -132,6 +225,28 @@ __device__ __forceinline__ double warp_sum(double v) {
         const double y = __shfl_down_sync(0xffffffffu, v, o);
         if (lane < o) v += y;
     }
+    return v;
+}
+// Sums of four values over the warp with six FP64 additions instead of twenty: at the first two
+// steps the lanes pass half of their values on and keep the other half.  Lane 0 holds the sum of
+// a, lane 8 of b, lane 16 of c, lane 24 of d (as do the seven lanes after each).
+__device__ __forceinline__ double warp_sum4(double a, double b, double c, double d) {
+    const int lane = threadIdx.x & 31;
+    const bool up = lane & 16, mid = lane & 8;
+    const double k0 = (up ? c : a) + __shfl_xor_sync(0xffffffffu, up ? a : c, 16);
+    const double k1 = (up ? d : b) + __shfl_xor_sync(0xffffffffu, up ? b : d, 16);
+    double v = (mid ? k1 : k0) + __shfl_xor_sync(0xffffffffu, mid ? k0 : k1, 8);
+    v += __shfl_xor_sync(0xffffffffu, v, 4);
+    v += __shfl_xor_sync(0xffffffffu, v, 2);
+    v += __shfl_xor_sync(0xffffffffu, v, 1);
+    return v;
+}
+// Sums of two values: lane 0 holds the sum of a, lane 16 of b.
+__device__ __forceinline__ double warp_sum2(double a, double b) {
+    const bool up = threadIdx.x & 16;
+    double v = (up ? b : a) + __shfl_xor_sync(0xffffffffu, up ? a : b, 16);
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
 }
 __device__ __forceinline__ double warp_max(double v) {

@@ -1225,6 +1225,7 @@ void upload_instances(mcg_ctx* c, const std::vector<InstIn>& ins) {
             conn_hash[h] = key;
         }
     // blocks that never straddle two instances
+    const int bdim = cf.precision == MCG_MIXED ? kMapBlock : kBeamBlock;
     std::vector<int4> nblk, bblk, irange(static_cast<size_t>(I));
     for (int k = 0; k < I; k++) {
         const InstHost& h = ih[size_t(k)];
@@ -1233,8 +1234,8 @@ void upload_instances(mcg_ctx* c, const std::vector<InstIn>& ins) {
             nblk.push_back(make_int4(h.node0 + f, std::min(kMapBlock, h.N - f), k, 0));
         irange[size_t(k)].y = int(nblk.size());
         irange[size_t(k)].z = int(bblk.size());
-        for (int f = 0; f < h.B; f += kMapBlock)
-            bblk.push_back(make_int4(h.beam0 + f, std::min(kMapBlock, h.B - f), k, 0));
+        for (int f = 0; f < h.B; f += bdim)
+            bblk.push_back(make_int4(h.beam0 + f, std::min(bdim, h.B - f), k, 0));
         irange[size_t(k)].w = int(bblk.size());
     }
     // contact-grid offsets: the instances' footprints (x-z extent with room to widen under
@@ -1344,6 +1345,7 @@ void upload_instances(mcg_ctx* c, const std::vector<InstIn>& ins) {
     T.I = I;
     T.n_nblk = int(nblk.size());
     T.n_bblk = int(bblk.size());
+    T.bdim = bdim;
     {
         int4* d = M.get<int4>(nblk.size());
         h2d(d, nblk.data(), nblk.size(), s);

@@ -54,6 +54,7 @@ struct DevTopo {
     int n_nblk, n_bblk;       // node blocks, beam blocks
     const int4* nblk;         // [n_nblk] first node, node count, instance, 0
     const int4* bblk;         // [n_bblk] first beam, beam count, instance, 0
+    int bdim;                 // beams per beam block: kBeamBlock (FP64) or kMapBlock (mixed)
     const int4* irange;       // [I] node blocks [x, y), beam blocks [z, w) of the instance
     const int* inst_n;        // [I] nodes of the instance
     const long long* inst_free;  // [I] unlocked DOFs of the instance
@@ -63,8 +64,10 @@ struct DevTopo {
     const uint8_t* trial_inst;  // [I] with trials == 2: 1 where the instance writes its trial states
 };
 
-// Elements per mapped block (the launch block size of the mapped kernels).
+// Elements per mapped block (the launch block size of the mapped kernels): node blocks, and the
+// beam blocks of the mixed form; the FP64 form's beam blocks (one warp per FP64 unit of an SM).
 constexpr int kMapBlock = 256;
+constexpr int kBeamBlock = 128;
 
 #if defined(__CUDACC__)
 // Position of a thread of a mapped block: element index, instance; valid == false past the

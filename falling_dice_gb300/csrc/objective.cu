@@ -120,49 +120,6 @@ __global__ void __launch_bounds__(kBlock) k_center(DevTopo t, const double* __re
     }
 }
 
-// ---- constitutive return maps: MC/src/sim.cpp:5-8 ------------------------------------------
-struct Ret1 { double force, p, a, dg, energy, hard; bool yielded; };
-// inv_kH = 1 / max(1e-20, k + H), precomputed per beam (the reference divides).
-__device__ __forceinline__ Ret1 return1(double total, double pc, double ac, double k, double y, double H,
-                                        double inv_kH) {
-    Ret1 r;
-    const double trial = k * (total - pc);
-    const double f = fabs(trial) - (y + H * ac);
-    if (f > 0) {
-        const double s = trial >= 0 ? 1.0 : -1.0;
-        r.dg = f * inv_kH;
-        r.p = pc + s * r.dg;
-        r.a = ac + r.dg;
-        r.yielded = true;
-    } else {
-        r.dg = 0; r.p = pc; r.a = ac; r.yielded = false;
-    }
-    r.force = k * (total - r.p);
-    r.energy = .5 * k * sqr(total - r.p);
-    r.hard = .5 * H * sqr(r.a);
-    return r;
-}
-struct Ret3 { d3 force, p; double a, dg, energy, hard; bool yielded; };
-__device__ __forceinline__ Ret3 return3(d3 t, d3 pc, double ac, double k, double y, double H, double inv_kH) {
-    Ret3 r;
-    const d3 trial = (t - pc) * k;
-    const double n = len(trial);
-    const double f = n - (y + H * ac);
-    if (f > 0 && n > 1e-20) {
-        const d3 d = trial * (1.0 / n);
-        r.dg = f * inv_kH;
-        r.p = pc + d * r.dg;
-        r.a = ac + r.dg;
-        r.yielded = true;
-    } else {
-        r.dg = 0; r.p = pc; r.a = ac; r.yielded = false;
-    }
-    r.force = (t - r.p) * k;
-    r.energy = .5 * k * len2(t - r.p);
-    r.hard = .5 * H * sqr(r.a);
-    return r;
-}
-
 __device__ __forceinline__ q4 ldq(const double4_32a* R, int i) {
     const double4_32a v = R[i];
     return q4{v.x, v.y, v.z, v.w};
@@ -175,44 +132,164 @@ __device__ __forceinline__ m3 ldm(const double4_32a* M, int i) {
     const double4_32a a = M[3 * size_t(i)], b = M[3 * size_t(i) + 1], c = M[3 * size_t(i) + 2];
     return m3{d3{a.x, a.y, a.z}, d3{b.x, b.y, b.z}, d3{c.x, c.y, c.z}};
 }
-// Unit quaternion by one reciprocal square root (the reference divides by the norm).
-__device__ __forceinline__ q4 qnorm_fast(q4 q) {
-    const double n2 = q.w * q.w + q.x * q.x + q.y * q.y + q.z * q.z;
-    if (n2 < 1e-60) return q4{1, 0, 0, 0};
-    const double r = rsqrt(n2);
-    return q4{q.w * r, q.x * r, q.y * r, q.z * r};
+
+// ---- constitutive return maps: MC/src/sim.cpp:5-8 ------------------------------------------
+// e: the trial elastic part (total - plastic), updated to the elastic part after the return;
+// inv_kH = 1 / max(1e-20, k + H), precomputed per beam (the reference divides).  Elastic and
+// hardening energies come as twice their value, k e^2 + H a^2: the factor 1/2 is applied once
+// per block.
+struct Ret1 { double force, p, a, dg, energy2; bool yielded; };
+__device__ __forceinline__ Ret1 return1(double e, double pc, double ac, double k, double y, double H, double inv_kH) {
+    Ret1 r{0, pc, ac, 0, 0, false};
+    r.force = k * e;
+    const double f = fabs(r.force) - fma(H, ac, y);
+    if (positive(f)) {
+        r.dg = f * inv_kH;
+        const double s = xor_sign(r.dg, r.force);
+        r.p = pc + s;
+        r.a = ac + r.dg;
+        e -= s;
+        r.force = k * e;
+        r.yielded = true;
+    }
+    r.energy2 = fma(r.force, e, (H * r.a) * r.a);
+    return r;
 }
-// normalize() of MC/include/core.hpp:39 with a reciprocal square root.
-__device__ __forceinline__ d3 unit_fast(d3 v) {
-    const double l2 = len2(v);
-    return (isfinite(l2) && l2 > 1e-30) ? v * rsqrt(l2) : d3{0, 1, 0};
+// The vector form.  The yield test needs |trial| = k |e| only where it yields: whether it can
+// is decided on the squares, k^2 |e|^2 > Y^2 (with a margin for their rounding), the square
+// root is taken for those beams and the test as the reference writes it decides.
+struct Ret3 { d3 force, p; double a, dg, energy2; bool yielded; };
+__device__ __forceinline__ Ret3 return3(d3 e, d3 pc, double ac, double k, double y, double H, double inv_kH) {
+    Ret3 r{{}, pc, ac, 0, 0, false};
+    double e2 = len2(e);
+    const double Y = fma(H, ac, y);
+    if (positive(fma((k * k) * (1.0 + 0x1p-48), e2, -Y * Y)) || negative_sign(Y)) {
+        const double rs = rsqrt_any(e2), n = k * (e2 * rs), f = n - Y;
+        if (positive(f) && less_bits(1e-20, n)) {
+            r.dg = f * inv_kH;
+            const d3 dp = e * (rs * r.dg);
+            r.p = pc + dp;
+            r.a = ac + r.dg;
+            e = e - dp;
+            e2 = len2(e);
+            r.yielded = true;
+        }
+    }
+    r.force = e * k;
+    r.energy2 = fma(k, e2, (H * r.a) * r.a);
+    return r;
+}
+
+// Length and inverse length of a chord from its square (from 2^-111 on by the estimate).  Both
+// are rounded as the reference's sqrt and division, the inverse by one correction with the
+// residual of 1 / sqrt(l2) as the start (Markstein, as sqrt_from): at rest the chord's tangent is
+// then the stored director bit for bit, and the shear vanishes exactly.
+__device__ __forceinline__ void chord_length(double l2, double& L, double& invL) {
+    if (rsqrt_range(l2)) {
+        const double y = rsqrt_est(l2);
+        L = sqrt_from(l2, y);
+        invL = fma(fma(-L, y, 1.0), y, y);
+    } else {
+        L = sqrt(l2);
+        invL = 1.0 / L;
+    }
+}
+
+// Rotation vector of the relative rotation Q = Ra^* Rb (MC/include/core.hpp:52 quatLog of the
+// normalized Q with w >= 0) and its squared length.  With s = |v| of the unit Q, the vector is
+// 2 asin(s) / s v: a polynomial in s^2 up to s^2 = 0.1 (angles up to 36.9 degrees; Chebyshev
+// interpolation, error 2e-18), so that the usual beam takes no square root, division or
+// arctangent; larger angles take atan2 as the reference does.  Q is a product of two unit
+// quaternions, so its norm differs from one by rounding only and one step corrects it.
+__device__ __forceinline__ d3 relative_rotation(q4 Ra, q4 Rb, double& phi2) {
+    q4 Q = qmul(conj(Ra), Rb);
+    const double v2 = Q.x * Q.x + Q.y * Q.y + Q.z * Q.z, n2 = fma(Q.w, Q.w, v2);
+    const double r = fma(-.5, n2, 1.5);
+    const double s2 = v2 * (r * r);
+    if (near_one(n2) && unsigned(__double2hiint(s2)) < 0x3fb99999u) {  // s2 < 0.1
+        double g = 0x1.c42a558b8b15bp-6;
+        g = fma(g, s2, 0x1.11d08867c9adep-6);
+        g = fma(g, s2, 0x1.80fd1940cecf2p-6);
+        g = fma(g, s2, 0x1.c90c2f25d23e5p-6);
+        g = fma(g, s2, 0x1.1c529e3ddf7c6p-5);
+        g = fma(g, s2, 0x1.6e8b80a6ac006p-5);
+        g = fma(g, s2, 0x1.f1c71d2f31c2ep-5);
+        g = fma(g, s2, 0x1.6db6db6c86271p-4);
+        g = fma(g, s2, 0x1.33333333342e1p-3);
+        g = fma(g, s2, 0x1.5555555555550p-2);
+        g = fma(g, s2, 2.0);
+        phi2 = (g * g) * s2;
+        g = xor_sign(g * r, Q.w);
+        return d3{Q.x * g, Q.y * g, Q.z * g};
+    }
+    Q = qnorm(Q);
+    if (Q.w < 0) Q = q4{-Q.w, -Q.x, -Q.y, -Q.z};
+    const double s = sqrt(Q.x * Q.x + Q.y * Q.y + Q.z * Q.z);
+    d3 phi{2 * Q.x, 2 * Q.y, 2 * Q.z};
+    if (!(s < 1e-12)) phi = d3{Q.x, Q.y, Q.z} * (2 * atan2(s, clampd(Q.w, -1, 1)) / s);
+    phi2 = len2(phi);
+    return phi;
+}
+
+// J_l^{-T}(phi) v (jl_inv_t) with the coefficient as a polynomial in phi2 = |phi|^2 up to 0.42
+// (every angle of relative_rotation's polynomial; Chebyshev interpolation, error 4e-17 against
+// 1/12, which enters multiplied by phi2).
+__device__ __forceinline__ d3 transport(d3 phi, double phi2, d3 v) {
+    if (unsigned(__double2hiint(phi2)) >= 0x3fdae000u) return jl_inv_t(phi, v);  // 0.4199
+    double A = 0x1.2bf59666dc69ep-31;
+    A = fma(A, phi2, 0x1.6684f73f8bd8ep-26);
+    A = fma(A, phi2, 0x1.bbd7b81461d47p-21);
+    A = fma(A, phi2, 0x1.1566aba745146p-15);
+    A = fma(A, phi2, 0x1.6c16c16c1de72p-10);
+    A = fma(A, phi2, 0x1.5555555555553p-4);
+    const d3 c1 = cross(phi, v), c2 = cross(phi, c1);
+    return d3{fma(A, c2.x, fma(.5, c1.x, v.x)), fma(A, c2.y, fma(.5, c1.y, v.y)), fma(A, c2.z, fma(.5, c1.z, v.z))};
+}
+
+// The beam's axis in the material frame: unit(Ra^T t), t a unit vector.
+__device__ __forceinline__ d3 material_axis(const m3& Ma, d3 t) {
+    const d3 a = mrot_t(Ma, t);
+    const double l2 = len2(a);
+    if (near_one(l2)) return a * fma(-.5, l2, 1.5);
+    return unit(a);
 }
 
 // ---- beam kernel: MC/src/sim.cpp:139-141 ---------------------------------------------------
-// kMinBlocks: CTAs per SM the register allocation must allow (an occupancy variant picked by
-// mcg_autotune; the arithmetic, and so the result, is the same in every variant).
+// Bound by the FP64 pipe (one warp instruction per 19 cycles and SM, beside which loads and the
+// other pipes are idle), so the formulas are written for few FP64 instructions: energies summed
+// as twice their value, shear from the director-chord differences (2 t - da - db = -(ma + mb)),
+// polynomials for the rotation vector and its transport, square roots from the FP32 estimate,
+// comparisons on bit patterns.
+// Measured at 184,400 beams (32x32x16): 391 -> 265 FP64 instructions per 32 beams, 0.159 ->
+// 0.109 ms (84 % of the FP64 pipe's instruction rate).
+// Blocks of kBeamBlock = 128 beams: one warp on each of an SM's four FP64 units, so that a
+// lattice of a few hundred beams spreads over several SMs.
+// kMinBlocks: units of 256 threads per SM the register allocation must allow (an occupancy
+// variant picked by mcg_autotune; the arithmetic, and so the result, is the same in every variant).
 template <int kMinBlocks>
-__global__ void __launch_bounds__(kBlock, kMinBlocks) k_beams(DevTopo t, Material m, const double* __restrict__ plastic,
-                                                              int trials, EvalBufs e) {
-    __shared__ double sm[3 * (kBlock / 32)];
+__global__ void __launch_bounds__(kBeamBlock, 2 * kMinBlocks) k_beams(DevTopo t, Material m,
+                                                                      const double* __restrict__ plastic, int trials,
+                                                                      EvalBufs e) {
+    __shared__ double sm[2 * (kBeamBlock / 32)];
     const MapPos mp = map_pos(t.bblk);
     if (!t.active[mp.inst]) return;
     if (trials == 2) trials = t.trial_inst[mp.inst];  // per instance (device-resident solver)
     const int b = mp.i;
     const int B = t.B;
-    double acc[3] = {0, 0, 0};  // energy, elastic, plastic
+    double elastic2 = 0, diss = 0, penalty = 0;  // twice the elastic energy, plastic dissipation
     if (mp.valid) {
         const int2 ab = t.ab[b];
         const d3 xa = ldx(e.x, ab.x), xb = ldx(e.x, ab.y);
-        // chord, length and tangent rounded as the reference (no fused multiply-add), so
-        // that a beam at its rest length has exactly zero strain here too
+        // chord, its square and tangent rounded as the reference (no fused multiply-add), so
+        // that a beam at its rest length has zero strain here too
         const d3 d{__dsub_rn(xb.x, xa.x), __dsub_rn(xb.y, xa.y), __dsub_rn(xb.z, xa.z)};
-        const double L = sqrt(__dadd_rn(__dadd_rn(__dmul_rn(d.x, d.x), __dmul_rn(d.y, d.y)), __dmul_rn(d.z, d.z)));
+        double L, invL;
+        chord_length(__dadd_rn(__dadd_rn(__dmul_rn(d.x, d.x), __dmul_rn(d.y, d.y)), __dmul_rn(d.z, d.z)), L, invL);
         double* sa = e.slotA + 6 * size_t(b);
         double* sb = e.slotB + 6 * size_t(b);
-        if (L < 1e-10) {
+        if (less_bits(L, 1e-10)) {
             // Degenerate element: penalty energy only, no gradient and a default trial.
-            acc[0] = 1e8 * sqr(1e-10 - L);
+            penalty = 1e8 * sqr(1e-10 - L);
 #pragma unroll
             for (int k = 0; k < 6; k++) { sa[k] = 0; sb[k] = 0; }
             if (trials) {
@@ -225,58 +302,44 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) k_beams(DevTopo t, Materia
             const double pl_epsp = plastic[b], pl_alpha = plastic[size_t(B) + b];
             const d3 rotp{plastic[2 * size_t(B) + b], plastic[3 * size_t(B) + b], plastic[4 * size_t(B) + b]};
             const double pl_alphaB = plastic[5 * size_t(B) + b], pl_alphaT = plastic[6 * size_t(B) + b];
-            const double invL = 1.0 / L;
             const d3 tt{__dmul_rn(d.x, invL), __dmul_rn(d.y, invL), __dmul_rn(d.z, invL)};
             // axial
             const double eps = (L - t.L0[b]) * t.invL0[b];
-            const Ret1 ax = return1(eps, pl_epsp, pl_alpha, m.E, t.sy[b], m.H, m.inv_EH);
-            const double aL = t.aL[b];
-            const double uax = aL * (ax.energy + ax.hard);
-            const double dax = t.aLsy[b] * ax.dg;
-            const double Nf = t.area[b] * ax.force;
-            d3 F = tt * Nf;
+            const Ret1 ax = return1(eps - pl_epsp, pl_epsp, pl_alpha, m.E, t.sy[b], m.H, m.inv_EH);
+            const double uax2 = t.aL[b] * ax.energy2;
+            if (ax.yielded) diss = t.aLsy[b] * ax.dg;
             // shear: the end directors against the chord (rotations by the nodes' matrices)
             const m3 Ma = ldm(e.M, ab.x), Mb = ldm(e.M, ab.y);
             const d3 e0{t.e0x[b], t.e0y[b], t.e0z[b]};
             const d3 da = mrot(Ma, e0), db = mrot(Mb, e0);
             const double cs = t.cs[b];
             const d3 ma = da - tt, mb = db - tt;
-            const double us = .5 * cs * (len2(ma) + len2(mb));
-            const d3 gt = ((tt * 2.0 - da) - db) * cs;
-            const d3 trans = (gt - tt * dot(gt, tt)) * invL;
-            F = F + trans;
-            d3 Ga = -(cross(da, tt) * cs);
-            d3 Gb = -(cross(db, tt) * cs);
+            const double us2 = len2(ma) + len2(mb);  // times cs
+            const d3 gm = ma + mb;
+            const double kt_ = cs * invL;
+            const double kf = fma(kt_, dot(gm, tt), t.area[b] * ax.force);
+            // F = t N + ((I - t t^T) g) / L with g = -cs (ma + mb)
+            const d3 F{fma(tt.x, kf, -(kt_ * gm.x)), fma(tt.y, kf, -(kt_ * gm.y)), fma(tt.z, kf, -(kt_ * gm.z))};
+            const d3 tc = tt * cs;
+            d3 Ga = cross(tc, da);
+            d3 Gb = cross(tc, db);
             // bending and torsion from the relative rotation Q = Ra^* Rb
-            const q4 Ra = ldq(e.R, ab.x), Rb = ldq(e.R, ab.y);
-            q4 Q = qnorm_fast(qmul(conj(Ra), Rb));
-            if (Q.w < 0) Q = q4{-Q.w, -Q.x, -Q.y, -Q.z};
-            d3 phi;
-            {  // log map (MC/include/core.hpp:52); Q is already unit
-                const double s2 = Q.x * Q.x + Q.y * Q.y + Q.z * Q.z;
-                const double sq = sqrt(s2);
-                if (sq < 1e-12) {
-                    phi = d3{2 * Q.x, 2 * Q.y, 2 * Q.z};
-                } else {
-                    const double ang = 2 * atan2(sq, clampd(Q.w, -1, 1));
-                    phi = d3{Q.x, Q.y, Q.z} * (ang / sq);
-                }
-            }
-            const d3 axis = unit_fast(mrot_t(Ma, tt));
+            double phi2;
+            const d3 phi = relative_rotation(ldq(e.R, ab.x), ldq(e.R, ab.y), phi2);
+            const d3 axis = material_axis(Ma, tt);
             const double tw = dot(phi, axis), ptw = dot(rotp, axis);
             const d3 bend = phi - axis * tw, pb = rotp - axis * ptw;
-            const double kb = t.kb[b], kt = t.kt[b], my = t.my[b], ty = t.ty[b];
-            const Ret3 br = return3(bend, pb, pl_alphaB, kb, my, t.hb[b], t.inv_kbh[b]);
-            const Ret1 tor = return1(tw, ptw, pl_alphaT, kt, ty, t.ht[b], t.inv_kth[b]);
+            const double kb = t.kb[b], kt = t.kt[b];
+            const Ret3 br = return3(bend - pb, pb, pl_alphaB, kb, t.my[b], t.hb[b], t.inv_kbh[b]);
+            const Ret1 tor = return1(tw - ptw, ptw, pl_alphaT, kt, t.ty[b], t.ht[b], t.inv_kth[b]);
             const d3 moment = br.force + axis * tor.force;
-            const double ur = br.energy + br.hard + tor.energy + tor.hard;
-            const double dr = my * br.dg + ty * tor.dg;
-            const d3 world = mrot(Ma, jl_inv_t(phi, moment));
+            double dr = 0;
+            if (br.yielded) dr = t.my[b] * br.dg;
+            if (tor.yielded) dr = fma(t.ty[b], tor.dg, dr);
+            const d3 world = mrot(Ma, transport(phi, phi2, moment));
             Ga = Ga - world;
             Gb = Gb + world;
-            acc[0] = (uax + dax) + us + (ur + dr);
-            acc[1] = uax + us + ur;
-            acc[2] = dax + dr;
+            elastic2 = fma(cs, us2, uax2) + (br.energy2 + tor.energy2);
             sa[0] = -F.x; sa[1] = -F.y; sa[2] = -F.z; sa[3] = Ga.x; sa[4] = Ga.y; sa[5] = Ga.z;
             sb[0] = F.x;  sb[1] = F.y;  sb[2] = F.z;  sb[3] = Gb.x; sb[4] = Gb.y; sb[5] = Gb.z;
             if (trials) {
@@ -294,19 +357,36 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) k_beams(DevTopo t, Materia
                 e.trial_aux[2 * S + b] = moment.x;
                 e.trial_aux[3 * S + b] = moment.y;
                 e.trial_aux[4 * S + b] = moment.z;
-                e.trial_aux[5 * S + b] = uax + us + ur;
-                e.trial_aux[6 * S + b] = dax + dr;
+                e.trial_aux[5 * S + b] = .5 * elastic2;
+                e.trial_aux[6 * S + b] = diss + dr;
                 e.trial_flags[b] = ax.yielded;
                 e.trial_flags[S + b] = br.yielded;
                 e.trial_flags[2 * S + b] = tor.yielded;
             }
+            diss += dr;
         }
     }
-    block_sum<3>(acc, sm);
+    const double v = warp_sum2(elastic2, diss);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if ((lane & 15) == 0) sm[(lane >> 4) * (kBeamBlock / 32) + warp] = v;
+    const bool degenerate = __syncthreads_or(__double_as_longlong(penalty) != 0);
     if (threadIdx.x == 0) {
-        e.part_beam[3 * blockIdx.x] = acc[0];
-        e.part_beam[3 * blockIdx.x + 1] = acc[1];
-        e.part_beam[3 * blockIdx.x + 2] = acc[2];
+        double el = 0, pl = 0;
+#pragma unroll
+        for (int w = 0; w < kBeamBlock / 32; w++) {
+            el += sm[w];
+            pl += sm[kBeamBlock / 32 + w];
+        }
+        el *= .5;
+        e.part_beam[3 * blockIdx.x] = el + pl;
+        e.part_beam[3 * blockIdx.x + 1] = el;
+        e.part_beam[3 * blockIdx.x + 2] = pl;
+    }
+    if (degenerate) {  // block-uniform, rare
+        __syncthreads();
+        double acc[1] = {penalty};
+        block_sum<1>(acc, sm);
+        if (threadIdx.x == 0) e.part_beam[3 * blockIdx.x] += acc[0];
     }
 }
 
@@ -716,19 +796,19 @@ void launch_commit(const DevTopo& t, const uint8_t* mask, const EvalBufs& e, dou
     k_commit_nodes<<<t.n_nblk, kBlock, 0, s>>>(t, mask, e.x, e.R, base_x, base_r);
     note_launches(1);
     if (t.B > 0 && plastic) {
-        k_commit_plastic<<<t.n_bblk, kBlock, 0, s>>>(t, mask, e.trial_next, plastic);
+        k_commit_plastic<<<t.n_bblk, t.bdim, 0, s>>>(t, mask, e.trial_next, plastic);
         note_launches(1);
     }
 }
 
 void launch_plastic_stats(const DevTopo& t, const double* plastic, double* part, double* out6, cudaStream_t s) {
     if (t.B == 0) return;
-    k_plastic_part<<<t.n_bblk, kBlock, 0, s>>>(t, plastic, part);
+    k_plastic_part<<<t.n_bblk, t.bdim, 0, s>>>(t, plastic, part);
     k_plastic_final<<<t.I, kBlock, 0, s>>>(t, part, out6);
     note_launches(2);
 }
 
-// Occupancy variants (CTAs per SM) of the FP64 beam kernel and of the gather.
+// Occupancy variants of the FP64 beam kernel (256-thread units per SM) and of the gather (CTAs per SM).
 constexpr int kBeamBlocks[] = {1, 2, 3};
 constexpr int kGatherBlocks[] = {1, 2, 4};
 
@@ -752,9 +832,9 @@ void launch_beams(const DevTopo& t, const Material& m, const double* plastic, in
     if (t.B == 0) return;
     const int tr = trials;  // 0, 1, or 2: per instance (t.trial_inst)
     switch (variant) {
-        case 1: k_beams<kBeamBlocks[1]><<<t.n_bblk, kBlock, 0, s>>>(t, m, plastic, tr, e); break;
-        case 2: k_beams<kBeamBlocks[2]><<<t.n_bblk, kBlock, 0, s>>>(t, m, plastic, tr, e); break;
-        default: k_beams<kBeamBlocks[0]><<<t.n_bblk, kBlock, 0, s>>>(t, m, plastic, tr, e); break;
+        case 1: k_beams<kBeamBlocks[1]><<<t.n_bblk, kBeamBlock, 0, s>>>(t, m, plastic, tr, e); break;
+        case 2: k_beams<kBeamBlocks[2]><<<t.n_bblk, kBeamBlock, 0, s>>>(t, m, plastic, tr, e); break;
+        default: k_beams<kBeamBlocks[0]><<<t.n_bblk, kBeamBlock, 0, s>>>(t, m, plastic, tr, e); break;
     }
     note_launches(1);
 }

@@ -22,8 +22,9 @@ ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 
 NVCC_FLAGS = ARCH + ["-O3", "-lineinfo", "-std=c++20", "-Xcompiler", "-fPIC", f"-I{INC}",
                      "--expt-relaxed-constexpr", "-Xptxas", "-warn-spills"]
-# Per-unit extra flags.  contact.cu must round like the reference: no FMA contraction.
-EXTRA = {"contact.cu": ["-fmad=false"]}
+# Per-unit extra flags.  contact.cu must round like the reference, objective.cu writes its fused
+# multiply-adds out (its occupancy variants must round identically): no FMA contraction.
+EXTRA = {"contact.cu": ["-fmad=false"], "objective.cu": ["-fmad=false"]}
 CXX_FLAGS = ["-O2", "-std=c++20", "-fPIC", "-ffp-contract=off", "-Wall", "-Wextra",
              f"-I{CUDA_HOME}/include", f"-I{INC}"]
 

@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "kernels.h"
+
 namespace mcg {
 
 constexpr int kBlock = 256;          // threads per CTA for the streaming kernels
@@ -126,6 +128,11 @@ __device__ __forceinline__ double xor_sign(double v, double s) {
 __device__ __forceinline__ double half_of(double v) {
     return __hiloint2double(__double2hiint(v) - 0x00100000, __double2loint(v));
 }
+// 2 v for a normal v below the largest exponent, or zero.
+__device__ __forceinline__ double twice(double v) {
+    const int hi = __double2hiint(v);
+    return __hiloint2double((hi & 0x7ff00000) ? hi + 0x00100000 : hi, __double2loint(v));
+}
 // |v - 1| < 2^-20: a squared norm whose square root is 1 + (v - 1) / 2 to FP64 precision when
 // it differs from one by rounding only.
 __device__ __forceinline__ bool near_one(double v) {
@@ -191,9 +198,23 @@ __device__ __forceinline__ q4 exp_map_small(d3 v, double v2) {
     c = fma(c, v2, 0x1p+0); s = fma(s, v2, 0x1p-1);
     return {c, v.x * s, v.y * s, v.z * s};
 }
+// Products with explicit fused multiply-adds, for units compiled without contraction: the
+// compiler then cannot fuse the same formula differently in two variants of a kernel, whose
+// results must agree bit for bit.
+__device__ __forceinline__ double fdot(d3 a, d3 b) { return fma(a.z, b.z, fma(a.y, b.y, a.x * b.x)); }
+__device__ __forceinline__ d3 fcross(d3 a, d3 b) {
+    return {fma(a.y, b.z, -(a.z * b.y)), fma(a.z, b.x, -(a.x * b.z)), fma(a.x, b.y, -(a.y * b.x))};
+}
+__device__ __forceinline__ d3 fmadd(d3 a, double s, d3 c) { return {fma(a.x, s, c.x), fma(a.y, s, c.y), fma(a.z, s, c.z)}; }
+__device__ __forceinline__ q4 fqmul(q4 a, q4 b) {
+    return {fma(-a.z, b.z, fma(-a.y, b.y, fma(-a.x, b.x, a.w * b.w))),
+            fma(-a.z, b.y, fma(a.y, b.z, fma(a.x, b.w, a.w * b.x))),
+            fma(a.z, b.x, fma(a.y, b.w, fma(-a.x, b.z, a.w * b.y))),
+            fma(a.z, b.w, fma(-a.y, b.x, fma(a.x, b.y, a.w * b.z)))};
+}
 // Unit quaternion of q when |q| differs from one by rounding only, else qnorm.
 __device__ __forceinline__ q4 qnorm_near(q4 q) {
-    const double n2 = q.w * q.w + q.x * q.x + q.y * q.y + q.z * q.z;
+    const double n2 = fma(q.z, q.z, fma(q.y, q.y, fma(q.x, q.x, q.w * q.w)));
     if (!near_one(n2)) return qnorm(q);
     const double r = fma(-.5, n2, 1.5);
     return {q.w * r, q.x * r, q.y * r, q.z * r};
@@ -202,11 +223,15 @@ __device__ __forceinline__ q4 qnorm_near(q4 q) {
 // Rotation matrix of a unit quaternion, rows as 32-byte records (x, y, z, pad).
 struct m3 { d3 r0, r1, r2; };
 __device__ __forceinline__ m3 quat_matrix(q4 q) {
-    const double x2 = 2 * q.x, y2 = 2 * q.y, z2 = 2 * q.z;
+    const double x2 = twice(q.x), y2 = twice(q.y), z2 = twice(q.z);
     const double wx = q.w * x2, wy = q.w * y2, wz = q.w * z2;
     return m3{d3{fma(-q.y, y2, fma(-q.z, z2, 1.0)), fma(q.x, y2, -wz), fma(q.x, z2, wy)},
               d3{fma(q.x, y2, wz), fma(-q.x, x2, fma(-q.z, z2, 1.0)), fma(q.y, z2, -wx)},
               d3{fma(q.x, z2, -wy), fma(q.y, z2, wx), fma(-q.x, x2, fma(-q.y, y2, 1.0))}};
+}
+__device__ __forceinline__ d3 fmrot(const m3& m, d3 v) { return d3{fdot(m.r0, v), fdot(m.r1, v), fdot(m.r2, v)}; }
+__device__ __forceinline__ d3 fmrot_t(const m3& m, d3 v) {
+    return fmadd(m.r2, v.z, fmadd(m.r1, v.y, m.r0 * v.x));
 }
 __device__ __forceinline__ d3 mrot(const m3& m, d3 v) { return d3{dot(m.r0, v), dot(m.r1, v), dot(m.r2, v)}; }
 __device__ __forceinline__ d3 mrot_t(const m3& m, d3 v) {
@@ -391,6 +416,89 @@ __device__ __forceinline__ double block_max(double v, double* smem) {
     }
     __syncthreads();
     return v;
+}
+
+// ---- maxima on the integer pipe -------------------------------------------------------------
+// Floats and doubles as integers of the same order; NaN counts as the lowest value, as fmax
+// skips it.
+__device__ __forceinline__ int order_key(float v) {
+    const int b = __float_as_int(v);
+    return v == v ? b ^ ((b >> 31) & 0x7fffffff) : int(0x80000000u);
+}
+__device__ __forceinline__ float order_value(int k) { return __int_as_float(k ^ ((k >> 31) & 0x7fffffff)); }
+__device__ __forceinline__ long long order_key(double v) {
+    const long long b = __double_as_longlong(v);
+    const bool nan = (unsigned long long)(b & 0x7fffffffffffffffLL) > 0x7ff0000000000000ULL;
+    return nan ? (long long)0x8000000000000000ULL : b ^ ((b >> 63) & 0x7fffffffffffffffLL);
+}
+__device__ __forceinline__ double order_value(long long k) {
+    return __longlong_as_double(k ^ ((k >> 63) & 0x7fffffffffffffffLL));
+}
+__device__ __forceinline__ int warp_max_key(int k) { return __reduce_max_sync(0xffffffffu, k); }
+__device__ __forceinline__ long long warp_max_key(long long k) {
+    const int hi = __reduce_max_sync(0xffffffffu, int(k >> 32));
+    const unsigned lo = __reduce_max_sync(0xffffffffu, int(k >> 32) == hi ? unsigned(k) : 0u);
+    return ((long long)hi << 32) | lo;
+}
+
+// ---- node state: bounds and block partials, shared by the FP64 and the mixed form ------------
+// Single-precision bounds of a node's position in the contact grid's frame (the instance's
+// offset added with outward rounding), and the extrema of the bounding box: x and z from the
+// outward-rounded bounds (they contain the FP64 positions), y exact (the permanent set reads it).
+struct StateBounds {
+    int f[4] = {int(0x80000000u), int(0x80000000u), int(0x80000000u), int(0x80000000u)};  // -min x, -min z, max x, max z
+    long long y[2] = {(long long)0x8000000000000000ULL, (long long)0x8000000000000000ULL};  // -min y, max y
+    __device__ __forceinline__ void take(double xx, double xy, double xz, float2 o, float4& xf_lo, float4& xf_hi) {
+        const float4 lo = make_float4(__fadd_rd(to_float<RoundTo::kDown>(xx), o.x), to_float<RoundTo::kDown>(xy),
+                                      __fadd_rd(to_float<RoundTo::kDown>(xz), o.y), 0.f);
+        const float4 hi = make_float4(__fadd_ru(to_float<RoundTo::kUp>(xx), o.x), to_float<RoundTo::kUp>(xy),
+                                      __fadd_ru(to_float<RoundTo::kUp>(xz), o.y), 0.f);
+        xf_lo = lo;
+        xf_hi = hi;
+        f[0] = order_key(-lo.x);
+        f[1] = order_key(-lo.z);
+        f[2] = order_key(hi.x);
+        f[3] = order_key(hi.z);
+        y[0] = order_key(-xy);
+        y[1] = order_key(xy);
+    }
+};
+struct StateParts {
+    double sum[3][kEvalBlock / 32];
+    long long y[2][kEvalBlock / 32];
+    int f[4][kEvalBlock / 32];
+};
+// The block's nine partials (sum, -min, max of the positions) into q.
+__device__ __forceinline__ void state_block_parts(const double (&acc)[3], const StateBounds& b, StateParts& sm, double* q) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const double v = warp_sum4(acc[0], acc[1], acc[2], 0.0);
+    if ((lane & 7) == 0 && lane < 24) sm.sum[lane >> 3][warp] = v;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const int m = warp_max_key(b.f[k]);
+        if (lane == 0) sm.f[k][warp] = m;
+    }
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        const long long m = warp_max_key(b.y[k]);
+        if (lane == 0) sm.y[k][warp] = m;
+    }
+    __syncthreads();
+    constexpr int nw = kEvalBlock / 32;
+    const int t = threadIdx.x;
+    if (t < 3) {
+        double s = sm.sum[t][0];
+        for (int w = 1; w < nw; w++) s += sm.sum[t][w];
+        q[t] = s;
+    } else if (t < 5) {
+        long long m = sm.y[t - 3][0];
+        for (int w = 1; w < nw; w++) m = max(m, sm.y[t - 3][w]);
+        q[t == 3 ? 4 : 7] = order_value(m);
+    } else if (t < 9) {
+        int m = sm.f[t - 5][0];
+        for (int w = 1; w < nw; w++) m = max(m, sm.f[t - 5][w]);
+        q[t == 5 ? 3 : t == 6 ? 5 : t == 7 ? 6 : 8] = double(order_value(m));
+    }
 }
 
 inline unsigned grid_for(long long n, int block = kBlock) {

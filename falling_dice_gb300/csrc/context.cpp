@@ -1226,7 +1226,8 @@ void upload_instances(mcg_ctx* c, const std::vector<InstIn>& ins) {
         }
     // blocks that never straddle two instances
     const int bdim = cf.precision == MCG_MIXED ? kMapBlock : kBeamBlock;
-    std::vector<int4> nblk, bblk, irange(static_cast<size_t>(I));
+    std::vector<int4> nblk, bblk, eblk, irange(static_cast<size_t>(I));
+    std::vector<int2> erange(static_cast<size_t>(I));
     for (int k = 0; k < I; k++) {
         const InstHost& h = ih[size_t(k)];
         irange[size_t(k)].x = int(nblk.size());
@@ -1237,6 +1238,10 @@ void upload_instances(mcg_ctx* c, const std::vector<InstIn>& ins) {
         for (int f = 0; f < h.B; f += bdim)
             bblk.push_back(make_int4(h.beam0 + f, std::min(bdim, h.B - f), k, 0));
         irange[size_t(k)].w = int(bblk.size());
+        erange[size_t(k)].x = int(eblk.size());
+        for (int f = 0; f < h.N; f += kEvalBlock)
+            eblk.push_back(make_int4(h.node0 + f, std::min(kEvalBlock, h.N - f), k, 0));
+        erange[size_t(k)].y = int(eblk.size());
     }
     // contact-grid offsets: the instances' footprints (x-z extent with room to widen under
     // compression) packed in rows, so that the shared grid stays small; offsets are
@@ -1346,6 +1351,7 @@ void upload_instances(mcg_ctx* c, const std::vector<InstIn>& ins) {
     T.n_nblk = int(nblk.size());
     T.n_bblk = int(bblk.size());
     T.bdim = bdim;
+    T.n_eblk = int(eblk.size());
     {
         int4* d = M.get<int4>(nblk.size());
         h2d(d, nblk.data(), nblk.size(), s);
@@ -1356,6 +1362,12 @@ void upload_instances(mcg_ctx* c, const std::vector<InstIn>& ins) {
         int4* r = M.get<int4>(irange.size());
         h2d(r, irange.data(), irange.size(), s);
         T.irange = r;
+        int4* eb = M.get<int4>(eblk.size());
+        h2d(eb, eblk.data(), eblk.size(), s);
+        T.eblk = eb;
+        int2* er = M.get<int2>(erange.size());
+        h2d(er, erange.data(), erange.size(), s);
+        T.erange = er;
         std::vector<int> nn(static_cast<size_t>(I));
         std::vector<long long> nf(static_cast<size_t>(I));
         std::vector<float2> off(static_cast<size_t>(I));
@@ -1446,15 +1458,15 @@ void upload_instances(mcg_ctx* c, const std::vector<InstIn>& ins) {
     e.M = V.get<double4_32a>(3 * size_t(N));
     e.xf_lo = V.get<float4>(size_t(N));
     e.xf_hi = V.get<float4>(size_t(N));
-    e.slotA = V.get<double>(6 * size_t(B));
-    e.slotB = V.get<double>(6 * size_t(B));
-    e.part_state = V.get<double>(9 * size_t(T.n_nblk));
+    e.slot = V.get<double>(12 * size_t(B));
+    e.part_state = V.get<double>(9 * size_t(T.n_eblk));
     e.part_beam = V.get<double>(3 * size_t(std::max(T.n_bblk, 1)));
     e.err = V.get<unsigned>(1);
     ck(cudaMemsetAsync(e.err, 0, sizeof(unsigned), s), "memset");
-    e.part_node = V.get<double>(kNodeParts * size_t(T.n_nblk));
+    e.part_node = V.get<double>(kNodeParts * size_t(T.n_eblk));
     e.part_fin = V.get<double>(size_t(kFinPartDoubles) * size_t(I));
     e.cen = V.get<double>(9 * size_t(I + 1));
+    e.cforce = V.get<double>(2 * size_t(I));
     e.tops = V.get<double>(size_t(I));
     e.out = V.get<EvalOut>(size_t(I));
     e.trial_next = V.get<double>(7 * size_t(B));
@@ -1462,8 +1474,7 @@ void upload_instances(mcg_ctx* c, const std::vector<InstIn>& ins) {
     e.trial_flags = V.get<uint8_t>(3 * size_t(B));
     c->mixed = cf.precision == MCG_MIXED;
     if (c->mixed) {
-        e.slotAf = V.get<float>(6 * size_t(B));
-        e.slotBf = V.get<float>(6 * size_t(B));
+        e.slotf = V.get<float>(12 * size_t(B));
         e.trial_nextf = V.get<float>(7 * size_t(B));
         e.trial_auxf = V.get<float>(7 * size_t(B));
         MixedBeams mb{};

@@ -56,6 +56,9 @@ struct DevTopo {
     const int4* bblk;         // [n_bblk] first beam, beam count, instance, 0
     int bdim;                 // beams per beam block: kBeamBlock (FP64) or kMapBlock (mixed)
     const int4* irange;       // [I] node blocks [x, y), beam blocks [z, w) of the instance
+    int n_eblk;               // evaluation node blocks
+    const int4* eblk;         // [n_eblk] first node, node count, instance, 0
+    const int2* erange;       // [I] evaluation node blocks [x, y) of the instance
     const int* inst_n;        // [I] nodes of the instance
     const long long* inst_free;  // [I] unlocked DOFs of the instance
     const float2* off;        // [I] (x, z) offset of the instance in the contact grid
@@ -68,6 +71,8 @@ struct DevTopo {
 // beam blocks of the mixed form; the FP64 form's beam blocks (one warp per FP64 unit of an SM).
 constexpr int kMapBlock = 256;
 constexpr int kBeamBlock = 128;
+// Nodes per evaluation node block (state and gather; the solver's vectors use kMapBlock).
+constexpr int kEvalBlock = 128;
 
 #if defined(__CUDACC__)
 // Position of a thread of a mapped block: element index, instance; valid == false past the
@@ -178,23 +183,23 @@ struct EvalBufs {
     double4_32a* M;             // [3N] rotation matrix rows of R (x, y, z, pad)
     float4* xf_lo;              // [N] position rounded down to single precision
     float4* xf_hi;              // [N] position rounded up
-    double* slotA;          // [6B] (-F, Ga) per beam, added to node a
-    double* slotB;          // [6B] (+F, Gb) per beam, added to node b
-    double* part_state;     // [9 * nb_nodes] sum, -min, max of x per block
+    double* slot;           // [12B] per beam: (-F, Ga), added to node a, then (+F, Gb), added to
+                            //   node b: entry 2 beam + role, the incidence list's numbering
+    double* part_state;     // [9 * n_eblk] sum, -min, max of x per block
     double* part_beam;      // [3 * nb_beams]
     unsigned* err;          // [1] a kernel's bounded wait gave up (the host reports it)
-    double* part_node;      // [kNodeParts * nb_nodes]
+    double* part_node;      // [kNodeParts * n_eblk]
     double* part_fin;       // [I * kFinPartDoubles] first-stage totals of the finalize
     double* cen;            // [9 (I + 1)] per instance mean, min, max of the node positions (min/max
                             //   in the contact grid's frame); then min/max over all instances
+    double* cforce;         // [2 I] centering force of the instance on each node (x, z)
     double* tops;           // [I] platen height per instance
     EvalOut* out;           // [I]
     double* trial_next;     // [7B] SoA
     double* trial_aux;      // [7B] SoA
     uint8_t* trial_flags;   // [3B] SoA
     // mixed-precision form
-    float* slotAf;          // [6B]
-    float* slotBf;          // [6B]
+    float* slotf;           // [12B] as slot
     float* trial_nextf;     // [7B] SoA
     float* trial_auxf;      // [7B] SoA
 };
@@ -227,8 +232,6 @@ extern std::atomic<long long> g_launch_count;
 inline void note_launches(int k) { g_launch_count += k; }
 
 // ---- launchers (objective.cu) ----------------------------------------------------------
-int nb_nodes(int N);
-int nb_beams(int B);
 void launch_state(const DevTopo& t, const PhysParams& p, const double* z, const double* base_x,
                   const double* base_r, EvalBufs& e, cudaStream_t s);
 // Occupancy variants of the beam kernels and the gather (CTAs per SM the register allocation
@@ -251,7 +254,7 @@ void launch_finalize(const DevTopo& t, const PhysParams& p, const ContactBufs* c
 // instances with mask[i] != 0 (mask == nullptr: all)
 void launch_commit(const DevTopo& t, const uint8_t* mask, const EvalBufs& e, double* base_x, double* base_r,
                    double* plastic, cudaStream_t s);
-void launch_center(const DevTopo& t, EvalBufs& e, cudaStream_t s);
+void launch_center(const DevTopo& t, const PhysParams& p, EvalBufs& e, cudaStream_t s);
 void launch_gather_mixed(const DevTopo& t, const PhysParams& p, const ContactBufs* c, double* grad, EvalBufs& e,
                          cudaStream_t s, int variant = 0);
 

@@ -1,6 +1,9 @@
 // objective.cu -- FP64 kernels of the energy/gradient evaluation
 // (the reference's Simulator::state + objective, MC/src/sim.cpp:136-172).
 //
+// Compiled without contraction: fused multiply-adds are written out where they are meant, so
+// that a kernel's occupancy variants round identically.
+//
 //   k_state    per node: z -> current position/orientation; block partial sums of x
 //   k_center   one block: mean position for the centering term
 //   k_beams    per beam: axial/shear/bending/torsion energy with return mapping,
@@ -16,27 +19,26 @@ namespace mcg {
 
 static_assert(kMapBlock == kBlock, "mapped blocks are launched with kBlock threads");
 
-int nb_nodes(int N) { return int(grid_for(N)); }
-int nb_beams(int B) { return int(grid_for(B)); }
-
 // ---- node state: MC/src/sim.cpp:136 -------------------------------------------------------
-__global__ void __launch_bounds__(kBlock) k_state(DevTopo t, PhysParams p, const double* __restrict__ z,
-                                                  const double* __restrict__ bx, const double* __restrict__ br,
-                                                  double4_32a* __restrict__ x4, double4_32a* __restrict__ R4,
-                                                  double4_32a* __restrict__ M4, float4* __restrict__ xf_lo,
-                                                  float4* __restrict__ xf_hi, double* __restrict__ part) {
-    __shared__ double sm[3 * kBlock];
-    __shared__ float smx[4 * (kBlock / 32)];
-    const MapPos mp = map_pos(t.nblk);
+// Bound by the FP64 pipe like the beam kernel: rotations up to one radian by polynomials
+// (larger ones by the general exponential), the quaternion normalized by one step when its norm
+// is one but for rounding, conversions and maxima on the integer pipe; 128-node blocks.  222 ->
+// 72 FP64 instructions per 32 nodes; 34,897 nodes: 24.1 -> 11.5 us.
+__global__ void __launch_bounds__(kEvalBlock) k_state(DevTopo t, PhysParams p, const double* __restrict__ z,
+                                                      const double* __restrict__ bx, const double* __restrict__ br,
+                                                      double4_32a* __restrict__ x4, double4_32a* __restrict__ R4,
+                                                      double4_32a* __restrict__ M4, float4* __restrict__ xf_lo,
+                                                      float4* __restrict__ xf_hi, double* __restrict__ part) {
+    __shared__ StateParts sm;
+    const MapPos mp = map_pos(t.eblk);
     if (!t.active[mp.inst]) return;  // block-uniform
     const int i = mp.i;
     double acc[3] = {0, 0, 0};
-    const float ninf = __int_as_float(0xff800000);
-    float mx[4] = {ninf, ninf, ninf, ninf};  // -min x, -min z, max x, max z (grid frame, FP32)
-    const double ninfd = __longlong_as_double(0xfff0000000000000LL);
-    double my[2] = {ninfd, ninfd};  // -min y, max y (FP64: the permanent set reads them)
+    StateBounds bounds;
     if (mp.valid) {
-        const double* zi = z + 6 * size_t(i);
+        const double2* z2 = reinterpret_cast<const double2*>(z + 6 * size_t(i));
+        const double2 za = z2[0], zb = z2[1], zc = z2[2];
+        const double zi[6] = {za.x, za.y, zb.x, zb.y, zc.x, zc.y};
         const uint8_t* li = t.locked + 6 * size_t(i);
         double tr[3], r[3];
 #pragma unroll
@@ -50,50 +52,34 @@ __global__ void __launch_bounds__(kBlock) k_state(DevTopo t, PhysParams p, const
         const double xx = __dadd_rn(bx[3 * size_t(i)], __dmul_rn(ts, tr[0]));
         const double xy = __dadd_rn(bx[3 * size_t(i) + 1], __dmul_rn(ts, tr[1]));
         const double xz = __dadd_rn(bx[3 * size_t(i) + 2], __dmul_rn(ts, tr[2]));
-        const q4 b{br[4 * size_t(i)], br[4 * size_t(i) + 1], br[4 * size_t(i) + 2], br[4 * size_t(i) + 3]};
-        const q4 R = qnorm(qmul(exp_map(d3{r[0], r[1], r[2]}), b));
+        const double4_32a b4 = reinterpret_cast<const double4_32a*>(br)[i];
+        const d3 rv{r[0], r[1], r[2]};
+        const double r2 = fdot(rv, rv);
+        const q4 e = unsigned(__double2hiint(r2)) < 0x3ff00000u ? exp_map_small(rv, r2) : exp_map(rv);
+        const q4 R = qnorm_near(fqmul(e, q4{b4.x, b4.y, b4.z, b4.w}));
         x4[i] = make_double4_32a(xx, xy, xz, 0.0);
-        // single-precision bounds of the position in the contact grid's frame (the
-        // instance's offset added with outward rounding)
-        const float2 o = t.off[mp.inst];
-        const float4 lo = make_float4(__fadd_rd(__double2float_rd(xx), o.x), __double2float_rd(xy),
-                                      __fadd_rd(__double2float_rd(xz), o.y), 0.f);
-        const float4 hi = make_float4(__fadd_ru(__double2float_ru(xx), o.x), __double2float_ru(xy),
-                                      __fadd_ru(__double2float_ru(xz), o.y), 0.f);
-        xf_lo[i] = lo;
-        xf_hi[i] = hi;
         R4[i] = make_double4_32a(R.w, R.x, R.y, R.z);
         const m3 M = quat_matrix(R);
         M4[3 * size_t(i)] = make_double4_32a(M.r0.x, M.r0.y, M.r0.z, 0.0);
         M4[3 * size_t(i) + 1] = make_double4_32a(M.r1.x, M.r1.y, M.r1.z, 0.0);
         M4[3 * size_t(i) + 2] = make_double4_32a(M.r2.x, M.r2.y, M.r2.z, 0.0);
+        bounds.take(xx, xy, xz, t.off[mp.inst], xf_lo[i], xf_hi[i]);
         acc[0] = xx; acc[1] = xy; acc[2] = xz;
-        // bounding box in the grid's frame: x and z from the outward-rounded bounds (they
-        // contain the FP64 positions), y exact; fmax/fmaxf skip NaN coordinates
-        mx[0] = -lo.x; mx[1] = -lo.z; mx[2] = hi.x; mx[3] = hi.z;
-        my[0] = -xy; my[1] = xy;
     }
-    block_sum_t<3>(acc, sm);
-    block_max_nf<4>(mx, smx);
-    block_max_t<2>(my, sm);
-    if (threadIdx.x == 0) {
-        double* q = part + 9 * size_t(blockIdx.x);
-        q[0] = acc[0]; q[1] = acc[1]; q[2] = acc[2];
-        q[3] = double(mx[0]); q[4] = my[0]; q[5] = double(mx[1]);
-        q[6] = double(mx[2]); q[7] = my[1]; q[8] = double(mx[3]);
-    }
+    state_block_parts(acc, bounds, sm, part + 9 * size_t(blockIdx.x));
 }
 
 // Mean position of each instance's nodes (MC/src/sim.cpp:143) and bounding boxes from the
 // k_state partials: block i < I writes instance i's cen[9i..9i+8] (mean, minimum, maximum);
 // block I the minimum and maximum over all instances at cen[9I + 3..8].
-__global__ void __launch_bounds__(kBlock) k_center(DevTopo t, const double* __restrict__ part,
-                                                   double* __restrict__ cen) {
+// Also the instance's centering force on each node (sim.cpp:143).
+__global__ void __launch_bounds__(kBlock) k_center(DevTopo t, double centering, const double* __restrict__ part,
+                                                   double* __restrict__ cen, double* __restrict__ cforce) {
     __shared__ double sm[6 * kBlock];
     const int inst = blockIdx.x;
-    int k0 = 0, k1 = t.n_nblk;
+    int k0 = 0, k1 = t.n_eblk;
     if (inst < t.I) {
-        const int4 r = t.irange[inst];
+        const int2 r = t.erange[inst];
         k0 = r.x;
         k1 = r.y;
     }
@@ -114,6 +100,8 @@ __global__ void __launch_bounds__(kBlock) k_center(DevTopo t, const double* __re
         if (inst < t.I) {
             const double inv = 1.0 / double(t.inst_n[inst]);
             c[0] = acc[0] * inv; c[1] = acc[1] * inv; c[2] = acc[2] * inv;
+            cforce[2 * inst] = centering * c[0] / double(t.inst_n[inst]);
+            cforce[2 * inst + 1] = centering * c[2] / double(t.inst_n[inst]);
         }
         c[3] = -mx[0]; c[4] = -mx[1]; c[5] = -mx[2];
         c[6] = mx[3]; c[7] = mx[4]; c[8] = mx[5];
@@ -161,17 +149,17 @@ __device__ __forceinline__ Ret1 return1(double e, double pc, double ac, double k
 struct Ret3 { d3 force, p; double a, dg, energy2; bool yielded; };
 __device__ __forceinline__ Ret3 return3(d3 e, d3 pc, double ac, double k, double y, double H, double inv_kH) {
     Ret3 r{{}, pc, ac, 0, 0, false};
-    double e2 = len2(e);
+    double e2 = fdot(e, e);
     const double Y = fma(H, ac, y);
     if (positive(fma((k * k) * (1.0 + 0x1p-48), e2, -Y * Y)) || negative_sign(Y)) {
         const double rs = rsqrt_any(e2), n = k * (e2 * rs), f = n - Y;
         if (positive(f) && less_bits(1e-20, n)) {
             r.dg = f * inv_kH;
-            const d3 dp = e * (rs * r.dg);
-            r.p = pc + dp;
+            const double f1 = rs * r.dg;
+            r.p = fmadd(e, f1, pc);
             r.a = ac + r.dg;
-            e = e - dp;
-            e2 = len2(e);
+            e = fmadd(e, -f1, e);
+            e2 = fdot(e, e);
             r.yielded = true;
         }
     }
@@ -202,8 +190,9 @@ __device__ __forceinline__ void chord_length(double l2, double& L, double& invL)
 // arctangent; larger angles take atan2 as the reference does.  Q is a product of two unit
 // quaternions, so its norm differs from one by rounding only and one step corrects it.
 __device__ __forceinline__ d3 relative_rotation(q4 Ra, q4 Rb, double& phi2) {
-    q4 Q = qmul(conj(Ra), Rb);
-    const double v2 = Q.x * Q.x + Q.y * Q.y + Q.z * Q.z, n2 = fma(Q.w, Q.w, v2);
+    q4 Q = fqmul(conj(Ra), Rb);
+    const d3 v{Q.x, Q.y, Q.z};
+    const double v2 = fdot(v, v), n2 = fma(Q.w, Q.w, v2);
     const double r = fma(-.5, n2, 1.5);
     const double s2 = v2 * (r * r);
     if (near_one(n2) && unsigned(__double2hiint(s2)) < 0x3fb99999u) {  // s2 < 0.1
@@ -242,14 +231,14 @@ __device__ __forceinline__ d3 transport(d3 phi, double phi2, d3 v) {
     A = fma(A, phi2, 0x1.1566aba745146p-15);
     A = fma(A, phi2, 0x1.6c16c16c1de72p-10);
     A = fma(A, phi2, 0x1.5555555555553p-4);
-    const d3 c1 = cross(phi, v), c2 = cross(phi, c1);
+    const d3 c1 = fcross(phi, v), c2 = fcross(phi, c1);
     return d3{fma(A, c2.x, fma(.5, c1.x, v.x)), fma(A, c2.y, fma(.5, c1.y, v.y)), fma(A, c2.z, fma(.5, c1.z, v.z))};
 }
 
 // The beam's axis in the material frame: unit(Ra^T t), t a unit vector.
 __device__ __forceinline__ d3 material_axis(const m3& Ma, d3 t) {
-    const d3 a = mrot_t(Ma, t);
-    const double l2 = len2(a);
+    const d3 a = fmrot_t(Ma, t);
+    const double l2 = fdot(a, a);
     if (near_one(l2)) return a * fma(-.5, l2, 1.5);
     return unit(a);
 }
@@ -285,13 +274,12 @@ __global__ void __launch_bounds__(kBeamBlock, 2 * kMinBlocks) k_beams(DevTopo t,
         const d3 d{__dsub_rn(xb.x, xa.x), __dsub_rn(xb.y, xa.y), __dsub_rn(xb.z, xa.z)};
         double L, invL;
         chord_length(__dadd_rn(__dadd_rn(__dmul_rn(d.x, d.x), __dmul_rn(d.y, d.y)), __dmul_rn(d.z, d.z)), L, invL);
-        double* sa = e.slotA + 6 * size_t(b);
-        double* sb = e.slotB + 6 * size_t(b);
+        double2* slot = reinterpret_cast<double2*>(e.slot) + 6 * size_t(b);
         if (less_bits(L, 1e-10)) {
             // Degenerate element: penalty energy only, no gradient and a default trial.
             penalty = 1e8 * sqr(1e-10 - L);
 #pragma unroll
-            for (int k = 0; k < 6; k++) { sa[k] = 0; sb[k] = 0; }
+            for (int k = 0; k < 6; k++) slot[k] = make_double2(0, 0);
             if (trials) {
 #pragma unroll
                 for (int k = 0; k < 7; k++) { e.trial_next[k * size_t(B) + b] = 0; e.trial_aux[k * size_t(B) + b] = 0; }
@@ -311,40 +299,44 @@ __global__ void __launch_bounds__(kBeamBlock, 2 * kMinBlocks) k_beams(DevTopo t,
             // shear: the end directors against the chord (rotations by the nodes' matrices)
             const m3 Ma = ldm(e.M, ab.x), Mb = ldm(e.M, ab.y);
             const d3 e0{t.e0x[b], t.e0y[b], t.e0z[b]};
-            const d3 da = mrot(Ma, e0), db = mrot(Mb, e0);
+            const d3 da = fmrot(Ma, e0), db = fmrot(Mb, e0);
             const double cs = t.cs[b];
             const d3 ma = da - tt, mb = db - tt;
-            const double us2 = len2(ma) + len2(mb);  // times cs
+            const double us2 = fma(mb.z, mb.z, fma(mb.y, mb.y, fma(mb.x, mb.x, fdot(ma, ma))));  // times cs
             const d3 gm = ma + mb;
             const double kt_ = cs * invL;
-            const double kf = fma(kt_, dot(gm, tt), t.area[b] * ax.force);
+            const double kf = fma(kt_, fdot(gm, tt), t.area[b] * ax.force);
             // F = t N + ((I - t t^T) g) / L with g = -cs (ma + mb)
             const d3 F{fma(tt.x, kf, -(kt_ * gm.x)), fma(tt.y, kf, -(kt_ * gm.y)), fma(tt.z, kf, -(kt_ * gm.z))};
             const d3 tc = tt * cs;
-            d3 Ga = cross(tc, da);
-            d3 Gb = cross(tc, db);
+            d3 Ga = fcross(tc, da);
+            d3 Gb = fcross(tc, db);
             // bending and torsion from the relative rotation Q = Ra^* Rb
             double phi2;
             const d3 phi = relative_rotation(ldq(e.R, ab.x), ldq(e.R, ab.y), phi2);
             const d3 axis = material_axis(Ma, tt);
-            const double tw = dot(phi, axis), ptw = dot(rotp, axis);
-            const d3 bend = phi - axis * tw, pb = rotp - axis * ptw;
+            const double tw = fdot(phi, axis), ptw = fdot(rotp, axis);
+            const d3 bend = fmadd(axis, -tw, phi), pb = fmadd(axis, -ptw, rotp);
             const double kb = t.kb[b], kt = t.kt[b];
             const Ret3 br = return3(bend - pb, pb, pl_alphaB, kb, t.my[b], t.hb[b], t.inv_kbh[b]);
             const Ret1 tor = return1(tw - ptw, ptw, pl_alphaT, kt, t.ty[b], t.ht[b], t.inv_kth[b]);
-            const d3 moment = br.force + axis * tor.force;
+            const d3 moment = fmadd(axis, tor.force, br.force);
             double dr = 0;
             if (br.yielded) dr = t.my[b] * br.dg;
             if (tor.yielded) dr = fma(t.ty[b], tor.dg, dr);
-            const d3 world = mrot(Ma, transport(phi, phi2, moment));
+            const d3 world = fmrot(Ma, transport(phi, phi2, moment));
             Ga = Ga - world;
             Gb = Gb + world;
             elastic2 = fma(cs, us2, uax2) + (br.energy2 + tor.energy2);
-            sa[0] = -F.x; sa[1] = -F.y; sa[2] = -F.z; sa[3] = Ga.x; sa[4] = Ga.y; sa[5] = Ga.z;
-            sb[0] = F.x;  sb[1] = F.y;  sb[2] = F.z;  sb[3] = Gb.x; sb[4] = Gb.y; sb[5] = Gb.z;
+            slot[0] = make_double2(-F.x, -F.y);
+            slot[1] = make_double2(-F.z, Ga.x);
+            slot[2] = make_double2(Ga.y, Ga.z);
+            slot[3] = make_double2(F.x, F.y);
+            slot[4] = make_double2(F.z, Gb.x);
+            slot[5] = make_double2(Gb.y, Gb.z);
             if (trials) {
                 const size_t S = size_t(B);
-                const d3 nrot = br.p + axis * tor.p;
+                const d3 nrot = fmadd(axis, tor.p, br.p);
                 e.trial_next[b] = ax.p;
                 e.trial_next[S + b] = ax.a;
                 e.trial_next[2 * S + b] = nrot.x;
@@ -468,17 +460,18 @@ __device__ __forceinline__ void sum_slots(const DevTopo& t, const EvalBufs& e, i
     if (!F32) {
 #pragma unroll 4
         for (int k = k0; k < k1; k++) {
-            const int v = t.inc[k];
-            const double* s = ((v & 1) ? e.slotB : e.slotA) + 6 * size_t(v >> 1);
-            gx.x += s[0]; gx.y += s[1]; gx.z += s[2];
-            gr.x += s[3]; gr.y += s[4]; gr.z += s[5];
+            const double2* s = reinterpret_cast<const double2*>(e.slot) + 3 * size_t(t.inc[k]);
+            const double2 a = s[0], b = s[1], c = s[2];
+            gx.x += a.x; gx.y += a.y; gx.z += b.x;
+            gr.x += b.y; gr.y += c.x; gr.z += c.y;
         }
     } else {
         float hi[6] = {0, 0, 0, 0, 0, 0}, lo[6] = {0, 0, 0, 0, 0, 0};
 #pragma unroll 4
         for (int k = k0; k < k1; k++) {
-            const int v = t.inc[k];
-            const float* s = ((v & 1) ? e.slotBf : e.slotAf) + 6 * size_t(v >> 1);
+            const float2* s2 = reinterpret_cast<const float2*>(e.slotf) + 3 * size_t(t.inc[k]);
+            const float2 p = s2[0], q = s2[1], r = s2[2];
+            const float s[6] = {p.x, p.y, q.x, q.y, r.x, r.y};
 #pragma unroll
             for (int j = 0; j < 6; j++) {  // two-sum
                 const float a = s[j], sum = hi[j] + a, bp = sum - hi[j];
@@ -486,31 +479,34 @@ __device__ __forceinline__ void sum_slots(const DevTopo& t, const EvalBufs& e, i
                 hi[j] = sum;
             }
         }
-        gx = d3{double(hi[0]) + double(lo[0]), double(hi[1]) + double(lo[1]), double(hi[2]) + double(lo[2])};
-        gr = d3{double(hi[3]) + double(lo[3]), double(hi[4]) + double(lo[4]), double(hi[5]) + double(lo[5])};
+        gx = d3{to_double(hi[0]) + to_double(lo[0]), to_double(hi[1]) + to_double(lo[1]), to_double(hi[2]) + to_double(lo[2])};
+        gr = d3{to_double(hi[3]) + to_double(lo[3]), to_double(hi[4]) + to_double(lo[4]), to_double(hi[5]) + to_double(lo[5])};
     }
 }
 
+// Per-warp totals of the gather.
+struct GatherParts {
+    double sum[5][kEvalBlock / 32];  // gravity E, |g|^2, platen E, reaction, self-contact E
+    int count[kEvalBlock / 32];
+    long long m[2][kEvalBlock / 32];  // max penetration, max |g| (bits of non-negative doubles)
+};
+
+// Bound by the FP64 pipe (the incident vectors' additions) and the latency of their loads.
+// Only what nearly every node has is reduced always (gravity energy and |g|^2, in five FP64
+// additions a warp); platen and contact totals where a node of the warp touches something.
+// 34,897 nodes with 41,722 contacts: 39 -> 33 us.
+// kMinBlocks: units of 256 threads per SM the register allocation must allow.
 template <bool F32, int kMinBlocks>
-__global__ void __launch_bounds__(kBlock, kMinBlocks) k_gather(DevTopo t, PhysParams p, ContactBufs c, int use_contacts,
-                                                               EvalBufs e, double* __restrict__ grad) {
-    __shared__ double sm[6 * kBlock];
-    __shared__ double cforce[2];
-    const MapPos mp = map_pos(t.nblk);
+__global__ void __launch_bounds__(kEvalBlock, 2 * kMinBlocks) k_gather(DevTopo t, PhysParams p, ContactBufs c,
+                                                                       int use_contacts, EvalBufs e,
+                                                                       double* __restrict__ grad) {
+    __shared__ GatherParts sm;
+    const MapPos mp = map_pos(t.eblk);
     if (!t.active[mp.inst]) return;  // block-uniform
     const int i = mp.i;
     const int N = t.N;
-    // centering force of the block's instance (sim.cpp:143), the same for all its nodes:
-    // one FP64 division per block (GB300's FP64 pipe is narrow)
-    if (threadIdx.x == 0) {
-        const double* cen = e.cen + 9 * size_t(mp.inst);
-        const double Ni = double(t.inst_n[mp.inst]);
-        cforce[0] = p.centering * cen[0] / Ni;
-        cforce[1] = p.centering * cen[2] / Ni;
-    }
-    __syncthreads();
-    double acc[6] = {0, 0, 0, 0, 0, 0};  // gravity E, platen E, reaction, contacts, self-contact E, |g|^2
-    double pen_max = 0;
+    double egrav = 0, g2 = 0, eplat = 0, reac = 0, econt = 0, pen_max = 0;
+    int count = 0;
     unsigned long long gbits = 0;  // max |g| as the bits of a non-negative double (integer max)
     if (mp.valid) {
         d3 gx{0, 0, 0}, gr{0, 0, 0};
@@ -518,11 +514,11 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) k_gather(DevTopo t, PhysPa
         const d3 xi = ldx(e.x, i);
         // gravity (sim.cpp:142)
         const double mg = t.mass[i] * p.gravity;
-        acc[0] = mg * xi.y;
+        egrav = mg * xi.y;
         gx.y += mg;
-        // centering (sim.cpp:143)
-        gx.x += cforce[0];
-        gx.z += cforce[1];
+        // centering (sim.cpp:143), the same force for all nodes of the instance
+        gx.x += e.cforce[2 * mp.inst];
+        gx.z += e.cforce[2 * mp.inst + 1];
         // self-contact forces on this node in ascending (lower shape, higher shape, slot)
         // order (the list is sorted by the contact pipeline), and the self-contact energy of
         // each contact on the first node of its lower shape: both independent of the order
@@ -531,10 +527,10 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) k_gather(DevTopo t, PhysPa
         if (cnt > 32 && c.long_sum) {  // summed by k_node_contact_long
             const double* q = c.long_sum + 6 * size_t(c.n_cursor[i]);
             gx = gx + d3{q[0], q[1], q[2]};
-            acc[4] += q[3];
-            acc[3] += q[4];
+            econt += q[3];
+            count += int(q[4]);
             pen_max = fmax(pen_max, q[5]);
-        } else if (use_contacts) {
+        } else if (cnt) {
             const uint32_t s0 = c.n_start[i];
             uint32_t k = 0;
             // four items at a time: their loads in flight together (a joint of a densely
@@ -551,59 +547,91 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks) k_gather(DevTopo t, PhysPa
 #pragma unroll
                 for (int j = 0; j < 4; j++) {
                     gx = gx + f[j];
-                    if (pen[j] >= 0) {
-                        acc[4] += .5 * p.contact_k * pen[j] * pen[j];
-                        acc[3] += 1;
+                    if (!negative_sign(pen[j])) {
+                        econt += .5 * p.contact_k * pen[j] * pen[j];
+                        count += 1;
                         pen_max = fmax(pen_max, pen[j]);
                     }
                 }
             }
-            for (; k < cnt; k++) add_contact_item(c, p, N, c.n_sorted[s0 + k], gx, acc[4], acc[3], pen_max);
+            for (; k < cnt; k++) {
+                double one = 0;
+                add_contact_item(c, p, N, c.n_sorted[s0 + k], gx, econt, one, pen_max);
+                count += one != 0;
+            }
         }
         // platens (sim.cpp:168-171)
         const double jr = p.joint_radius, kc = p.contact_k;
         const double pb = jr - xi.y;
-        if (pb > 0) {
+        if (positive(pb)) {
             const double mm = kc * pb;
-            acc[1] += .5 * kc * pb * pb;
+            eplat += .5 * kc * pb * pb;
             pen_max = fmax(pen_max, pb);
-            acc[3] += 1;
+            count += 1;
             gx.y -= mm;
         }
         const double pt = xi.y + jr - e.tops[mp.inst];
-        if (pt > 0) {
+        if (positive(pt)) {
             const double mm = kc * pt;
-            acc[1] += .5 * kc * pt * pt;
-            acc[2] += mm;
+            eplat += .5 * kc * pt * pt;
+            reac += mm;
             pen_max = fmax(pen_max, pt);
-            acc[3] += 1;
+            count += 1;
             gx.y += mm;
         }
         // pack, scale and lock (sim.cpp:172)
         const double ts = p.translation_scale;
         const uint8_t* li = t.locked + 6 * size_t(i);
-        double* g = grad + 6 * size_t(i);
-        const double gv[6] = {ts * gx.x, ts * gx.y, ts * gx.z, gr.x, gr.y, gr.z};
+        double gv[6] = {ts * gx.x, ts * gx.y, ts * gx.z, gr.x, gr.y, gr.z};
 #pragma unroll
         for (int k = 0; k < 6; k++) {
-            g[k] = li[k] ? 0.0 : gv[k];
+            if (li[k]) gv[k] = 0.0;
             // residual over free DOFs for the solver's convergence test (sim.cpp:44-45)
-            if (!li[k]) {
-                acc[5] += gv[k] * gv[k];
-                // fmax(gmax, |g|) on the bit patterns; a NaN (above the infinity pattern) is
-                // skipped as fmax skips it
-                const unsigned long long b = (unsigned long long)__double_as_longlong(gv[k]) & 0x7fffffffffffffffULL;
-                if (b <= 0x7ff0000000000000ULL && b > gbits) gbits = b;
-            }
+            g2 = fma(gv[k], gv[k], g2);
+            // fmax(gmax, |g|) on the bit patterns; a NaN (above the infinity pattern) is
+            // skipped as fmax skips it
+            const unsigned long long b = (unsigned long long)__double_as_longlong(gv[k]) & 0x7fffffffffffffffULL;
+            if (b <= 0x7ff0000000000000ULL && b > gbits) gbits = b;
         }
+        double2* g = reinterpret_cast<double2*>(grad + 6 * size_t(i));
+        g[0] = make_double2(gv[0], gv[1]);
+        g[1] = make_double2(gv[2], gv[3]);
+        g[2] = make_double2(gv[4], gv[5]);
     }
-    block_sum_t<6>(acc, sm);
-    double m2[2] = {pen_max, __longlong_as_double((long long)gbits)};
-    block_max_t<2>(m2, sm);
-    if (threadIdx.x == 0) {
-        double* q = e.part_node + kNodeParts * size_t(blockIdx.x);
-        q[0] = acc[0]; q[1] = acc[1]; q[2] = acc[2]; q[3] = m2[0]; q[4] = acc[3]; q[5] = acc[4];
-        q[6] = acc[5]; q[7] = m2[1];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const double v = warp_sum2(egrav, g2);
+    const long long gm = warp_max_key((long long)gbits);
+    double w = 0;
+    long long pm = 0;
+    int cn = 0;
+    if (__any_sync(0xffffffffu, count != 0)) {
+        w = warp_sum4(eplat, reac, econt, 0.0);
+        pm = warp_max_key(__double_as_longlong(pen_max));
+        cn = __reduce_add_sync(0xffffffffu, count);
+    }
+    if (lane == 0) {
+        sm.m[0][warp] = pm;
+        sm.m[1][warp] = gm;
+        sm.count[warp] = cn;
+    }
+    if ((lane & 15) == 0) sm.sum[lane >> 4][warp] = v;
+    if ((lane & 7) == 0 && lane < 24) sm.sum[2 + (lane >> 3)][warp] = w;
+    __syncthreads();
+    constexpr int nw = kEvalBlock / 32;
+    const int tid = threadIdx.x;
+    double* q = e.part_node + kNodeParts * size_t(blockIdx.x);
+    if (tid < 5) {
+        double s = sm.sum[tid][0];
+        for (int k = 1; k < nw; k++) s += sm.sum[tid][k];
+        q[tid == 0 ? 0 : tid == 1 ? 6 : tid == 2 ? 1 : tid == 3 ? 2 : 5] = s;
+    } else if (tid < 7) {
+        long long m = sm.m[tid - 5][0];
+        for (int k = 1; k < nw; k++) m = max(m, sm.m[tid - 5][k]);
+        q[tid == 5 ? 3 : 7] = __longlong_as_double(m);
+    } else if (tid == 7) {
+        int n = 0;
+        for (int k = 0; k < nw; k++) n += sm.count[k];
+        q[4] = double(n);
     }
 }
 
@@ -621,13 +649,14 @@ __global__ void __launch_bounds__(kBlock) k_finalize_parts(DevTopo t, const doub
     const int inst = blockIdx.y, f = blockIdx.x;
     if (!t.active[inst]) return;
     const int4 r = t.irange[inst];
+    const int2 er = t.erange[inst];
     double acc[6] = {0, 0, 0, 0, 0, 0};  // beamE, elastic, plastic, gravityE, platenE, reaction
     double cacc[3] = {0, 0, 0};          // self-contact E, contacts (platen and self), |g|^2
     double m2[2] = {0, 0};               // max penetration, max |g|
     for (int k = r.z + f + kFinFan * int(threadIdx.x); k < r.w; k += kFinFan * int(blockDim.x)) {
         acc[0] += pbeam[3 * k]; acc[1] += pbeam[3 * k + 1]; acc[2] += pbeam[3 * k + 2];
     }
-    for (int k = r.x + f + kFinFan * int(threadIdx.x); k < r.y; k += kFinFan * int(blockDim.x)) {
+    for (int k = er.x + f + kFinFan * int(threadIdx.x); k < er.y; k += kFinFan * int(blockDim.x)) {
         const double* q = pnode + kNodeParts * size_t(k);
         acc[3] += q[0]; acc[4] += q[1]; acc[5] += q[2];
         m2[0] = fmax(m2[0], q[3]);
@@ -781,13 +810,13 @@ __global__ void __launch_bounds__(kBlock) k_plastic_final(DevTopo t, const doubl
 // ---- launchers ------------------------------------------------------------------------------
 void launch_state(const DevTopo& t, const PhysParams& p, const double* z, const double* base_x,
                   const double* base_r, EvalBufs& e, cudaStream_t s) {
-    k_state<<<t.n_nblk, kBlock, 0, s>>>(t, p, z, base_x, base_r, e.x, e.R, e.M, e.xf_lo, e.xf_hi, e.part_state);
+    k_state<<<t.n_eblk, kEvalBlock, 0, s>>>(t, p, z, base_x, base_r, e.x, e.R, e.M, e.xf_lo, e.xf_hi, e.part_state);
     note_launches(1);
-    launch_center(t, e, s);
+    launch_center(t, p, e, s);
 }
 
-void launch_center(const DevTopo& t, EvalBufs& e, cudaStream_t s) {
-    k_center<<<t.I + 1, kBlock, 0, s>>>(t, e.part_state, e.cen);
+void launch_center(const DevTopo& t, const PhysParams& p, EvalBufs& e, cudaStream_t s) {
+    k_center<<<t.I + 1, kBlock, 0, s>>>(t, p.centering, e.part_state, e.cen, e.cforce);
     note_launches(1);
 }
 
@@ -808,7 +837,7 @@ void launch_plastic_stats(const DevTopo& t, const double* plastic, double* part,
     note_launches(2);
 }
 
-// Occupancy variants of the FP64 beam kernel (256-thread units per SM) and of the gather (CTAs per SM).
+// Occupancy variants of the FP64 beam kernel (256-thread units per SM) and of the gather.
 constexpr int kBeamBlocks[] = {1, 2, 3};
 constexpr int kGatherBlocks[] = {1, 2, 4};
 
@@ -851,9 +880,9 @@ void gather_variant(const DevTopo& t, const PhysParams& p, const ContactBufs* c,
         (k_node_contact_long<<<kLongListBlocks, kBlock, 0, s>>>(t, p, cc), note_launches(1));
     }
     switch (variant) {
-        case 1: k_gather<F32, kGatherBlocks[1]><<<t.n_nblk, kBlock, 0, s>>>(t, p, cc, uc, e, grad); break;
-        case 2: k_gather<F32, kGatherBlocks[2]><<<t.n_nblk, kBlock, 0, s>>>(t, p, cc, uc, e, grad); break;
-        default: k_gather<F32, kGatherBlocks[0]><<<t.n_nblk, kBlock, 0, s>>>(t, p, cc, uc, e, grad); break;
+        case 1: k_gather<F32, kGatherBlocks[1]><<<t.n_eblk, kEvalBlock, 0, s>>>(t, p, cc, uc, e, grad); break;
+        case 2: k_gather<F32, kGatherBlocks[2]><<<t.n_eblk, kEvalBlock, 0, s>>>(t, p, cc, uc, e, grad); break;
+        default: k_gather<F32, kGatherBlocks[0]><<<t.n_eblk, kEvalBlock, 0, s>>>(t, p, cc, uc, e, grad); break;
     }
     note_launches(1);
 }

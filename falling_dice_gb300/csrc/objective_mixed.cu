@@ -169,29 +169,27 @@ __device__ __forceinline__ f3 rotvec_f(float qw, f3 qv) {
 // ---- node state --------------------------------------------------------------------------
 // u = s t (FP32), e = exp(r) as (w - 1, v) (FP32), x = x_base + u (FP64, for contact,
 // platen and centering), FP32 position bounds; block partial sums and extrema of x.
-__global__ void __launch_bounds__(kBlock) k_state_mixed(DevTopo t, double ts, const double* __restrict__ z,
+__global__ void __launch_bounds__(kEvalBlock) k_state_mixed(DevTopo t, double ts, const double* __restrict__ z,
                                                         const double* __restrict__ bx, float4* __restrict__ UE,
                                                         double4_32a* __restrict__ x4,
                                                         float4* __restrict__ xf_lo, float4* __restrict__ xf_hi,
                                                         double* __restrict__ part) {
-    __shared__ double sm[3 * kBlock];
-    __shared__ float smx[4 * (kBlock / 32)];
-    const MapPos mp = map_pos(t.nblk);
+    __shared__ StateParts sm;
+    const MapPos mp = map_pos(t.eblk);
     if (!t.active[mp.inst]) return;
     const int i = mp.i;
     double acc[3] = {0, 0, 0};
-    const float ninf = __int_as_float(0xff800000);
-    float mx[4] = {ninf, ninf, ninf, ninf};  // -min x, -min z, max x, max z (grid frame, FP32)
-    const double ninfd = __longlong_as_double(0xfff0000000000000LL);
-    double my[2] = {ninfd, ninfd};  // -min y, max y (FP64: the permanent set reads them)
+    StateBounds bounds;
     if (mp.valid) {
-        const double* zi = z + 6 * size_t(i);
+        const double2* z2 = reinterpret_cast<const double2*>(z + 6 * size_t(i));
+        const double2 za = z2[0], zb = z2[1], zc = z2[2];
+        const double zi[6] = {za.x, za.y, zb.x, zb.y, zc.x, zc.y};
         const uint8_t* li = t.locked + 6 * size_t(i);
         float tr[3], r[3];
 #pragma unroll
         for (int d = 0; d < 3; d++) {
-            tr[d] = li[d] ? 0.f : float(zi[d] * ts);
-            r[d] = li[d + 3] ? 0.f : float(zi[d + 3]);
+            tr[d] = li[d] ? 0.f : to_float<RoundTo::kNearest>(zi[d] * ts);
+            r[d] = li[d + 3] ? 0.f : to_float<RoundTo::kNearest>(zi[d + 3]);
         }
         UE[2 * size_t(i)] = make_float4(tr[0], tr[1], tr[2], 0.f);
         const float th2 = r[0] * r[0] + r[1] * r[1] + r[2] * r[2];
@@ -207,32 +205,14 @@ __global__ void __launch_bounds__(kBlock) k_state_mixed(DevTopo t, double ts, co
             sv = 2.f * s4 * c4 / th;
         }
         UE[2 * size_t(i) + 1] = make_float4(wm1, r[0] * sv, r[1] * sv, r[2] * sv);
-        const double xx = bx[3 * size_t(i)] + double(tr[0]);
-        const double xy = bx[3 * size_t(i) + 1] + double(tr[1]);
-        const double xz = bx[3 * size_t(i) + 2] + double(tr[2]);
+        const double xx = bx[3 * size_t(i)] + to_double(tr[0]);
+        const double xy = bx[3 * size_t(i) + 1] + to_double(tr[1]);
+        const double xz = bx[3 * size_t(i) + 2] + to_double(tr[2]);
         x4[i] = make_double4_32a(xx, xy, xz, 0.0);
-        const float2 o = t.off[mp.inst];
-        const float4 lo = make_float4(__fadd_rd(__double2float_rd(xx), o.x), __double2float_rd(xy),
-                                      __fadd_rd(__double2float_rd(xz), o.y), 0.f);
-        const float4 hi = make_float4(__fadd_ru(__double2float_ru(xx), o.x), __double2float_ru(xy),
-                                      __fadd_ru(__double2float_ru(xz), o.y), 0.f);
-        xf_lo[i] = lo;
-        xf_hi[i] = hi;
+        bounds.take(xx, xy, xz, t.off[mp.inst], xf_lo[i], xf_hi[i]);
         acc[0] = xx; acc[1] = xy; acc[2] = xz;
-        // bounding box in the grid's frame: x and z from the outward-rounded bounds (they
-        // contain the FP64 positions), y exact; fmax/fmaxf skip NaN coordinates
-        mx[0] = -lo.x; mx[1] = -lo.z; mx[2] = hi.x; mx[3] = hi.z;
-        my[0] = -xy; my[1] = xy;
     }
-    block_sum_t<3>(acc, sm);
-    block_max_nf<4>(mx, smx);
-    block_max_t<2>(my, sm);
-    if (threadIdx.x == 0) {
-        double* q = part + 9 * size_t(blockIdx.x);
-        q[0] = acc[0]; q[1] = acc[1]; q[2] = acc[2];
-        q[3] = double(mx[0]); q[4] = my[0]; q[5] = double(mx[1]);
-        q[6] = double(mx[2]); q[7] = my[1]; q[8] = double(mx[3]);
-    }
+    state_block_parts(acc, bounds, sm, part + 9 * size_t(blockIdx.x));
 }
 
 // ---- per-increment base terms (FP64, once per commit) ----------------------------------------
@@ -324,12 +304,11 @@ __device__ __forceinline__ void beam_mixed(const Material& mat, const MixedBeams
     const float q = c0 + 2.f * fdot(d0, du) + fdot(du, du);  // |d|^2 - L0^2
     const f3 d = d0 + du;
     const float L = sqrtf(fmaxf(L0 * L0 + q, 0.f));
-    float* sa = e.slotAf + 6 * size_t(b);
-    float* sb = e.slotBf + 6 * size_t(b);
+    float4* slot = reinterpret_cast<float4*>(e.slotf) + 3 * size_t(b);
     if (L < 1e-10f) {
         ue = 1e8f * (1e-10f - L) * (1e-10f - L);
 #pragma unroll
-        for (int k = 0; k < 6; k++) { sa[k] = 0.f; sb[k] = 0.f; }
+        for (int k = 0; k < 3; k++) slot[k] = make_float4(0.f, 0.f, 0.f, 0.f);
         if (trials) {
 #pragma unroll
             for (int k = 0; k < 7; k++) { e.trial_nextf[k * size_t(B) + b] = 0.f; e.trial_auxf[k * size_t(B) + b] = 0.f; }
@@ -405,8 +384,9 @@ __device__ __forceinline__ void beam_mixed(const Material& mat, const MixedBeams
         Gb = Gb + world;
         ue = uax + us + ur;
         up = dax + dr;
-        sa[0] = -F.x; sa[1] = -F.y; sa[2] = -F.z; sa[3] = Ga.x; sa[4] = Ga.y; sa[5] = Ga.z;
-        sb[0] = F.x;  sb[1] = F.y;  sb[2] = F.z;  sb[3] = Gb.x; sb[4] = Gb.y; sb[5] = Gb.z;
+        slot[0] = make_float4(-F.x, -F.y, -F.z, Ga.x);
+        slot[1] = make_float4(Ga.y, Ga.z, F.x, F.y);
+        slot[2] = make_float4(F.z, Gb.x, Gb.y, Gb.z);
         if (trials) {
             const size_t S = size_t(B);
             const f3 nrot = br.p + axis * tor.p;
@@ -635,10 +615,10 @@ __global__ void k_f32_to_f64(long long n, const float* __restrict__ a, double* _
 
 void launch_state_mixed(const DevTopo& t, const PhysParams& p, const double* z, const double* base_x,
                         const MixedNodes& mn, EvalBufs& e, cudaStream_t s) {
-    k_state_mixed<<<t.n_nblk, kBlock, 0, s>>>(t, p.translation_scale, z, base_x, mn.UE, e.x, e.xf_lo, e.xf_hi,
+    k_state_mixed<<<t.n_eblk, kEvalBlock, 0, s>>>(t, p.translation_scale, z, base_x, mn.UE, e.x, e.xf_lo, e.xf_hi,
                                               e.part_state);
     note_launches(1);
-    launch_center(t, e, s);
+    launch_center(t, p, e, s);
 }
 
 // Variants of the mixed beam kernel: the plain kernel at 3, 4, 5 or 6 CTAs per SM, and the

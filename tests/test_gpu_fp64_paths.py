@@ -67,3 +67,22 @@ def test_a_nan_position_gives_the_reference_outcome(mcg, mco):
     z[free[17]] = np.nan
     r = sol.objective(z, lat.geometry.top0 + 0.01)
     assert r["energy"] == np.inf and not np.any(r["grad"])
+
+
+@pytest.mark.parametrize("cells", [(1, 1, 30), (1, 1, 31), (1, 1, 32), (3, 3, 3), (4, 4, 4), (3, 7, 7), (5, 6, 5)])
+def test_node_counts_around_the_block_size(mcg, mco, cells):
+    """Cubic lattices of 64 .. 256 nodes (124, 128, 132; blocks of 128 nodes) between both platens
+    and with self-contact on: totals, extrema and residual norms of full and partial blocks."""
+    cfg, spec = workloads.bcc(cells)
+    spec.kind = abi.MCG_LATTICE_CUBIC
+    lat = mcg.generate_lattice(spec, cfg)
+    sol, orc = mcg.Solver(cfg, lat), mco.Model("mco", cfg, lattice=lat)
+    z, pl = mcg.random_state(lat, 0.2, 0.1, 0.02, 21)
+    for m in (sol, orc):
+        m.set_state(plastic=pl)
+    top = lat.geometry.top0 - 0.1 * lat.geometry.height
+    r, o = sol.objective(z, top), orc.objective(z, top, False)
+    s = {"energy": o["energy"], "grad": o["grad"],
+         "diag": np.array([o["diag"][k] for k in ("elastic", "plastic", "contact", "reaction", "max_pen", "contacts")])}
+    check_eval(r, s, cells)
+    assert np.array_equal(sol.contact_pairs(), orc.contact_pairs(z))

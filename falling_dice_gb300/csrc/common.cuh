@@ -463,6 +463,23 @@ struct StateBounds {
         y[1] = order_key(xy);
     }
 };
+// Whether a node may have moved farther than `skin` from its position at the list's build: the
+// displacement bounded from its FP32 interval [l, h] and the stored lower end r of its interval at
+// the build (one FP32 ulp wide at most), all rounded upward.  A list built with boxes grown by
+// `skin` holds every pair whose boxes overlap at any state where no node has moved farther than
+// skin (Euclidean, so no farther on any axis): each current box lies inside the build's.
+__device__ __forceinline__ bool moved_beyond(float skin, float4 l, float4 h, float4 r) {
+    const float ulp = 1.2e-7f * fmaxf(fmaxf(fabsf(r.x), fabsf(r.y)), fabsf(r.z)) + 1e-30f;
+    const float dx = __fadd_ru(fmaxf(__fsub_ru(h.x, r.x), __fsub_ru(r.x, l.x)), ulp);
+    const float dy = __fadd_ru(fmaxf(__fsub_ru(h.y, r.y), __fsub_ru(r.y, l.y)), ulp);
+    const float dz = __fadd_ru(fmaxf(__fsub_ru(h.z, r.z), __fsub_ru(r.z, l.z)), ulp);
+    const float d2 = __fadd_ru(__fadd_ru(__fmul_ru(dx, dx), __fmul_ru(dy, dy)), __fmul_ru(dz, dz));
+    return !(__fsqrt_ru(d2) <= skin);  // also when not finite
+}
+// All threads of the block: asks for a build when one of its nodes has moved.
+__device__ __forceinline__ void ask_build(const BuildArgs& b, bool moved) {
+    if (__any_sync(0xffffffffu, moved) && (threadIdx.x & 31) == 0) b.flags[1] = 1u;
+}
 struct StateParts {
     double sum[3][kEvalBlock / 32];
     long long y[2][kEvalBlock / 32];

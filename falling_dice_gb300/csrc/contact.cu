@@ -13,21 +13,21 @@
 // handed out by the bin's atomic counter).  The pair pass gives each occupied bin to one
 // warp, which enumerates the bin's pairs in the order the atomics handed out: the candidate
 // list's order can vary from run to run, its content cannot, and nothing computed from it
-// depends on the order (contact forces and energies are summed per node in shape-pair
-// order, and pair sets are reported sorted).  A pair is examined only in the cell that is the
+// depends on the order (pair sets are reported sorted).  A pair is examined only in the cell that is the
 // minimum corner of the intersection of the two shapes' cell ranges: every pair that
 // shares a cell is examined exactly once -- the reference's `tested` set without a set.
 // A conservative FP32 AABB test and the local-shape exclusion (sim.cpp:24-39) run before
 // the FP64 narrow phase.
 //
-// Output order.  Candidate pairs are appended to one flat list in chunks staged per warp;
-// the narrow phase flags the candidates in contact, a scan places them, and the contact
-// list keeps the candidate order.  Per-node force lists are built with counters and sorted by contact
-// key (lower shape, higher shape, slot), so every sum is independent of the list order.
+// Sums without an order.  Candidates, kept candidates and contacts are appended to flat lists in
+// whatever order the warps arrive; a contact's forces and energy are added to its nodes' records
+// as fixed-point integers (NodeContact), whose sums are exact and the same in any order.  So no
+// result depends on the lists' order, and no list is counted, scanned, filled or sorted per
+// node.
 //
-// No host synchronisation: sizes that can overflow a buffer (a bin's slots, bins,
-// candidates, contacts, a shape spanning too many cells) raise a flag instead of writing out of bounds, and the
-// host repeats the evaluation with larger buffers (or coarser cells) when it sees one.
+// No host synchronisation: sizes that can overflow a buffer (a bin's slots, bins, candidates,
+// contacts, a shape spanning too many cells) raise a flag instead of writing out of bounds, and
+// the host repeats the evaluation with larger buffers (or coarser cells) when it sees one.
 #include "common.cuh"
 #include "kernels.h"
 
@@ -36,14 +36,13 @@ namespace mcg {
 namespace {
 
 constexpr long long kMaxCellsPerShape = 1 << 12;
-constexpr float kBoxQuanta = 32000.f;   // quantization steps across the grid extent
 constexpr uint32_t kBoxMax = 32767u;    // 15-bit box coordinates
 constexpr uint32_t kGuard2 = 0x80008000u;
 constexpr uint32_t kShapeBits = 29;     // shape id below, first-cell flags above
 constexpr int kPairWarps = kBlock / 32;
 constexpr int kPairGrab = 2;             // bins a warp claims at a time (<= 32)
 constexpr int kPairRanks = 128;          // bins up to this size are enumerated from registers
-constexpr int kStreamBlocks = 8 * 152;
+constexpr int kStreamBlocks = 4 * 152;   // grid of the list kernels (256 threads, grid-stride)
 
 __device__ __forceinline__ uint32_t spread3_10(uint32_t v) {  // 10 bits -> every third bit
     v &= 0x3ffu;
@@ -215,193 +214,86 @@ __device__ __noinline__ PairHit narrow_phase(const DevTopo& t, const PhysParams&
     return h;
 }
 
-// ---- candidate-list reuse -------------------------------------------------------------------
-// The list built with boxes inflated by `skin` holds every pair whose boxes overlap at any
-// state where no node has moved farther than skin (Euclidean, so no farther on any axis)
-// from its position at the build: each current box lies inside the inflated box of the
-// build.  flags[1] = rebuild now.
-// A node's displacement is bounded from its FP32 interval [lo, hi] and the stored lower end
-// of its interval at the build (one FP32 ulp wide at most), rounding upward.
-__global__ void __launch_bounds__(kBlock) k_skin_check(DevTopo t, int N, const float4* __restrict__ xf_lo,
-                                                       const float4* __restrict__ xf_hi,
-                                                       const float4* __restrict__ xref, float skin,
-                                                       uint32_t* __restrict__ flags) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (!(skin > 0.f)) {  // no reuse: every evaluation builds, no position to compare
-        if (i == 0) atomicOr(flags + 1, 1u);
-        return;
-    }
-    bool moved = false;
-    if (i == 0 && flags[2]) moved = true;
-    if (i < N && !moved && t.active[t.node_inst[i]]) {
-        const float4 l = xf_lo[i], h = xf_hi[i], r = xref[i];
-        // per-axis bounds of the move, then its Euclidean length, all rounded upward
-        const float ulp = 1.2e-7f * fmaxf(fmaxf(fabsf(r.x), fabsf(r.y)), fabsf(r.z)) + 1e-30f;
-        const float dx = __fadd_ru(fmaxf(__fsub_ru(h.x, r.x), __fsub_ru(r.x, l.x)), ulp);
-        const float dy = __fadd_ru(fmaxf(__fsub_ru(h.y, r.y), __fsub_ru(r.y, l.y)), ulp);
-        const float dz = __fadd_ru(fmaxf(__fsub_ru(h.z, r.z), __fsub_ru(r.z, l.z)), ulp);
-        const float d2 = __fadd_ru(__fadd_ru(__fmul_ru(dx, dx), __fmul_ru(dy, dy)), __fmul_ru(dz, dz));
-        moved = !(__fsqrt_ru(d2) <= skin);  // also when not finite
-    }
-    if (__any_sync(0xffffffffu, moved) && (threadIdx.x & 31) == 0) atomicOr(flags + 1, 1u);
-}
-
-// After a rebuild: the build positions and the end of a forced rebuild.  A build that
-// overflowed a buffer (bins, bin slots, cell span, candidates) left an incomplete list:
-// the next evaluation must build again, whatever the skin says, so that the overflow is
-// raised again there (the overflow bits are per evaluation; a caller that enqueues several
-// evaluations before reading sees only the last one's).
-__global__ void __launch_bounds__(kBlock) k_skin_commit(int N, const float4* __restrict__ xf_lo,
-                                                        float4* __restrict__ xref, uint32_t* __restrict__ flags) {
-    if (!flags[1]) return;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < N) xref[i] = xf_lo[i];
-    if (i == 0)
-        flags[2] = (flags[0] & uint32_t(kOverEntries | kOverBins | kOverSpan | kOverCandidates)) ? 1u : 0u;
-}
-
-__global__ void __launch_bounds__(kBlock) k_zero_gated(long long n, uint32_t* __restrict__ a,
-                                                       const uint32_t* __restrict__ gate) {
-    if (!*gate) return;
-    for (long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (long long)gridDim.x * blockDim.x)
-        a[k] = 0;
-}
-
 // ---- kernels -------------------------------------------------------------------------------
-// Grid origin, extent and bin numbering from the node bounding box (e.cen[3..8]).
-__global__ void k_grid_params(const double* __restrict__ cen, double pad, double cell, long long bin_cap, int* grid,
-                              uint32_t* flags, uint32_t* ncand, uint32_t* nentries) {
-    if (threadIdx.x != 0 || blockIdx.x != 0 || !flags[1]) return;
-    flags[4]++;  // builds since the buffers were allocated
-    *ncand = 0;  // the candidate list and entry counts of this build
-    nentries[0] = 0;
-    nentries[1] = 0;
-    nentries[2] = 0;
-    bool ok = true;
-    long long lo[3], dim[3];
-    for (int d = 0; d < 3; d++) {
-        const double a = floor((cen[3 + d] - pad) / cell) - 1.0;
-        const double b = floor((cen[6 + d] + pad) / cell) + 1.0;
-        if (!isfinite(a) || !isfinite(b) || fabs(a) > 1e9 || fabs(b) > 1e9) {
-            ok = false;
-            lo[d] = 0;
-            dim[d] = 1;
-            continue;
-        }
-        lo[d] = (long long)a;
-        dim[d] = (long long)b - lo[d] + 1;
-    }
-    int bits = 0;
-    for (int d = 0; d < 3; d++)
-        while ((1LL << bits) < dim[d]) bits++;
-    long long nb;
-    int mode;
-    if (bits <= 10 && (1LL << (3 * bits)) <= bin_cap && (1LL << (3 * bits)) <= 4 * dim[0] * dim[1] * dim[2]) {
-        mode = 0;
-        nb = 1LL << (3 * bits);
-    } else {
-        mode = 1;
-        nb = dim[0] * dim[1] * dim[2];
-    }
-    grid[9] = int(nb < (1LL << 30) ? nb : (1LL << 30));
-    if (ok && nb > bin_cap) {  // the host enlarges the bins or coarsens the cells
-        atomicOr(flags, uint32_t(kOverBins));
-        ok = false;
-    }
-    for (int d = 0; d < 3; d++) {
-        grid[d] = int(lo[d]);
-        grid[3 + d] = int(dim[d]);
-        // box quantization: kBoxQuanta steps across the grid's extent on each axis
-        grid[10 + d] = __float_as_int(float(double(kBoxQuanta) / (double(dim[d]) * cell)));
-        grid[13 + d] = __float_as_int(float(double(lo[d]) * cell));
-    }
-    grid[6] = mode;
-    grid[7] = ok ? 1 : 0;
-    grid[8] = ok ? int(nb) : 0;
-}
-
-// Per-shape bounding box and cell range, in single precision rounded outward: the box
-// contains the reference's double-precision box (sim.cpp:154), and cell indices are a
-// monotone function of it, so two shapes whose reference boxes overlap share a cell.
-// The pair-test record holds the box quantized to 15 bits per axis (floor minus one
-// quantum for the low side, ceil plus one for the high side, so the quantized box contains
-// the FP32 box whatever the rounding of the scaling) with a guard bit over each high
-// value, and the first cell packed as three 10-bit fields.
-__global__ void __launch_bounds__(kBlock) k_shape_prep(DevTopo t, PhysParams p, const float4* __restrict__ xf_lo,
-                                                       const float4* __restrict__ xf_hi, const int* __restrict__ grid,
-                                                       int4* __restrict__ cell_lo, int4* __restrict__ cell_hi,
-                                                       uint4* __restrict__ rec, float skin,
-                                                       uint32_t* __restrict__ flags) {
+// Boxes and bin entries of every shape, when the candidate list is rebuilt (flags[1], decided by
+// the state and center kernels).
+// The box is in single precision rounded outward: it contains the reference's double-precision
+// box (sim.cpp:154), and cell indices are a monotone function of it, so two shapes whose
+// reference boxes overlap share a cell.  The pair-test record holds the box quantized to 15 bits
+// per axis (floor minus one quantum for the low side, ceil plus one for the high side, so the
+// quantized box contains the FP32 box whatever the rounding of the scaling) with a guard bit over
+// each high value, and the first cell packed as three 10-bit fields.
+// Entries: one per cell of the shape's range, written straight into the bin's slot that the bin
+// counter hands out (all counters are zero here: the pair pass clears each bin it reads), four
+// returning atomics in flight per thread.  A bin that fills up keeps counting (kOverEntries, and
+// the largest count in counts[kLargestBin] so the host can size bin_slots).
+__global__ void __launch_bounds__(kBlock) k_shapes(DevTopo t, PhysParams p, const float4* __restrict__ xf_lo,
+                                                   const float4* __restrict__ xf_hi, float skin, ContactBufs c) {
     const int S = t.N + t.B;
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= S || !flags[1]) return;
+    if (s >= S || !c.flags[1]) return;
+    const int* __restrict__ grid = c.grid;
     const int2 nd = shape_nodes(t, uint32_t(s));
     const int n1 = nd.y >= 0 ? nd.y : nd.x;
+    if (!grid[7] || !t.active[t.node_inst[nd.x]]) return;  // inactive instances take no part
     const float4 al = xf_lo[nd.x], ah = xf_hi[nd.x], bl = xf_lo[n1], bh = xf_hi[n1];
     const float pad = __fadd_ru(s < t.N ? p.joint_padf : t.padf[s - t.N], skin);
     const float lo[3] = {__fsub_rd(fminf(al.x, bl.x), pad), __fsub_rd(fminf(al.y, bl.y), pad),
                          __fsub_rd(fminf(al.z, bl.z), pad)};
     const float hi[3] = {__fadd_ru(fmaxf(ah.x, bh.x), pad), __fadd_ru(fmaxf(ah.y, bh.y), pad),
                          __fadd_ru(fmaxf(ah.z, bh.z), pad)};
-    const bool finite_box = isfinite(lo[0]) && isfinite(lo[1]) && isfinite(lo[2]) && isfinite(hi[0]) &&
-                            isfinite(hi[1]) && isfinite(hi[2]);
-    if (!grid[7] || !finite_box || !t.active[t.node_inst[nd.x]]) {  // inactive instances take no part
-        cell_lo[s] = make_int4(0, 0, 0, 0);
-        cell_hi[s] = make_int4(-1, -1, -1, 0);
-        rec[s] = make_uint4(0, 0, 0, 0);
-        if (!finite_box) atomicOr(flags, uint32_t(kNonFinite));
+    if (!(isfinite(lo[0]) && isfinite(lo[1]) && isfinite(lo[2]) && isfinite(hi[0]) && isfinite(hi[1]) &&
+          isfinite(hi[2]))) {
+        atomicOr(c.flags, uint32_t(kNonFinite));
         return;
     }
-    int c0[3], c1[3];
+    int c0[3], dim[3];
     uint32_t q0[3], q1[3];
-    long long n = 1;
     bool wide = false;
 #pragma unroll
     for (int d = 0; d < 3; d++) {
-        const float dim = float(grid[3 + d] - 1);
+        const float top = float(grid[3 + d] - 1);
         const float org = float(grid[d]);
-        c0[d] = int(fminf(fmaxf(floorf(lo[d] * p.inv_cell_f) - org, 0.f), dim));
-        c1[d] = int(fminf(fmaxf(floorf(hi[d] * p.inv_cell_f) - org, 0.f), dim));
-        n *= (long long)(c1[d] - c0[d] + 1);
-        wide |= c1[d] - c0[d] >= 1024;
+        c0[d] = int(fminf(fmaxf(floorf(lo[d] * p.inv_cell_f) - org, 0.f), top));
+        dim[d] = int(fminf(fmaxf(floorf(hi[d] * p.inv_cell_f) - org, 0.f), top)) - c0[d] + 1;
+        wide |= dim[d] > 1024;
         const float qs = __int_as_float(grid[10 + d]), qo = __int_as_float(grid[13 + d]);
         q0[d] = uint32_t(fminf(fmaxf(floorf((lo[d] - qo) * qs) - 1.f, 0.f), float(kBoxMax)));
         q1[d] = uint32_t(fminf(fmaxf(ceilf((hi[d] - qo) * qs) + 1.f, 0.f), float(kBoxMax)));
     }
-    if (n > kMaxCellsPerShape || wide) {  // the host coarsens the grid and evaluates again
-        atomicOr(flags, uint32_t(kOverSpan));
-        n = 0;
-        c1[0] = c0[0] - 1;
+    if (wide || (long long)dim[0] * dim[1] * dim[2] > kMaxCellsPerShape) {
+        atomicOr(c.flags, uint32_t(kOverSpan));  // the host coarsens the grid and evaluates again
+        return;
     }
-    cell_lo[s] = make_int4(c0[0], c0[1], c0[2], 0);
-    cell_hi[s] = make_int4(c1[0], c1[1], c1[2], 0);
-    rec[s] = make_uint4(q0[0] | (q0[1] << 16), (q1[0] | (q1[1] << 16)) | kGuard2, q0[2] | ((q1[2] | 0x8000u) << 16),
-                        pack_cell(c0[0], c0[1], c0[2]));
-}
-
-// Entries of shape s: one per cell of its range, written straight into the bin's slot that
-// the bin counter hands out.  A bin that fills up keeps counting (kOverEntries, and the
-// largest count in nentries[1] so the host can size bin_slots).
-__global__ void __launch_bounds__(kBlock) k_emit(int S, const int* __restrict__ grid, const int4* __restrict__ cell_lo,
-                                                 const int4* __restrict__ cell_hi, int bin_slots,
-                                                 uint32_t* __restrict__ bin_count, uint32_t* __restrict__ bin_items,
-                                                 uint32_t* __restrict__ nentries, uint32_t* __restrict__ flags) {
-    if (!flags[1]) return;
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s < S) {
-        const int4 lo = cell_lo[s], hi = cell_hi[s];
-        for (int j = lo.y; j <= hi.y; j++)
-            for (int k = lo.z; k <= hi.z; k++)
-                for (int i = lo.x; i <= hi.x; i++) {
-                    const uint32_t b = bin_of(grid, i, j, k);
-                    const uint32_t slot = atomicAdd(&bin_count[b], 1u);
-                    if (slot < uint32_t(bin_slots)) {
-                        bin_items[size_t(b) * size_t(bin_slots) + slot] = uint32_t(s);
-                    } else {
-                        atomicOr(flags, uint32_t(kOverEntries));
-                        atomicMax(nentries + 1, slot + 1);
-                    }
+    c.rec[s] = make_uint4(q0[0] | (q0[1] << 16), (q1[0] | (q1[1] << 16)) | kGuard2, q0[2] | ((q1[2] | 0x8000u) << 16),
+                          pack_cell(c0[0], c0[1], c0[2]));
+    const int n = dim[0] * dim[1] * dim[2];
+    int i = 0, j = 0, k = 0;  // the next cell of the range
+    for (int e0 = 0; e0 < n; e0 += 4) {
+        uint32_t bin[4], slot[4];
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            if (e0 + e >= n) break;
+            bin[e] = bin_of(grid, c0[0] + i, c0[1] + j, c0[2] + k);
+            slot[e] = atomicAdd(&c.bin_count[bin[e]], 1u);
+            if (++i == dim[0]) {
+                i = 0;
+                if (++j == dim[1]) {
+                    j = 0;
+                    k++;
                 }
+            }
+        }
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            if (e0 + e >= n) break;
+            if (slot[e] < uint32_t(c.bin_slots)) {
+                c.bin_items[size_t(bin[e]) * size_t(c.bin_slots) + slot[e]] = uint32_t(s);
+            } else {
+                atomicOr(c.flags, uint32_t(kOverEntries));
+                atomicMax(c.counts + kLargestBin, slot[e] + 1);
+            }
+        }
     }
 }
 
@@ -517,7 +409,7 @@ __device__ __forceinline__ void rotate_pairs(const PairRec& me, const uint4* __r
 // Candidate pairs of every bin holding two or more shapes.  Warps claim the grid's bins
 // kPairGrab at a time (single bins near the end) from a cursor (flags[3]) and skip the empty
 // ones (one ballot), so bins of uneven size balance over the grid; they count the build's
-// cell entries and occupied bins into nentries[0] and [2] on the way, and append their
+// cell entries and occupied bins on the way, clear the bin counters, and append their
 // candidate pairs (lower shape, higher shape) to the flat list in warp-sized batches, one
 // atomic on ncand per batch, without a counting pass.  The list's length is the number of
 // pairs, whatever the order.
@@ -530,12 +422,12 @@ __device__ __forceinline__ void rotate_pairs(const PairRec& me, const uint4* __r
 //   larger    the same by groups of 32: each group is staged in turn and then meets every
 //             later group, staged 32 records at a time.
 __global__ void __launch_bounds__(kBlock, 6) k_bin_pairs(DevTopo t, const int* __restrict__ grid,
-                                                      const uint32_t* __restrict__ bin_count, int bin_slots,
-                                                      uint32_t* __restrict__ nentries,
+                                                      uint32_t* __restrict__ bin_count, int bin_slots,
+                                                      uint32_t* __restrict__ counts,
                                                       const uint32_t* __restrict__ bin_items,
                                                       const uint4* __restrict__ rec, long long cand_cap,
-                                                      uint2* __restrict__ cand, uint32_t* __restrict__ ncand,
-                                                      uint32_t* __restrict__ flags) {
+                                                      uint2* __restrict__ cand, uint32_t* __restrict__ flags) {
+    uint32_t* __restrict__ ncand = counts + kCand;
     __shared__ uint4 rec_all[kPairWarps][kPairRanks];  // the bin's records, staged for the partner reads
     __shared__ int2 nd_all[kPairWarps][kPairRanks];
     if (!flags[1]) return;
@@ -560,6 +452,7 @@ __global__ void __launch_bounds__(kBlock, 6) k_bin_pairs(DevTopo t, const int* _
         b0 = __shfl_sync(0xffffffffu, b0, 0);
         if (b0 >= nbins) break;
         const uint32_t cnt = lane < int(grab) && b0 + lane < nbins ? bin_count[b0 + lane] : 0u;
+        if (cnt) bin_count[b0 + lane] = 0;  // zero for the next build
         if (b0 + grab >= single_from) grab = 1;
         entries += cnt;
         unsigned todo = __ballot_sync(0xffffffffu, cnt >= 2);  // the claimed bins holding pairs
@@ -657,8 +550,8 @@ __global__ void __launch_bounds__(kBlock, 6) k_bin_pairs(DevTopo t, const int* _
     }
     entries = __reduce_add_sync(0xffffffffu, entries);
     if (lane == 0) {
-        if (entries) atomicAdd(nentries, entries);
-        if (occupied) atomicAdd(nentries + 2, occupied);
+        if (entries) atomicAdd(counts + kEntries, entries);
+        if (occupied) atomicAdd(counts + kOccupied, occupied);
     }
 }
 
@@ -681,6 +574,7 @@ struct DistBounds {
     bool far_ok;      // far is a valid lower bound (the closest points are not within 1e-7 m)
     float far;        // certified lower bound on the distance, already less its error
     float near;       // certified upper bound on the distance between points at (s, tt)
+    bool near_ok;     // near bounds the reference's distance too (below)
     float pad_sum;    // pad_a + pad_b >= the reference's target
     float target_lo;  // <= the reference's target ra + rb + margin
 };
@@ -727,6 +621,11 @@ __device__ __forceinline__ DistBounds dist_bounds(const DevTopo& t, const PhysPa
     r.pad_sum = (pa + pb) * 1.000001f;
     // the pads less one margin exceed the target by at most two FP32 roundings
     r.target_lo = (pa + pb - float(p.contact_margin)) * 0.999999f;
+    // The reference takes s = 0 where a e - b^2 <= 1e-20, whatever the angle (sim.cpp:14): its points
+    // then lie up to sqrt(1e-20 / min(a, e)) farther apart than the closest ones.  Struts of a
+    // millimetre stay far inside the allowance; for tiny ones only the exact test can tell.
+    const float shorter = fminf(a, e);
+    r.near_ok = shorter == 0.f || err * err * shorter >= 1e-20f;
     r.near = isfinite(nn) ? sqrtf(nn) * 1.000001f + err : __int_as_float(0x7f800000);
     r.far_ok = nn > 1e-14f;  // false also when not finite
     r.far = 0.f;
@@ -745,215 +644,180 @@ __device__ __forceinline__ DistBounds dist_bounds(const DevTopo& t, const PhysPa
 __device__ __forceinline__ int distance_class(const DevTopo& t, const PhysParams& p, const float4* __restrict__ xf,
                                               uint32_t sa, uint32_t sb) {
     const DistBounds d = dist_bounds(t, p, xf, sa, sb);
-    if (d.near < d.target_lo) return 1;
+    if (d.near_ok && d.near < d.target_lo) return 1;
     return d.far_ok && d.far > d.pad_sum ? -1 : 0;
 }
 
-// Candidate filter, once per list build: keeps, in order, the candidates of one
-// instance whose certified distance lower bound at the build does not exceed the pads plus
-// `reach` (2 skin: every point of a segment whose endpoints move at most skin moves at most
-// skin, so two segments close a gap by at most 2 skin) and whose nodes are not connected (sim.cpp:24-39).  Pass 0: keep bits and counts per chunk of 32; pass 1 (after a scan of the
-// counts): the kept candidates, compacted.
-template <int pass>
-__global__ void __launch_bounds__(kBlock) k_filter(DevTopo t, PhysParams p, const float4* __restrict__ xf,
-                                                   long long cand_cap, const uint2* __restrict__ cand,
-                                                   const uint32_t* __restrict__ ncand, float reach,
-                                                   uint32_t* __restrict__ fbits, uint32_t* __restrict__ fcount,
-                                                   const uint32_t* __restrict__ foff, uint2* __restrict__ cand2,
-                                                   const uint32_t* __restrict__ gate) {
-    if (!*gate) return;
+constexpr int kBatch = 4;  // candidates per lane behind one list atomic
+
+// Appends the flagged candidates of a warp's batch to a list of capacity cap: bit u of `keep`
+// stands for this lane's candidate u.  One atomic per warp and batch.  All lanes call it.
+template <typename Put>
+__device__ __forceinline__ void append_batch(uint32_t keep, uint32_t* __restrict__ count, long long cap, Put put) {
     const int lane = threadIdx.x & 31;
-    const unsigned below = (1u << lane) - 1u;
-    const uint32_t total = uint32_t(min((long long)*ncand, cand_cap));
-    const long long nchunk = (total + 31) / 32;
-    const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
-    for (long long ch = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; ch < nchunk; ch += warps) {
-        const uint32_t g = uint32_t(ch * 32 + lane);
-        if constexpr (pass == 1) {
-            if (!fbits[ch]) continue;  // warp-uniform
+    const uint32_t below = (1u << lane) - 1u;
+    uint32_t m[kBatch], total = 0;
+#pragma unroll
+    for (int u = 0; u < kBatch; u++) {
+        m[u] = __ballot_sync(0xffffffffu, keep >> u & 1u);
+        total += __popc(m[u]);
+    }
+    if (total == 0) return;  // warp-uniform
+    uint32_t base = 0;
+    if (lane == 0) base = atomicAdd(count, total);
+    base = __shfl_sync(0xffffffffu, base, 0);
+#pragma unroll
+    for (int u = 0; u < kBatch; u++) {
+        if (keep >> u & 1u) {
+            const long long at = (long long)base + __popc(m[u] & below);
+            if (at < cap) put(at, u);
         }
-        if constexpr (pass == 0) {
-            bool keep = false;
-            if (g < total) {
-                const uint2 q = cand[g];
-                const int2 na = shape_nodes(t, q.x), nb = shape_nodes(t, q.y);
-                if (t.node_inst[na.x] == t.node_inst[nb.x]) {
-                    const DistBounds d = dist_bounds(t, p, xf, q.x, q.y);
-                    keep = !(d.far_ok && d.far > d.pad_sum + reach);
-                    // local pairs (sim.cpp:24-39) never make contact: dropped here, once per
-                    // build, so the narrow phase of every evaluation needs no hash lookups
-                    if (keep) keep = !any_connected(t, na, nb);
-                }
-            }
-            const unsigned m = __ballot_sync(0xffffffffu, keep);
-            if (lane == 0) {
-                fbits[ch] = m;
-                fcount[ch] = __popc(m);
-            }
-        } else {
-            const unsigned m = fbits[ch];
-            if (m & (1u << lane)) cand2[foff[ch] + __popc(m & below)] = cand[g];
-        }
+        base += __popc(m[u]);
     }
 }
 
-// Narrow phase over the filtered list (flat, in order), one candidate per thread.
-// Pass 0: test every candidate; one hit bit per candidate and the hit count per chunk of
-// 32.  Pass 1 (after a scan of the chunk counts of the list's length): the hits' candidate
-// indices, compacted in candidate order (into c_a, overwritten by k_contacts).
-template <int pass>
-__global__ void __launch_bounds__(kBlock) k_narrow(DevTopo t, PhysParams p, const double4_32a* __restrict__ x,
-                                                   const float4* __restrict__ xf, const uint2* __restrict__ cand2,
-                                                   const uint32_t* __restrict__ ntotal,
-                                                   uint32_t* __restrict__ hitbits, uint32_t* __restrict__ hcount,
-                                                   const uint32_t* __restrict__ hoff, ContactBufs c) {
+// Candidate filter, once per list build: keeps the candidates of one instance whose certified
+// distance lower bound at the build does not exceed the pads plus `reach` (2 skin: every point
+// of a segment whose endpoints move at most skin moves at most skin, so two segments close a gap
+// by at most 2 skin) and whose nodes are not connected (sim.cpp:24-39; local pairs never make
+// contact, so the narrow phase of every evaluation needs no hash lookups).
+// The kernel also ends the build: it stores the positions that later evaluations measure their
+// moves from, and the end of a forced rebuild.  A build that overflowed a buffer (bins, bin
+// slots, cell span, candidates) left an incomplete list: the next evaluation must build again,
+// whatever the skin says, so that the overflow is raised again there (the overflow bits are per
+// evaluation; a caller that enqueues several evaluations before reading sees only the last one's).
+__global__ void __launch_bounds__(kBlock) k_filter(DevTopo t, PhysParams p, const float4* __restrict__ xf, float reach,
+                                                   ContactBufs c) {
+    if (!c.flags[1]) return;
+    const long long thread = (long long)blockIdx.x * blockDim.x + threadIdx.x, threads = (long long)gridDim.x * blockDim.x;
+    for (long long i = thread; i < t.N; i += threads) c.xref[i] = xf[i];
+    if (thread == 0)
+        c.flags[2] = (c.flags[0] & uint32_t(kOverEntries | kOverBins | kOverSpan | kOverCandidates)) ? 1u : 0u;
     const int lane = threadIdx.x & 31;
-    const unsigned below = (1u << lane) - 1u;
-    const uint32_t total = *ntotal;
-    const long long nchunk = (total + 31) / 32;
-    const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
-    for (long long ch = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; ch < nchunk; ch += warps) {
-        const uint32_t g = uint32_t(ch * 32 + lane);
-        if constexpr (pass == 1) {
-            // the hits' candidates, compacted in order: contact o is candidate hits[o]
-            const unsigned m = hitbits[ch];
-            if (m & (1u << lane)) {
-                const uint32_t o = hoff[ch] + __popc(m & below);
-                if (o < uint32_t(c.contact_cap)) c.c_a[o] = g;
-            }
-        } else {
-            bool hit = false;
-            if (g < total) {
-                const uint2 q = cand2[g];  // not a local pair (k_filter)
+    const uint32_t total = uint32_t(min((long long)c.counts[kCand], c.cand_cap));
+    for (long long b0 = thread / 32 * 32 * kBatch; b0 < total; b0 += threads * kBatch) {
+        uint2 q[kBatch];
+        uint32_t keep = 0;
+#pragma unroll
+        for (int u = 0; u < kBatch; u++)
+            if (b0 + 32 * u + lane < total) q[u] = c.cand[b0 + 32 * u + lane];
+#pragma unroll
+        for (int u = 0; u < kBatch; u++) {
+            if (b0 + 32 * u + lane >= total) continue;
+            const int2 na = shape_nodes(t, q[u].x), nb = shape_nodes(t, q[u].y);
+            if (t.I > 1 && t.node_inst[na.x] != t.node_inst[nb.x]) continue;
+            const DistBounds d = dist_bounds(t, p, xf, q[u].x, q[u].y);
+            if (!(d.far_ok && d.far > d.pad_sum + reach) && !any_connected(t, na, nb)) keep |= 1u << u;
+        }
+        append_batch(keep, c.counts + kKept, c.cand_cap, [&](long long at, int u) { c.cand2[at] = q[u]; });
+    }
+}
+
+// Narrow phase over the filtered list: the pairs in contact (of the evaluated instances) are
+// appended to the contact list; more than its capacity raises kOverContacts.
+__global__ void __launch_bounds__(kBlock) k_narrow(DevTopo t, PhysParams p, const double4_32a* __restrict__ x,
+                                                   const float4* __restrict__ xf, ContactBufs c) {
+    const long long thread = (long long)blockIdx.x * blockDim.x + threadIdx.x, threads = (long long)gridDim.x * blockDim.x;
+    const int lane = threadIdx.x & 31;
+    const uint32_t total = uint32_t(min((long long)c.counts[kKept], c.cand_cap));
+    for (long long g0 = thread / 32 * 32; g0 < total; g0 += threads) {
+        bool hit = false;
+        uint2 q = make_uint2(0, 0);
+        if (g0 + lane < total) {
+            q = c.cand2[g0 + lane];  // not a local pair (k_filter)
+            if (t.I == 1 || t.active[t.node_inst[shape_nodes(t, q.x).x]]) {
                 const int cls = distance_class(t, p, xf, q.x, q.y);
                 if (cls > 0) hit = true;  // certainly within the target
                 else if (cls == 0) hit = narrow_phase(t, p, x, q.x, q.y).hit;
             }
-            const unsigned m = __ballot_sync(0xffffffffu, hit);
-            if (lane == 0) {
-                hitbits[ch] = m;
-                hcount[ch] = __popc(m);
-            }
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, hit);
+        if (!m) continue;  // warp-uniform
+        uint32_t base = 0;
+        if (lane == 0) {
+            base = atomicAdd(c.counts + kContacts, uint32_t(__popc(m)));
+            if ((long long)base + __popc(m) > c.contact_cap) atomicOr(c.flags, uint32_t(kOverContacts));
+        }
+        const long long at = (long long)__shfl_sync(0xffffffffu, base, 0) + __popc(m & ((1u << lane) - 1u));
+        if (hit && at < c.contact_cap) {
+            c.c_a[at] = q.x;
+            c.c_b[at] = q.y;
         }
     }
 }
 
-// The contacts, one hit per thread (dense: the FP64 closest points run with full warps):
-// contact o is candidate c_a[o] of the filtered list, written in candidate order.
-__global__ void __launch_bounds__(kBlock) k_contacts(DevTopo t, PhysParams p, const double4_32a* __restrict__ x,
-                                                     const uint2* __restrict__ cand2,
-                                                     const uint32_t* __restrict__ total, ContactBufs c) {
-    const long long nc = min((long long)*total, c.contact_cap);
+// Adds v to a fixed-point sum of quantum 2^e0 (kSumLimbs signed counters of 32 bits each, which
+// hold 2^31 additions): the 53-bit mantissa lands in at most three limbs, added with v's sign.
+// Bits below the quantum are dropped; false when v is not finite or beyond the top limb.
+__device__ __forceinline__ bool add_fixed(long long* __restrict__ sum, double v, int e0) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+    const int e = int(b >> 52) & 0x7ff;
+    if (e == 0) return true;       // zero (or subnormal, far below any quantum in use)
+    if (e == 0x7ff) return false;
+    unsigned long long m = (b & 0xfffffffffffffULL) | 0x10000000000000ULL;
+    int at = e - 1023 - 52 - e0;   // bit position of the mantissa's lowest bit
+    if (at < 0) {
+        m = at <= -64 ? 0 : m >> -at;
+        at = 0;
+    }
+    const int limb = at >> 5, sh = at & 31;
+    const unsigned long long lo = m << sh;
+    const unsigned parts[3] = {unsigned(lo), unsigned(lo >> 32), sh ? unsigned(m >> (64 - sh)) : 0u};
+    const bool minus = b >> 63;
+    bool ok = true;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        if (!parts[k]) continue;
+        if (limb + k >= kSumLimbs) {
+            ok = false;
+            continue;
+        }
+        const long long d = minus ? -(long long)parts[k] : (long long)parts[k];
+        atomicAdd(reinterpret_cast<unsigned long long*>(sum + limb + k), (unsigned long long)d);
+    }
+    return ok;
+}
+
+// The contacts, one per thread (dense: the FP64 closest points run with full warps): the forces
+// of the penalty (sim.cpp:163-164, addShapeGradient sim.cpp:23: capsule ends split the force
+// (1 - u, u)) onto the nodes' fixed-point sums, the contact's energy, count and penetration onto
+// the first node of its lower shape.
+__global__ void __launch_bounds__(64) k_contacts(DevTopo t, PhysParams p, const double4_32a* __restrict__ x,
+                                                 ContactBufs c) {
+    const long long nc = min((long long)c.counts[kContacts], c.contact_cap);
     for (long long o = (long long)blockIdx.x * blockDim.x + threadIdx.x; o < nc; o += (long long)gridDim.x * blockDim.x) {
-        const uint2 q = cand2[c.c_a[o]];
-        const PairHit h = narrow_phase(t, p, x, q.x, q.y);
-        c.c_a[o] = q.x;
-        c.c_b[o] = q.y;
-        c.c_s[o] = h.s;
-        c.c_t[o] = h.t;
-        c.c_n[3 * size_t(o)] = h.n.x;
-        c.c_n[3 * size_t(o) + 1] = h.n.y;
-        c.c_n[3 * size_t(o) + 2] = h.n.z;
-        c.c_pen[o] = h.pen;
-    }
-}
-
-__device__ __forceinline__ int slot_node(const DevTopo& t, uint32_t shape, int slot) {
-    if (shape < uint32_t(t.N)) return slot == 0 ? int(shape) : -1;
-    const int2 ab = t.ab[shape - uint32_t(t.N)];
-    return slot == 0 ? ab.x : ab.y;
-}
-
-// Per-node item counts; a contact list longer than its capacity flags kOverContacts.
-__global__ void __launch_bounds__(kBlock) k_node_count(DevTopo t, const uint32_t* __restrict__ total, ContactBufs c) {
-    if (blockIdx.x == 0 && threadIdx.x == 0 && (long long)*total > c.contact_cap)
-        atomicOr(c.flags, uint32_t(kOverContacts));
-    const long long nc = min((long long)*total, c.contact_cap);
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nc; i += (long long)gridDim.x * blockDim.x)
-        for (int slot = 0; slot < 4; slot++) {
-            const int node = slot_node(t, slot < 2 ? c.c_a[i] : c.c_b[i], slot & 1);
-            if (node >= 0) atomicAdd(&c.n_count[node], 1u);
-        }
-}
-
-__global__ void __launch_bounds__(kBlock) k_node_fill(DevTopo t, const uint32_t* __restrict__ total, ContactBufs c) {
-    const long long nc = min((long long)*total, c.contact_cap);
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nc; i += (long long)gridDim.x * blockDim.x)
-        for (int slot = 0; slot < 4; slot++) {
-            const int node = slot_node(t, slot < 2 ? c.c_a[i] : c.c_b[i], slot & 1);
-            if (node < 0) continue;
-            const uint32_t pos = atomicAdd(&c.n_cursor[node], 1u);
-            c.n_items[c.n_start[node] + pos] = (uint32_t(i) << 2) | uint32_t(slot);
-        }
-}
-
-// Per-node contact lists in canonical order: by the contact's (lower shape, higher shape)
-// and the slot, which no two items of one node share.  The gather sums each list in this
-// order, so forces do not depend on the order of the contact list.
-__device__ __forceinline__ unsigned long long item_key(const ContactBufs& c, uint32_t item) {
-    const uint32_t ci = item >> 2;
-    return ((unsigned long long)c.c_a[ci] << 31) | ((unsigned long long)c.c_b[ci] << 2) | (item & 3u);
-}
-
-// One warp per node with contacts: lists of up to 32 items ranked by shuffles; longer lists
-// are queued.
-__global__ void __launch_bounds__(kBlock) k_node_sort(int N, ContactBufs c) {
-    const int lane = threadIdx.x & 31;
-    const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
-    const long long groups = (N + 31) / 32;
-    // warp w takes the groups of 32 consecutive nodes w, w + warps, ...; one ballot finds the
-    // group's nodes that have contacts (most have none)
-    for (long long g = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; g < groups; g += warps) {
-        const long long i0 = g * 32;
-        const uint32_t mine = i0 + lane < N ? c.n_count[i0 + lane] : 0u;
-        unsigned todo = __ballot_sync(0xffffffffu, mine != 0);
-        while (todo) {
-            const int b = __ffs(todo) - 1;
-            todo &= todo - 1;
-            const long long i = i0 + b;
-            const uint32_t cnt = __shfl_sync(0xffffffffu, mine, b), s0 = c.n_start[i];
-            if (cnt > 32) {
-                if (lane == 0) {
-                    const uint32_t at = atomicAdd(c.n_long, 1u);
-                    c.n_long[1 + at] = uint32_t(i);
-                    c.n_cursor[i] = at;  // the fill is done with it
+        const uint32_t sa = c.c_a[o], sb = c.c_b[o];
+        const PairHit h = narrow_phase(t, p, x, sa, sb);
+        if (!h.hit) continue;
+        const double mag = p.contact_k * h.pen;
+        bool ok = true;
+#pragma unroll
+        for (int side = 0; side < 2; side++) {
+            const uint32_t shape = side ? sb : sa;
+            const bool capsule = shape >= uint32_t(t.N);
+            const int2 nd = shape_nodes(t, shape);
+            const d3 v = h.n * (side ? -mag : mag);
+            const double u = side ? h.t : h.s;
+#pragma unroll
+            for (int end = 0; end < 2; end++) {
+                if (end && !capsule) break;
+                const int node = end ? nd.y : nd.x;
+                const d3 f = !capsule ? v : end ? v * u : v * (1 - u);
+                NodeContact& r = c.n_sum[node];
+                ok &= add_fixed(r.f[0], f.x, c.force_e0);
+                ok &= add_fixed(r.f[1], f.y, c.force_e0);
+                ok &= add_fixed(r.f[2], f.z, c.force_e0);
+                if (side == 0 && end == 0) {
+                    ok &= add_fixed(r.energy, .5 * p.contact_k * h.pen * h.pen, c.energy_e0);
+                    atomicMax(&r.pen, (unsigned long long)__double_as_longlong(h.pen));  // pen > 0
+                    atomicAdd(c.n_count + node, 1ULL | (1ULL << 32));
+                } else {
+                    atomicAdd(c.n_count + node, 1ULL);
                 }
-                continue;
             }
-            uint32_t item = 0;
-            unsigned long long key = ~0ull;
-            if (lane < int(cnt)) {
-                item = c.n_items[s0 + lane];
-                key = item_key(c, item);
-            }
-            uint32_t rank = 0;
-            for (uint32_t q = 0; q < cnt; q++) rank += __shfl_sync(0xffffffffu, key, int(q)) < key;
-            if (lane < int(cnt)) c.n_sorted[s0 + rank] = item;
         }
-    }
-}
-
-constexpr int kLongCap = 2048;  // keys staged in shared memory per long list
-
-// One block per queued node (longer lists): each item's rank is the number of smaller keys.
-__global__ void __launch_bounds__(kBlock) k_node_sort_long(ContactBufs c) {
-    __shared__ unsigned long long keys[kLongCap];
-    const uint32_t nl = c.n_long[0];
-    for (uint32_t j = blockIdx.x; j < nl; j += gridDim.x) {
-        const uint32_t i = c.n_long[1 + j];
-        const uint32_t cnt = c.n_count[i], s0 = c.n_start[i];
-        const bool staged = cnt <= uint32_t(kLongCap);
-        if (staged)
-            for (uint32_t e = threadIdx.x; e < cnt; e += blockDim.x) keys[e] = item_key(c, c.n_items[s0 + e]);
-        __syncthreads();
-        for (uint32_t e = threadIdx.x; e < cnt; e += blockDim.x) {
-            const uint32_t item = c.n_items[s0 + e];
-            const unsigned long long k = staged ? keys[e] : item_key(c, item);
-            uint32_t r = 0;
-            for (uint32_t q = 0; q < cnt; q++) r += (staged ? keys[q] : item_key(c, c.n_items[s0 + q])) < k;
-            c.n_sorted[s0 + r] = item;
-        }
-        __syncthreads();
+        // not finite: the evaluation's energy must be, too (the gather reads the flag)
+        if (!ok) atomicOr(c.n_count + shape_nodes(t, sa).x, kContactNotFinite);
     }
 }
 
@@ -965,55 +829,21 @@ int contact_pair_blocks(long long shapes) {
     return int(b < 1 ? 1 : (b > 8 * 152 ? 8 * 152 : b));
 }
 
-void launch_contacts(const DevTopo& t, const PhysParams& p, const EvalBufs& e, ContactBufs& c, double pad,
-                     float skin, cudaStream_t s, cudaEvent_t pairs_begin, cudaEvent_t pairs_end) {
-    const int S = t.N + t.B;
-    const uint32_t* gate = c.flags + 1;
-    cudaMemsetAsync(c.flags, 0, 2 * sizeof(uint32_t), s);
-    cudaMemsetAsync(c.flags + 3, 0, sizeof(uint32_t), s);  // the pair pass's bin cursor
-    (k_skin_check<<<grid_for(t.N), kBlock, 0, s>>>(t, t.N, e.xf_lo, e.xf_hi, c.xref, skin, c.flags), note_launches(1));
+void launch_contacts(const DevTopo& t, const PhysParams& p, const EvalBufs& e, ContactBufs& c, float skin,
+                     cudaStream_t s, cudaEvent_t pairs_begin, cudaEvent_t pairs_end) {
+    const float grow = skin > 0.f ? skin : 0.f;
     // candidate list (only when rebuilding)
-    (k_zero_gated<<<kStreamBlocks, kBlock, 0, s>>>(c.bin_cap + 1, c.bin_count, gate), note_launches(1));
-    (k_grid_params<<<1, 32, 0, s>>>(e.cen + 9 * size_t(t.I), pad + double(skin > 0.f ? skin : 0.f), p.broad_cell,
-                                    c.bin_cap, c.grid, c.flags, c.ncand, c.nentries),
-     note_launches(1));
-    (k_shape_prep<<<grid_for(S), kBlock, 0, s>>>(t, p, e.xf_lo, e.xf_hi, c.grid, c.cell_lo, c.cell_hi, c.rec,
-                                                 skin > 0.f ? skin : 0.f, c.flags), note_launches(1));
-    (k_emit<<<grid_for(S), kBlock, 0, s>>>(S, c.grid, c.cell_lo, c.cell_hi, c.bin_slots, c.bin_count, c.bin_items,
-                                           c.nentries, c.flags), note_launches(1));
-    // occupied bins, then the candidate list
+    (k_shapes<<<grid_for((long long)t.N + t.B), kBlock, 0, s>>>(t, p, e.xf_lo, e.xf_hi, grow, c), note_launches(1));
     if (pairs_begin) cudaEventRecord(pairs_begin, s);
-    (k_bin_pairs<<<c.pair_blocks, kBlock, 0, s>>>(t, c.grid, c.bin_count, c.bin_slots, c.nentries, c.bin_items,
-                                                c.rec, c.cand_cap, c.cand, c.ncand, c.flags),
+    (k_bin_pairs<<<c.pair_blocks, kBlock, 0, s>>>(t, c.grid, c.bin_count, c.bin_slots, c.counts, c.bin_items, c.rec,
+                                                c.cand_cap, c.cand, c.flags),
      note_launches(1));
     if (pairs_end) cudaEventRecord(pairs_end, s);
-    // filtered list (only when rebuilding)
-    const long long chunks = c.cand_cap / 32;
-    const float reach = skin > 0.f ? 2.0001f * skin : 0.f;  // >= 2 skin
-    (k_filter<0><<<kStreamBlocks, kBlock, 0, s>>>(t, p, e.xf_lo, c.cand_cap, c.cand, c.ncand, reach, c.fbits,
-                                                c.fcount, c.foff, c.cand2, gate), note_launches(1));
-    exclusive_scan_u32(c.fcount, c.foff, chunks, c.scan_tmp, s, gate, c.ncand, 31, 5);
-    (k_filter<1><<<kStreamBlocks, kBlock, 0, s>>>(t, p, e.xf_lo, c.cand_cap, c.cand, c.ncand, reach, c.fbits,
-                                                c.fcount, c.foff, c.cand2, gate), note_launches(1));
-    (k_skin_commit<<<grid_for(t.N), kBlock, 0, s>>>(t.N, e.xf_lo, c.xref, c.flags), note_launches(1));
-    // narrow phase over the filtered list: hit bits and counts per chunk, scan, contacts
-    const uint32_t* nkept = c.foff + chunks;
-    (k_narrow<0><<<kStreamBlocks, kBlock, 0, s>>>(t, p, e.x, e.xf_lo, c.cand2, nkept, c.hitbits, c.hcount, c.hoff, c),
+    (k_filter<<<kStreamBlocks, kBlock, 0, s>>>(t, p, e.xf_lo, skin > 0.f ? 2.0001f * skin : 0.f, c),  // >= 2 skin
      note_launches(1));
-    exclusive_scan_u32(c.hcount, c.hoff, chunks, c.scan_tmp, s, nullptr, nkept, 31, 5);
-    (k_narrow<1><<<kStreamBlocks, kBlock, 0, s>>>(t, p, e.x, e.xf_lo, c.cand2, nkept, c.hitbits, c.hcount, c.hoff, c),
-     note_launches(1));
-    // one warp per block: the few thousand contacts spread over every SM's FP64 pipe
-    (k_contacts<<<8 * kStreamBlocks, 32, 0, s>>>(t, p, e.x, c.cand2, c.hoff + chunks, c), note_launches(1));
-    const uint32_t* total = c.hoff + chunks;
-    cudaMemsetAsync(c.n_count, 0, size_t(t.N + 1) * sizeof(uint32_t), s);
-    cudaMemsetAsync(c.n_cursor, 0, size_t(t.N) * sizeof(uint32_t), s);
-    (k_node_count<<<kStreamBlocks, kBlock, 0, s>>>(t, total, c), note_launches(1));
-    exclusive_scan_u32(c.n_count, c.n_start, t.N, c.scan_tmp, s);
-    (k_node_fill<<<kStreamBlocks, kBlock, 0, s>>>(t, total, c), note_launches(1));
-    cudaMemsetAsync(c.n_long, 0, sizeof(uint32_t), s);
-    (k_node_sort<<<kStreamBlocks, kBlock, 0, s>>>(t.N, c), note_launches(1));
-    (k_node_sort_long<<<kStreamBlocks, kBlock, 0, s>>>(c), note_launches(1));
+    // every evaluation: the pairs in contact, then their forces
+    (k_narrow<<<kStreamBlocks, kBlock, 0, s>>>(t, p, e.x, e.xf_lo, c), note_launches(1));
+    (k_contacts<<<2 * kStreamBlocks, 64, 0, s>>>(t, p, e.x, c), note_launches(1));
 }
 
 }  // namespace mcg

@@ -313,11 +313,10 @@ struct mcg_ctx {
         contact_mem.release();
         const long long S = (long long)N + B;
         ContactBufs c{};
-        c.cell_lo = contact_mem.get<int4>(size_t(S));
-        c.cell_hi = contact_mem.get<int4>(size_t(S));
         c.rec = contact_mem.get<uint4>(size_t(S));
         c.grid = contact_mem.get<int>(16);
         c.flags = contact_mem.get<uint32_t>(5);
+        c.counts = contact_mem.get<uint32_t>(kContactCounts);
         c.xref = contact_mem.get<float4>(size_t(std::max(N, 1)));
         int slots = 8;
         while (slots < bin_slots && slots < (1 << 20)) slots <<= 1;
@@ -325,59 +324,56 @@ struct mcg_ctx {
         c.bin_cap = bin_cap;
         c.bin_count = contact_mem.get<uint32_t>(size_t(bin_cap + 1));
         c.bin_items = contact_mem.get<uint32_t>(size_t(bin_cap) * size_t(slots));
-        c.nentries = contact_mem.get<uint32_t>(3);
         c.pair_blocks = pair_blocks_for(S);
         c.cand_cap = std::max<long long>(1024, (cand_cap + 31) / 32 * 32);
         c.cand = contact_mem.get<uint2>(size_t(c.cand_cap));
-        c.ncand = contact_mem.get<uint32_t>(1);
-        const long long chunks = c.cand_cap / 32;
         c.cand2 = contact_mem.get<uint2>(size_t(c.cand_cap));
-        c.fbits = contact_mem.get<uint32_t>(size_t(chunks));
-        c.fcount = contact_mem.get<uint32_t>(size_t(chunks + 1));
-        c.foff = contact_mem.get<uint32_t>(size_t(chunks + 1));
-        c.hitbits = contact_mem.get<uint32_t>(size_t(chunks));
-        c.hcount = contact_mem.get<uint32_t>(size_t(chunks + 1));
-        c.hoff = contact_mem.get<uint32_t>(size_t(chunks + 1));
         c.contact_cap = contact_cap;
         c.c_a = contact_mem.get<uint32_t>(size_t(contact_cap));
         c.c_b = contact_mem.get<uint32_t>(size_t(contact_cap));
-        c.c_s = contact_mem.get<double>(size_t(contact_cap));
-        c.c_t = contact_mem.get<double>(size_t(contact_cap));
-        c.c_n = contact_mem.get<double>(size_t(3 * contact_cap));
-        c.c_pen = contact_mem.get<double>(size_t(contact_cap));
-        c.n_count = contact_mem.get<uint32_t>(size_t(N + 1));
-        c.n_start = contact_mem.get<uint32_t>(size_t(N + 1));
-        c.n_cursor = contact_mem.get<uint32_t>(size_t(N));
-        c.n_items = contact_mem.get<uint32_t>(size_t(4 * contact_cap));
-        c.n_sorted = contact_mem.get<uint32_t>(size_t(4 * contact_cap));
-        c.n_long = contact_mem.get<uint32_t>(size_t(N + 1));
-        c.long_sum = contact_mem.get<double>(6 * size_t(std::max(N, 1)));
-        c.scan_tmp_bytes = scan_tmp_bytes(std::max({(long long)N + 1, chunks + 1}));
-        c.scan_tmp = contact_mem.get<unsigned char>(c.scan_tmp_bytes);
+        c.n_count = contact_mem.get<unsigned long long>(size_t(N));
+        c.n_sum = contact_mem.get<NodeContact>(size_t(N));
+        set_sum_quanta(c);
         ck(cudaMemsetAsync(c.flags, 0, 5 * sizeof(uint32_t), stream), "memset");
-        ck(cudaMemsetAsync(c.ncand, 0, sizeof(uint32_t), stream), "memset");
-        ck(cudaMemsetAsync(c.nentries, 0, 3 * sizeof(uint32_t), stream), "memset");
+        ck(cudaMemsetAsync(c.counts, 0, kContactCounts * sizeof(uint32_t), stream), "memset");
+        ck(cudaMemsetAsync(c.bin_count, 0, size_t(bin_cap + 1) * sizeof(uint32_t), stream), "memset");
+        ck(cudaMemsetAsync(c.n_count, 0, size_t(N) * sizeof(unsigned long long), stream), "memset");
+        ck(cudaMemsetAsync(c.n_sum, 0, size_t(N) * sizeof(NodeContact), stream), "memset");
         ck(cudaMemsetAsync(c.flags + 2, 1, 1, stream), "memset");  // the first evaluation builds the list
         cb = c;
     }
-    long long contact_chunks() const { return cb.cand_cap / 32; }
+    // Quanta of the nodes' contact sums, from the configuration alone (so that a lattice sums alike
+    // alone and in a batch): stiffness times a reference length no penetration exceeds by much
+    // (the joint radius with the margin, or a cell), times that length again for the energy.
+    void set_sum_quanta(ContactBufs& c) const {
+        double T = std::max(std::abs(jr) + std::abs(cfg.contact_margin), std::abs(cfg.cell_size));
+        if (!(T > 0) || !std::isfinite(T)) T = 1.0;
+        auto exponent = [](double v) {
+            return v > 0 && std::isfinite(v) ? std::max(-900, std::min(900, std::ilogb(v))) - kSumQuantumBits : -kSumQuantumBits;
+        };
+        c.force_e0 = exponent(std::abs(cfg.contact_stiffness) * T);
+        c.energy_e0 = exponent(std::abs(cfg.contact_stiffness) * T * T);
+    }
+    // What the state and center kernels need to decide on a rebuild of cb's candidate list.
+    BuildArgs build_args(const ContactBufs& c, float skin) const {
+        if (!phys.self_contact) return BuildArgs{};
+        return BuildArgs{c.xref, c.flags, c.counts, c.grid, rmax + cfg.contact_margin + double(skin > 0.f ? skin : 0.f),
+                         broad_cell, c.bin_cap, skin};
+    }
 
     // Grows whatever the last evaluation overflowed; false when nothing did.
     bool grow_contacts(int flags) {
         if (!(flags & (kOverEntries | kOverContacts | kOverBins | kOverSpan | kOverCandidates))) return false;
-        uint32_t need[3] = {0, 0, 0};
+        uint32_t need[kContactCounts] = {};
         int grid[16];
-        ck(cudaMemcpyAsync(&need[0], cb.nentries + 1, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream), "copy");
-        ck(cudaMemcpyAsync(&need[1], cb.hoff + contact_chunks(), sizeof(uint32_t), cudaMemcpyDeviceToHost, stream),
-           "copy");
-        ck(cudaMemcpyAsync(&need[2], cb.ncand, sizeof(uint32_t), cudaMemcpyDeviceToHost, stream), "copy");
+        ck(cudaMemcpyAsync(need, cb.counts, sizeof(need), cudaMemcpyDeviceToHost, stream), "copy");
         ck(cudaMemcpyAsync(grid, cb.grid, sizeof(grid), cudaMemcpyDeviceToHost, stream), "copy");
         sync();
         long long slots = cb.bin_slots, ccap = cb.contact_cap, bcap = cb.bin_cap, kcap = cb.cand_cap;
-        if (flags & kOverCandidates) kcap = std::max(kcap, (long long)need[2] + need[2] / 4 + 1024);
+        if (flags & kOverCandidates) kcap = std::max(kcap, (long long)need[kCand] + need[kCand] / 4 + 1024);
         if (flags & kOverSpan) broad_cell *= 2;
-        if (flags & kOverEntries) slots = std::max(slots, (long long)need[0] + need[0] / 4);
-        if (flags & kOverContacts) ccap = std::max(ccap, (long long)need[1] + need[1] / 4 + 1024);
+        if (flags & kOverEntries) slots = std::max(slots, (long long)need[kLargestBin] + need[kLargestBin] / 4);
+        if (flags & kOverContacts) ccap = std::max(ccap, (long long)need[kContacts] + need[kContacts] / 4 + 1024);
         if (flags & kOverBins) {
             const long long want = (long long)grid[9] + grid[9] / 4 + 1024;
             if (want <= (1LL << 28)) bcap = std::max(bcap, want);
@@ -487,16 +483,17 @@ struct mcg_ctx {
         p.broad_cell = broad_cell;
         p.inv_cell_f = float(1.0 / broad_cell);
         mark(0);
-        if (mixed) launch_state_mixed(topo, p, dz, d_baseX, mn, ev, stream);
-        else launch_state(topo, p, dz, d_baseX, d_baseR, ev, stream);
+        const BuildArgs ba = build_args(cb, contact_skin);
+        if (mixed) launch_state_mixed(topo, p, dz, d_baseX, mn, ba, ev, stream);
+        else launch_state(topo, p, dz, d_baseX, d_baseR, ba, ev, stream);
         mark(1);
         if (mixed) launch_beams_mixed(topo, mat, mb, mn, trials, ev, stream, beam_variant);
         else launch_beams(topo, mat, d_plastic, trials, ev, stream, beam_variant);
         mark(2);
         const ContactBufs* cptr = nullptr;
         if (p.self_contact) {
-            launch_contacts(topo, p, ev, cb, rmax + cfg.contact_margin, contact_skin, stream,
-                            timing ? ev_t[3] : nullptr, timing ? ev_t[4] : nullptr);
+            launch_contacts(topo, p, ev, cb, contact_skin, stream, timing ? ev_t[3] : nullptr,
+                            timing ? ev_t[4] : nullptr);
             cptr = &cb;
         } else {
             mark(3);
@@ -529,27 +526,20 @@ struct mcg_ctx {
             read_outs();
         }
         if (hp.outs[0].overflow) throw Fail(MCG_ERR_CAPACITY, "contact buffers could not be sized");
-        if (cfg.self_contact) last_contacts = hp.u32[0];
+        last_contacts = hp.outs[0].pairs;
         contacts_stale = false;
         return hp.outs;
     }
-    long long read_contact_count() {
-        d2h(hp.u32, cb.hoff + contact_chunks(), 1, stream);
-        sync();
-        return hp.u32[0];
-    }
     void read_outs() {
         d2h(hp.outs, ev.out, size_t(I), stream);
-        if (cfg.self_contact) d2h(hp.u32, cb.hoff + contact_chunks(), 1, stream);
-        d2h(hp.u32 + 6, ev.err, 1, stream);
         sync();
         check_kernel_error();
     }
-    // A kernel's bounded wait that gave up (ev.err, read into hp.u32[6] with the totals)
+    // A kernel's bounded wait that gave up (ev.err, copied into the totals)
     // leaves its evaluation invalid: an error, after which the context stays usable.
     void check_kernel_error() {
-        if (!hp.u32[6]) return;
-        hp.u32[6] = 0;
+        if (!hp.outs[0].kernel_error) return;
+        hp.outs[0].kernel_error = 0;
         ck(cudaMemsetAsync(ev.err, 0, sizeof(unsigned), stream), "memset");
         sync();
         throw Fail(MCG_ERR_CUDA, "a staging wait of the beam kernel gave up; the evaluation is invalid");
@@ -558,7 +548,7 @@ struct mcg_ctx {
     EvalOut read_out() {
         read_outs();
         if (hp.outs[0].overflow) eval_read(last_z, last_trials, last_grad);
-        else if (cfg.self_contact) last_contacts = hp.u32[0];
+        else last_contacts = hp.outs[0].pairs;
         contacts_stale = false;
         return hp.outs[0];
     }
@@ -810,8 +800,6 @@ struct mcg_ctx {
             d2h(hp.mins, d_mins, size_t(I), stream);
             d2h(hp.mz, d_mz, 1, stream);
             d2h(hp.outs, ev.out, size_t(I), stream);
-            if (cfg.self_contact) d2h(hp.u32, cb.hoff + contact_chunks(), 1, stream);
-            d2h(hp.u32 + 6, ev.err, 1, stream);
             sync();
             check_launch();
             check_kernel_error();
@@ -835,7 +823,7 @@ struct mcg_ctx {
                 throw Fail(MCG_ERR_CUDA, "the device-resident round loop ran no round");
             break;
         }
-        if (cfg.self_contact) last_contacts = hp.u32[0];
+        last_contacts = hp.outs[0].pairs;
         contacts_stale = false;
         return true;
     }
@@ -871,7 +859,7 @@ struct mcg_ctx {
         PhysParams p = phys;
         DevTopo all = topo;  // the committed instances' states (others are recomputed before use)
         all.active = d_all;
-        launch_state(all, p, d_zfinal, d_baseX, d_baseR, ev, stream);
+        launch_state(all, p, d_zfinal, d_baseX, d_baseR, BuildArgs{}, ev, stream);
         if (mixed) {
             launch_commit(topo, d_mask, ev, d_baseX, d_baseR, nullptr, stream);
             launch_plastic_mixed(topo, d_mask, nullptr, ev.trial_nextf, mb, stream);
@@ -1465,6 +1453,7 @@ void upload_instances(mcg_ctx* c, const std::vector<InstIn>& ins) {
     ck(cudaMemsetAsync(e.err, 0, sizeof(unsigned), s), "memset");
     e.part_node = V.get<double>(kNodeParts * size_t(T.n_eblk));
     e.part_fin = V.get<double>(size_t(kFinPartDoubles) * size_t(I));
+    ck(cudaMemsetAsync(e.part_fin, 0, size_t(kFinPartDoubles) * size_t(I) * sizeof(double), s), "memset");
     e.cen = V.get<double>(9 * size_t(I + 1));
     e.cforce = V.get<double>(2 * size_t(I));
     e.tops = V.get<double>(size_t(I));
@@ -1831,8 +1820,9 @@ int mcg_read_result(mcg_ctx* c, double* energy, double* grad, mcg_diag* diag) {
 namespace mcg {
 
 // One evaluation whose self-contact scratch is `fixed` (caller-provided, never grown) and
-// which allocates nothing: the building block of mcg_objective_noalloc (noalloc.cu).
-int objective_with_fixed_contacts(mcg_ctx* c, ContactBufs& fixed, const double* z, double top, double* energy,
+// which allocates nothing: the building block of mcg_objective_noalloc (noalloc.cu).  The first
+// zero_bytes of the scratch, from fixed.flags on, must be zero between evaluations.
+int objective_with_fixed_contacts(mcg_ctx* c, ContactBufs& fixed, size_t zero_bytes, const double* z, double top, double* energy,
                                   double* grad, mcg_diag* diag) {
     return guarded(c, [&] {
         need_single(c);
@@ -1846,13 +1836,19 @@ int objective_with_fixed_contacts(mcg_ctx* c, ContactBufs& fixed, const double* 
         PhysParams p = c->phys;
         p.broad_cell = c->broad_cell;
         p.inv_cell_f = float(1.0 / c->broad_cell);
-        if (c->mixed) launch_state_mixed(c->topo, p, c->d_zin, c->d_baseX, c->mn, c->ev, s);
-        else launch_state(c->topo, p, c->d_zin, c->d_baseX, c->d_baseR, c->ev, s);
+        if (p.self_contact) {
+            // the scratch holds whatever its last user left: the state between evaluations
+            c->set_sum_quanta(fixed);
+            ck(cudaMemsetAsync(fixed.flags, 0, zero_bytes, s), "memset");
+        }
+        const BuildArgs ba = c->build_args(fixed, 0.f);  // always rebuilds
+        if (c->mixed) launch_state_mixed(c->topo, p, c->d_zin, c->d_baseX, c->mn, ba, c->ev, s);
+        else launch_state(c->topo, p, c->d_zin, c->d_baseX, c->d_baseR, ba, c->ev, s);
         if (c->mixed) launch_beams_mixed(c->topo, c->mat, c->mb, c->mn, false, c->ev, s, c->beam_variant);
         else launch_beams(c->topo, c->mat, c->d_plastic, false, c->ev, s, c->beam_variant);
         const ContactBufs* cptr = nullptr;
         if (p.self_contact) {
-            launch_contacts(c->topo, p, c->ev, fixed, c->rmax + c->cfg.contact_margin, 0.f, s);  // always rebuilds
+            launch_contacts(c->topo, p, c->ev, fixed, 0.f, s);
             cptr = &fixed;
         }
         if (c->mixed) launch_gather_mixed(c->topo, p, cptr, c->d_grad, c->ev, s, c->gather_variant);
@@ -1984,13 +1980,10 @@ int mcg_contact_stats(mcg_ctx* c, int64_t* out5) {
         if (!out5) throw Fail(MCG_ERR_INVALID, "null output");
         if (c->contacts_stale)
             throw Fail(MCG_ERR_STATE, "the last evaluation was mcg_objective_noalloc's, whose contact statistics are not kept");
-        d2h(c->hp.u32, c->cb.nentries, 1, c->stream);
-        d2h(c->hp.u32 + 1, c->cb.nentries + 2, 1, c->stream);
-        d2h(c->hp.u32 + 2, c->cb.ncand, 1, c->stream);
-        d2h(c->hp.u32 + 3, c->cb.foff + c->contact_chunks(), 1, c->stream);
-        d2h(c->hp.u32 + 4, c->cb.hoff + c->contact_chunks(), 1, c->stream);
+        d2h(c->hp.u32, c->cb.counts, kContactCounts, c->stream);
         c->sync();
-        for (int k = 0; k < 5; k++) out5[k] = c->hp.u32[k];
+        const int order[5] = {kEntries, kOccupied, kCand, kKept, kContacts};
+        for (int k = 0; k < 5; k++) out5[k] = c->hp.u32[order[k]];
     });
 }
 

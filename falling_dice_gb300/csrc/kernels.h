@@ -101,7 +101,8 @@ struct EvalOut {
     int contacts, nonfinite;
     double beam_energy, node_energy, center_energy, contact_energy, platen_energy;
     int overflow;                    // ContactFlag bits that invalidate this evaluation
-    int pad_;
+    unsigned kernel_error;           // a kernel's bounded wait gave up (EvalBufs::err)
+    unsigned pairs, pad_;            // self-contacts of all instances (ContactCount kContacts)
     double rms, gmax;                // residual over free DOFs: sqrt(mean g^2), max |g| (sim.cpp:44-45)
 };
 
@@ -116,66 +117,81 @@ enum ContactFlag : uint32_t {
     kOverCandidates = 32 // more narrow-phase candidates than cand_cap
 };
 
+// Counters of the contact pipeline (ContactBufs::counts).
+enum ContactCount : int {
+    kCand,        // candidates of the last build (may exceed cand_cap)
+    kKept,        // candidates kept by its filter
+    kEntries,     // its cell entries
+    kLargestBin,  // its largest bin count above bin_slots (0 when every bin fitted)
+    kOccupied,    // its bins holding two or more entries
+    kContacts,    // contacts of the last evaluation (may exceed contact_cap)
+    kContactCounts
+};
+
+// Contact forces and energy of one node, summed as integers so that the sums are exact and do
+// not depend on their order: a value is a signed multiple of a quantum (2^force_e0, 2^energy_e0),
+// its bits spread over limbs of 32 bits with room for 2^31 additions each.  The gather reads the
+// record of a node whose n_count is not zero and clears both.
+constexpr int kSumLimbs = 4;
+constexpr int kSumQuantumBits = 90;  // the quantum lies 2^-90 below stiffness times the reference length
+struct NodeContact {
+    long long f[3][kSumLimbs];
+    long long energy[kSumLimbs];  // of the contacts whose lower shape's first node this is
+    unsigned long long pen;       // their largest penetration (bits of a non-negative double)
+    unsigned long long pad_;
+};
+// n_count: force items in the low 31 bits, contacts counted at this node from bit 32 on; this
+// bit: a contact's force or energy was not finite.
+constexpr unsigned long long kContactNotFinite = 1ULL << 31;
+
 struct ContactBufs {
     // per shape (S = N + B)
-    int4* cell_lo;          // [S] first cell (i, j, k) relative to the grid origin
-    int4* cell_hi;          // [S] last cell
     uint4* rec;             // [S] pair-test record: quantized AABB (3 words), packed first cell
     int* grid;              // [16]: origin i,j,k; dims i,j,k; mode; valid; bins; bins needed;
                             //       box quantization scale x,y,z and origin x,y,z (float bits)
     uint32_t* flags;        // [5]: [0] ContactFlag bits of this evaluation, [1] candidate list
                             //      rebuilt by this evaluation, [2] rebuild forced (by the host,
                             //      or by a build that overflowed), [3] the pair pass's
-                            //      occupied-bin cursor, [4] builds since allocation
+                            //      occupied-bin cursor, [4] builds since allocation.  [0] and
+                            //      [1] are zero between evaluations (cleared by the finalize)
+    uint32_t* counts;       // [kContactCounts]
     float4* xref;           // [N] node positions (FP32, rounded down) when the list was built
     // bins of fixed capacity: the shapes of bin b at bin_items[b * bin_slots ...]
     long long bin_cap;
     int bin_slots;          // entries a bin holds, a power of two
-    uint32_t* bin_count;    // [bin_cap+1] entries counted per bin (may exceed bin_slots)
+    uint32_t* bin_count;    // [bin_cap+1] entries counted per bin (may exceed bin_slots); zero
+                            //             between builds
     uint32_t* bin_items;    // [bin_cap * bin_slots]
-    uint32_t* nentries;     // [3]: [0] cell entries of the last build, [1] the largest bin count
-                            //      above bin_slots (0 when every bin fitted), [2] bins holding
-                            //      two or more entries
     // narrow-phase candidates: one flat list, appended by the pair grid's warps in chunks
     int pair_blocks;        // blocks of the pair grid (8 warps each)
     long long cand_cap;     // candidate slots, a multiple of 32
     uint2* cand;            // [cand_cap] (lower shape, higher shape)
-    uint32_t* ncand;        // [1] candidates found by the last build (may exceed cand_cap)
-    // filtered candidates (the ones that can reach contact before the next build), in order
-    uint2* cand2;           // [cand_cap]
-    uint32_t* fbits;        // [chunks] keep bit per candidate (chunks = cand_cap / 32)
-    uint32_t* fcount;       // [chunks + 1] kept per chunk
-    uint32_t* foff;         // [chunks + 1] scan of fcount; foff[chunks] = filtered list length
-    // narrow phase, per chunk of 32 consecutive filtered candidates
-    uint32_t* hitbits;      // [chunks] contact bit per candidate
-    uint32_t* hcount;       // [chunks + 1] contacts per chunk
-    uint32_t* hoff;         // [chunks + 1] scan of hcount; hoff[chunks] = contact count
+    uint2* cand2;           // [cand_cap] the ones that can reach contact before the next build
     long long contact_cap;
     uint32_t* c_a;          // lower shape index
     uint32_t* c_b;          // higher shape index
-    double* c_s;            // closest-point parameters on a and b
-    double* c_t;
-    double* c_n;            // [3 * cap] unit normal from a to b
-    double* c_pen;          // penetration
-    // per-node contact force lists (CSR built per evaluation)
-    uint32_t* n_count;      // [N+1]
-    uint32_t* n_start;      // [N+1]
-    uint32_t* n_cursor;     // [N] fill cursor; then, for a node in n_long, its place there
-    uint32_t* n_items;      // [4 * contact_cap]  (contact << 2 | slot), in arrival order
-    uint32_t* n_sorted;     // [4 * contact_cap]  the same per node, by (lower shape, higher shape, slot)
-    uint32_t* n_long;       // [N + 1] count, then the nodes whose lists exceed one warp
-    // [6 * N] or null: per node of n_long (by its place there), the sums of its list --
-    // force (3), self-contact energy, contacts, largest penetration -- taken by the gather
-    // instead of walking the list (null: the gather walks every list)
-    double* long_sum;
-    void* scan_tmp;
-    size_t scan_tmp_bytes;
+    unsigned long long* n_count;  // [N] zero between evaluations
+    NodeContact* n_sum;           // [N] zero between evaluations
+    int force_e0, energy_e0;      // exponents of the sums' quanta
+};
+
+// The candidate-list decision of an evaluation, made by its state and center kernels: rebuild
+// when some node has moved farther than the skin since the last build, or always with no skin,
+// or when forced (flags[2]); then the grid of the build.
+struct BuildArgs {
+    const float4* xref;
+    uint32_t* flags;   // null: no self-contact
+    uint32_t* counts;
+    int* grid;
+    double pad, cell;  // shape boxes reach at most pad beyond the nodes; grid cell
+    long long bin_cap;
+    float skin;        // <= 0: rebuild at every evaluation
 };
 
 // per node block: gravity E, platen E, reaction, max penetration, contacts, self-contact E,
 // sum of squared free gradient entries, max |free gradient entry|
 constexpr int kNodeParts = 8;
-constexpr int kFinPartDoubles = 32 * 11;  // per instance: 32 first-stage blocks x 11 totals
+constexpr int kFinPartDoubles = 32 * 11 + 1;  // per instance: 32 first-stage blocks x 11 totals, a counter
 
 struct EvalBufs {
     double4_32a* x;             // [N]
@@ -233,7 +249,7 @@ inline void note_launches(int k) { g_launch_count += k; }
 
 // ---- launchers (objective.cu) ----------------------------------------------------------
 void launch_state(const DevTopo& t, const PhysParams& p, const double* z, const double* base_x,
-                  const double* base_r, EvalBufs& e, cudaStream_t s);
+                  const double* base_r, const BuildArgs& b, EvalBufs& e, cudaStream_t s);
 // Occupancy variants of the beam kernels and the gather (CTAs per SM the register allocation
 // allows; the arithmetic is the same in every variant).  Variant 0 is the default.
 enum class ShapeKernel { kBeams, kBeamsMixed, kGather };
@@ -254,13 +270,13 @@ void launch_finalize(const DevTopo& t, const PhysParams& p, const ContactBufs* c
 // instances with mask[i] != 0 (mask == nullptr: all)
 void launch_commit(const DevTopo& t, const uint8_t* mask, const EvalBufs& e, double* base_x, double* base_r,
                    double* plastic, cudaStream_t s);
-void launch_center(const DevTopo& t, const PhysParams& p, EvalBufs& e, cudaStream_t s);
+void launch_center(const DevTopo& t, const PhysParams& p, const BuildArgs& b, EvalBufs& e, cudaStream_t s);
 void launch_gather_mixed(const DevTopo& t, const PhysParams& p, const ContactBufs* c, double* grad, EvalBufs& e,
                          cudaStream_t s, int variant = 0);
 
 // ---- mixed-precision form (objective_mixed.cu) ------------------------------------------
 void launch_state_mixed(const DevTopo& t, const PhysParams& p, const double* z, const double* base_x,
-                        const MixedNodes& mn, EvalBufs& e, cudaStream_t s);
+                        const MixedNodes& mn, const BuildArgs& b, EvalBufs& e, cudaStream_t s);
 void launch_beams_mixed(const DevTopo& t, const Material& m, const MixedBeams& mb, const MixedNodes& mn, int trials,
                         EvalBufs& e, cudaStream_t s, int variant = 0);
 void launch_rebase_mixed(const DevTopo& t, const double* base_x, const double* base_r, MixedBeams& mb,
@@ -281,22 +297,11 @@ void launch_plastic_stats(const DevTopo& t, const double* plastic, double* part,
 // ---- contact pipeline (contact.cu) ------------------------------------------------------
 // Blocks of the pair / narrow-phase grid for a model of `shapes` shapes (8 warps each).
 int contact_pair_blocks(long long shapes);
-// The whole broad/narrow phase: grid, entries, bins, pairs, contact list, node lists.
-// The candidate list is rebuilt only when a node has moved more than skin (m, per axis)
-// since the last build, or the host forced it (flags[2]); skin <= 0 rebuilds every time.
+// The whole broad/narrow phase after the state and center kernels: bins, pairs and filtered
+// candidates (only when the list is rebuilt), contacts and their forces.
 // pairs_begin / pairs_end (may be null) are recorded around the pair enumeration.
-void launch_contacts(const DevTopo& t, const PhysParams& p, const EvalBufs& e, ContactBufs& c, double pad,
-                     float skin, cudaStream_t s, cudaEvent_t pairs_begin = nullptr, cudaEvent_t pairs_end = nullptr);
-
-// ---- scan (sort.cu) -----------------------------------------------------------------------
-size_t scan_tmp_bytes(long long n);
-// Exclusive scan of n uint32 values; out[n] receives the total.
-// Exclusive scan of n counts into out[0..n] (out[n] = total).  With a gate, every kernel
-// returns at once when *gate is 0 (the output keeps its previous contents).  With dn, only
-// the first min(n, (*dn + add) >> shift) counts are scanned (a count known on the device;
-// the total also goes to out[n]).
-void exclusive_scan_u32(const uint32_t* in, uint32_t* out, long long n, void* tmp, cudaStream_t s,
-                        const uint32_t* gate = nullptr, const uint32_t* dn = nullptr, int add = 0, int shift = 0);
+void launch_contacts(const DevTopo& t, const PhysParams& p, const EvalBufs& e, ContactBufs& c, float skin,
+                     cudaStream_t s, cudaEvent_t pairs_begin = nullptr, cudaEvent_t pairs_end = nullptr);
 
 // ---- L-BFGS vector kernels (lbfgs.cu), all instances of a context per launch --------------
 // Operations an instance takes part in during one solver step (SolveCtl::flags).

@@ -25,7 +25,7 @@
 // and keeps it in the context (a context created after a cudaDeviceReset looks it up again).
 //
 // All calls on a device share the one array, which keeps the previous call's contents;
-// every buffer that must start at zero is cleared by the evaluation itself.  Two calls whose
+// every buffer that must start at zero is cleared before the evaluation.  Two calls whose
 // work overlaps on the GPU (two contexts on two host threads, or two streams) race on the
 // array: callers must order them.
 #include <cuda_runtime.h>
@@ -36,7 +36,7 @@
 
 namespace mcg {
 
-int objective_with_fixed_contacts(mcg_ctx* c, ContactBufs& fixed, const double* z, double top, double* energy,
+int objective_with_fixed_contacts(mcg_ctx* c, ContactBufs& fixed, size_t zero_bytes, const double* z, double top, double* energy,
                                   double* grad, mcg_diag* diag);
 int ctx_counts(const mcg_ctx* c, int* n_nodes, int* n_beams, int* device);
 void** ctx_noalloc_scratch(mcg_ctx* c);
@@ -71,8 +71,9 @@ cudaError_t scratch_address(mcg_ctx* ctx, unsigned char** out) {
     return cudaSuccess;
 }
 
-// Carves the contact buffers out of the array; false if they do not fit.
-bool carve(unsigned char* base, long long N, long long S, ContactBufs& c) {
+// Carves the contact buffers out of the array, first those that must be zero between evaluations
+// (zero_bytes); false if they do not fit.
+bool carve(unsigned char* base, long long N, long long S, ContactBufs& c, size_t& zero_bytes) {
     size_t off = 0;
     auto take = [&](size_t bytes) {
         unsigned char* p = base + off;
@@ -80,47 +81,25 @@ bool carve(unsigned char* base, long long N, long long S, ContactBufs& c) {
         return p;
     };
     c = ContactBufs{};
-    c.cell_lo = reinterpret_cast<int4*>(take(size_t(S) * sizeof(int4)));
-    c.cell_hi = reinterpret_cast<int4*>(take(size_t(S) * sizeof(int4)));
-    c.rec = reinterpret_cast<uint4*>(take(size_t(S) * sizeof(uint4)));
-    c.grid = reinterpret_cast<int*>(take(16 * sizeof(int)));
-    c.flags = reinterpret_cast<uint32_t*>(take(5 * 4));
-    c.xref = reinterpret_cast<float4*>(take(size_t(N > 0 ? N : 1) * sizeof(float4)));
     c.bin_cap = kNoAllocBins;
     c.bin_slots = kNoAllocBinSlots;
+    c.flags = reinterpret_cast<uint32_t*>(take(5 * 4));
+    c.counts = reinterpret_cast<uint32_t*>(take(kContactCounts * 4));
     c.bin_count = reinterpret_cast<uint32_t*>(take(size_t(kNoAllocBins + 1) * 4));
+    c.n_count = reinterpret_cast<unsigned long long*>(take(size_t(N) * 8));
+    c.n_sum = reinterpret_cast<NodeContact*>(take(size_t(N) * sizeof(NodeContact)));
+    zero_bytes = off;
+    c.rec = reinterpret_cast<uint4*>(take(size_t(S) * sizeof(uint4)));
+    c.grid = reinterpret_cast<int*>(take(16 * sizeof(int)));
+    c.xref = reinterpret_cast<float4*>(take(size_t(N > 0 ? N : 1) * sizeof(float4)));
     c.bin_items = reinterpret_cast<uint32_t*>(take(size_t(kNoAllocBins) * kNoAllocBinSlots * 4));
-    c.nentries = reinterpret_cast<uint32_t*>(take(3 * 4));
     c.pair_blocks = contact_pair_blocks(S);
     c.cand_cap = kNoAllocCandidates;
     c.cand = reinterpret_cast<uint2*>(take(size_t(kNoAllocCandidates) * sizeof(uint2)));
-    c.ncand = reinterpret_cast<uint32_t*>(take(4));
-    const long long chunks = kNoAllocCandidates / 32;
     c.cand2 = reinterpret_cast<uint2*>(take(size_t(kNoAllocCandidates) * sizeof(uint2)));
-    c.fbits = reinterpret_cast<uint32_t*>(take(size_t(chunks) * 4));
-    c.fcount = reinterpret_cast<uint32_t*>(take(size_t(chunks + 1) * 4));
-    c.foff = reinterpret_cast<uint32_t*>(take(size_t(chunks + 1) * 4));
-    c.hitbits = reinterpret_cast<uint32_t*>(take(size_t(chunks) * 4));
-    c.hcount = reinterpret_cast<uint32_t*>(take(size_t(chunks + 1) * 4));
-    c.hoff = reinterpret_cast<uint32_t*>(take(size_t(chunks + 1) * 4));
     c.contact_cap = kNoAllocContacts;
     c.c_a = reinterpret_cast<uint32_t*>(take(size_t(kNoAllocContacts) * 4));
     c.c_b = reinterpret_cast<uint32_t*>(take(size_t(kNoAllocContacts) * 4));
-    c.c_s = reinterpret_cast<double*>(take(size_t(kNoAllocContacts) * 8));
-    c.c_t = reinterpret_cast<double*>(take(size_t(kNoAllocContacts) * 8));
-    c.c_n = reinterpret_cast<double*>(take(size_t(3 * kNoAllocContacts) * 8));
-    c.c_pen = reinterpret_cast<double*>(take(size_t(kNoAllocContacts) * 8));
-    c.n_count = reinterpret_cast<uint32_t*>(take(size_t(N + 1) * 4));
-    c.n_start = reinterpret_cast<uint32_t*>(take(size_t(N + 1) * 4));
-    c.n_cursor = reinterpret_cast<uint32_t*>(take(size_t(N) * 4));
-    c.n_items = reinterpret_cast<uint32_t*>(take(size_t(4 * kNoAllocContacts) * 4));
-    c.n_sorted = reinterpret_cast<uint32_t*>(take(size_t(4 * kNoAllocContacts) * 4));
-    c.n_long = reinterpret_cast<uint32_t*>(take(size_t(N + 1) * 4));
-    c.long_sum = nullptr;  // the gather walks every list (no room for the long lists' sums)
-    long long scan_n = N + 1;
-    if (chunks + 1 > scan_n) scan_n = chunks + 1;
-    c.scan_tmp_bytes = scan_tmp_bytes(scan_n);
-    c.scan_tmp = take(c.scan_tmp_bytes);
     return off <= kNoAllocScratchBytes;
 }
 
@@ -150,9 +129,10 @@ extern "C" int mcg_objective_noalloc(mcg_ctx* ctx, const double* z, double top, 
         return MCG_ERR_CUDA;
     }
     ContactBufs fixed;
-    if (!carve(base, N, (long long)N + B, fixed)) {
+    size_t zero_bytes = 0;
+    if (!carve(base, N, (long long)N + B, fixed, zero_bytes)) {
         ctx_set_error(ctx, "mcg_objective_noalloc: internal scratch layout exceeds the array");
         return MCG_ERR_CAPACITY;
     }
-    return objective_with_fixed_contacts(ctx, fixed, z, top, energy, grad, diag);
+    return objective_with_fixed_contacts(ctx, fixed, zero_bytes, z, top, energy, grad, diag);
 }

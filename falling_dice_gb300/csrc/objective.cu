@@ -5,13 +5,13 @@
 // that a kernel's occupancy variants round identically.
 //
 //   k_state    per node: z -> current position/orientation; block partial sums of x
-//   k_center   one block: mean position for the centering term
+//   k_center   per instance: mean position for the centering term; the contact grid
 //   k_beams    per beam: axial/shear/bending/torsion energy with return mapping,
 //              the two end 6-vectors of its gradient, optional trial state
 //   k_gather   per node: deterministic CSR sum of the incident beams' end vectors in
-//              ascending beam order, gravity, centering, self-contact contributions
-//              (sorted), platen contact; packs, scales and locks the 6-DOF gradient
-//   k_finalize one block: fixed-order totals, diagnostics, non-finite guard
+//              ascending beam order, gravity, centering, the node's self-contact sums,
+//              platen contact; packs, scales and locks the 6-DOF gradient
+//   k_finalize fixed-order totals, diagnostics, non-finite guard
 #include "common.cuh"
 #include "kernels.h"
 
@@ -28,13 +28,15 @@ __global__ void __launch_bounds__(kEvalBlock) k_state(DevTopo t, PhysParams p, c
                                                       const double* __restrict__ bx, const double* __restrict__ br,
                                                       double4_32a* __restrict__ x4, double4_32a* __restrict__ R4,
                                                       double4_32a* __restrict__ M4, float4* __restrict__ xf_lo,
-                                                      float4* __restrict__ xf_hi, double* __restrict__ part) {
+                                                      float4* __restrict__ xf_hi, double* __restrict__ part,
+                                                      BuildArgs build) {
     __shared__ StateParts sm;
     const MapPos mp = map_pos(t.eblk);
     if (!t.active[mp.inst]) return;  // block-uniform
     const int i = mp.i;
     double acc[3] = {0, 0, 0};
     StateBounds bounds;
+    bool moved = false;
     if (mp.valid) {
         const double2* z2 = reinterpret_cast<const double2*>(z + 6 * size_t(i));
         const double2 za = z2[0], zb = z2[1], zc = z2[2];
@@ -63,19 +65,72 @@ __global__ void __launch_bounds__(kEvalBlock) k_state(DevTopo t, PhysParams p, c
         M4[3 * size_t(i)] = make_double4_32a(M.r0.x, M.r0.y, M.r0.z, 0.0);
         M4[3 * size_t(i) + 1] = make_double4_32a(M.r1.x, M.r1.y, M.r1.z, 0.0);
         M4[3 * size_t(i) + 2] = make_double4_32a(M.r2.x, M.r2.y, M.r2.z, 0.0);
-        bounds.take(xx, xy, xz, t.off[mp.inst], xf_lo[i], xf_hi[i]);
+        float4 lo, hi;
+        bounds.take(xx, xy, xz, t.off[mp.inst], lo, hi);
+        xf_lo[i] = lo;
+        xf_hi[i] = hi;
+        if (build.flags && build.skin > 0.f) moved = moved_beyond(build.skin, lo, hi, build.xref[i]);
         acc[0] = xx; acc[1] = xy; acc[2] = xz;
     }
+    if (build.flags) ask_build(build, moved);
     state_block_parts(acc, bounds, sm, part + 9 * size_t(blockIdx.x));
 }
 
+// The grid of a rebuilt candidate list: origin, extent and bin numbering from the node bounding
+// box ext = (min x, y, z, max x, y, z), by a whole block (thread d the axis d: the divisions are
+// the cost).  grid[]: 0-2 origin cell, 3-5 dims, 6 mode (0 Morton, 1 row-major), 7 valid, 8 number
+// of bins, 9 bins needed, 10-15 box quantization.
+constexpr float kBoxQuanta = 32000.f;  // box quantization steps across the grid extent
+__device__ void grid_params(const BuildArgs& b, const double* ext) {
+    __shared__ long long dims[3];
+    __shared__ int good[3];
+    const int d = threadIdx.x;
+    if (d < 3) {
+        const double lo = floor((ext[d] - b.pad) / b.cell) - 1.0;
+        const double hi = floor((ext[3 + d] + b.pad) / b.cell) + 1.0;
+        const bool ok = isfinite(lo) && isfinite(hi) && fabs(lo) <= 1e9 && fabs(hi) <= 1e9;
+        const long long l = ok ? (long long)lo : 0, dim = ok ? (long long)hi - l + 1 : 1;
+        good[d] = ok;
+        dims[d] = dim;
+        b.grid[d] = int(l);
+        b.grid[3 + d] = int(dim);
+        b.grid[10 + d] = __float_as_int(float(double(kBoxQuanta) / (double(dim) * b.cell)));
+        b.grid[13 + d] = __float_as_int(float(double(l) * b.cell));
+    }
+    __syncthreads();
+    if (d != 0) return;
+    bool ok = good[0] && good[1] && good[2];
+    int bits = 0;
+    for (int k = 0; k < 3; k++)
+        if (dims[k] > 1) bits = max(bits, 64 - __clzll(dims[k] - 1));
+    const double dense = double(dims[0]) * double(dims[1]) * double(dims[2]);
+    long long nb = dense < 1e18 ? dims[0] * dims[1] * dims[2] : 1LL << 60;
+    int mode = 1;
+    if (bits <= 10 && (1LL << (3 * bits)) <= b.bin_cap && (1LL << (3 * bits)) <= 4 * nb) {
+        mode = 0;
+        nb = 1LL << (3 * bits);
+    }
+    b.grid[9] = int(nb < (1LL << 30) ? nb : (1LL << 30));
+    if (ok && nb > b.bin_cap) {  // the host enlarges the bins or coarsens the cells
+        atomicOr(b.flags, uint32_t(kOverBins));
+        ok = false;
+    }
+    b.grid[6] = mode;
+    b.grid[7] = ok ? 1 : 0;
+    b.grid[8] = ok ? int(nb) : 0;
+}
+
 // Mean position of each instance's nodes (MC/src/sim.cpp:143) and bounding boxes from the
-// k_state partials: block i < I writes instance i's cen[9i..9i+8] (mean, minimum, maximum);
-// block I the minimum and maximum over all instances at cen[9I + 3..8].
-// Also the instance's centering force on each node (sim.cpp:143).
+// k_state partials: block i < I writes instance i's cen[9i..9i+8] (mean, minimum, maximum) and
+// its centering force on each node (sim.cpp:143); block I the minimum and maximum over all
+// instances at cen[9I + 3..8], and it decides whether this evaluation rebuilds the candidate
+// list: every kernel of the build returns at once when it does not.
 __global__ void __launch_bounds__(kBlock) k_center(DevTopo t, double centering, const double* __restrict__ part,
-                                                   double* __restrict__ cen, double* __restrict__ cforce) {
+                                                   double* __restrict__ cen, double* __restrict__ cforce,
+                                                   BuildArgs build) {
     __shared__ double sm[6 * kBlock];
+    __shared__ double ext[6];
+    __shared__ int rebuild;
     const int inst = blockIdx.x;
     int k0 = 0, k1 = t.n_eblk;
     if (inst < t.I) {
@@ -84,28 +139,57 @@ __global__ void __launch_bounds__(kBlock) k_center(DevTopo t, double centering, 
         k1 = r.y;
     }
     double acc[3] = {0, 0, 0};
-    const double ninf = __longlong_as_double(0xfff0000000000000LL);
-    double mx[6] = {ninf, ninf, ninf, ninf, ninf, ninf};
+    const long long lowest = (long long)0x8000000000000000ULL;
+    long long mx[6] = {lowest, lowest, lowest, lowest, lowest, lowest};  // maxima on the integer pipe
 #pragma unroll 4
     for (int k = k0 + int(threadIdx.x); k < k1; k += blockDim.x) {
         const double* q = part + 9 * size_t(k);
-        acc[0] += q[0]; acc[1] += q[1]; acc[2] += q[2];
-#pragma unroll
-        for (int j = 0; j < 6; j++) mx[j] = fmax(mx[j], q[3 + j]);
-    }
-    block_sum_t<3>(acc, sm);
-    block_max_t<6>(mx, sm);
-    if (threadIdx.x == 0) {
-        double* c = cen + 9 * size_t(inst);
         if (inst < t.I) {
-            const double inv = 1.0 / double(t.inst_n[inst]);
-            c[0] = acc[0] * inv; c[1] = acc[1] * inv; c[2] = acc[2] * inv;
-            cforce[2 * inst] = centering * c[0] / double(t.inst_n[inst]);
-            cforce[2 * inst + 1] = centering * c[2] / double(t.inst_n[inst]);
+            acc[0] += q[0]; acc[1] += q[1]; acc[2] += q[2];
         }
-        c[3] = -mx[0]; c[4] = -mx[1]; c[5] = -mx[2];
-        c[6] = mx[3]; c[7] = mx[4]; c[8] = mx[5];
+#pragma unroll
+        for (int j = 0; j < 6; j++) mx[j] = max(mx[j], order_key(q[3 + j]));
     }
+    if (inst < t.I) block_sum_t<3>(acc, sm);
+    long long* smx = reinterpret_cast<long long*>(sm);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int j = 0; j < 6; j++) {
+        const long long m = warp_max_key(mx[j]);
+        if (lane == 0) smx[j * (kBlock / 32) + warp] = m;
+    }
+    __syncthreads();
+    double* c = cen + 9 * size_t(inst);
+    if (threadIdx.x < 6) {
+        const int j = threadIdx.x;
+        long long m = smx[j * (kBlock / 32)];
+        for (int w = 1; w < kBlock / 32; w++) m = max(m, smx[j * (kBlock / 32) + w]);
+        const double v = order_value(m);
+        ext[j] = j < 3 ? -v : v;
+        c[3 + j] = ext[j];
+    }
+    if (inst < t.I) {
+        if (threadIdx.x == 0) {
+            const double n = double(t.inst_n[inst]), inv = 1.0 / n;
+            c[0] = acc[0] * inv; c[1] = acc[1] * inv; c[2] = acc[2] * inv;
+            cforce[2 * inst] = centering * c[0] / n;
+            cforce[2 * inst + 1] = centering * c[2] / n;
+        }
+        return;
+    }
+    if (!build.flags) return;
+    if (threadIdx.x == 0) {
+        rebuild = build.flags[1] || build.flags[2] || !(build.skin > 0.f);
+        build.counts[kContacts] = 0;
+        if (rebuild) {
+            build.flags[1] = 1;
+            build.flags[3] = 0;  // the pair pass's bin cursor
+            build.flags[4]++;    // builds since the buffers were allocated
+            for (int k : {int(kCand), int(kKept), int(kEntries), int(kLargestBin), int(kOccupied)}) build.counts[k] = 0;
+        }
+    }
+    __syncthreads();
+    if (rebuild) grid_params(build, ext);
 }
 
 __device__ __forceinline__ q4 ldq(const double4_32a* R, int i) {
@@ -382,71 +466,24 @@ __global__ void __launch_bounds__(kBeamBlock, 2 * kMinBlocks) k_beams(DevTopo t,
     }
 }
 
-// Contribution of one contact slot to its node (MC/src/sim.cpp:23 addShapeGradient):
-// slots 0/1 are shape a's ends, 2/3 shape b's; capsule ends split the force (1-u, u).
-__device__ __forceinline__ d3 contact_slot_force(const ContactBufs& c, const PhysParams& p, int N,
-                                                 uint32_t item) {
-    const uint32_t ci = item >> 2, slot = item & 3u;
-    const d3 n{c.c_n[3 * size_t(ci)], c.c_n[3 * size_t(ci) + 1], c.c_n[3 * size_t(ci) + 2]};
-    const double mag = p.contact_k * c.c_pen[ci];
-    const bool side_b = slot >= 2;
-    const uint32_t shape = side_b ? c.c_b[ci] : c.c_a[ci];
-    const bool capsule = shape >= uint32_t(N);
-    const d3 v = n * (side_b ? -mag : mag);
-    if (!capsule) return v;
-    const double u = side_b ? c.c_t[ci] : c.c_s[ci];
-    return (slot & 1u) ? v * u : v * (1 - u);
-}
-
-// One item of a node's contact list: its force, and for slot 0 (the first node of the
-// lower shape, present for every contact) the contact's penalty energy, count and
-// penetration (sim.cpp:163-164).
-__device__ __forceinline__ void add_contact_item(const ContactBufs& c, const PhysParams& p, int N, uint32_t item,
-                                                 d3& gx, double& energy, double& count, double& pen_max) {
-    gx = gx + contact_slot_force(c, p, N, item);
-    if ((item & 3u) == 0) {
-        const double pen = c.c_pen[item >> 2];
-        energy += .5 * p.contact_k * pen * pen;
-        count += 1;
-        pen_max = fmax(pen_max, pen);
-    }
-}
-
-// The sums of each long list (n_long) for the gather, one warp per node: lane l takes items
-// l, l + 32, ... in list order, then the lanes' partial sums meet in a fixed butterfly, so
-// the sums do not depend on the order of the queue or of the contact list.  A node of a
-// densely compressed lattice holds a few hundred items; walked by one thread in the gather,
-// its dependent loads set the gather's time.
-__global__ void __launch_bounds__(kBlock) k_node_contact_long(DevTopo t, PhysParams p, ContactBufs c) {
-    const int lane = threadIdx.x & 31;
-    const uint32_t nl = c.n_long[0];
-    const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
-    for (long long j = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; j < nl; j += warps) {
-        const uint32_t i = c.n_long[1 + j];
-        const uint32_t s0 = c.n_start[i], cnt = c.n_count[i];
-        d3 f{0, 0, 0};
-        double energy = 0, count = 0, pen_max = 0;
-        for (uint32_t k = uint32_t(lane); k < cnt; k += 32)
-            add_contact_item(c, p, t.N, c.n_sorted[s0 + k], f, energy, count, pen_max);
+// Value of a fixed-point sum (NodeContact): carries propagated, sign taken out, the magnitude's
+// two halves converted and scaled by the quantum 2^e0.
+__device__ __forceinline__ double fixed_value(const long long* l, int e0) {
+    unsigned a[4];
+    long long t = 0;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            f.x += __shfl_xor_sync(0xffffffffu, f.x, o);
-            f.y += __shfl_xor_sync(0xffffffffu, f.y, o);
-            f.z += __shfl_xor_sync(0xffffffffu, f.z, o);
-            energy += __shfl_xor_sync(0xffffffffu, energy, o);
-            count += __shfl_xor_sync(0xffffffffu, count, o);
-            pen_max = fmax(pen_max, __shfl_xor_sync(0xffffffffu, pen_max, o));
-        }
-        if (lane == 0) {
-            double* q = c.long_sum + 6 * size_t(j);
-            q[0] = f.x;
-            q[1] = f.y;
-            q[2] = f.z;
-            q[3] = energy;
-            q[4] = count;
-            q[5] = pen_max;
-        }
+    for (int k = 0; k < kSumLimbs; k++) {
+        t = l[k] + (t >> 32);
+        a[k] = unsigned(t);
     }
+    const bool minus = t < 0;
+    unsigned long long lo = ((unsigned long long)a[1] << 32) | a[0], hi = ((unsigned long long)a[3] << 32) | a[2];
+    if (minus) {
+        lo = ~lo + 1;
+        hi = ~hi + (lo == 0);
+    }
+    const double v = fma(double(hi), 0x1p64, double(lo)) * __hiloint2double((e0 + 1023) << 20, 0);
+    return minus ? -v : v;
 }
 
 // ---- per-node gather: the scatter of MC/src/sim.cpp:139-172, as a deterministic CSR sum ---
@@ -519,46 +556,21 @@ __global__ void __launch_bounds__(kEvalBlock, 2 * kMinBlocks) k_gather(DevTopo t
         // centering (sim.cpp:143), the same force for all nodes of the instance
         gx.x += e.cforce[2 * mp.inst];
         gx.z += e.cforce[2 * mp.inst + 1];
-        // self-contact forces on this node in ascending (lower shape, higher shape, slot)
-        // order (the list is sorted by the contact pipeline), and the self-contact energy of
-        // each contact on the first node of its lower shape: both independent of the order
-        // of the contact list
-        const uint32_t cnt = use_contacts ? c.n_count[i] : 0u;
-        if (cnt > 32 && c.long_sum) {  // summed by k_node_contact_long
-            const double* q = c.long_sum + 6 * size_t(c.n_cursor[i]);
-            gx = gx + d3{q[0], q[1], q[2]};
-            econt += q[3];
-            count += int(q[4]);
-            pen_max = fmax(pen_max, q[5]);
-        } else if (cnt) {
-            const uint32_t s0 = c.n_start[i];
-            uint32_t k = 0;
-            // four items at a time: their loads in flight together (a joint of a densely
-            // compressed lattice can hold a few hundred items), the additions in list order
-            for (; k + 4 <= cnt; k += 4) {
-                d3 f[4];
-                double pen[4];
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    const uint32_t item = c.n_sorted[s0 + k + j];
-                    f[j] = contact_slot_force(c, p, N, item);
-                    pen[j] = (item & 3u) == 0 ? c.c_pen[item >> 2] : -1.0;  // a contact's pen > 0
-                }
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    gx = gx + f[j];
-                    if (!negative_sign(pen[j])) {
-                        econt += .5 * p.contact_k * pen[j] * pen[j];
-                        count += 1;
-                        pen_max = fmax(pen_max, pen[j]);
-                    }
-                }
+        // self-contact: the node's fixed-point sums, cleared for the next evaluation
+        const unsigned long long items = use_contacts ? c.n_count[i] : 0ULL;
+        if (items) {
+            NodeContact& r = c.n_sum[i];
+            gx.x += fixed_value(r.f[0], c.force_e0);
+            gx.y += fixed_value(r.f[1], c.force_e0);
+            gx.z += fixed_value(r.f[2], c.force_e0);
+            if (items >> 32) {
+                econt = fixed_value(r.energy, c.energy_e0);
+                pen_max = __longlong_as_double((long long)r.pen);
             }
-            for (; k < cnt; k++) {
-                double one = 0;
-                add_contact_item(c, p, N, c.n_sorted[s0 + k], gx, econt, one, pen_max);
-                count += one != 0;
-            }
+            if (items & kContactNotFinite) econt = __longlong_as_double(0x7ff8000000000000LL);
+            count = int(items >> 32);
+            r = NodeContact{};
+            c.n_count[i] = 0;
         }
         // platens (sim.cpp:168-171)
         const double jr = p.joint_radius, kc = p.contact_k;
@@ -604,7 +616,7 @@ __global__ void __launch_bounds__(kEvalBlock, 2 * kMinBlocks) k_gather(DevTopo t
     double w = 0;
     long long pm = 0;
     int cn = 0;
-    if (__any_sync(0xffffffffu, count != 0)) {
+    if (__any_sync(0xffffffffu, count != 0 || __double_as_longlong(econt) != 0)) {
         w = warp_sum4(eplat, reac, econt, 0.0);
         pm = warp_max_key(__double_as_longlong(pen_max));
         cn = __reduce_add_sync(0xffffffffu, count);
@@ -636,103 +648,121 @@ __global__ void __launch_bounds__(kEvalBlock, 2 * kMinBlocks) k_gather(DevTopo t
 }
 
 // ---- totals and the non-finite guard ---------------------------------------------------------
-// Two stages, so the FP64 additions spread over many SMs (GB300's FP64 pipe is narrow).
-// Stage 1: block (f, inst) sums the instance's block partials k = first + f + kFinFan j.
+// One launch: an instance of few block partials is summed by one block, a larger one by kFinFan
+// blocks (block f takes the partials first + f + kFinFan j), the last of which to finish sums
+// their results in order, so the FP64 additions spread over many SMs.  Which way an instance
+// goes depends on its own size only, so it sums alike alone and in a batch.
 constexpr int kFinFan = 32;
 constexpr int kFinVals = 11;  // beamE, elastic, plastic, gravityE, platenE, reaction, contactE,
                               // contacts, |g|^2, max penetration, max |g|
-static_assert(kFinPartDoubles == kFinFan * kFinVals, "first-stage totals buffer");
-__global__ void __launch_bounds__(kBlock) k_finalize_parts(DevTopo t, const double* __restrict__ pbeam,
-                                                           const double* __restrict__ pnode,
-                                                           double* __restrict__ fpart) {
+constexpr int kFinSingle = 512;  // block partials one block sums: two per thread
+static_assert(kFinPartDoubles == kFinFan * kFinVals + 1, "first-stage totals and their counter");
+__global__ void __launch_bounds__(kBlock) k_finalize(DevTopo t, PhysParams p, EvalBufs e, uint32_t* __restrict__ flags,
+                                                     const uint32_t* __restrict__ counts, double* __restrict__ grad) {
     __shared__ double sm[9 * kBlock];
+    __shared__ double tot[kFinVals];
+    __shared__ int state;  // 0 done, 1 this block sums up, 2 the gradient is to be cleared
     const int inst = blockIdx.y, f = blockIdx.x;
-    if (!t.active[inst]) return;
+    EvalOut* out = e.out + inst;
+    if (inst == 0 && f == 0 && threadIdx.x == 0) {  // of the whole evaluation, whether instance 0 is active or not
+        out->overflow = flags ? int(flags[0] & ~uint32_t(kNonFinite)) : 0;
+        out->pairs = counts ? counts[kContacts] : 0u;
+        out->kernel_error = *e.err;
+        if (flags) flags[0] = flags[1] = 0;  // for the next evaluation
+    }
     const int4 r = t.irange[inst];
     const int2 er = t.erange[inst];
-    double acc[6] = {0, 0, 0, 0, 0, 0};  // beamE, elastic, plastic, gravityE, platenE, reaction
-    double cacc[3] = {0, 0, 0};          // self-contact E, contacts (platen and self), |g|^2
-    double m2[2] = {0, 0};               // max penetration, max |g|
-    for (int k = r.z + f + kFinFan * int(threadIdx.x); k < r.w; k += kFinFan * int(blockDim.x)) {
-        acc[0] += pbeam[3 * k]; acc[1] += pbeam[3 * k + 1]; acc[2] += pbeam[3 * k + 2];
+    const int fan = (r.w - r.z) + (er.y - er.x) <= kFinSingle ? 1 : kFinFan;
+    if (!t.active[inst] || f >= fan) return;
+    double all[9] = {};  // sums: beamE, elastic, plastic, gravityE, platenE, reaction, contactE, contacts, |g|^2
+    long long m2[2] = {0, 0};  // max penetration, max |g| (bits of non-negative doubles)
+    for (int k = r.z + f + fan * int(threadIdx.x); k < r.w; k += fan * int(blockDim.x)) {
+        const double* q = e.part_beam + 3 * size_t(k);
+        all[0] += q[0]; all[1] += q[1]; all[2] += q[2];
     }
-    for (int k = er.x + f + kFinFan * int(threadIdx.x); k < er.y; k += kFinFan * int(blockDim.x)) {
-        const double* q = pnode + kNodeParts * size_t(k);
-        acc[3] += q[0]; acc[4] += q[1]; acc[5] += q[2];
-        m2[0] = fmax(m2[0], q[3]);
-        cacc[1] += q[4];
-        cacc[0] += q[5];
-        cacc[2] += q[6];
-        m2[1] = fmax(m2[1], q[7]);
+    for (int k = er.x + f + fan * int(threadIdx.x); k < er.y; k += fan * int(blockDim.x)) {
+        const double* q = e.part_node + kNodeParts * size_t(k);
+        all[3] += q[0]; all[4] += q[1]; all[5] += q[2];
+        m2[0] = max(m2[0], __double_as_longlong(q[3]));
+        all[7] += q[4];
+        all[6] += q[5];
+        all[8] += q[6];
+        m2[1] = max(m2[1], __double_as_longlong(q[7]));
     }
-    double all[9] = {acc[0], acc[1], acc[2], acc[3], acc[4], acc[5], cacc[0], cacc[1], cacc[2]};
     block_sum_t<9>(all, sm);
-    block_max_t<2>(m2, sm);
-    if (threadIdx.x == 0) {
-        double* o = fpart + kFinVals * (size_t(inst) * kFinFan + f);
-        for (int k = 0; k < 9; k++) o[k] = all[k];
-        o[9] = m2[0]; o[10] = m2[1];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    long long* smx = reinterpret_cast<long long*>(sm);
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        const long long m = warp_max_key(m2[k]);
+        if (lane == 0) smx[k * (kBlock / 32) + warp] = m;
     }
-}
-
-// Stage 2, one block per instance: the kFinFan stage-1 results in order, the energy in the
-// reference's group order, diagnostics, non-finite guard.
-__global__ void __launch_bounds__(kBlock) k_finalize(DevTopo t, PhysParams p, const double* __restrict__ fpart,
-                                                     const double* __restrict__ cen,
-                                                     const uint32_t* __restrict__ flags, EvalOut* out_all) {
-    static_assert(kFinFan == 32, "one stage-1 result per lane");
-    const int inst = blockIdx.x;
-    if (!t.active[inst]) return;
-    const double* q = fpart + kFinVals * (size_t(inst) * kFinFan + threadIdx.x);
-    double acc[6], cacc[3];  // beamE, elastic, plastic, gravityE, platenE, reaction; contactE,
-                             // contacts, |g|^2
-#pragma unroll
-    for (int k = 0; k < 6; k++) acc[k] = warp_sum(q[k]);
-#pragma unroll
-    for (int k = 0; k < 3; k++) cacc[k] = warp_sum(q[6 + k]);
-    const double pmax = warp_max(q[9]), gmax = warp_max(q[10]);
-    if (threadIdx.x != 0) return;
+    __syncthreads();
     if (threadIdx.x == 0) {
-        const double* c = cen + 9 * size_t(inst);
+        for (int w = 1; w < kBlock / 32; w++) {
+            smx[0] = max(smx[0], smx[w]);
+            smx[kBlock / 32] = max(smx[kBlock / 32], smx[kBlock / 32 + w]);
+        }
+        for (int k = 0; k < 9; k++) tot[k] = all[k];
+        tot[9] = __longlong_as_double(smx[0]);
+        tot[10] = __longlong_as_double(smx[kBlock / 32]);
+        state = 1;
+        if (fan > 1) {
+            double* fp = e.part_fin + size_t(kFinPartDoubles) * inst;
+            for (int k = 0; k < kFinVals; k++) fp[kFinVals * f + k] = tot[k];
+            __threadfence();
+            unsigned* done = reinterpret_cast<unsigned*>(fp + kFinPartDoubles - 1);
+            state = atomicAdd(done, 1u) == unsigned(fan) - 1u;
+            if (state) *done = 0;
+            __threadfence();
+        }
+    }
+    __syncthreads();
+    if (!state) return;
+    if (fan > 1) {
+        const double* fp = e.part_fin + size_t(kFinPartDoubles) * inst;
+        for (int k = warp; k < kFinVals; k += kBlock / 32) {
+            const double v = __ldcg(fp + kFinVals * lane + k);
+            const double s = k < 9 ? warp_sum(v) : warp_max(v);
+            if (lane == 0) tot[k] = s;
+        }
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        const double* c = e.cen + 9 * size_t(inst);
         const double center = .5 * p.centering * (sqr(c[0]) + sqr(c[2]));
-        const double contactE = cacc[0];
         // Group order of the reference's accumulation: beams, gravity, centering,
         // self-contact, platens (sim.cpp:139-171).
-        double energy = acc[0];
-        energy += acc[3];
+        double energy = tot[0];
+        energy += tot[3];
         energy += center;
-        energy += contactE;
-        energy += acc[4];
+        energy += tot[6];
+        energy += tot[4];
         const int nonfinite = isfinite(energy) ? 0 : 1;
-        EvalOut* out = out_all + inst;
         out->energy = nonfinite ? __longlong_as_double(0x7ff0000000000000LL) : energy;
-        out->elastic = acc[1];
-        out->plastic = acc[2];
-        out->contact = contactE + acc[4];
-        out->reaction = acc[5];
-        out->max_pen = pmax;
-        out->contacts = int(cacc[1]);
+        out->elastic = tot[1];
+        out->plastic = tot[2];
+        out->contact = tot[6] + tot[4];
+        out->reaction = tot[5];
+        out->max_pen = tot[9];
+        out->contacts = int(tot[7]);
         out->nonfinite = nonfinite;
-        out->beam_energy = acc[0];
-        out->node_energy = acc[3];
+        out->beam_energy = tot[0];
+        out->node_energy = tot[3];
         out->center_energy = center;
-        out->contact_energy = contactE;
-        out->platen_energy = acc[4];
-        out->overflow = flags ? int(flags[0] & ~uint32_t(kNonFinite)) : 0;
-        // a non-finite evaluation has a zero gradient (k_zero_if_nonfinite)
+        out->contact_energy = tot[6];
+        out->platen_energy = tot[4];
+        // a non-finite evaluation has a zero gradient
         const long long nf = t.inst_free[inst];
-        out->rms = nonfinite ? 0.0 : (nf ? sqrt(cacc[2] / double(nf)) : 0.0);
-        out->gmax = nonfinite ? 0.0 : gmax;
+        out->rms = nonfinite ? 0.0 : (nf ? sqrt(tot[8] / double(nf)) : 0.0);
+        out->gmax = nonfinite ? 0.0 : tot[10];
+        state = nonfinite ? 2 : 0;
     }
-}
-
-// Non-finite energy: the instance's whole gradient is zero (sim.cpp:172).
-__global__ void __launch_bounds__(kBlock) k_zero_if_nonfinite(DevTopo t, const EvalOut* __restrict__ out,
-                                                              double* __restrict__ grad) {
-    const MapPos mp = map_pos(t.nblk);
-    if (!mp.valid || !t.active[mp.inst] || !out[mp.inst].nonfinite) return;
-#pragma unroll
-    for (int k = 0; k < 6; k++) grad[6 * size_t(mp.i) + k] = 0;
+    __syncthreads();
+    if (state == 2) {  // non-finite energy: the instance's whole gradient is zero (sim.cpp:172)
+        double* g = grad + 6 * size_t(t.eblk[er.x].x);
+        for (long long k = threadIdx.x; k < 6LL * t.inst_n[inst]; k += blockDim.x) g[k] = 0;
+    }
 }
 
 // ---- commit (MC/src/sim.cpp:212): base state <- current state, plastic <- trial ----------
@@ -809,14 +839,14 @@ __global__ void __launch_bounds__(kBlock) k_plastic_final(DevTopo t, const doubl
 
 // ---- launchers ------------------------------------------------------------------------------
 void launch_state(const DevTopo& t, const PhysParams& p, const double* z, const double* base_x,
-                  const double* base_r, EvalBufs& e, cudaStream_t s) {
-    k_state<<<t.n_eblk, kEvalBlock, 0, s>>>(t, p, z, base_x, base_r, e.x, e.R, e.M, e.xf_lo, e.xf_hi, e.part_state);
+                  const double* base_r, const BuildArgs& b, EvalBufs& e, cudaStream_t s) {
+    k_state<<<t.n_eblk, kEvalBlock, 0, s>>>(t, p, z, base_x, base_r, e.x, e.R, e.M, e.xf_lo, e.xf_hi, e.part_state, b);
     note_launches(1);
-    launch_center(t, p, e, s);
+    launch_center(t, p, b, e, s);
 }
 
-void launch_center(const DevTopo& t, const PhysParams& p, EvalBufs& e, cudaStream_t s) {
-    k_center<<<t.I + 1, kBlock, 0, s>>>(t, p.centering, e.part_state, e.cen, e.cforce);
+void launch_center(const DevTopo& t, const PhysParams& p, const BuildArgs& b, EvalBufs& e, cudaStream_t s) {
+    k_center<<<t.I + 1, kBlock, 0, s>>>(t, p.centering, e.part_state, e.cen, e.cforce, b);
     note_launches(1);
 }
 
@@ -868,17 +898,12 @@ void launch_beams(const DevTopo& t, const Material& m, const double* plastic, in
     note_launches(1);
 }
 
-constexpr int kLongListBlocks = 4 * 152;  // eight long lists per block, grid-stride
-
 template <bool F32>
 void gather_variant(const DevTopo& t, const PhysParams& p, const ContactBufs* c, double* grad, EvalBufs& e,
                     cudaStream_t s, int variant) {
     ContactBufs cc{};
     if (c) cc = *c;
     const int uc = c ? 1 : 0;
-    if (c && c->long_sum) {
-        (k_node_contact_long<<<kLongListBlocks, kBlock, 0, s>>>(t, p, cc), note_launches(1));
-    }
     switch (variant) {
         case 1: k_gather<F32, kGatherBlocks[1]><<<t.n_eblk, kEvalBlock, 0, s>>>(t, p, cc, uc, e, grad); break;
         case 2: k_gather<F32, kGatherBlocks[2]><<<t.n_eblk, kEvalBlock, 0, s>>>(t, p, cc, uc, e, grad); break;
@@ -899,10 +924,8 @@ void launch_gather_mixed(const DevTopo& t, const PhysParams& p, const ContactBuf
 
 void launch_finalize(const DevTopo& t, const PhysParams& p, const ContactBufs* c, double* grad, EvalBufs& e,
                      cudaStream_t s) {
-    k_finalize_parts<<<dim3(kFinFan, t.I), kBlock, 0, s>>>(t, e.part_beam, e.part_node, e.part_fin);
-    k_finalize<<<t.I, 32, 0, s>>>(t, p, e.part_fin, e.cen, c ? c->flags : nullptr, e.out);
-    k_zero_if_nonfinite<<<t.n_nblk, kBlock, 0, s>>>(t, e.out, grad);
-    note_launches(3);
+    k_finalize<<<dim3(kFinFan, t.I), kBlock, 0, s>>>(t, p, e, c ? c->flags : nullptr, c ? c->counts : nullptr, grad);
+    note_launches(1);
 }
 
 }  // namespace mcg

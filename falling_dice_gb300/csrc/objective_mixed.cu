@@ -173,13 +173,14 @@ __global__ void __launch_bounds__(kEvalBlock) k_state_mixed(DevTopo t, double ts
                                                         const double* __restrict__ bx, float4* __restrict__ UE,
                                                         double4_32a* __restrict__ x4,
                                                         float4* __restrict__ xf_lo, float4* __restrict__ xf_hi,
-                                                        double* __restrict__ part) {
+                                                        double* __restrict__ part, BuildArgs build) {
     __shared__ StateParts sm;
     const MapPos mp = map_pos(t.eblk);
     if (!t.active[mp.inst]) return;
     const int i = mp.i;
     double acc[3] = {0, 0, 0};
     StateBounds bounds;
+    bool moved = false;
     if (mp.valid) {
         const double2* z2 = reinterpret_cast<const double2*>(z + 6 * size_t(i));
         const double2 za = z2[0], zb = z2[1], zc = z2[2];
@@ -209,9 +210,14 @@ __global__ void __launch_bounds__(kEvalBlock) k_state_mixed(DevTopo t, double ts
         const double xy = bx[3 * size_t(i) + 1] + to_double(tr[1]);
         const double xz = bx[3 * size_t(i) + 2] + to_double(tr[2]);
         x4[i] = make_double4_32a(xx, xy, xz, 0.0);
-        bounds.take(xx, xy, xz, t.off[mp.inst], xf_lo[i], xf_hi[i]);
+        float4 lo, hi;
+        bounds.take(xx, xy, xz, t.off[mp.inst], lo, hi);
+        xf_lo[i] = lo;
+        xf_hi[i] = hi;
+        if (build.flags && build.skin > 0.f) moved = moved_beyond(build.skin, lo, hi, build.xref[i]);
         acc[0] = xx; acc[1] = xy; acc[2] = xz;
     }
+    if (build.flags) ask_build(build, moved);
     state_block_parts(acc, bounds, sm, part + 9 * size_t(blockIdx.x));
 }
 
@@ -614,11 +620,11 @@ __global__ void k_f32_to_f64(long long n, const float* __restrict__ a, double* _
 }  // namespace
 
 void launch_state_mixed(const DevTopo& t, const PhysParams& p, const double* z, const double* base_x,
-                        const MixedNodes& mn, EvalBufs& e, cudaStream_t s) {
+                        const MixedNodes& mn, const BuildArgs& b, EvalBufs& e, cudaStream_t s) {
     k_state_mixed<<<t.n_eblk, kEvalBlock, 0, s>>>(t, p.translation_scale, z, base_x, mn.UE, e.x, e.xf_lo, e.xf_hi,
-                                              e.part_state);
+                                                  e.part_state, b);
     note_launches(1);
-    launch_center(t, p, e, s);
+    launch_center(t, p, b, e, s);
 }
 
 // Variants of the mixed beam kernel: the plain kernel at 3, 4, 5 or 6 CTAs per SM, and the

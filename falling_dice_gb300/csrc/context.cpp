@@ -240,6 +240,18 @@ struct mcg_ctx {
     uint8_t* d_trial = nullptr;   // per-instance trial mask of the loop's evaluations
     MzStatus* d_mz = nullptr;
     cudaGraphExec_t loop_exec = nullptr;
+    // Captured evaluations run the contact pipeline (integer work) beside the beam kernel (FP64
+    // pipe or memory): its branch of the graph is captured on this stream, whose priority lets
+    // the pipeline's short kernels in between the beam kernel's blocks.
+    cudaStream_t fork = nullptr;
+    cudaEvent_t fork_ev[2] = {};
+    void make_fork() {
+        if (fork) return;
+        int least = 0, greatest = 0;
+        ck(cudaDeviceGetStreamPriorityRange(&least, &greatest), "cudaDeviceGetStreamPriorityRange");
+        for (cudaEvent_t& e : fork_ev) ck(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
+        ck(cudaStreamCreateWithPriority(&fork, cudaStreamNonBlocking, greatest), "cudaStreamCreate");
+    }
     cudaStream_t side = nullptr;  // captures the bodies of the loop's conditional nodes
     bool device_loop = true;
     std::string loop_error;
@@ -277,6 +289,9 @@ struct mcg_ctx {
         for (auto& e : ev_t)
             if (e) cudaEventDestroy(e);
         if (side) cudaStreamDestroy(side);
+        if (fork) cudaStreamDestroy(fork);
+        for (cudaEvent_t e : fork_ev)
+            if (e) cudaEventDestroy(e);
         if (stream) cudaStreamDestroy(stream);
     }
 
@@ -449,7 +464,7 @@ struct mcg_ctx {
     // ev.out[0..I).  Enqueues only: no host synchronisation.
     void eval(const double* dz, bool trials, double* d_gout) {
         if (!use_graphs || timing) {
-            eval_launches(dz, trials, d_gout);
+            eval_launches(dz, trials, d_gout, false);
         } else {
             const EvalGraph* found = nullptr;
             for (const EvalGraph& g : graphs)
@@ -458,8 +473,9 @@ struct mcg_ctx {
                 cudaGraph_t graph = nullptr;
                 cudaGraphExec_t exec = nullptr;
                 const long long before = g_launch_count.load();
+                make_fork();
                 ck(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal), "cudaStreamBeginCapture");
-                eval_launches(dz, trials, d_gout);
+                eval_launches(dz, trials, d_gout, true);
                 ck(cudaStreamEndCapture(stream, &graph), "cudaStreamEndCapture");
                 const long long kernels = g_launch_count.load() - before;
                 g_launch_count -= kernels;  // counted when the graph runs
@@ -478,7 +494,8 @@ struct mcg_ctx {
     }
 
     // trials: 0 none, 1 every instance, 2 the instances of d_trial (device-resident loop)
-    void eval_launches(const double* dz, int trials, double* d_gout) {
+    // forked: captured launches, the contact pipeline on its own branch beside the beam kernel
+    void eval_launches(const double* dz, int trials, double* d_gout, bool forked) {
         PhysParams p = phys;
         p.broad_cell = broad_cell;
         p.inv_cell_f = float(1.0 / broad_cell);
@@ -486,15 +503,24 @@ struct mcg_ctx {
         const BuildArgs ba = build_args(cb, contact_skin);
         if (mixed) launch_state_mixed(topo, p, dz, d_baseX, mn, ba, ev, stream);
         else launch_state(topo, p, dz, d_baseX, d_baseR, ba, ev, stream);
+        const ContactBufs* cptr = p.self_contact ? &cb : nullptr;
+        const bool branch = forked && cptr;
+        cudaStream_t cs = branch ? fork : stream;
+        if (branch) {
+            ck(cudaEventRecord(fork_ev[0], stream), "cudaEventRecord");
+            ck(cudaStreamWaitEvent(fork, fork_ev[0], 0), "cudaStreamWaitEvent");
+        }
+        launch_center(topo, p, ba, ev, cs);
+        if (branch) launch_contacts(topo, p, ev, cb, contact_skin, cs);
         mark(1);
         if (mixed) launch_beams_mixed(topo, mat, mb, mn, trials, ev, stream, beam_variant);
         else launch_beams(topo, mat, d_plastic, trials, ev, stream, beam_variant);
         mark(2);
-        const ContactBufs* cptr = nullptr;
-        if (p.self_contact) {
-            launch_contacts(topo, p, ev, cb, contact_skin, stream, timing ? ev_t[3] : nullptr,
-                            timing ? ev_t[4] : nullptr);
-            cptr = &cb;
+        if (branch) {
+            ck(cudaEventRecord(fork_ev[1], fork), "cudaEventRecord");
+            ck(cudaStreamWaitEvent(stream, fork_ev[1], 0), "cudaStreamWaitEvent");
+        } else if (cptr) {
+            launch_contacts(topo, p, ev, cb, contact_skin, stream, timing ? ev_t[3] : nullptr, timing ? ev_t[4] : nullptr);
         } else {
             mark(3);
             mark(4);
@@ -719,6 +745,7 @@ struct mcg_ctx {
     // IF(multi) two-loop; IF(any direction) descent fix; IF(steepest) retry; B; prepare;
     // evaluation (trial states per instance); C; IF(accept) accept step }.
     void build_loop() {
+        make_fork();
         if (!side) ck(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking), "cudaStreamCreate");
         const double mt = cfg.max_translation_step / cfg.translation_scale, mr = cfg.max_rotation_step;
         const MzDev md = mz_dev();
@@ -760,7 +787,7 @@ struct mcg_ctx {
                 });
                 launch_mz_eval(md, stream);
                 bl_prepare(topo, d_ctl, d_hist, d_z, d_best, d_zeval, d_p, d_zfinal, stream);
-                eval_launches(d_zeval, 2, d_geval);
+                eval_launches(d_zeval, 2, d_geval, true);
                 launch_mz_decide(md, P, hpost, h_loop, stream);
                 capture_if(hpost, [&](cudaStream_t s2) {
                     bl_accept(topo, d_ctl, d_hist, H, d_z, d_g, d_zeval, d_geval, d_S, d_Y, 6LL * N, d_best, d_rho,
@@ -860,6 +887,7 @@ struct mcg_ctx {
         DevTopo all = topo;  // the committed instances' states (others are recomputed before use)
         all.active = d_all;
         launch_state(all, p, d_zfinal, d_baseX, d_baseR, BuildArgs{}, ev, stream);
+        launch_center(all, p, BuildArgs{}, ev, stream);
         if (mixed) {
             launch_commit(topo, d_mask, ev, d_baseX, d_baseR, nullptr, stream);
             launch_plastic_mixed(topo, d_mask, nullptr, ev.trial_nextf, mb, stream);
@@ -1844,6 +1872,7 @@ int objective_with_fixed_contacts(mcg_ctx* c, ContactBufs& fixed, size_t zero_by
         const BuildArgs ba = c->build_args(fixed, 0.f);  // always rebuilds
         if (c->mixed) launch_state_mixed(c->topo, p, c->d_zin, c->d_baseX, c->mn, ba, c->ev, s);
         else launch_state(c->topo, p, c->d_zin, c->d_baseX, c->d_baseR, ba, c->ev, s);
+        launch_center(c->topo, p, ba, c->ev, s);
         if (c->mixed) launch_beams_mixed(c->topo, c->mat, c->mb, c->mn, false, c->ev, s, c->beam_variant);
         else launch_beams(c->topo, c->mat, c->d_plastic, false, c->ev, s, c->beam_variant);
         const ContactBufs* cptr = nullptr;

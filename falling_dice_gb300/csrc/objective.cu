@@ -842,7 +842,6 @@ void launch_state(const DevTopo& t, const PhysParams& p, const double* z, const 
                   const double* base_r, const BuildArgs& b, EvalBufs& e, cudaStream_t s) {
     k_state<<<t.n_eblk, kEvalBlock, 0, s>>>(t, p, z, base_x, base_r, e.x, e.R, e.M, e.xf_lo, e.xf_hi, e.part_state, b);
     note_launches(1);
-    launch_center(t, p, b, e, s);
 }
 
 void launch_center(const DevTopo& t, const PhysParams& p, const BuildArgs& b, EvalBufs& e, cudaStream_t s) {

@@ -624,7 +624,6 @@ void launch_state_mixed(const DevTopo& t, const PhysParams& p, const double* z, 
     k_state_mixed<<<t.n_eblk, kEvalBlock, 0, s>>>(t, p.translation_scale, z, base_x, mn.UE, e.x, e.xf_lo, e.xf_hi,
                                                   e.part_state, b);
     note_launches(1);
-    launch_center(t, p, b, e, s);
 }
 
 // Variants of the mixed beam kernel: the plain kernel at 3, 4, 5 or 6 CTAs per SM, and the

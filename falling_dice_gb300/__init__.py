@@ -315,7 +315,7 @@ class Solver:
         return n.value
 
     def set_contact_cell(self, cell):
-        """Contact-grid cell size in metres (0: the reference's)."""
+        """Contact-grid cell size in metres (0: the default, mcg_set_contact_cell)."""
         self._check(self.lib.mcg_set_contact_cell(self.h, float(cell)), "mcg_set_contact_cell")
 
     def autotune(self, z=None, tops=None, reps=3):
@@ -342,7 +342,7 @@ class Solver:
                     "mcg_set_kernel_shapes")
 
     def set_contact_shapes(self, cell, pair_blocks):
-        """Grid cell (m, 0: the reference's) and pair-enumeration blocks (0: default), as
+        """Grid cell (m, 0: the default) and pair-enumeration blocks (0: default), as
         autotune() reports them."""
         self._check(self.lib.mcg_set_contact_shapes(self.h, float(cell), int(pair_blocks)),
                     "mcg_set_contact_shapes")

@@ -37,11 +37,11 @@ namespace {
 
 constexpr long long kMaxCellsPerShape = 1 << 12;
 constexpr uint32_t kBoxMax = 32767u;    // 15-bit box coordinates
-constexpr uint32_t kGuard2 = 0x80008000u;
-constexpr uint32_t kShapeBits = 29;     // shape id below, first-cell flags above
-constexpr int kPairWarps = kBlock / 32;
-constexpr int kPairGrab = 2;             // bins a warp claims at a time (<= 32)
-constexpr int kPairRanks = 128;          // bins up to this size are enumerated from registers
+constexpr int kPairThreads = 128;
+constexpr int kPairWarps = kPairThreads / 32;
+constexpr int kPairGroups = 4;           // groups of 32 shapes of a bin staged at a time
+constexpr int kChunk = 32 * kPairGroups;  // shapes of a unit of pair work (ContactBufs::units)
+constexpr int kLevelBits = 5;            // box levels inside a bin: 2^kLevelBits = 32 per axis
 constexpr int kStreamBlocks = 4 * 152;   // grid of the list kernels (256 threads, grid-stride)
 
 __device__ __forceinline__ uint32_t spread3_10(uint32_t v) {  // 10 bits -> every third bit
@@ -221,11 +221,12 @@ __device__ __noinline__ PairHit narrow_phase(const DevTopo& t, const PhysParams&
 // box (sim.cpp:154), and cell indices are a monotone function of it, so two shapes whose
 // reference boxes overlap share a cell.  The pair-test record holds the box quantized to 15 bits
 // per axis (floor minus one quantum for the low side, ceil plus one for the high side, so the
-// quantized box contains the FP32 box whatever the rounding of the scaling) with a guard bit over
-// each high value, and the first cell packed as three 10-bit fields.
+// quantized box contains the FP32 box whatever the rounding of the scaling) and the first cell
+// packed as three 10-bit fields.
 // Entries: one per cell of the shape's range, written straight into the bin's slot that the bin
-// counter hands out (all counters are zero here: the pair pass clears each bin it reads), four
-// returning atomics in flight per thread.  A bin that fills up keeps counting (kOverEntries, and
+// counter hands out (all counters are zero here: the filter clears them at the end of a build), four
+// returning atomics in flight per thread; the entry that begins a chunk of its bin lists the
+// chunk as a unit of pair work.  A bin that fills up keeps counting (kOverEntries, and
 // the largest count in counts[kLargestBin] so the host can size bin_slots).
 __global__ void __launch_bounds__(kBlock) k_shapes(DevTopo t, PhysParams p, const float4* __restrict__ xf_lo,
                                                    const float4* __restrict__ xf_hi, float skin, ContactBufs c) {
@@ -265,7 +266,7 @@ __global__ void __launch_bounds__(kBlock) k_shapes(DevTopo t, PhysParams p, cons
         atomicOr(c.flags, uint32_t(kOverSpan));  // the host coarsens the grid and evaluates again
         return;
     }
-    c.rec[s] = make_uint4(q0[0] | (q0[1] << 16), (q1[0] | (q1[1] << 16)) | kGuard2, q0[2] | ((q1[2] | 0x8000u) << 16),
+    c.rec[s] = make_uint4(q0[0] | (q0[1] << 16), q1[0] | (q1[1] << 16), q0[2] | (q1[2] << 16),
                           pack_cell(c0[0], c0[1], c0[2]));
     const int n = dim[0] * dim[1] * dim[2];
     int i = 0, j = 0, k = 0;  // the next cell of the range
@@ -289,6 +290,8 @@ __global__ void __launch_bounds__(kBlock) k_shapes(DevTopo t, PhysParams p, cons
             if (e0 + e >= n) break;
             if (slot[e] < uint32_t(c.bin_slots)) {
                 c.bin_items[size_t(bin[e]) * size_t(c.bin_slots) + slot[e]] = uint32_t(s);
+                if (slot[e] % kChunk == 0)  // the first shape of a chunk of the bin
+                    c.units[atomicAdd(c.counts + kUnits, 1u)] = make_uint2(bin[e], slot[e] / kChunk);
             } else {
                 atomicOr(c.flags, uint32_t(kOverEntries));
                 atomicMax(c.counts + kLargestBin, slot[e] + 1);
@@ -297,265 +300,272 @@ __global__ void __launch_bounds__(kBlock) k_shapes(DevTopo t, PhysParams p, cons
     }
 }
 
-// One shape as the pair test sees it inside one bin: id with the first-cell flags in the
-// top three bits (bit d set when the shape's first cell on axis d is the bin's cell), the
-// quantized box words and the shape's nodes (a joint's node twice).
-struct PairRec {
-    uint32_t id, w0, w1, w2;
-    int n0, n1;
+// ---- pair enumeration inside a bin ---------------------------------------------------------
+// 32 x 32 pairs at a time, one bit each.  Inside its bin a shape's box is reduced to 32 levels
+// per axis, by one monotone map per axis, so overlapping boxes have overlapping level ranges.
+// The low level is 0 exactly when the shape's first cell on that axis lies before the bin, so
+// that "the bin is the pair's first common cell" (each pair is examined once, the reference's
+// `tested` set without a set) reads: one of the two low levels is not 0.
+// For a group of 32 shapes the warp makes, per axis, the tables
+//   below[l] = the shapes whose low level is at most l, above[l] = those whose high level is at
+//   least l,
+// one bit per shape and one entry per level (32 entries: reads of different levels hit different
+// banks).  A shape's box partners in the group are then below[its high] & above[its low] over
+// the axes, without the below[0] (not starting here) where the shape does not start here either.
+// The tables come from bit planes: a bit transpose across the warp turns the 32 shapes' levels
+// into one word per level bit, and lane l compares its own number with all 32 levels by one
+// three-input logic operation per bit.
+struct PairRow {
+    uint32_t id;
+    int n0, n1;       // the shape's nodes (a joint's node twice)
+    uint32_t levels;  // low levels in bits 5 d, high levels in bits 15 + 5 d
 };
 
-__device__ __forceinline__ PairRec load_rec(const DevTopo& t, uint32_t s, const uint4* __restrict__ rec, uint32_t ccp) {
+// The bin's frame: level of the quantized coordinate q on axis d is (q - base) scale + 1, clamped
+// and rounded.
+struct BinFrame {
+    float base[3], scale[3];
+    uint32_t cell;  // packed cell of the bin
+};
+
+__device__ __forceinline__ uint32_t level_of(const BinFrame& f, int d, uint32_t q) {
+    // integer to float and back by adding powers of two: conversions run at a quarter of the rate
+    const float v = (__int_as_float(int(0x4b000000u | q)) - 8388608.f - f.base[d]) * f.scale[d] + 1.f;
+    return uint32_t(__float_as_int(fminf(fmaxf(v, 1.f), float((1 << kLevelBits) - 1)) + 8388608.f)) & 31u;
+}
+
+__device__ __forceinline__ PairRow load_row(const DevTopo& t, uint32_t s, const uint4* __restrict__ rec, const BinFrame& f) {
     const uint4 r = rec[s];
     const int2 nd = s < uint32_t(t.N) ? make_int2(int(s), int(s)) : t.ab[s - uint32_t(t.N)];
-    // cell spans are below 1024 per axis, so the 10-bit fields compare exactly
-    const uint32_t e = ~(r.w ^ ccp);
-    const uint32_t f = ((e & 0x3ffu) == 0x3ffu) | (((e & 0xffc00u) == 0xffc00u) << 1) |
-                       (((e & 0x3ff00000u) == 0x3ff00000u) << 2);
-    return PairRec{s | (f << kShapeBits), r.x, r.y, r.z, nd.x, nd.y};
+    const uint32_t before = r.w ^ f.cell;  // cell spans are below 1024 per axis: a field is 0 where the first cell is the bin's
+    PairRow row{s, nd.x, nd.y, 0};
+    if (!(before & 0x3ffu)) row.levels |= level_of(f, 0, r.x & 0x7fffu);
+    if (!(before & 0xffc00u)) row.levels |= level_of(f, 1, r.x >> 16) << 5;
+    if (!(before & 0x3ff00000u)) row.levels |= level_of(f, 2, r.z & 0x7fffu) << 10;
+    row.levels |= level_of(f, 0, r.y & 0x7fffu) << 15 | level_of(f, 1, r.y >> 16) << 20 | level_of(f, 2, r.z >> 16) << 25;
+    return row;
 }
 
-// Broad-phase filter of one pair in its bin: the bin is the first common cell (the OR of
-// the flags has all three bits), the quantized boxes overlap, and no node is shared.
-// Box overlap by guarded subtraction: with a guard bit over each 15-bit high value,
-// (hi | guard) - lo keeps the guard exactly when hi >= lo, two axes per word.
-__device__ __forceinline__ bool pair_test(const PairRec& A, const PairRec& B) {
-    const bool first = (A.id | B.id) >= 0xe0000000u;
-    const uint32_t d1 = B.w1 - A.w0, d2 = A.w1 - B.w0;
-    const uint32_t d3 = __byte_perm(B.w2, A.w2, 0x7632) - __byte_perm(A.w2, B.w2, 0x5410);
-    const bool box = (d1 & d2 & d3 & kGuard2) == kGuard2;
-    const bool share = A.n0 == B.n0 || A.n0 == B.n1 || A.n1 == B.n0 || A.n1 == B.n1;
-    return first && box && !share;
-}
-
-
-constexpr uint32_t kIdMask = (1u << kShapeBits) - 1u;
-
-// Appends every lane's hits to the flat candidate list: lane l's hits are the set bits of
-// `bits`, bit k standing for its pair with the record partner(k) returns; the lanes' counts
-// are placed by a warp scan behind one atomic on ncand.  Past cand_cap the pairs are counted
-// but not stored and kOverCandidates is raised.  All lanes of the warp call it.
-template <typename Partner>
-__device__ __forceinline__ void append_bits(uint32_t bits, uint32_t me, Partner partner, int lane,
-                                            long long cand_cap, uint2* __restrict__ cand,
-                                            uint32_t* __restrict__ ncand, uint32_t* __restrict__ flags) {
-    const uint32_t cnt = uint32_t(__popc(bits));
-    uint32_t incl = cnt;
+// Transposes a 32 x 32 bit matrix held one row per lane: afterwards bit j of lane k is bit k of
+// lane j's argument.
+__device__ __forceinline__ uint32_t transpose_bits(uint32_t x, int lane) {
+    uint32_t m = 0x0000ffffu;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += v;
+    for (int s = 16; s > 0; s >>= 1) {
+        const uint32_t y = __shfl_xor_sync(0xffffffffu, x, s);
+        x = (lane & s) ? (x & ~m) | ((y & ~m) >> s) : (x & m) | ((y & m) << s);
+        m ^= m << (s >> 1);
     }
-    const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-    if (total == 0) return;  // warp-uniform
-    uint32_t base = 0;
-    if (lane == 0) {
-        base = atomicAdd(ncand, total);
-        if ((long long)base + total > cand_cap) atomicOr(flags, uint32_t(kOverCandidates));
-    }
-    long long at = (long long)__shfl_sync(0xffffffffu, base, 0) + (incl - cnt);
-    while (bits) {
-        const int k = __ffs(bits) - 1;
-        bits &= bits - 1;
-        const uint32_t o = partner(k);
-        if (at < cand_cap) cand[at] = make_uint2(min(me, o), max(me, o));
-        at++;
-    }
+    return x;
 }
 
-// Every unordered pair of the records at ranks base .. base + m - 1 (m <= 32; lane i holds
-// rank base + i in `me`, and all of them are staged in shared memory), by rotation: in
-// round k lane i meets rank base + (i + k) mod m, k = 1 .. m/2 (the last round of an even m
-// only from the lower half), the partner's record read from shared memory.  Hits are kept as
-// one bit per round and appended at the end.
-__device__ __forceinline__ void rotate_pairs(const PairRec& me, const uint4* __restrict__ srec,
-                                             const int2* __restrict__ snd, int base, int m, int lane,
-                                             long long cand_cap, uint2* __restrict__ cand,
-                                             uint32_t* __restrict__ ncand, uint32_t* __restrict__ flags) {
-    const int half = m >> 1;
-    uint32_t bits = 0;
-    if (m == 32) {
-        // a full group (the common case): partners (lane + k) & 31, every lane active but in
-        // the last round, fully unrolled so that the hit bits' shifts are constants
+// A warp's shared memory: the staged groups' tables, levels and shapes (the last place holds the
+// shapes of a row group that is not staged), the queue of meeting boxes and the candidates on
+// their way to the list.
+constexpr int kPairOut = 64, kPairRound = 8;
+struct PairShared {
+    int4 shape[kPairGroups + 1][32];  // id, nodes
+    uint32_t below[kPairGroups][3][32], above[kPairGroups][3][32];
+    uint32_t levels[kPairGroups][32];
+    uint2 out[kPairOut];
+    uint16_t queue[32 * kPairRound + 32];  // row rank << 8 | column rank
+};
+
+// Pairs of meeting boxes come a few per lane and unevenly; queued, they are checked for a shared
+// node (three quarters of them share one in a cubic+BCC lattice) 32 at a time.  Candidates go on
+// to the flat list with one atomic and coalesced stores per flush; past cand_cap they are counted
+// but not stored and kOverCandidates is raised.
+struct PairQueue {
+    PairShared& s;
+    int nq, n;  // pairs queued, candidates held: the same in all lanes
+    long long cand_cap;
+    uint2* cand;
+    uint32_t *ncand, *flags;
+    __device__ __forceinline__ void flush(int lane) {
+        __syncwarp();
+        uint32_t base = 0;
+        if (lane == 0 && n) {
+            base = atomicAdd(ncand, uint32_t(n));
+            if ((long long)base + n > cand_cap) atomicOr(flags, uint32_t(kOverCandidates));
+        }
+        base = __shfl_sync(0xffffffffu, base, 0);
+        for (int i = lane; i < n; i += 32)
+            if ((long long)base + i < cand_cap) cand[(long long)base + i] = s.out[i];
+        n = 0;
+        __syncwarp();
+    }
+    // Checks the last min(32, nq) queued pairs.
+    __device__ __forceinline__ void check(int lane) {
+        const int m = min(32, nq);
+        nq -= m;
+        bool keep = false;
+        int4 p{}, q{};
+        if (lane < m) {
+            const uint32_t code = s.queue[nq + lane];
+            p = (&s.shape[0][0])[code >> 8];
+            q = (&s.shape[0][0])[code & 255u];
+            keep = p.y != q.y && p.y != q.z && p.z != q.y && p.z != q.z;
+        }
+        const unsigned k = __ballot_sync(0xffffffffu, keep);
+        if (keep) s.out[n + __popc(k & ((1u << lane) - 1u))] = make_uint2(min(uint32_t(p.x), uint32_t(q.x)), max(uint32_t(p.x), uint32_t(q.x)));
+        n += __popc(k);
+        if (n > kPairOut - 32) flush(lane);
+    }
+    // Bit j of `bits`: the row of rank `row` meets column 32 h + j.  All lanes call it.
+    __device__ __forceinline__ void add(uint32_t bits, uint32_t row, uint32_t h, int lane) {
+        const uint32_t code = row << 8 | h << 5;
+        while (__any_sync(0xffffffffu, bits != 0)) {
+            // up to kPairRound pairs per lane, placed by a warp scan
+            const int cnt = min(__popc(bits), kPairRound);
+            int incl = cnt;
 #pragma unroll
-        for (int k = 1; k <= 16; k++) {
-            const int src = base + ((lane + k) & 31);
-            const uint4 r = srec[src];
-            const int2 q = snd[src];
-            const PairRec o{r.x, r.y, r.z, r.w, q.x, q.y};
-            const bool hit = pair_test(me, o) && (k < 16 || lane < 16);
-            bits |= uint32_t(hit) << (k - 1);
-        }
-    } else {
-        int src = lane;
-        for (int k = 1; k <= half; k++) {
-            src = src + 1 < m ? src + 1 : 0;  // (lane + k) mod m for lanes below m
-            const uint4 r = srec[base + src];
-            const int2 q = snd[base + src];
-            const PairRec o{r.x, r.y, r.z, r.w, q.x, q.y};
-            const bool active = lane < m && !((m & 1) == 0 && k == half && lane >= half);
-            bits |= uint32_t(active && pair_test(me, o)) << (k - 1);
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += v;
+            }
+            uint16_t* at = s.queue + nq + (incl - cnt);
+            nq += __shfl_sync(0xffffffffu, incl, 31);
+            for (int k = 0; k < cnt; k++) {
+                at[k] = uint16_t(code | uint32_t(__ffs(bits) - 1));
+                bits &= bits - 1;
+            }
+            __syncwarp();
+            while (nq >= 32) check(lane);
+            __syncwarp();
         }
     }
-    append_bits(bits, me.id & kIdMask,
-                [&](int k) {
-                    int j = lane + k + 1;
-                    j = j >= m ? j - m : j;
-                    return srec[base + j].x & kIdMask;
-                },
-                lane, cand_cap, cand, ncand, flags);
+};
+
+// The row's box partners in group g whose first common cell is the bin.
+__device__ __forceinline__ uint32_t meet(const PairShared& s, int g, uint32_t levels) {
+    uint32_t hit = 0xffffffffu;
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+        const uint32_t lo = levels >> (5 * d) & 31u, hi = levels >> (15 + 5 * d) & 31u;
+        const uint32_t starts = lo ? 0xffffffffu : ~s.below[g][d][0];
+        hit &= s.below[g][d][hi] & s.above[g][d][lo] & starts;
+    }
+    return hit;
 }
 
-// Candidate pairs of every bin holding two or more shapes.  Warps claim the grid's bins
-// kPairGrab at a time (single bins near the end) from a cursor (flags[3]) and skip the empty
-// ones (one ballot), so bins of uneven size balance over the grid; they count the build's
-// cell entries and occupied bins on the way, clear the bin counters, and append their
-// candidate pairs (lower shape, higher shape) to the flat list in warp-sized batches, one
-// atomic on ncand per batch, without a counting pass.  The list's length is the number of
-// pairs, whatever the order.
-// Enumeration inside a bin, entries in bin order:
-//   n <= 128  the entries in groups of 32, lane i holding entry 32 g + i of group g and every
-//             record staged in shared memory: the pairs inside each group by rotation
-//             (rotate_pairs), then each full group against every record of the later groups
-//             (one record read by all lanes per round), hits kept as bits over windows of 32
-//             partners;
-//   larger    the same by groups of 32: each group is staged in turn and then meets every
-//             later group, staged 32 records at a time.
-__global__ void __launch_bounds__(kBlock, 6) k_bin_pairs(DevTopo t, const int* __restrict__ grid,
-                                                      uint32_t* __restrict__ bin_count, int bin_slots,
-                                                      uint32_t* __restrict__ counts,
-                                                      const uint32_t* __restrict__ bin_items,
-                                                      const uint4* __restrict__ rec, long long cand_cap,
-                                                      uint2* __restrict__ cand, uint32_t* __restrict__ flags) {
-    uint32_t* __restrict__ ncand = counts + kCand;
-    __shared__ uint4 rec_all[kPairWarps][kPairRanks];  // the bin's records, staged for the partner reads
-    __shared__ int2 nd_all[kPairWarps][kPairRanks];
+// Candidate pairs of every bin holding two or more shapes.  A unit of work is a chunk of
+// kPairGroups groups of 32 shapes of a bin: a warp stages the chunk's groups, and every group of
+// the bin up to the staged ones (those of earlier chunks reread) meets them, one 32 x 32 block
+// per step.  Warps claim units from a cursor (flags[3]), from the end of the list, where the later
+// chunks of large bins are (they take longest), so units of uneven size balance over the grid;
+// they count the build's cell entries and occupied bins on the way.
+// An integer kernel, bound by instruction issue: its time follows the staged groups, the blocks
+// and the meeting boxes.
+__global__ void __launch_bounds__(kPairThreads, 7) k_bin_pairs(DevTopo t, const int* __restrict__ grid,
+                                                               const uint32_t* __restrict__ bin_count, int bin_slots,
+                                                               uint32_t* __restrict__ counts,
+                                                               const uint2* __restrict__ unit_list,
+                                                               const uint32_t* __restrict__ bin_items,
+                                                               const uint4* __restrict__ rec, long long cand_cap,
+                                                               uint2* __restrict__ cand, uint32_t* __restrict__ flags) {
+    __shared__ PairShared shared[kPairWarps];
     if (!flags[1]) return;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const uint32_t nbins = uint32_t(grid[8]);
-    uint4* srec = rec_all[w];
-    int2* snd = nd_all[w];
-    uint32_t* cursor = flags + 3;
-    auto stage_rec = [&](const PairRec& r, int rank) {
-        srec[rank] = make_uint4(r.id, r.w0, r.w1, r.w2);
-        snd[rank] = make_int2(r.n0, r.n1);
-    };
+    const int lane = threadIdx.x & 31;
+    const uint32_t units = counts[kUnits];
+    PairShared& s = shared[threadIdx.x >> 5];
+    PairQueue out{s, 0, 0, cand_cap, cand, counts + kCand, flags};
+    const float quanta[3] = {kBoxQuanta / float(grid[3]), kBoxQuanta / float(grid[4]), kBoxQuanta / float(grid[5])};
+    BinFrame frame;
+#pragma unroll
+    for (int d = 0; d < 3; d++) frame.scale[d] = float((1 << kLevelBits) - 2) / quanta[d];
+    uint32_t mine[kLevelBits];  // the bits of the lane's number, expanded
+#pragma unroll
+    for (int k = 0; k < kLevelBits; k++) mine[k] = (lane >> k & 1) ? 0xffffffffu : 0u;
     uint32_t entries = 0, occupied = 0;  // this lane's share of the build's counts
-    // kPairGrab bins per claim, then single bins for the last 4 per warp of the grid, so that
-    // a few heavy bins do not end up queued behind one warp
-    const uint32_t tail = 4u * gridDim.x * kPairWarps;
-    const uint32_t single_from = nbins > tail ? nbins - tail : 0u;
-    uint32_t grab = kPairGrab;  // warp-uniform
+    // several units a claim while each warp of the grid still has many claims to come
+    const uint32_t warps = kPairWarps * gridDim.x, grab = units > 16 * warps ? 4u : units > 8 * warps ? 2u : 1u;
     for (;;) {
-        uint32_t b0 = 0;
-        if (lane == 0) b0 = atomicAdd(cursor, grab);
-        b0 = __shfl_sync(0xffffffffu, b0, 0);
-        if (b0 >= nbins) break;
-        const uint32_t cnt = lane < int(grab) && b0 + lane < nbins ? bin_count[b0 + lane] : 0u;
-        if (cnt) bin_count[b0 + lane] = 0;  // zero for the next build
-        if (b0 + grab >= single_from) grab = 1;
-        entries += cnt;
-        unsigned todo = __ballot_sync(0xffffffffu, cnt >= 2);  // the claimed bins holding pairs
-        occupied += lane == 0 ? uint32_t(__popc(todo)) : 0u;
+        uint32_t u0 = 0;
+        if (lane == 0) u0 = atomicAdd(flags + 3, grab);
+        u0 = __shfl_sync(0xffffffffu, u0, 0);
+        if (u0 >= units) break;
+        uint2 unit = make_uint2(0, 0);
+        uint32_t cnt = 0;
+        if (uint32_t(lane) < grab && u0 + lane < units) {
+            unit = unit_list[units - 1 - (u0 + lane)];
+            cnt = bin_count[unit.x];
+            if (unit.y == 0) {
+                entries += cnt;
+                occupied += cnt >= 2;
+            }
+        }
+        // a full bin repeats the build (kOverEntries), so clamping only keeps reads in bounds
+        cnt = min(cnt, uint32_t(bin_slots));
+        unsigned todo = __ballot_sync(0xffffffffu, cnt >= 2);
         while (todo) {
             const int j = __ffs(todo) - 1;
             todo &= todo - 1;
-            const uint32_t b = b0 + uint32_t(j);
-            // a full bin repeats the build (kOverEntries), so clamping only keeps reads in bounds
-            const int n = int(min(__shfl_sync(0xffffffffu, cnt, j), uint32_t(bin_slots)));
+            const uint32_t b = __shfl_sync(0xffffffffu, unit.x, j);
+            const int n = int(__shfl_sync(0xffffffffu, cnt, j));
+            const int g0 = kPairGroups * int(__shfl_sync(0xffffffffu, unit.y, j));  // first staged group
             const uint32_t* items = bin_items + size_t(b) * size_t(bin_slots);
             const int3 cc = cell_of(grid, b);
-            const uint32_t ccp = pack_cell(cc.x, cc.y, cc.z);
-            __syncwarp();  // the previous bin's partner reads are done
-            if (n <= kPairRanks) {
-                // ranks 32 g + lane in group g = 0 .. G-1, all staged in shared memory
-                const int G = (n + 31) >> 5;
-                for (int g = 0; g < G; g++)
-                    if (32 * g + lane < n) stage_rec(load_rec(t, items[32 * g + lane], rec, ccp), 32 * g + lane);
-                __syncwarp();
-                for (int g = 0; g < G; g++) {
-                    const int mg = min(32, n - 32 * g);
-                    PairRec me{};
-                    if (lane < mg) {
-                        const uint4 q = srec[32 * g + lane];
-                        const int2 nq = snd[32 * g + lane];
-                        me = PairRec{q.x, q.y, q.z, q.w, nq.x, nq.y};
-                    }
-                    rotate_pairs(me, srec, snd, 32 * g, mg, lane, cand_cap, cand, ncand, flags);  // within group g
-                    // group g (full: a later group exists) against the records of the later
-                    // groups, 32 partners per window of hit bits
-                    for (int r0 = 32 * (g + 1); r0 < n; r0 += 32) {
-                        const int rn = min(32, n - r0);
-                        uint32_t bits = 0;
-                        if (rn == 32) {  // a full window: constant shifts
+            frame.cell = pack_cell(cc.x, cc.y, cc.z);
+            frame.base[0] = float(cc.x) * quanta[0];
+            frame.base[1] = float(cc.y) * quanta[1];
+            frame.base[2] = float(cc.z) * quanta[2];
+            const int left = n - 32 * g0;  // shapes from the first staged one on
+            const int m = min((left + 31) >> 5, kPairGroups);
+            __syncwarp();  // the last reads of the staged groups are done
+            for (int g = 0; g < m; g++) {
+                PairRow row{0, 0, 0, 0};
+                if (32 * g + lane < left) row = load_row(t, items[32 * (g0 + g) + lane], rec, frame);
+                s.shape[g][lane] = make_int4(int(row.id), row.n0, row.n1, 0);
+                s.levels[g][lane] = row.levels;
+                const uint32_t plane = transpose_bits(row.levels, lane);
 #pragma unroll
-                            for (int k = 0; k < 32; k++) {
-                                const uint4 q = srec[r0 + k];
-                                const int2 nq = snd[r0 + k];
-                                const PairRec o{q.x, q.y, q.z, q.w, nq.x, nq.y};
-                                bits |= uint32_t(pair_test(me, o)) << k;
-                            }
-                        } else {
-#pragma unroll 4
-                            for (int k = 0; k < rn; k++) {
-                                const uint4 q = srec[r0 + k];
-                                const int2 nq = snd[r0 + k];
-                                const PairRec o{q.x, q.y, q.z, q.w, nq.x, nq.y};
-                                bits |= uint32_t(pair_test(me, o)) << k;
-                            }
-                        }
-                        append_bits(bits, me.id & kIdMask, [&](int k) { return srec[r0 + k].x & kIdMask; }, lane,
-                                    cand_cap, cand, ncand, flags);
+                for (int d = 0; d < 3; d++) {
+                    uint32_t le = 0xffffffffu, ge = 0xffffffffu;
+#pragma unroll
+                    for (int k = 0; k < kLevelBits; k++) {
+                        const uint32_t pl = __shfl_sync(0xffffffffu, plane, 5 * d + k);
+                        const uint32_t ph = __shfl_sync(0xffffffffu, plane, 15 + 5 * d + k);
+                        le = (mine[k] & ~pl) | (~(mine[k] ^ pl) & le);
+                        ge = (ph & ~mine[k]) | (~(ph ^ mine[k]) & ge);
                     }
+                    s.below[g][d][lane] = le;
+                    s.above[g][d][lane] = ge;
                 }
-            } else {
-                // large bin: its groups of 32 entries in turn.  Group g is staged in shared
-                // ranks 0..31 (lane i holding entry 32 g + i) and its pairs found by
-                // rotation; each later group is then staged in ranks 32..63 and met 32
-                // partners per window of hit bits.  A group with a later group is full, so
-                // every lane holds an entry there.
-                const int G = (n + 31) >> 5;
-                for (int g = 0; g < G; g++) {
-                    const int mg = min(32, n - 32 * g);
-                    __syncwarp();  // the previous group's partner reads are done
-                    if (lane < mg) stage_rec(load_rec(t, items[32 * g + lane], rec, ccp), lane);
-                    __syncwarp();
-                    PairRec me{};
-                    if (lane < mg) {
-                        const uint4 q = srec[lane];
-                        const int2 nq = snd[lane];
-                        me = PairRec{q.x, q.y, q.z, q.w, nq.x, nq.y};
-                    }
-                    rotate_pairs(me, srec, snd, 0, mg, lane, cand_cap, cand, ncand, flags);
-                    for (int h = g + 1; h < G; h++) {
-                        const int rn = min(32, n - 32 * h);
-                        __syncwarp();
-                        if (lane < rn) stage_rec(load_rec(t, items[32 * h + lane], rec, ccp), 32 + lane);
-                        __syncwarp();
-                        uint32_t bits = 0;
-#pragma unroll 4
-                        for (int k = 0; k < rn; k++) {
-                            const uint4 q = srec[32 + k];
-                            const int2 nq = snd[32 + k];
-                            const PairRec o{q.x, q.y, q.z, q.w, nq.x, nq.y};
-                            bits |= uint32_t(pair_test(me, o)) << k;
-                        }
-                        append_bits(bits, me.id & kIdMask, [&](int k) { return srec[32 + k].x & kIdMask; }, lane,
-                                    cand_cap, cand, ncand, flags);
-                    }
-                }
-                __syncwarp();
             }
+            __syncwarp();
+            for (int g = 0; g < m; g++) {
+                const uint32_t levels = s.levels[g][lane];
+                const bool valid = 32 * g + lane < left;
+                for (int h = g; h < m; h++) {
+                    uint32_t bits = meet(s, h, levels);
+                    if (left - 32 * h < 32) bits &= (1u << (left - 32 * h)) - 1u;
+                    if (h == g) bits &= ~1u << lane;  // each pair of a group once: j > lane
+                    out.add(valid ? bits : 0u, uint32_t(32 * g + lane), uint32_t(h), lane);
+                }
+            }
+            for (int g = 0; g < g0; g++) {  // groups (full) of earlier chunks
+                const PairRow row = load_row(t, items[32 * g + lane], rec, frame);
+                if (out.nq) out.check(lane);  // the queue refers to the row group replaced here
+                __syncwarp();
+                s.shape[kPairGroups][lane] = make_int4(int(row.id), row.n0, row.n1, 0);
+                __syncwarp();
+                for (int h = 0; h < m; h++) {
+                    uint32_t bits = meet(s, h, row.levels);
+                    if (left - 32 * h < 32) bits &= (1u << (left - 32 * h)) - 1u;
+                    out.add(bits, uint32_t(32 * kPairGroups + lane), uint32_t(h), lane);
+                }
+            }
+            if (out.nq) out.check(lane);  // the queue refers to the staged groups
         }
     }
+    out.flush(lane);
     entries = __reduce_add_sync(0xffffffffu, entries);
+    occupied = __reduce_add_sync(0xffffffffu, occupied);
     if (lane == 0) {
         if (entries) atomicAdd(counts + kEntries, entries);
         if (occupied) atomicAdd(counts + kOccupied, occupied);
     }
 }
-
-
 
 // Certified single-precision distance bounds of a candidate pair.  A pair certainly farther
 // apart than pad_a + pad_b (>= the reference's target ra + rb + margin) fails the reference's
@@ -681,8 +691,8 @@ __device__ __forceinline__ void append_batch(uint32_t keep, uint32_t* __restrict
 // of a segment whose endpoints move at most skin moves at most skin, so two segments close a gap
 // by at most 2 skin) and whose nodes are not connected (sim.cpp:24-39; local pairs never make
 // contact, so the narrow phase of every evaluation needs no hash lookups).
-// The kernel also ends the build: it stores the positions that later evaluations measure their
-// moves from, and the end of a forced rebuild.  A build that overflowed a buffer (bins, bin
+// The kernel also ends the build: it clears the bins, stores the positions that later evaluations
+// measure their moves from, and the end of a forced rebuild.  A build that overflowed a buffer (bins, bin
 // slots, cell span, candidates) left an incomplete list: the next evaluation must build again,
 // whatever the skin says, so that the overflow is raised again there (the overflow bits are per
 // evaluation; a caller that enqueues several evaluations before reading sees only the last one's).
@@ -691,6 +701,7 @@ __global__ void __launch_bounds__(kBlock) k_filter(DevTopo t, PhysParams p, cons
     if (!c.flags[1]) return;
     const long long thread = (long long)blockIdx.x * blockDim.x + threadIdx.x, threads = (long long)gridDim.x * blockDim.x;
     for (long long i = thread; i < t.N; i += threads) c.xref[i] = xf[i];
+    for (long long i = thread; i < c.grid[8]; i += threads) c.bin_count[i] = 0;  // for the next build
     if (thread == 0)
         c.flags[2] = (c.flags[0] & uint32_t(kOverEntries | kOverBins | kOverSpan | kOverCandidates)) ? 1u : 0u;
     const int lane = threadIdx.x & 31;
@@ -824,9 +835,13 @@ __global__ void __launch_bounds__(64) k_contacts(DevTopo t, PhysParams p, const 
 }  // namespace
 
 
+long long pair_units(long long bins, int slots) { return bins * ((slots + kChunk - 1) / kChunk); }
+
+// One unit of pair work per warp or so (a bin at the default cell holds about 100 shapes, each in
+// about three bins), and no more blocks than the GPU holds at a time.
 int contact_pair_blocks(long long shapes) {
-    const long long b = shapes / 256;
-    return int(b < 1 ? 1 : (b > 8 * 152 ? 8 * 152 : b));
+    const long long b = shapes / 128;
+    return int(b < 1 ? 1 : (b > 4 * 152 ? 4 * 152 : b));
 }
 
 void launch_contacts(const DevTopo& t, const PhysParams& p, const EvalBufs& e, ContactBufs& c, float skin,
@@ -835,7 +850,8 @@ void launch_contacts(const DevTopo& t, const PhysParams& p, const EvalBufs& e, C
     // candidate list (only when rebuilding)
     (k_shapes<<<grid_for((long long)t.N + t.B), kBlock, 0, s>>>(t, p, e.xf_lo, e.xf_hi, grow, c), note_launches(1));
     if (pairs_begin) cudaEventRecord(pairs_begin, s);
-    (k_bin_pairs<<<c.pair_blocks, kBlock, 0, s>>>(t, c.grid, c.bin_count, c.bin_slots, c.counts, c.bin_items, c.rec,
+    (k_bin_pairs<<<8 / kPairWarps * c.pair_blocks, kPairThreads, 0, s>>>(t, c.grid, c.bin_count, c.bin_slots, c.counts, c.units, c.bin_items,
+                                                           c.rec,
                                                 c.cand_cap, c.cand, c.flags),
      note_launches(1));
     if (pairs_end) cudaEventRecord(pairs_end, s);

@@ -312,7 +312,12 @@ struct mcg_ctx {
     double broad_cell = 0;   // current grid cell (the reference's size unless coarsened)
     float contact_skin = 0;  // candidate-list reuse distance (m); 0 rebuilds every evaluation
     int pair_blocks_set = 0; // blocks of the pair enumeration; 0: contact_pair_blocks(shapes)
-    double default_cell() const { return std::max(2.8 * jr, .72 * cfg.cell_size); }
+    double reference_cell() const { return std::max(2.8 * jr, .72 * cfg.cell_size); }
+    // The default grid cell, twice the reference's: a shape then lies in 2.8 cells instead of six,
+    // and the pair pass takes a bin's shapes 32 x 32 pairs at a time.  64x64x32 cubic+BCC, boxes and
+    // entries / pairs: 94 / 428 us at the reference's cell, 69 / 301 at 1.5 times, 53 / 225 at twice,
+    // 59 / 215 at 2.5 times; the densely compressed 32x32x16 lattice does not gain beyond that.
+    double default_cell() const { return 2 * reference_cell(); }
     int pair_blocks_for(long long shapes) const {
         return pair_blocks_set > 0 ? pair_blocks_set : contact_pair_blocks(shapes);
     }
@@ -339,6 +344,7 @@ struct mcg_ctx {
         c.bin_cap = bin_cap;
         c.bin_count = contact_mem.get<uint32_t>(size_t(bin_cap + 1));
         c.bin_items = contact_mem.get<uint32_t>(size_t(bin_cap) * size_t(slots));
+        c.units = contact_mem.get<uint2>(size_t(pair_units(bin_cap, slots)));
         c.pair_blocks = pair_blocks_for(S);
         c.cand_cap = std::max<long long>(1024, (cand_cap + 31) / 32 * 32);
         c.cand = contact_mem.get<uint2>(size_t(c.cand_cap));
@@ -370,10 +376,10 @@ struct mcg_ctx {
         c.energy_e0 = exponent(std::abs(cfg.contact_stiffness) * T * T);
     }
     // What the state and center kernels need to decide on a rebuild of cb's candidate list.
-    BuildArgs build_args(const ContactBufs& c, float skin) const {
+    BuildArgs build_args(const ContactBufs& c, float skin, double cell) const {
         if (!phys.self_contact) return BuildArgs{};
         return BuildArgs{c.xref, c.flags, c.counts, c.grid, rmax + cfg.contact_margin + double(skin > 0.f ? skin : 0.f),
-                         broad_cell, c.bin_cap, skin};
+                         cell, c.bin_cap, skin};
     }
 
     // Grows whatever the last evaluation overflowed; false when nothing did.
@@ -500,7 +506,7 @@ struct mcg_ctx {
         p.broad_cell = broad_cell;
         p.inv_cell_f = float(1.0 / broad_cell);
         mark(0);
-        const BuildArgs ba = build_args(cb, contact_skin);
+        const BuildArgs ba = build_args(cb, contact_skin, broad_cell);
         if (mixed) launch_state_mixed(topo, p, dz, d_baseX, mn, ba, ev, stream);
         else launch_state(topo, p, dz, d_baseX, d_baseR, ba, ev, stream);
         const ContactBufs* cptr = p.self_contact ? &cb : nullptr;
@@ -1438,7 +1444,7 @@ void upload_instances(mcg_ctx* c, const std::vector<InstIn>& ins) {
     P.contact_k = cf.contact_stiffness;
     P.contact_margin = cf.contact_margin;
     P.joint_radius = c->jr;
-    P.broad_cell = std::max(2.8 * c->jr, .72 * cf.cell_size);
+    P.broad_cell = c->default_cell();
     P.top = ih[0].geom.top0;
     P.self_contact = cf.self_contact ? 1 : 0;
     P.joint_padf = round_up_float(c->jr + cf.contact_margin);
@@ -1554,7 +1560,8 @@ void upload_instances(mcg_ctx* c, const std::vector<InstIn>& ins) {
         long long bin_cap = std::min(1LL << (3 * bits), 1LL << 27);
         // row-major bins when the Morton range does not fit or is mostly empty
         if ((1LL << bits) < dmax || bin_cap > 4 * dense) bin_cap = std::min(dense, 1LL << 28);
-        c->alloc_contacts(64, std::max<long long>(S / 2, 4096), bin_cap, std::max<long long>(4 * S, 4096));
+        // a cubic+BCC lattice's bins hold about 100 shapes at rest
+        c->alloc_contacts(256, std::max<long long>(S / 2, 4096), bin_cap, std::max<long long>(4 * S, 4096));
     }
     // solver vectors
     DevArena& Q = c->solver_mem;
@@ -1862,14 +1869,15 @@ int objective_with_fixed_contacts(mcg_ctx* c, ContactBufs& fixed, size_t zero_by
         c->upload_tops();
         c->set_active(std::vector<uint8_t>(1, 1));
         PhysParams p = c->phys;
-        p.broad_cell = c->broad_cell;
-        p.inv_cell_f = float(1.0 / c->broad_cell);
+        // its bins are few and small: the reference's cell unless another was set
+        p.broad_cell = c->broad_cell == c->default_cell() ? c->reference_cell() : c->broad_cell;
+        p.inv_cell_f = float(1.0 / p.broad_cell);
         if (p.self_contact) {
             // the scratch holds whatever its last user left: the state between evaluations
             c->set_sum_quanta(fixed);
             ck(cudaMemsetAsync(fixed.flags, 0, zero_bytes, s), "memset");
         }
-        const BuildArgs ba = c->build_args(fixed, 0.f);  // always rebuilds
+        const BuildArgs ba = c->build_args(fixed, 0.f, p.broad_cell);  // always rebuilds
         if (c->mixed) launch_state_mixed(c->topo, p, c->d_zin, c->d_baseX, c->mn, ba, c->ev, s);
         else launch_state(c->topo, p, c->d_zin, c->d_baseX, c->d_baseR, ba, c->ev, s);
         launch_center(c->topo, p, ba, c->ev, s);

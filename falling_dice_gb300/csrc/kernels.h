@@ -117,6 +117,8 @@ enum ContactFlag : uint32_t {
     kOverCandidates = 32 // more narrow-phase candidates than cand_cap
 };
 
+constexpr float kBoxQuanta = 32000.f;  // quantization steps of shape boxes across the contact grid's extent
+
 // Counters of the contact pipeline (ContactBufs::counts).
 enum ContactCount : int {
     kCand,        // candidates of the last build (may exceed cand_cap)
@@ -124,6 +126,7 @@ enum ContactCount : int {
     kEntries,     // its cell entries
     kLargestBin,  // its largest bin count above bin_slots (0 when every bin fitted)
     kOccupied,    // its bins holding two or more entries
+    kUnits,       // its units of pair work
     kContacts,    // contacts of the last evaluation (may exceed contact_cap)
     kContactCounts
 };
@@ -152,7 +155,7 @@ struct ContactBufs {
     uint32_t* flags;        // [5]: [0] ContactFlag bits of this evaluation, [1] candidate list
                             //      rebuilt by this evaluation, [2] rebuild forced (by the host,
                             //      or by a build that overflowed), [3] the pair pass's
-                            //      occupied-bin cursor, [4] builds since allocation.  [0] and
+                            //      cursor, [4] builds since allocation.  [0] and
                             //      [1] are zero between evaluations (cleared by the finalize)
     uint32_t* counts;       // [kContactCounts]
     float4* xref;           // [N] node positions (FP32, rounded down) when the list was built
@@ -162,6 +165,7 @@ struct ContactBufs {
     uint32_t* bin_count;    // [bin_cap+1] entries counted per bin (may exceed bin_slots); zero
                             //             between builds
     uint32_t* bin_items;    // [bin_cap * bin_slots]
+    uint2* units;           // [pair_units()] (bin, chunk of the bin's shapes) with an entry
     // narrow-phase candidates: one flat list, appended by the pair grid's warps in chunks
     int pair_blocks;        // blocks of the pair grid (8 warps each)
     long long cand_cap;     // candidate slots, a multiple of 32
@@ -297,6 +301,8 @@ void launch_plastic_stats(const DevTopo& t, const double* plastic, double* part,
 // ---- contact pipeline (contact.cu) ------------------------------------------------------
 // Blocks of the pair / narrow-phase grid for a model of `shapes` shapes (8 warps each).
 int contact_pair_blocks(long long shapes);
+// Units of pair work that `bins` bins of `slots` entries can hold.
+long long pair_units(long long bins, int slots);
 // The whole broad/narrow phase after the state and center kernels: bins, pairs and filtered
 // candidates (only when the list is rebuilt), contacts and their forces.
 // pairs_begin / pairs_end (may be null) are recorded around the pair enumeration.

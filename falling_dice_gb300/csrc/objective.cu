@@ -80,7 +80,6 @@ __global__ void __launch_bounds__(kEvalBlock) k_state(DevTopo t, PhysParams p, c
 // box ext = (min x, y, z, max x, y, z), by a whole block (thread d the axis d: the divisions are
 // the cost).  grid[]: 0-2 origin cell, 3-5 dims, 6 mode (0 Morton, 1 row-major), 7 valid, 8 number
 // of bins, 9 bins needed, 10-15 box quantization.
-constexpr float kBoxQuanta = 32000.f;  // box quantization steps across the grid extent
 __device__ void grid_params(const BuildArgs& b, const double* ext) {
     __shared__ long long dims[3];
     __shared__ int good[3];
@@ -185,7 +184,7 @@ __global__ void __launch_bounds__(kBlock) k_center(DevTopo t, double centering, 
             build.flags[1] = 1;
             build.flags[3] = 0;  // the pair pass's bin cursor
             build.flags[4]++;    // builds since the buffers were allocated
-            for (int k : {int(kCand), int(kKept), int(kEntries), int(kLargestBin), int(kOccupied)}) build.counts[k] = 0;
+            for (int k : {int(kCand), int(kKept), int(kEntries), int(kLargestBin), int(kOccupied), int(kUnits)}) build.counts[k] = 0;
         }
     }
     __syncthreads();

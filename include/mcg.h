@@ -300,19 +300,19 @@ int mcg_batch_run(mcg_ctx* ctx, mcg_frame* frames, int32_t capacity, int32_t* co
  * the default after mcg_upload_topology is cell_size / 32. */
 int mcg_set_contact_skin(mcg_ctx* ctx, double skin);
 
-/* Cell size of the self-contact grid in metres (no reference counterpart; 0: the
- * reference's max(2.8 joint radius, 0.72 cell_size)).  Pair sets and results do not depend
+/* Cell size of the self-contact grid in metres (no reference counterpart; 0: the default,
+ * twice the reference's max(2.8 joint radius, 0.72 cell_size)).  Pair sets and results do not depend
  * on it: a pair is examined once whatever the grid, and the narrow phase decides. */
 int mcg_set_contact_cell(mcg_ctx* ctx, double cell);
 
 /* Both broad-phase shapes at once, as mcg_autotune reports them (no reference counterpart):
- * the grid cell in metres (0: the reference's) and the blocks of the pair enumeration (0: a
+ * the grid cell in metres (0: the default) and the blocks of the pair enumeration (0: a
  * default from the lattice size), e.g. to re-apply a tuning without timing again. */
 int mcg_set_contact_shapes(mcg_ctx* ctx, double cell, int32_t pair_blocks);
 
 /* Shapes of the evaluation's kernels picked by measurement (no reference counterpart).
  * First the self-contact broad phase: grid cells 0.9, 1, 1.1, 1.25 and 1.4 times the
- * reference's max(2.8 joint radius, 0.72 cell_size), and pair-enumeration grids of 152 ..
+ * default (mcg_set_contact_cell), and pair-enumeration grids of 152 ..
  * 1216 blocks (at most one warp per 32 shapes) besides the default; then the occupancy of the
  * beam kernel (FP64: 1, 2 or 3 times 256 threads per SM; mixed: 3, 4, 5 or 6, and -3 or
  * -4 for the mixed kernel whose beam records arrive in shared memory by bulk copies, two

@@ -172,6 +172,12 @@ def write_summary_json(frames, cfg, mass_kg, path, material=abi.REFERENCE_MATERI
         raise MCGError(rc, f"cannot write {path}")
 
 
+def _frame_buffer(n):
+    """n uninitialised frames (the library writes the ones it reports; a run's capacity is tens of
+    megabytes for a batch, of which a few frames are used)."""
+    return (abi.Frame * n).from_buffer(np.empty(n * C.sizeof(abi.Frame), np.uint8))
+
+
 class Solver:
     """One device context holding one lattice: the reference Simulator's energy/gradient,
     minimize, commit and run, on the GPU."""
@@ -207,22 +213,22 @@ class Solver:
                                            _ptr(_f64(plastic))), "mcg_set_state")
 
     def get_state(self):
-        bx = np.zeros(3 * self.n_nodes)
-        br = np.zeros(4 * self.n_nodes)
-        pl = np.zeros(7 * self.n_beams)
+        bx = np.empty(3 * self.n_nodes)
+        br = np.empty(4 * self.n_nodes)
+        pl = np.empty(7 * self.n_beams)
         self._check(self.lib.mcg_get_state(self.h, _ptr(bx), _ptr(br), _ptr(pl)), "mcg_get_state")
         return bx, br, pl
 
     def objective(self, z, top, trials=False):
         z = _f64(z)
         e = C.c_double()
-        grad = np.zeros(6 * self.n_nodes)
+        grad = np.empty(6 * self.n_nodes)
         diag = abi.Diag()
         nxt = aux = flags = None
         if trials:
-            nxt = np.zeros(7 * self.n_beams)
-            aux = np.zeros(7 * self.n_beams)
-            flags = np.zeros(3 * self.n_beams, np.uint8)
+            nxt = np.empty(7 * self.n_beams)
+            aux = np.empty(7 * self.n_beams)
+            flags = np.empty(3 * self.n_beams, np.uint8)
         self._check(self.lib.mcg_objective(self.h, _ptr(z), top, int(trials), C.byref(e), _ptr(grad),
                                            C.byref(diag), _ptr(nxt), _ptr(aux), _ptr(flags, _u8)),
                     "mcg_objective")
@@ -239,7 +245,7 @@ class Solver:
 
     def read_result(self, grad=True):
         e = C.c_double()
-        g = np.zeros(6 * self.n_nodes) if grad else None
+        g = np.empty(6 * self.n_nodes) if grad else None
         diag = abi.Diag()
         self._check(self.lib.mcg_read_result(self.h, C.byref(e), _ptr(g), C.byref(diag)), "mcg_read_result")
         return {"energy": e.value, "grad": g, "diag": diag.as_dict()}
@@ -268,7 +274,7 @@ class Solver:
 
     def run(self, verbose=False):
         cap = self.cfg.load_steps + self.cfg.unload_steps + 1 + 4096
-        frames = (abi.Frame * cap)()
+        frames = _frame_buffer(cap)
         count = C.c_int32()
         rc = self.lib.mcg_run(self.h, frames, cap, C.byref(count), int(verbose))
         if rc not in (abi.MCG_OK, abi.MCG_ERR_EQUILIBRIUM):
@@ -403,7 +409,7 @@ class BatchSolver(Solver):
         z = _f64(z)
         tops = _f64(tops)
         e = np.zeros(self.count)
-        grad = np.zeros(6 * self.n_nodes)
+        grad = np.empty(6 * self.n_nodes)
         diags = (abi.Diag * self.count)()
         self._check(self.lib.mcg_batch_objective(self.h, _ptr(z), _ptr(tops), _ptr(e), _ptr(grad), diags),
                     "mcg_batch_objective")
@@ -411,7 +417,7 @@ class BatchSolver(Solver):
 
     def run(self, verbose=False):
         cap = self.cfg.load_steps + self.cfg.unload_steps + 1 + 4096
-        frames = (abi.Frame * (cap * self.count))()
+        frames = _frame_buffer(cap * self.count)
         counts = np.zeros(self.count, np.int32)
         status = np.zeros(self.count, np.int32)
         self._check(self.lib.mcg_batch_run(self.h, frames, cap, _ptr(counts, _i32), _ptr(status, _i32)),

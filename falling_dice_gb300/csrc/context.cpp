@@ -1724,11 +1724,8 @@ int mcg_set_state(mcg_ctx* c, const double* bx, const double* br, const double* 
         if (bx) h2d(c->d_baseX, bx, 3 * size_t(c->N), s);
         if (br) h2d(c->d_baseR, br, 4 * size_t(c->N), s);
         if (pl) {
-            const size_t B = size_t(c->B);
-            std::vector<double> soa(7 * B);
-            for (size_t b = 0; b < B; b++)
-                for (int k = 0; k < 7; k++) soa[size_t(k) * B + b] = pl[7 * b + size_t(k)];
-            h2d(c->d_plastic, soa.data(), soa.size(), s);
+            h2d(c->ev.slot, pl, 7 * size_t(c->B), s);  // the beams' slots are free between evaluations
+            launch_from_records7(c->B, c->ev.slot, c->d_plastic, s);
             if (c->mixed) launch_plastic_mixed(c->topo, nullptr, c->d_plastic, nullptr, c->mb, s);
             c->sync();
         }
@@ -1745,12 +1742,8 @@ int mcg_get_state(mcg_ctx* c, double* bx, double* br, double* pl) {
         if (bx) d2h(bx, c->d_baseX, 3 * size_t(c->N), s);
         if (br) d2h(br, c->d_baseR, 4 * size_t(c->N), s);
         if (pl) {
-            const size_t B = size_t(c->B);
-            std::vector<double> soa(7 * B);
-            d2h(soa.data(), c->d_plastic, soa.size(), s);
-            c->sync();
-            for (size_t b = 0; b < B; b++)
-                for (int k = 0; k < 7; k++) pl[7 * b + size_t(k)] = soa[size_t(k) * B + b];
+            launch_records7(c->B, c->d_plastic, c->ev.slot, s);
+            d2h(pl, c->ev.slot, 7 * size_t(c->B), s);
         }
         c->sync();
     });
@@ -1771,26 +1764,21 @@ int mcg_objective(mcg_ctx* c, const double* z, double top, int trials, double* e
         if (trials) c->have_final = false;
         if (energy) *energy = o.energy;
         fill_diag(diag, o);
-        if (trials && c->mixed) {
-            launch_f32_to_f64(7LL * c->B, c->ev.trial_nextf, c->ev.trial_next, s);
-            launch_f32_to_f64(7LL * c->B, c->ev.trial_auxf, c->ev.trial_aux, s);
-        }
-        if (trials && (trial_next || trial_aux || trial_flags)) {
-            std::vector<double> soa(7 * B);
-            auto aos = [&](const double* d, double* out) {
-                d2h(soa.data(), d, soa.size(), s);
-                c->sync();
-                for (size_t b = 0; b < B; b++)
-                    for (int k = 0; k < 7; k++) out[7 * b + size_t(k)] = soa[size_t(k) * B + b];
-            };
-            if (trial_next) aos(c->ev.trial_next, trial_next);
-            if (trial_aux) aos(c->ev.trial_aux, trial_aux);
+        if (trials) {  // in the ABI's layout, through the beams' slots (the gather has read them)
+            double* rec = c->ev.slot;
+            if (trial_next) {
+                if (c->mixed) launch_records7(c->B, c->ev.trial_nextf, rec, s);
+                else launch_records7(c->B, c->ev.trial_next, rec, s);
+                d2h(trial_next, rec, 7 * B, s);
+            }
+            if (trial_aux) {
+                if (c->mixed) launch_records7(c->B, c->ev.trial_auxf, rec, s);
+                else launch_records7(c->B, c->ev.trial_aux, rec, s);
+                d2h(trial_aux, rec, 7 * B, s);
+            }
             if (trial_flags) {
-                std::vector<uint8_t> f(3 * B);
-                d2h(f.data(), c->ev.trial_flags, f.size(), s);
-                c->sync();
-                for (size_t b = 0; b < B; b++)
-                    for (int k = 0; k < 3; k++) trial_flags[3 * b + size_t(k)] = f[size_t(k) * B + b];
+                launch_records3(c->B, c->ev.trial_flags, reinterpret_cast<uint8_t*>(rec), s);
+                d2h(trial_flags, reinterpret_cast<const uint8_t*>(rec), 3 * B, s);
             }
         }
         c->sync();

@@ -275,6 +275,11 @@ void launch_finalize(const DevTopo& t, const PhysParams& p, const ContactBufs* c
 void launch_commit(const DevTopo& t, const uint8_t* mask, const EvalBufs& e, double* base_x, double* base_r,
                    double* plastic, cudaStream_t s);
 void launch_center(const DevTopo& t, const PhysParams& p, const BuildArgs& b, EvalBufs& e, cudaStream_t s);
+// Per-beam arrays (7 values, 3 flags; structure of arrays) to and from consecutive values per beam.
+void launch_records7(long long B, const double* soa, double* aos, cudaStream_t s);
+void launch_records7(long long B, const float* soa, double* aos, cudaStream_t s);
+void launch_records3(long long B, const uint8_t* soa, uint8_t* aos, cudaStream_t s);
+void launch_from_records7(long long B, const double* aos, double* soa, cudaStream_t s);
 void launch_gather_mixed(const DevTopo& t, const PhysParams& p, const ContactBufs* c, double* grad, EvalBufs& e,
                          cudaStream_t s, int variant = 0);
 
@@ -293,7 +298,6 @@ void launch_plastic_mixed(const DevTopo& t, const uint8_t* mask, const double* p
                           MixedBeams& mb, cudaStream_t s);
 void launch_plastic_mixed_to_f64(const DevTopo& t, const uint8_t* mask, const MixedBeams& mb, double* plastic64,
                                  cudaStream_t s);
-void launch_f32_to_f64(long long n, const float* a, double* o, cudaStream_t s);
 // out6[6 i..]: per instance sum|epsp|, max|epsp|, sum|rotp|, max|rotp|, #|epsp|>1e-5, #|rotp|>1e-4
 // (part: 6 doubles per beam block)
 void launch_plastic_stats(const DevTopo& t, const double* plastic, double* part, double* out6, cudaStream_t s);

@@ -836,6 +836,23 @@ __global__ void __launch_bounds__(kBlock) k_plastic_final(DevTopo t, const doubl
     }
 }
 
+// ---- per-beam records in the ABI's layout ----------------------------------------------------
+// K values per beam: structure of arrays (device) <-> K consecutive values per beam (host), so
+// that a host array is one copy.  Thread i handles the i-th value of the written layout.
+template <int K, typename In, typename Out>
+__global__ void __launch_bounds__(kBlock) k_to_records(long long B, const In* __restrict__ soa, Out* __restrict__ aos) {
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < K * B; i += (long long)gridDim.x * blockDim.x) {
+        const long long b = i / K;
+        aos[i] = Out(soa[(i - K * b) * B + b]);
+    }
+}
+__global__ void __launch_bounds__(kBlock) k_from_records7(long long B, const double* __restrict__ aos, double* __restrict__ soa) {
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < 7 * B; i += (long long)gridDim.x * blockDim.x) {
+        const long long k = i / B;
+        soa[i] = aos[7 * (i - k * B) + k];
+    }
+}
+
 // ---- launchers ------------------------------------------------------------------------------
 void launch_state(const DevTopo& t, const PhysParams& p, const double* z, const double* base_x,
                   const double* base_r, const BuildArgs& b, EvalBufs& e, cudaStream_t s) {
@@ -863,6 +880,21 @@ void launch_plastic_stats(const DevTopo& t, const double* plastic, double* part,
     k_plastic_part<<<t.n_bblk, t.bdim, 0, s>>>(t, plastic, part);
     k_plastic_final<<<t.I, kBlock, 0, s>>>(t, part, out6);
     note_launches(2);
+}
+
+static unsigned record_grid(long long n) { return grid_for(n < 16 * 152 * kBlock ? n : 16 * 152 * kBlock); }
+
+void launch_records7(long long B, const double* soa, double* aos, cudaStream_t s) {
+    if (B) (k_to_records<7><<<record_grid(7 * B), kBlock, 0, s>>>(B, soa, aos), note_launches(1));
+}
+void launch_records7(long long B, const float* soa, double* aos, cudaStream_t s) {
+    if (B) (k_to_records<7><<<record_grid(7 * B), kBlock, 0, s>>>(B, soa, aos), note_launches(1));
+}
+void launch_records3(long long B, const uint8_t* soa, uint8_t* aos, cudaStream_t s) {
+    if (B) (k_to_records<3><<<record_grid(3 * B), kBlock, 0, s>>>(B, soa, aos), note_launches(1));
+}
+void launch_from_records7(long long B, const double* aos, double* soa, cudaStream_t s) {
+    if (B) (k_from_records7<<<record_grid(7 * B), kBlock, 0, s>>>(B, aos, soa), note_launches(1));
 }
 
 // Occupancy variants of the FP64 beam kernel (256-thread units per SM) and of the gather.

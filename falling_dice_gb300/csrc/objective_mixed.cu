@@ -612,10 +612,6 @@ __global__ void __launch_bounds__(kBlock) k_plastic_to_f64(DevTopo t, const uint
     soa7[b] = p.x; soa7[S + b] = p.y; soa7[2 * S + b] = r.x; soa7[3 * S + b] = r.y; soa7[4 * S + b] = r.z;
     soa7[5 * S + b] = p.z; soa7[6 * S + b] = p.w;
 }
-__global__ void k_f32_to_f64(long long n, const float* __restrict__ a, double* __restrict__ o) {
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        o[i] = a[i];
-}
 
 }  // namespace
 
@@ -697,12 +693,6 @@ void launch_plastic_mixed_to_f64(const DevTopo& t, const uint8_t* mask, const Mi
                                  cudaStream_t s) {
     if (!t.B) return;
     k_plastic_to_f64<<<t.n_bblk, kBlock, 0, s>>>(t, mask, mb.P0, mb.P1, plastic64);
-    note_launches(1);
-}
-
-void launch_f32_to_f64(long long n, const float* a, double* o, cudaStream_t s) {
-    if (n <= 0) return;
-    k_f32_to_f64<<<grid_for(n < 152 * 8 * kBlock ? n : 152 * 8 * kBlock), kBlock, 0, s>>>(n, a, o);
     note_launches(1);
 }
 

@@ -207,8 +207,14 @@ struct mcg_ctx {
     int H = 0;
     double *d_z = nullptr, *d_zeval = nullptr, *d_p = nullptr, *d_g = nullptr, *d_geval = nullptr,
            *d_best = nullptr, *d_zfinal = nullptr, *d_S = nullptr, *d_Y = nullptr;
-    double *d_rho = nullptr, *d_alpha = nullptr, *d_part = nullptr, *d_dg = nullptr, *d_dots3 = nullptr,
-           *d_pstats = nullptr;
+    double *d_rho = nullptr, *d_alpha = nullptr, *d_coef = nullptr, *d_gram = nullptr, *d_part = nullptr,
+           *d_dg = nullptr, *d_h0 = nullptr, *d_pstats = nullptr;
+    unsigned* d_done = nullptr;
+    LbfgsBufs lbfgs() const {
+        return LbfgsBufs{d_z, d_best, d_zeval, d_zfinal, d_p, d_g, d_S, d_Y, d_geval, 6LL * N, std::max(H, 1), d_hist, d_rho,
+                         d_gram, d_alpha, d_coef, d_h0, d_dg, d_part, d_done,
+                         cfg.max_translation_step / cfg.translation_scale, cfg.max_rotation_step};
+    }
     SolveCtl* d_ctl = nullptr;
     int2* d_hist = nullptr;       // per instance: history pairs held, oldest slot
     uint8_t* d_mask = nullptr;
@@ -226,7 +232,6 @@ struct mcg_ctx {
         sync();  // the host vector may change before the copy runs
     }
     std::vector<Minimizer> mins;
-    std::vector<uint8_t> fused;  // the instance's direction is computed by one CTA
     bool have_final = false;  // instance 0 has a final state from minimize, not yet committed
 
     // ---- the device-resident round loop ------------------------------------------------
@@ -236,7 +241,6 @@ struct mcg_ctx {
     // synchronising after every round.  Off while timing phases (direct launches) or when
     // the graph cannot be built (loop_error says why); the host-stepped rounds then run.
     Minimizer* d_mins = nullptr;
-    uint8_t* d_fused = nullptr;
     uint8_t* d_trial = nullptr;   // per-instance trial mask of the loop's evaluations
     MzStatus* d_mz = nullptr;
     cudaGraphExec_t loop_exec = nullptr;
@@ -635,27 +639,24 @@ struct mcg_ctx {
     // device (sim.cpp:191, 205-206); the host reads back once per round: the evaluation's
     // totals and each instance's dg.  False when no instance had work.
     bool minimize_round() {
-        const double mt = cfg.max_translation_step / cfg.translation_scale, mr = cfg.max_rotation_step;
         const MzParams P = mz_params();
+        const LbfgsBufs L = lbfgs();
         // A. search directions: two-loop (sim.cpp:184-190), or steepest descent for the retry
         //    after a failed line search (:193-196)
-        bool any_dir = false, any_multi = false, any_sd = false;
+        bool any_dir = false, any_sd = false;
         clear_ctl(0);
         SolveCtl* ca = ctl_stage(0);
         for (int i = 0; i < I; i++) {
-            const int f = mz_stage_direction(mins[size_t(i)], fused[size_t(i)] != 0);
+            const int f = mz_stage_direction(mins[size_t(i)]);
             ca[i].flags = f;
-            any_dir |= f == kOpDirFused || f == kOpDirection;
-            any_multi |= f == kOpDirection;
+            any_dir |= f == kOpDirection;
             any_sd |= f == kOpSteepest;
         }
         if (any_dir || any_sd) {
             upload_ctl(0);
-            replay(1 | (any_dir ? 2 : 0) | (any_multi ? 4 : 0) | (any_sd ? 8 : 0), [&] {
-                if (any_dir)
-                    bl_direction(topo, d_ctl, d_hist, std::max(H, 1), any_multi, d_p, d_g, d_S, d_Y, 6LL * N, d_rho,
-                                 d_alpha, d_part, d_dg, mt, mr, stream);
-                if (any_sd) bl_steepest(topo, d_ctl, d_hist, d_p, d_g, d_part, d_dg, mt, mr, stream);
+            replay(1 | (any_dir ? 2 : 0) | (any_sd ? 4 : 0), [&] {
+                if (any_dir) bl_direction(topo, d_ctl, L, stream);
+                if (any_sd) bl_steepest(topo, d_ctl, L, stream);
             });
         }
         // B. one evaluation per instance: the start point, a line-search candidate
@@ -680,7 +681,7 @@ struct mcg_ctx {
         set_active(a);
         upload_ctl(1);
         upload_tops();
-        replay(16, [&] { bl_prepare(topo, d_ctl, d_hist, d_z, d_best, d_zeval, d_p, d_zfinal, stream); });
+        replay(16, [&] { bl_prepare(topo, d_ctl, L, stream); });
         d2h(hp.dg, d_dg, size_t(I), stream);  // read back with the evaluation's totals
         const EvalOut* out = eval_read(d_zeval, trials, d_geval);
         // C. decisions (the reference's, per instance) and the vectors they imply
@@ -694,10 +695,7 @@ struct mcg_ctx {
         }
         if (any_post) {
             upload_ctl(2);
-            replay(32, [&] {
-                bl_accept(topo, d_ctl, d_hist, H, d_z, d_g, d_zeval, d_geval, d_S, d_Y, 6LL * N, d_best, d_rho,
-                          d_part, d_dots3, stream);
-            });
+            replay(32, [&] { bl_accept(topo, d_ctl, L, stream); });
         }
         check_launch();
         return true;
@@ -734,7 +732,6 @@ struct mcg_ctx {
         MzDev d{};
         d.I = I;
         d.mins = d_mins;
-        d.fused = d_fused;
         d.ctl = d_ctl;
         d.active = d_active;
         d.trial_inst = d_trial;
@@ -747,13 +744,12 @@ struct mcg_ctx {
         return d;
     }
 
-    // The round loop as one graph: WHILE(loop) { A; IF(fused) one-CTA directions;
-    // IF(multi) two-loop; IF(any direction) descent fix; IF(steepest) retry; B; prepare;
-    // evaluation (trial states per instance); C; IF(accept) accept step }.
+    // The round loop as one graph: WHILE(loop) { A; IF(any direction) directions; IF(steepest)
+    // retry; B; prepare; evaluation (trial states per instance); C; IF(accept) accept step }.
     void build_loop() {
         make_fork();
         if (!side) ck(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking), "cudaStreamCreate");
-        const double mt = cfg.max_translation_step / cfg.translation_scale, mr = cfg.max_rotation_step;
+        const LbfgsBufs L = lbfgs();
         const MzDev md = mz_dev();
         const MzParams P = mz_params();
         cudaGraph_t g = nullptr;
@@ -769,36 +765,21 @@ struct mcg_ctx {
             cudaGraphNode_t wnode;
             ck(cudaGraphAddNode(&wnode, g, nullptr, nullptr, 0, &wp), "cudaGraphAddNode (WHILE)");
             cudaGraph_t body = wp.conditional.phGraph_out[0];
-            cudaGraphConditionalHandle hf, hm, hd, hs, hpost;
-            for (cudaGraphConditionalHandle* h : {&hf, &hm, &hd, &hs, &hpost})
+            cudaGraphConditionalHandle hd, hs, hpost;
+            for (cudaGraphConditionalHandle* h : {&hd, &hs, &hpost})
                 ck(cudaGraphConditionalHandleCreate(h, body, 0, cudaGraphCondAssignDefault), "conditional handle");
             const long long before = g_launch_count.load();
             ck(cudaStreamBeginCaptureToGraph(stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal),
                "cudaStreamBeginCaptureToGraph");
             try {
-                const int Hs = std::max(H, 1);
-                launch_mz_direction(md, hf, hm, hd, hs, stream);
-                capture_if(hf, [&](cudaStream_t s2) {
-                    bl_direction_fused(topo, d_ctl, d_hist, Hs, d_p, d_g, d_S, d_Y, 6LL * N, d_rho, d_dg, mt, mr, s2);
-                });
-                capture_if(hm, [&](cudaStream_t s2) {
-                    bl_direction_multi(topo, d_ctl, d_hist, Hs, d_p, d_g, d_S, d_Y, 6LL * N, d_rho, d_alpha, d_part,
-                                       d_dg, mt, mr, s2);
-                });
-                capture_if(hd, [&](cudaStream_t s2) {
-                    bl_descent_fix(topo, d_ctl, d_hist, d_p, d_g, d_part, d_dg, mt, mr, s2);
-                });
-                capture_if(hs, [&](cudaStream_t s2) {
-                    bl_steepest(topo, d_ctl, d_hist, d_p, d_g, d_part, d_dg, mt, mr, s2);
-                });
+                launch_mz_direction(md, hd, hs, stream);
+                capture_if(hd, [&](cudaStream_t s2) { bl_direction(topo, d_ctl, L, s2); });
+                capture_if(hs, [&](cudaStream_t s2) { bl_steepest(topo, d_ctl, L, s2); });
                 launch_mz_eval(md, stream);
-                bl_prepare(topo, d_ctl, d_hist, d_z, d_best, d_zeval, d_p, d_zfinal, stream);
+                bl_prepare(topo, d_ctl, L, stream);
                 eval_launches(d_zeval, 2, d_geval, true);
                 launch_mz_decide(md, P, hpost, h_loop, stream);
-                capture_if(hpost, [&](cudaStream_t s2) {
-                    bl_accept(topo, d_ctl, d_hist, H, d_z, d_g, d_zeval, d_geval, d_S, d_Y, 6LL * N, d_best, d_rho,
-                              d_part, d_dots3, s2);
-                });
+                capture_if(hpost, [&](cudaStream_t s2) { bl_accept(topo, d_ctl, L, s2); });
             } catch (...) {
                 cudaGraph_t junk = nullptr;
                 cudaStreamEndCapture(stream, &junk);
@@ -1248,22 +1229,18 @@ void upload_instances(mcg_ctx* c, const std::vector<InstIn>& ins) {
         }
     // blocks that never straddle two instances
     const int bdim = cf.precision == MCG_MIXED ? kMapBlock : kBeamBlock;
-    std::vector<int4> nblk, bblk, eblk, irange(static_cast<size_t>(I));
-    std::vector<int2> erange(static_cast<size_t>(I));
+    std::vector<int4> bblk, eblk, sblk;
+    std::vector<int2> brange, erange, srange;
+    auto add_blocks = [](std::vector<int4>& blk, std::vector<int2>& range, int first, int count, int size, int k) {
+        const int b0 = int(blk.size());
+        for (int f = 0; f < count; f += size) blk.push_back(make_int4(first + f, std::min(size, count - f), k, 0));
+        range.push_back(make_int2(b0, int(blk.size())));
+    };
     for (int k = 0; k < I; k++) {
         const InstHost& h = ih[size_t(k)];
-        irange[size_t(k)].x = int(nblk.size());
-        for (int f = 0; f < h.N; f += kMapBlock)
-            nblk.push_back(make_int4(h.node0 + f, std::min(kMapBlock, h.N - f), k, 0));
-        irange[size_t(k)].y = int(nblk.size());
-        irange[size_t(k)].z = int(bblk.size());
-        for (int f = 0; f < h.B; f += bdim)
-            bblk.push_back(make_int4(h.beam0 + f, std::min(bdim, h.B - f), k, 0));
-        irange[size_t(k)].w = int(bblk.size());
-        erange[size_t(k)].x = int(eblk.size());
-        for (int f = 0; f < h.N; f += kEvalBlock)
-            eblk.push_back(make_int4(h.node0 + f, std::min(kEvalBlock, h.N - f), k, 0));
-        erange[size_t(k)].y = int(eblk.size());
+        add_blocks(bblk, brange, h.beam0, h.B, bdim, k);
+        add_blocks(eblk, erange, h.node0, h.N, kEvalBlock, k);
+        add_blocks(sblk, srange, h.node0, h.N, solve_block_nodes(h.N), k);
     }
     // contact-grid offsets: the instances' footprints (x-z extent with room to widen under
     // compression) packed in rows, so that the shared grid stays small; offsets are
@@ -1370,26 +1347,27 @@ void upload_instances(mcg_ctx* c, const std::vector<InstIn>& ins) {
         T.padf = dp;
     }
     T.I = I;
-    T.n_nblk = int(nblk.size());
     T.n_bblk = int(bblk.size());
     T.bdim = bdim;
     T.n_eblk = int(eblk.size());
+    T.n_sblk = int(sblk.size());
     {
-        int4* d = M.get<int4>(nblk.size());
-        h2d(d, nblk.data(), nblk.size(), s);
-        T.nblk = d;
-        int4* e = M.get<int4>(bblk.size());
-        h2d(e, bblk.data(), bblk.size(), s);
-        T.bblk = e;
-        int4* r = M.get<int4>(irange.size());
-        h2d(r, irange.data(), irange.size(), s);
-        T.irange = r;
-        int4* eb = M.get<int4>(eblk.size());
-        h2d(eb, eblk.data(), eblk.size(), s);
-        T.eblk = eb;
-        int2* er = M.get<int2>(erange.size());
-        h2d(er, erange.data(), erange.size(), s);
-        T.erange = er;
+        auto up4 = [&](const std::vector<int4>& v) {
+            int4* d = M.get<int4>(v.size());
+            h2d(d, v.data(), v.size(), s);
+            return static_cast<const int4*>(d);
+        };
+        auto up2 = [&](const std::vector<int2>& v) {
+            int2* d = M.get<int2>(v.size());
+            h2d(d, v.data(), v.size(), s);
+            return static_cast<const int2*>(d);
+        };
+        T.bblk = up4(bblk);
+        T.eblk = up4(eblk);
+        T.sblk = up4(sblk);
+        T.brange = up2(brange);
+        T.erange = up2(erange);
+        T.srange = up2(srange);
         std::vector<int> nn(static_cast<size_t>(I));
         std::vector<long long> nf(static_cast<size_t>(I));
         std::vector<float2> off(static_cast<size_t>(I));
@@ -1574,9 +1552,13 @@ void upload_instances(mcg_ctx* c, const std::vector<InstIn>& ins) {
     c->d_Y = Q.get<double>(size_t(Hs) * n);
     c->d_rho = Q.get<double>(size_t(I) * Hs);
     c->d_alpha = Q.get<double>(size_t(I) * Hs);
-    c->d_part = Q.get<double>(std::max(lbfgs_part_doubles(std::max(T.n_nblk, T.n_bblk)), 6 * size_t(T.n_bblk) + 8));
+    c->d_coef = Q.get<double>(size_t(I) * Hs);
+    c->d_gram = Q.get<double>(size_t(I) * Hs * Hs);
+    c->d_done = Q.get<unsigned>(4 * size_t(I));
+    ck(cudaMemsetAsync(c->d_done, 0, 4 * size_t(I) * sizeof(unsigned), s), "memset");
+    c->d_part = Q.get<double>(std::max(lbfgs_part_doubles(T.n_sblk, Hs), 6 * size_t(T.n_bblk) + 8));
     c->d_dg = Q.get<double>(size_t(I));
-    c->d_dots3 = Q.get<double>(3 * size_t(I));
+    c->d_h0 = Q.get<double>(size_t(I));
     c->d_pstats = Q.get<double>(6 * size_t(I));
     c->d_ctl = Q.get<SolveCtl>(size_t(I));
     c->d_hist = Q.get<int2>(size_t(I));
@@ -1584,16 +1566,8 @@ void upload_instances(mcg_ctx* c, const std::vector<InstIn>& ins) {
     ck(cudaMemsetAsync(c->d_rho, 0, size_t(I) * Hs * sizeof(double), s), "memset");
     c->d_mask = Q.get<uint8_t>(size_t(I));
     c->mins.assign(size_t(I), Minimizer{});
-    c->fused.assign(size_t(I), 0);
-    for (int k = 0; k < I; k++) {
-        const int4 r = irange[size_t(k)];
-        c->fused[size_t(k)] = r.y - r.x <= fused_direction_limit() && c->H <= 64;
-    }
     c->d_mins = Q.get<Minimizer>(size_t(I));
     c->d_mz = Q.get<MzStatus>(1);
-    c->d_fused = Q.get<uint8_t>(size_t(I));
-    h2d(c->d_fused, c->fused.data(), size_t(I), s);
-
     ck(cudaMemsetAsync(c->d_z, 0, n * sizeof(double), s), "memset");
     if (c->mixed) {
         prepare_beams_mixed(c->device);
@@ -2118,6 +2092,22 @@ int mcg_autotune(mcg_ctx* c, const double* z, const double* tops, int32_t reps, 
         cudaEvent_t t0 = nullptr, t1 = nullptr;
         ck(cudaEventCreate(&t0), "cudaEventCreate");
         ck(cudaEventCreate(&t1), "cudaEventCreate");
+        // ms per evaluation, the best of three batches of reps (a small lattice's evaluation takes
+        // tens of microseconds: one disturbed batch would decide)
+        auto time_evals = [&] {
+            c->eval(c->d_zin, false, c->d_grad);  // captures the graph
+            double best = 1e300;
+            for (int batch = 0; batch < 3; batch++) {
+                ck(cudaEventRecord(t0, s), "cudaEventRecord");
+                for (int r = 0; r < reps; r++) c->eval(c->d_zin, false, c->d_grad);
+                ck(cudaEventRecord(t1, s), "cudaEventRecord");
+                c->read_outs();
+                float ms = 0;
+                ck(cudaEventElapsedTime(&ms, t0, t1), "cudaEventElapsedTime");
+                best = std::min(best, double(ms) / reps);
+            }
+            return best;
+        };
         struct Pick { double cell; int blocks; double ms; };
         std::vector<Pick> timed;
         double ms_default = 0;
@@ -2139,15 +2129,8 @@ int mcg_autotune(mcg_ctx* c, const double* z, const double* tops, int32_t reps, 
                                std::memcmp(g.data(), ref_g.data(), n * sizeof(double)) != 0) {
                         throw Fail(MCG_ERR_MISMATCH, "broad-phase shapes changed an evaluation");
                     }
-                    c->eval(c->d_zin, false, c->d_grad);  // captures the graph
-                    ck(cudaEventRecord(t0, s), "cudaEventRecord");
-                    for (int r = 0; r < reps; r++) c->eval(c->d_zin, false, c->d_grad);
-                    ck(cudaEventRecord(t1, s), "cudaEventRecord");
-                    c->read_outs();
+                    const double per = time_evals();
                     if (c->hp.outs[0].overflow) throw Fail(MCG_ERR_CAPACITY, "contact buffers overflowed in tuning");
-                    float ms = 0;
-                    ck(cudaEventElapsedTime(&ms, t0, t1), "cudaEventElapsedTime");
-                    const double per = double(ms) / reps;
                     if (tried == 0) ms_default = per;
                     tried++;
                     timed.push_back(Pick{c->broad_cell, c->pair_blocks_for(S), per});
@@ -2225,14 +2208,7 @@ int mcg_autotune(mcg_ctx* c, const double* z, const double* tops, int32_t reps, 
             }
             c->set_kernel_variants(bv, gv);
             // the whole evaluation with the chosen shapes
-            c->eval(c->d_zin, false, c->d_grad);  // captures the graph
-            ck(cudaEventRecord(t0, s), "cudaEventRecord");
-            for (int r = 0; r < reps; r++) c->eval(c->d_zin, false, c->d_grad);
-            ck(cudaEventRecord(t1, s), "cudaEventRecord");
-            c->read_outs();
-            float ms = 0;
-            ck(cudaEventElapsedTime(&ms, t0, t1), "cudaEventElapsedTime");
-            best_ms = double(ms) / reps;
+            best_ms = std::min(best_ms, time_evals());
         } catch (...) {
             cudaEventDestroy(t0);
             cudaEventDestroy(t1);

@@ -51,14 +51,16 @@ struct DevTopo {
     // so every block partial belongs to one instance and per-instance totals are sums over
     // an instance's own blocks, in the same order as for that lattice alone.
     int I;
-    int n_nblk, n_bblk;       // node blocks, beam blocks
-    const int4* nblk;         // [n_nblk] first node, node count, instance, 0
+    int n_bblk;               // beam blocks
     const int4* bblk;         // [n_bblk] first beam, beam count, instance, 0
     int bdim;                 // beams per beam block: kBeamBlock (FP64) or kMapBlock (mixed)
-    const int4* irange;       // [I] node blocks [x, y), beam blocks [z, w) of the instance
+    const int2* brange;       // [I] beam blocks [x, y) of the instance
     int n_eblk;               // evaluation node blocks
     const int4* eblk;         // [n_eblk] first node, node count, instance, 0
     const int2* erange;       // [I] evaluation node blocks [x, y) of the instance
+    int n_sblk;               // solver blocks: at most kSolveBlocks runs of nodes per instance
+    const int4* sblk;         // [n_sblk] first node, node count, instance, 0
+    const int2* srange;       // [I] solver blocks [x, y) of the instance
     const int* inst_n;        // [I] nodes of the instance
     const long long* inst_free;  // [I] unlocked DOFs of the instance
     const float2* off;        // [I] (x, z) offset of the instance in the contact grid
@@ -67,12 +69,14 @@ struct DevTopo {
     const uint8_t* trial_inst;  // [I] with trials == 2: 1 where the instance writes its trial states
 };
 
-// Elements per mapped block (the launch block size of the mapped kernels): node blocks, and the
-// beam blocks of the mixed form; the FP64 form's beam blocks (one warp per FP64 unit of an SM).
+// Elements per mapped block (the launch block size of the mapped kernels): the beam blocks of the
+// mixed form; the FP64 form's beam blocks (one warp per FP64 unit of an SM).
 constexpr int kMapBlock = 256;
 constexpr int kBeamBlock = 128;
-// Nodes per evaluation node block (state and gather; the solver's vectors use kMapBlock).
+// Nodes per evaluation node block (state and gather).
 constexpr int kEvalBlock = 128;
+// Solver blocks an instance's vectors are divided into at most: one per SM.
+constexpr int kSolveBlocks = 152;
 
 #if defined(__CUDACC__)
 // Position of a thread of a mapped block: element index, instance; valid == false past the
@@ -328,8 +332,7 @@ enum SolveOp : int {
     kOpAccept = 512,       // s, y, curvature dots, z = zeval, g = geval
     kOpPair = 1024,        // with kOpAccept: store (s, y) in history slot `target`
     kOpKeepBestAfter = 2048, // with kOpAccept: best = the accepted z
-    kOpDirFused = 4096,      // as kOpDirection, by one CTA for the instance (small instances)
-    kOpResetHistory = 8192   // the history starts empty (a new minimization)
+    kOpResetHistory = 4096   // the history starts empty (a new minimization)
 };
 // Per-instance solver control, written by the host before each step.  The history state
 // (pairs held m, oldest slot head) lives on the device (int2 per instance) and is filled in
@@ -340,38 +343,36 @@ struct SolveCtl {
     int m, head;       // (device history, loaded by the kernels)
     int pad_;
 };
-size_t lbfgs_part_doubles(int n_nblk);
-// Largest instance (in node blocks) whose direction one CTA computes (kOpDirFused).
-int fused_direction_limit();
-// Two-loop recursion (sim.cpp:184-187) into p for the kOpDirFused (one CTA each) and, with
-// multi, the kOpDirection instances; then p = clamp(lock(-p)) and dg[i] = <g, p>; where
-// not dg < 0, steepest descent with the history cleared (sim.cpp:191).
-// History: H slots of `stride` doubles, state hist[I], rho and alpha [I * H].
-void bl_direction(const DevTopo& t, const SolveCtl* ctl, int2* hist, int H, bool multi, double* p, const double* g,
-                  const double* S, const double* Y, long long stride, const double* rho, double* alpha, double* part,
-                  double* dg, double mt, double mr, cudaStream_t s);
-// The pieces of bl_direction, for callers that launch them under separate conditions: the
-// one-CTA directions (kOpDirFused), the multi-block two-loop (kOpDirection), and the
-// steepest-descent fallback of either kind where <g, p> >= 0.
-void bl_direction_fused(const DevTopo& t, const SolveCtl* ctl, int2* hist, int H, double* p, const double* g,
-                        const double* S, const double* Y, long long stride, const double* rho, double* dg, double mt,
-                        double mr, cudaStream_t s);
-void bl_direction_multi(const DevTopo& t, const SolveCtl* ctl, int2* hist, int H, double* p, const double* g,
-                        const double* S, const double* Y, long long stride, const double* rho, double* alpha,
-                        double* part, double* dg, double mt, double mr, cudaStream_t s);
-void bl_descent_fix(const DevTopo& t, const SolveCtl* ctl, int2* hist, double* p, const double* g, double* part,
-                    double* dg, double mt, double mr, cudaStream_t s);
+// The solver's vectors and scalars on the device: history H slots of `stride` doubles.
+struct LbfgsBufs {
+    double *z, *best, *zeval, *zfinal, *p, *g, *S, *Y;
+    const double* geval;
+    long long stride;
+    int H;               // history slots (at least 1)
+    int2* hist;          // [I] history pairs held, oldest slot
+    double* rho;         // [I H] 1 / <s, y> per slot
+    double* gram;        // [I H H] <s_i, y_j> at [slot i][slot j], pair i not newer than j
+    double *alpha, *coef;  // [I H] the two loops' coefficients, oldest pair first
+    double* h0;          // [I] initial scale of the newest pair: clamp(s.y / y.y, 1e-7, 1e4), else 0.1
+    double* dg;          // [I] <g, p>
+    double* part;        // [lbfgs_part_doubles] block partials
+    unsigned* done;      // [4 I] blocks that have arrived, per pass; zero between passes
+    double mt, mr;       // largest translation (in units of the scale) and rotation of a step
+};
+size_t lbfgs_part_doubles(int n_sblk, int H);
+// Nodes per solver block of an instance of n nodes.
+int solve_block_nodes(int n);
+// Two-loop recursion (sim.cpp:184-187) into p for the kOpDirection instances; then
+// p = clamp(lock(-p)) and dg = <g, p>; where not dg < 0, steepest descent with the history
+// cleared (sim.cpp:191).
+void bl_direction(const DevTopo& t, const SolveCtl* ctl, const LbfgsBufs& v, cudaStream_t s);
 // The steepest-descent retry for the kOpSteepest instances: history cleared,
-// p = clamp(lock(-g)), dg[i] = <g, p> (sim.cpp:193-196).
-void bl_steepest(const DevTopo& t, const SolveCtl* ctl, int2* hist, double* p, const double* g, double* part,
-                 double* dg, double mt, double mr, cudaStream_t s);
+// p = clamp(lock(-g)), dg = <g, p> (sim.cpp:193-196).
+void bl_steepest(const DevTopo& t, const SolveCtl* ctl, const LbfgsBufs& v, cudaStream_t s);
 // kOpResetHistory / kOpZero / kOpRestore / kOpKeepBest / kOpCandidate / kOpEvalAtZ / kOpFinal
-void bl_prepare(const DevTopo& t, const SolveCtl* ctl, int2* hist, double* z, double* best, double* zeval,
-                const double* p, double* zfinal, cudaStream_t s);
-// kOpTakeGrad / kOpAccept (+kOpPair, kOpKeepBestAfter); out3[3 i..] = <s, y>, <s, s>, <y, y>;
-// then the history update of the accepted instances (sim.cpp:205-206).
-void bl_accept(const DevTopo& t, const SolveCtl* ctl, int2* hist, int H, double* z, double* g, const double* zeval,
-               const double* geval, double* S, double* Y, long long stride, double* best, double* rho, double* part,
-               double* out3, cudaStream_t s);
+void bl_prepare(const DevTopo& t, const SolveCtl* ctl, const LbfgsBufs& v, cudaStream_t s);
+// kOpTakeGrad / kOpAccept (+kOpPair, kOpKeepBestAfter), h0 and the history
+// update of the accepted instances (sim.cpp:205-206).
+void bl_accept(const DevTopo& t, const SolveCtl* ctl, const LbfgsBufs& v, cudaStream_t s);
 
 }  // namespace mcg

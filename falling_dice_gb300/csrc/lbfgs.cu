@@ -3,14 +3,35 @@
 // instance of a context at once.
 //
 // Vectors hold 6 entries per node in the ABI layout; all instances' nodes are stored one
-// after another and every kernel runs over the node blocks of the context (a block never
-// straddles two instances).  Each instance has its own solver state (history count, ring
-// head, line-search step, which operations it takes part in), written by the host into a
-// small control array before each step.  Dot products are per-block partial sums (each
-// thread its node's six products in order, then a fixed tree) and one block per instance
-// summing its blocks in order: the same partition whether an instance is solved alone or
-// with others, so a batch reproduces the separate runs bit for bit.  The two-loop scalars
-// (alpha_h, H0) never leave the device.
+// after another and every kernel runs over the solver blocks of the context (DevTopo::sblk: runs
+// of a few 64-node units of one instance, at most kSolveBlocks per instance, a partition that
+// depends on the instance alone).  Each instance has its own solver state (history count, ring
+// head, line-search step, which operations it takes part in) in a small control array.  Dot
+// products are per-block partial sums (a fixed tree), summed in order by the last of the
+// instance's blocks to finish: a batch reproduces the separate runs bit for bit.
+//
+// The two-loop recursion (sim.cpp:184-187) takes 2 m dependent dot products over the vectors,
+// each a pass of its own.  Here each loop is one pass: with q = g - sum_j alpha_j y_j substituted
+// into alpha_i = rho_i <s_i, q>, the alphas solve a triangular system whose matrix are the products
+// <s_i, y_j> of the history, one column of which is new per accepted pair; likewise the second
+// loop's coefficients.  Three passes make a direction:
+//   k_dir_dots   <s_i, g> and the newest column <s_i, y_new>; then alpha (last block);
+//   k_dir_first  q = g - sum alpha_i y_i and <y_i, q>; then the second loop's coefficients;
+//   k_dir_second p = clamp(lock(-(H0 q + sum c_i s_i))) and <g, p>; then the descent check.
+// The same products and sums as the recursion's; measured against extended precision over the
+// histories of three specimens' minimizations the direction's error is the recursion's (ratio of
+// geometric means 0.99, 1.14, 0.99).
+//
+// What bounds a pass: latency for a small lattice (the chain of loads, the block's reduction, the
+// instance's counter, the last block's totals and solve: 8 us a pass at 343 nodes), the FP64 units
+// from 10^4 nodes on (81 instructions per 32 half-nodes of the second pass; 17 us a pass at 17 500
+// nodes, history 10).  So the nodes are spread one 64-node block per SM while they last (one warp
+// per FP64 unit, few partials for the last block to sum), a thread keeps the loads of all its
+// history in flight, and the scalar solves run in the last block instead of in launches of their
+// own.  Whole minimizations against one pass per dot product: 6x6x6 cubic (18 rounds) 3.3 -> 1.6 ms,
+// 32x32x16 cubic+BCC mixed (14 rounds) 3.4 -> 2.6 ms, a load/unload run of 6 lattices 6.4 -> 4.5 ms.
+// With 64 blocks an instance 32x32x16 takes 98 us a direction, with 152 51; with 304 55 (the last
+// block's totals).
 #include "common.cuh"
 #include "kernels.h"
 
@@ -18,12 +39,12 @@ namespace mcg {
 
 namespace {
 
-__device__ __forceinline__ const double* hist_slot(const double* base, long long stride, int slot) {
-    return base + stride * slot;
-}
-
-// Slot of the h-th oldest history pair of an instance.
-__device__ __forceinline__ int ring_slot(const SolveCtl& c, int H, int h) { return (c.head + h) % H; }
+constexpr int kThreads = 256;            // one half-node (3 DOFs) per thread at a time
+constexpr int kUnit = 64;                // nodes of a solver block of a small instance: a warp per FP64 unit
+constexpr int kWarps = kThreads / 32;
+constexpr int kDotPairs = 4;             // history pairs a block of the first pass takes
+constexpr int kSmallHistory = 16;        // histories whose products are solved from shared memory
+constexpr int kRegHistory = 12;          // histories whose vectors a thread holds in registers (the default is 10)
 
 // An instance's control record with its history state (pairs held, oldest slot), which
 // lives on the device: the solver kernels update it themselves.
@@ -34,619 +55,472 @@ __device__ __forceinline__ SolveCtl load_ctl(const SolveCtl* __restrict__ ctl, c
     c.head = h.y;
     return c;
 }
-
-// One instance's sum of its block partials part[k * nblk + b], b in its node-block range,
-// for k < K (one block per instance; fixed order).
-template <int K>
-__device__ __forceinline__ void instance_sum(const DevTopo& t, const double* __restrict__ part, int inst,
-                                             double (&acc)[K], double* sm) {
-    const int4 r = t.irange[inst];
-#pragma unroll
-    for (int k = 0; k < K; k++) acc[k] = 0;
-    for (int b = r.x + int(threadIdx.x); b < r.y; b += blockDim.x)
-#pragma unroll
-        for (int k = 0; k < K; k++) acc[k] += part[size_t(k) * t.n_nblk + b];
-    block_sum<K>(acc, sm);
+// Slot of the h-th oldest history pair of an instance.
+__device__ __forceinline__ int ring_slot(const SolveCtl& c, int H, int h) {
+    const int s = c.head + h;
+    return s < H ? s : s - H;
 }
 
-__device__ __forceinline__ double dot6(const double* a, const double* b) {
-    double s = a[0] * b[0];
-    s += a[1] * b[1];
-    s += a[2] * b[2];
-    s += a[3] * b[3];
-    s += a[4] * b[4];
-    s += a[5] * b[5];
-    return s;
+__device__ __forceinline__ d3 ld3(const double* v) { return d3{v[0], v[1], v[2]}; }
+__device__ __forceinline__ void st3(double* v, d3 a) {
+    v[0] = a.x;
+    v[1] = a.y;
+    v[2] = a.z;
 }
 
-// ---- two-loop recursion (sim.cpp:184-187) -----------------------------------------------
-// Step j of loop LOOP for the instances computing a direction with j < m.  Every block of
-// an instance sums the instance's partials of step j's dot product (in `cur`, same order in
-// each block) into the coefficient and updates its nodes of p; when j + 1 < m it then writes
-// its partial of step j + 1's dot product with the updated p to `nxt`.
-//   loop 1 (newest first, h = m - 1 - j): alpha = rho <s, p> (kept), p -= alpha y;
-//   loop 2 (oldest first, h = j):         beta = rho <y, p>, p += s (alpha - beta).
-template <int LOOP>
-__global__ void __launch_bounds__(kBlock) k_tl_step(DevTopo t, const SolveCtl* __restrict__ ctl,
-                                                    const int2* __restrict__ hist, int H, int j,
-                                                    double* __restrict__ p, const double* __restrict__ S,
-                                                    const double* __restrict__ Y, long long stride,
-                                                    const double* __restrict__ rho, double* __restrict__ alpha,
-                                                    const double* __restrict__ cur, double* __restrict__ nxt) {
-    __shared__ double sm[kBlock / 32];
-    __shared__ double coef;
-    const MapPos mp = map_pos(t.nblk);
-    const SolveCtl c = load_ctl(ctl, hist, mp.inst);
-    if (!(c.flags & kOpDirection) || j >= c.m) return;  // block-uniform
-    const int h = LOOP == 1 ? c.m - 1 - j : j;
-    const int slot = ring_slot(c, H, h);
-    double acc[1];
-    instance_sum<1>(t, cur, mp.inst, acc, sm);
+// Whether this is the last of `total` blocks to arrive at an instance's counter; then every
+// block's earlier writes are visible.  All threads call it.
+__device__ __forceinline__ bool last_block(unsigned* counter, unsigned total) {
+    __shared__ int last;
+    __threadfence();
+    __syncthreads();
     if (threadIdx.x == 0) {
-        const double r = rho[size_t(mp.inst) * H + slot] * acc[0];
-        if (LOOP == 1) {
-            coef = r;
-            if (blockIdx.x == t.irange[mp.inst].x) alpha[size_t(mp.inst) * H + h] = r;
-        } else {
-            coef = alpha[size_t(mp.inst) * H + h] - r;
-        }
+        last = atomicAdd(counter, 1u) == total - 1u;
+        if (last) *counter = 0;  // for the next pass
     }
     __syncthreads();
-    const double k = coef;
-    double pn[6] = {0, 0, 0, 0, 0, 0};
-    if (mp.valid) {
-        double* pi = p + 6 * size_t(mp.i);
-        if (LOOP == 1) {
-            const double* y = hist_slot(Y, stride, slot) + 6 * size_t(mp.i);
-#pragma unroll
-            for (int d = 0; d < 6; d++) pn[d] = pi[d] - k * y[d];
-        } else {
-            const double* sv = hist_slot(S, stride, slot) + 6 * size_t(mp.i);
-#pragma unroll
-            for (int d = 0; d < 6; d++) pn[d] = pi[d] + sv[d] * k;
-        }
-#pragma unroll
-        for (int d = 0; d < 6; d++) pi[d] = pn[d];
-    }
-    if (j + 1 >= c.m) return;  // block-uniform
-    const int slot2 = ring_slot(c, H, LOOP == 1 ? c.m - 2 - j : j + 1);
-    const double* v = hist_slot(LOOP == 1 ? S : Y, stride, slot2);
-    double a2[1] = {0};
-    if (mp.valid) a2[0] = dot6(v + 6 * size_t(mp.i), pn);
-    block_sum<1>(a2, sm);
-    if (threadIdx.x == 0) nxt[blockIdx.x] = a2[0];
+    if (last) __threadfence();
+    return last;
 }
 
-// Partials of <s, y> and <y, y> of the newest pair (for H0, into h0part), the copy p = g
-// that starts the recursion and the partial of loop 1's first dot product <s, g> (into
-// part0).
-__global__ void __launch_bounds__(kBlock) k_tl_start(DevTopo t, const SolveCtl* __restrict__ ctl, const int2* __restrict__ hist, int H,
-                                                     double* __restrict__ p, const double* __restrict__ g,
-                                                     const double* __restrict__ S, const double* __restrict__ Y,
-                                                     long long stride, double* __restrict__ h0part,
-                                                     double* __restrict__ part0) {
-    __shared__ double sm[3 * (kBlock / 32)];
-    const MapPos mp = map_pos(t.nblk);
-    const SolveCtl c = load_ctl(ctl, hist, mp.inst);
-    if (!(c.flags & kOpDirection)) return;
-    if (mp.valid)
-#pragma unroll
-        for (int d = 0; d < 6; d++) p[6 * size_t(mp.i) + d] = g[6 * size_t(mp.i) + d];
-    if (c.m == 0) return;
-    const int slot = ring_slot(c, H, c.m - 1);
-    double acc[3] = {0, 0, 0};
-    if (mp.valid) {
-        const double* s = hist_slot(S, stride, slot) + 6 * size_t(mp.i);
-        const double* y = hist_slot(Y, stride, slot) + 6 * size_t(mp.i);
-        acc[0] = dot6(s, y);
-        acc[1] = dot6(y, y);
-        acc[2] = dot6(s, g + 6 * size_t(mp.i));
-    }
-    block_sum<3>(acc, sm);
-    if (threadIdx.x == 0) {
-        h0part[blockIdx.x] = acc[0];
-        h0part[size_t(t.n_nblk) + blockIdx.x] = acc[1];
-        part0[blockIdx.x] = acc[2];
-    }
-}
-
-// p *= H0, H0 = clamp(sy/yy, 1e-7, 1e4) when both are positive, else 0.1 (sim.cpp:186), and
-// the partial of loop 2's first dot product <y, p> (into part0).
-__global__ void __launch_bounds__(kBlock) k_tl_scale(DevTopo t, const SolveCtl* __restrict__ ctl, const int2* __restrict__ hist,
-                                                     int H, double* __restrict__ p, const double* __restrict__ Y,
-                                                     long long stride, const double* __restrict__ h0part,
-                                                     double* __restrict__ part0) {
-    __shared__ double sm[2 * (kBlock / 32)];
-    __shared__ double h0;
-    const MapPos mp = map_pos(t.nblk);
-    const SolveCtl c = load_ctl(ctl, hist, mp.inst);
-    if (!(c.flags & kOpDirection)) return;
-    if (c.m > 0) {
-        double acc[2];
-        instance_sum<2>(t, h0part, mp.inst, acc, sm);
-        if (threadIdx.x == 0) {
-            double v = .10;
-            if (acc[0] > 1e-20 && acc[1] > 1e-20) v = clampd(acc[0] / acc[1], 1e-7, 1e4);
-            h0 = v;
-        }
-    } else if (threadIdx.x == 0) {
-        h0 = .10;
+// Block partial of up to four values into q[k * stride] (thread k writes value k).
+template <int NV>
+__device__ __forceinline__ void block_part(double a, double b, double c, double d, double* q, size_t stride,
+                                           double (*sm)[kWarps]) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (NV <= 2) {
+        const double v = warp_sum2(a, b);
+        if ((lane & 15) == 0) sm[lane >> 4][warp] = v;
+    } else {
+        const double v = warp_sum4(a, b, c, d);
+        if ((lane & 7) == 0) sm[lane >> 3][warp] = v;
     }
     __syncthreads();
-    const double k = h0;
-    double pn[6] = {0, 0, 0, 0, 0, 0};
-    if (mp.valid)
-#pragma unroll
-        for (int d = 0; d < 6; d++) {
-            pn[d] = p[6 * size_t(mp.i) + d] * k;
-            p[6 * size_t(mp.i) + d] = pn[d];
-        }
-    if (c.m == 0) return;  // block-uniform
-    const double* v = hist_slot(Y, stride, ring_slot(c, H, 0));
-    double a2[1] = {0};
-    if (mp.valid) a2[0] = dot6(v + 6 * size_t(mp.i), pn);
-    block_sum<1>(a2, sm);
-    if (threadIdx.x == 0) part0[blockIdx.x] = a2[0];
-}
-
-// Direction finish for the instances with `bit` set: p = clamp(lock(-src)) per node
-// (sim.cpp:188-190, clampDirection sim.cpp:46), and the partial of <g, p>.
-__global__ void __launch_bounds__(kBlock) k_finish(DevTopo t, const SolveCtl* __restrict__ ctl, int bit,
-                                                   double* __restrict__ p, const double* __restrict__ src,
-                                                   const double* __restrict__ g, double mt, double mr,
-                                                   double* __restrict__ part) {
-    __shared__ double sm[kBlock / 32];
-    const MapPos mp = map_pos(t.nblk);
-    if (!(ctl[mp.inst].flags & bit)) return;
-    double acc[1] = {0};
-    if (mp.valid) {
-        const size_t b = 6 * size_t(mp.i);
-        const uint8_t* lk = t.locked + b;
-        double v[6];
-#pragma unroll
-        for (int k = 0; k < 6; k++) {
-            v[k] = -src[b + k];
-            if (lk[k]) v[k] = 0;
-        }
-        const double lt = sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
-        if (lt > mt) {
-            const double f = mt / lt;
-            v[0] *= f; v[1] *= f; v[2] *= f;
-        }
-        const double lr = sqrt(v[3] * v[3] + v[4] * v[4] + v[5] * v[5]);
-        if (lr > mr) {
-            const double f = mr / lr;
-            v[3] *= f; v[4] *= f; v[5] *= f;
-        }
-#pragma unroll
-        for (int k = 0; k < 6; k++) {
-            v[k] = lk[k] ? 0.0 : v[k];
-            p[b + k] = v[k];
-        }
-        acc[0] = dot6(g + b, v);
+    if (threadIdx.x < NV) {
+        double s = sm[threadIdx.x][0];
+        for (int w = 1; w < kWarps; w++) s += sm[threadIdx.x][w];
+        q[threadIdx.x * stride] = s;
     }
-    block_sum<1>(acc, sm);
-    if (threadIdx.x == 0) part[blockIdx.x] = acc[0];
+    __syncthreads();
 }
 
-// One block per instance with `bit` set: out[K i + k] = sum of its partials.
-template <int K>
-__global__ void __launch_bounds__(kBlock) k_inst_final(DevTopo t, const SolveCtl* __restrict__ ctl, int bit,
-                                                       const double* __restrict__ part, double* __restrict__ out) {
-    __shared__ double sm[K * (kBlock / 32)];
-    const int inst = blockIdx.x;
-    if (!(ctl[inst].flags & bit)) return;
-    double acc[K];
-    instance_sum<K>(t, part, inst, acc, sm);
-    if (threadIdx.x == 0)
+// Totals of nv values' partials over the instance's nb (<= kSolveBlocks) blocks, value k at
+// part[k * stride + first ...], into out[k]; four values a warp at a time.
+__device__ __forceinline__ void part_totals(const double* part, size_t stride, int first, int nb, int nv, double* out) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int k0 = 4 * warp; k0 < nv; k0 += 4 * kWarps) {
+        double v[4] = {0, 0, 0, 0};
 #pragma unroll
-        for (int k = 0; k < K; k++) out[size_t(K) * inst + k] = acc[k];
+        for (int j = 0; j < 4; j++)
+            if (k0 + j < nv) {
+                const double* p = part + (k0 + j) * stride + first;
+#pragma unroll
+                for (int b = 0; b < kSolveBlocks; b += 32)
+                    if (b + lane < nb) v[j] += __ldcg(p + b + lane);
+            }
+        const double s = warp_sum4(v[0], v[1], v[2], v[3]);
+        if ((lane & 7) == 0 && k0 + (lane >> 3) < nv) out[k0 + (lane >> 3)] = s;
+    }
+    __syncthreads();
+}
+
+// ---- direction, first pass ------------------------------------------------------------------
+// Block (b, k): the partials of <s, g> and <s, y_new> for history pairs 4 k ... 4 k + 3; the last
+// block of the instance stores the newest column of the products and solves the first loop's
+// alphas, newest to oldest: alpha_i = rho_i (<s_i, g> - sum_{j > i} alpha_j <s_i, y_j>).
+__global__ void __launch_bounds__(kThreads) k_dir_dots(DevTopo t, const SolveCtl* __restrict__ ctl, LbfgsBufs v) {
+    __shared__ double sm[4][kWarps];
+    __shared__ double val[2 * 64], R[kSmallHistory][kSmallHistory + 1];
+    const int H = v.H;
+    const int4 q = t.sblk[blockIdx.x];
+    const int inst = q.z, h0 = kDotPairs * blockIdx.y;
+    const SolveCtl c = load_ctl(ctl, v.hist, inst);
+    const int m = c.m;
+    if (!(c.flags & kOpDirection) || h0 >= m) return;  // block-uniform (none when m == 0)
+    const int newest = ring_slot(c, H, m - 1);
+    const double* s[kDotPairs];
+#pragma unroll
+    for (int k = 0; k < kDotPairs; k++) s[k] = v.S + v.stride * ring_slot(c, H, min(h0 + k, m - 1)) + 6 * size_t(q.x);
+    const double* y = v.Y + v.stride * newest + 6 * size_t(q.x);
+    const double* g = v.g + 6 * size_t(q.x);
+    double d[2 * kDotPairs] = {};
+    for (int i = threadIdx.x; i < 2 * q.y; i += kThreads) {
+        const d3 b = ld3(g + 3 * i), e = ld3(y + 3 * i);
+        d3 a[kDotPairs];
+#pragma unroll
+        for (int k = 0; k < kDotPairs; k++)
+            if (h0 + k < m) a[k] = ld3(s[k] + 3 * i);
+#pragma unroll
+        for (int k = 0; k < kDotPairs; k++)
+            if (h0 + k < m) {
+                d[2 * k] = fma(a[k].z, b.z, fma(a[k].y, b.y, fma(a[k].x, b.x, d[2 * k])));
+                d[2 * k + 1] = fma(a[k].z, e.z, fma(a[k].y, e.y, fma(a[k].x, e.x, d[2 * k + 1])));
+            }
+    }
+#pragma unroll
+    for (int k = 0; k < 2 * kDotPairs; k += 4)
+        if (2 * h0 + k < 2 * m)
+            block_part<4>(d[k], d[k + 1], d[k + 2], d[k + 3], v.part + size_t(2 * h0 + k) * t.n_sblk + blockIdx.x, t.n_sblk, sm);
+    const int2 r = t.srange[inst];
+    const int nb = r.y - r.x;
+    if (!last_block(v.done + 4 * inst, unsigned(nb * ((m + kDotPairs - 1) / kDotPairs)))) return;
+    part_totals(v.part, t.n_sblk, r.x, nb, 2 * m, val);
+    double* gram = v.gram + size_t(inst) * H * H;  // <s_i, y_j> at [slot i][slot j], i not newer than j
+    const bool small = m <= kSmallHistory;
+    for (int i = threadIdx.x; i < m; i += kThreads) gram[ring_slot(c, H, i) * H + newest] = val[2 * i + 1];
+    if (small)
+        for (int k = threadIdx.x; k < m * m; k += kThreads) {
+            const int i = k / m, j = k - i * m;
+            if (i <= j) R[i][j] = j == m - 1 ? val[2 * i + 1] : gram[ring_slot(c, H, i) * H + ring_slot(c, H, j)];
+        }
+    __syncthreads();
+    if (threadIdx.x >= 32) return;
+    const int lane = threadIdx.x, nu = m > 32 ? 2 : 1;
+    const double* rho = v.rho + size_t(inst) * H;
+    double a[2], rh[2];  // history pairs lane and lane + 32
+    for (int u = 0; u < 2; u++) {
+        const int i = lane + 32 * u;
+        a[u] = i < m ? val[2 * i] : 0;
+        rh[u] = i < m ? rho[ring_slot(c, H, i)] : 0;
+    }
+    for (int i = m - 1; i >= 0; i--) {
+        const double al = __shfl_sync(0xffffffffu, i < 32 ? rh[0] * a[0] : rh[1] * a[1], i & 31);
+        if (lane == (i & 31)) v.alpha[size_t(inst) * H + i] = al;
+        for (int u = 0; u < nu; u++) {
+            const int j = lane + 32 * u;
+            if (j >= i) continue;
+            const double rji = small ? R[j][i] : i == m - 1 ? val[2 * j + 1] : gram[ring_slot(c, H, j) * H + ring_slot(c, H, i)];
+            a[u] = fma(-al, rji, a[u]);
+        }
+    }
+}
+
+// H0 of the direction: k_accept's for the newest pair, 0.1 without history (sim.cpp:186).
+__device__ __forceinline__ double initial_scale(const LbfgsBufs& v, int inst, int m) { return m > 0 ? v.h0[inst] : .10; }
+
+// ---- direction, second pass -----------------------------------------------------------------
+// q = g - sum alpha_i y_i (newest first, into p) and the partials of <y_i, q>; the last block of
+// the instance solves the second loop's coefficients, oldest to newest:
+// c_i = alpha_i - rho_i (H0 <y_i, q> + sum_{j < i} c_j <s_j, y_i>).
+__global__ void __launch_bounds__(kThreads) k_dir_first(DevTopo t, const SolveCtl* __restrict__ ctl, LbfgsBufs v) {
+    __shared__ double sm[4][kWarps];
+    __shared__ double al[64], val[64], R[kSmallHistory][kSmallHistory + 1];
+    const int H = v.H;
+    const int4 q = t.sblk[blockIdx.x];
+    const int inst = q.z;
+    const SolveCtl c = load_ctl(ctl, v.hist, inst);
+    if (!(c.flags & kOpDirection)) return;
+    const int m = c.m;
+    for (int i = threadIdx.x; i < m; i += kThreads) al[i] = v.alpha[size_t(inst) * H + i];
+    __syncthreads();
+    double* p = v.p + 6 * size_t(q.x);
+    const double* g = v.g + 6 * size_t(q.x);
+    if (m <= kRegHistory) {
+        // every load of the thread's half-node in flight at once, the y_i used for both sums
+        const double* Y[kRegHistory];
+#pragma unroll
+        for (int h = 0; h < kRegHistory; h++) Y[h] = v.Y + v.stride * (h < m ? ring_slot(c, H, h) : 0) + 6 * size_t(q.x);
+        double d[kRegHistory] = {};
+        for (int i = threadIdx.x; i < 2 * q.y; i += kThreads) {
+            d3 a = ld3(g + 3 * i), y[kRegHistory];
+#pragma unroll
+            for (int h = 0; h < kRegHistory; h++)
+                if (h < m) y[h] = ld3(Y[h] + 3 * i);
+#pragma unroll
+            for (int h = kRegHistory - 1; h >= 0; h--)
+                if (h < m) a = fmadd(y[h], -al[h], a);
+            st3(p + 3 * i, a);
+#pragma unroll
+            for (int h = 0; h < kRegHistory; h++)
+                if (h < m) d[h] = fma(a.z, y[h].z, fma(a.y, y[h].y, fma(a.x, y[h].x, d[h])));
+        }
+        if (m == 0) return;  // block-uniform: no history, p = g
+        __shared__ double wsum[kRegHistory][kWarps];
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+        for (int h = 0; h < kRegHistory; h += 4)
+            if (h < m) {
+                const double s4 = warp_sum4(d[h], d[h + 1], d[h + 2], d[h + 3]);
+                if ((lane & 7) == 0) wsum[h + (lane >> 3)][warp] = s4;
+            }
+        __syncthreads();
+        for (int h = threadIdx.x; h < m; h += kThreads) {
+            double s = wsum[h][0];
+            for (int w = 1; w < kWarps; w++) s += wsum[h][w];
+            v.part[size_t(h) * t.n_sblk + blockIdx.x] = s;
+        }
+    } else {
+        for (int i = threadIdx.x; i < 2 * q.y; i += kThreads) {
+            d3 a = ld3(g + 3 * i);
+            for (int h = m - 1; h >= 0; h--)
+                a = fmadd(ld3(v.Y + v.stride * ring_slot(c, H, h) + 6 * size_t(q.x) + 3 * i), -al[h], a);
+            st3(p + 3 * i, a);
+        }
+        for (int h = 0; h < m; h += 4) {
+            double d[4] = {0, 0, 0, 0};
+            for (int i = threadIdx.x; i < 2 * q.y; i += kThreads) {
+                const d3 a = ld3(p + 3 * i);
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    if (h + k >= m) break;
+                    const d3 y = ld3(v.Y + v.stride * ring_slot(c, H, h + k) + 6 * size_t(q.x) + 3 * i);
+                    d[k] = fma(a.z, y.z, fma(a.y, y.y, fma(a.x, y.x, d[k])));
+                }
+            }
+            block_part<4>(d[0], d[1], d[2], d[3], v.part + size_t(h) * t.n_sblk + blockIdx.x, t.n_sblk, sm);
+        }
+    }
+    const int2 r = t.srange[inst];
+    const int nb = r.y - r.x;
+    if (!last_block(v.done + 4 * inst + 1, unsigned(nb))) return;
+    part_totals(v.part, t.n_sblk, r.x, nb, m, val);
+    const double* gram = v.gram + size_t(inst) * H * H;
+    const bool small = m <= kSmallHistory;
+    if (small)
+        for (int k = threadIdx.x; k < m * m; k += kThreads) {
+            const int i = k / m, j = k - i * m;
+            if (i < j) R[i][j] = gram[ring_slot(c, H, i) * H + ring_slot(c, H, j)];
+        }
+    __syncthreads();
+    if (threadIdx.x >= 32) return;
+    const int lane = threadIdx.x, nu = m > 32 ? 2 : 1;
+    const double* rho = v.rho + size_t(inst) * H;
+    const double h0 = initial_scale(v, inst, m);
+    double a[2], rh[2], u0[2];
+    for (int u = 0; u < 2; u++) {
+        const int i = lane + 32 * u;
+        a[u] = i < m ? h0 * val[i] : 0;
+        rh[u] = i < m ? rho[ring_slot(c, H, i)] : 0;
+        u0[u] = i < m ? al[i] : 0;
+    }
+    for (int i = 0; i < m; i++) {
+        const double co = __shfl_sync(0xffffffffu, i < 32 ? fma(-rh[0], a[0], u0[0]) : fma(-rh[1], a[1], u0[1]), i & 31);
+        if (lane == (i & 31)) v.coef[size_t(inst) * H + i] = co;
+        for (int u = 0; u < nu; u++) {
+            const int j = lane + 32 * u;
+            if (j <= i || j >= m) continue;
+            const double rij = small ? R[i][j] : gram[ring_slot(c, H, i) * H + ring_slot(c, H, j)];
+            a[u] = fma(co, rij, a[u]);
+        }
+    }
+}
+
+// p = clamp(lock(v)) of one half of a node (translations or rotations; sim.cpp:188-190, 46).
+__device__ __forceinline__ d3 clamp_half(d3 a, const uint8_t* lk, double limit) {
+    if (lk[0]) a.x = 0;
+    if (lk[1]) a.y = 0;
+    if (lk[2]) a.z = 0;
+    const double l2 = fdot(a, a);
+    // the length is taken only where its square can exceed the limit's
+    if (!(limit >= 0 && l2 <= limit * limit * (1 - 0x1p-40))) {
+        const double l = sqrt(l2);
+        if (l > limit) a = a * (limit / l);
+    }
+    return a;
+}
+
+// p = clamp(lock(-src)) over the run of half-nodes and this thread's part of <g, p>.
+__device__ __forceinline__ double steepest_part(const DevTopo& t, const double* g, double* p, int first, int halves,
+                                                double mt, double mr) {
+    double d = 0;
+    for (int i = threadIdx.x; i < halves; i += kThreads) {
+        const size_t o = 6 * size_t(first) + 3 * size_t(i);
+        const d3 b = ld3(g + o), a = clamp_half(-b, t.locked + o, (i & 1) ? mr : mt);
+        st3(p + o, a);
+        d = fma(a.z, b.z, fma(a.y, b.y, fma(a.x, b.x, d)));
+    }
+    return d;
+}
+
+// ---- direction, third pass ------------------------------------------------------------------
+// p = clamp(lock(-(H0 q + sum c_i s_i))) and the partial of <g, p>; the last block of the instance
+// sums dg.  Not a descent direction (sim.cpp:191): that block takes steepest descent instead and
+// clears the history.
+__global__ void __launch_bounds__(kThreads) k_dir_second(DevTopo t, const SolveCtl* __restrict__ ctl, LbfgsBufs v) {
+    __shared__ double sm[4][kWarps];
+    __shared__ double co[64], total[1];
+    const int H = v.H;
+    const int4 q = t.sblk[blockIdx.x];
+    const int inst = q.z;
+    const SolveCtl c = load_ctl(ctl, v.hist, inst);
+    if (!(c.flags & kOpDirection)) return;
+    const int m = c.m;
+    for (int i = threadIdx.x; i < m; i += kThreads) co[i] = v.coef[size_t(inst) * H + i];
+    const double h0 = initial_scale(v, inst, m);
+    __syncthreads();
+    double d = 0;
+    for (int i = threadIdx.x; i < 2 * q.y; i += kThreads) {
+        const size_t o = 6 * size_t(q.x) + 3 * size_t(i);
+        d3 a = ld3(v.p + o);
+        if (m <= kRegHistory) {  // every load in flight at once
+            d3 sv[kRegHistory];
+#pragma unroll
+            for (int h = 0; h < kRegHistory; h++)
+                if (h < m) sv[h] = ld3(v.S + v.stride * ring_slot(c, H, h) + o);
+            a = a * h0;
+#pragma unroll
+            for (int h = 0; h < kRegHistory; h++)
+                if (h < m) a = fmadd(sv[h], co[h], a);
+        } else {
+            a = a * h0;
+            for (int h = 0; h < m; h++) a = fmadd(ld3(v.S + v.stride * ring_slot(c, H, h) + o), co[h], a);
+        }
+        a = clamp_half(-a, t.locked + o, (i & 1) ? v.mr : v.mt);
+        st3(v.p + o, a);
+        const d3 b = ld3(v.g + o);
+        d = fma(a.z, b.z, fma(a.y, b.y, fma(a.x, b.x, d)));
+    }
+    block_part<1>(d, 0, 0, 0, v.part + blockIdx.x, t.n_sblk, sm);
+    const int2 r = t.srange[inst];
+    const int nb = r.y - r.x;
+    if (!last_block(v.done + 4 * inst + 2, unsigned(nb))) return;
+    part_totals(v.part, t.n_sblk, r.x, nb, 1, total);
+    const double dg = total[0];
+    if (dg < 0) {
+        if (threadIdx.x == 0) v.dg[inst] = dg;
+        return;
+    }
+    const double e = steepest_part(t, v.g, v.p, t.sblk[r.x].x, 2 * t.inst_n[inst], v.mt, v.mr);
+    block_part<1>(e, 0, 0, 0, total, 1, sm);
+    if (threadIdx.x == 0) {
+        v.dg[inst] = total[0];
+        v.hist[inst].x = 0;
+    }
+}
+
+// The steepest-descent retry (sim.cpp:193-196): history cleared, p = clamp(lock(-g)), dg.
+__global__ void __launch_bounds__(kThreads) k_steepest(DevTopo t, const SolveCtl* __restrict__ ctl, LbfgsBufs v) {
+    __shared__ double sm[4][kWarps];
+    __shared__ double total[1];
+    const int4 q = t.sblk[blockIdx.x];
+    const int inst = q.z;
+    if (!(ctl[inst].flags & kOpSteepest)) return;
+    const double d = steepest_part(t, v.g, v.p, q.x, 2 * q.y, v.mt, v.mr);
+    block_part<1>(d, 0, 0, 0, v.part + blockIdx.x, t.n_sblk, sm);
+    const int2 r = t.srange[inst];
+    if (!last_block(v.done + 4 * inst + 2, unsigned(r.y - r.x))) return;
+    part_totals(v.part, t.n_sblk, r.x, r.y - r.x, 1, total);
+    if (threadIdx.x == 0) {
+        v.dg[inst] = total[0];
+        v.hist[inst].x = 0;
+    }
 }
 
 // ---- vectors around an evaluation ------------------------------------------------------------
 // Per node, in this order for each instance's flags: z = 0 (kOpZero), z = best (kOpRestore),
 // best = z (kOpKeepBest), zeval = z + step p with locked entries 0 (kOpCandidate, sim.cpp:179)
-// or zeval = z (kOpEvalAtZ), zfinal = z (kOpFinal).
-__global__ void __launch_bounds__(kBlock) k_prepare(DevTopo t, const SolveCtl* __restrict__ ctl,
-                                                    double* __restrict__ z, double* __restrict__ best,
-                                                    double* __restrict__ zeval, const double* __restrict__ p,
-                                                    double* __restrict__ zfinal) {
-    const MapPos mp = map_pos(t.nblk);
+// or zeval = z (kOpEvalAtZ), zfinal = z (kOpFinal); a new minimization starts with an empty
+// history (kOpResetHistory).
+__global__ void __launch_bounds__(kEvalBlock) k_prepare(DevTopo t, const SolveCtl* __restrict__ ctl, LbfgsBufs v) {
+    const MapPos mp = map_pos(t.eblk);
     const SolveCtl c = ctl[mp.inst];
+    if ((c.flags & kOpResetHistory) && threadIdx.x == 0 && int(blockIdx.x) == t.erange[mp.inst].x)
+        v.hist[mp.inst] = make_int2(0, 0);
     if (!mp.valid || !(c.flags & (kOpZero | kOpRestore | kOpKeepBest | kOpCandidate | kOpEvalAtZ | kOpFinal))) return;
-    const size_t b = 6 * size_t(mp.i);
+    const size_t o = 6 * size_t(mp.i);
+    double a[6];
 #pragma unroll
     for (int k = 0; k < 6; k++) {
-        double v = z[b + k];
-        if (c.flags & kOpZero) v = 0;
-        if (c.flags & kOpRestore) v = best[b + k];
-        z[b + k] = v;
-        if (c.flags & kOpKeepBest) best[b + k] = v;
-        if (c.flags & kOpCandidate) zeval[b + k] = t.locked[b + k] ? 0.0 : v + c.step * p[b + k];
-        if (c.flags & kOpEvalAtZ) zeval[b + k] = v;
-        if (c.flags & kOpFinal) zfinal[b + k] = v;
+        a[k] = (c.flags & kOpZero) ? 0.0 : v.z[o + k];
+        if (c.flags & kOpRestore) a[k] = v.best[o + k];
     }
+#pragma unroll
+    for (int k = 0; k < 6; k++) {
+        if (c.flags & (kOpZero | kOpRestore)) v.z[o + k] = a[k];
+        if (c.flags & kOpKeepBest) v.best[o + k] = a[k];
+        if (c.flags & kOpEvalAtZ) v.zeval[o + k] = a[k];
+        if (c.flags & kOpFinal) v.zfinal[o + k] = a[k];
+    }
+    if (!(c.flags & kOpCandidate)) return;
+    double p[6];
+#pragma unroll
+    for (int k = 0; k < 6; k++) p[k] = v.p[o + k];
+#pragma unroll
+    for (int k = 0; k < 6; k++) v.zeval[o + k] = t.locked[o + k] ? 0.0 : fma(c.step, p[k], a[k]);
 }
 
 // After an evaluation: g = geval for the instances that evaluated at z (kOpTakeGrad), and
 // for accepted trials (kOpAccept, sim.cpp:205-206) s = zeval - z, y = geval - g into the
-// history slot `target` (kOpPair), the partials of <s, y>, <s, s>, <y, y>, then z = zeval,
-// g = geval; best = z afterwards when kOpKeepBestAfter.
-__global__ void __launch_bounds__(kBlock) k_accept(DevTopo t, const SolveCtl* __restrict__ ctl, const int2* __restrict__ hist,
-                                                   int H, double* __restrict__ z, double* __restrict__ g,
-                                                   const double* __restrict__ zeval, const double* __restrict__ geval,
-                                                   double* __restrict__ S, double* __restrict__ Y, long long stride,
-                                                   double* __restrict__ best, double* __restrict__ part) {
-    __shared__ double sm[3 * (kBlock / 32)];
-    const MapPos mp = map_pos(t.nblk);
-    const SolveCtl c = load_ctl(ctl, hist, mp.inst);
+// next history slot (kOpPair), the partials of <s, y>, <s, s>, <y, y>, then z = zeval,
+// g = geval; best = z afterwards when kOpKeepBestAfter.  The last block of the instance sums the
+// products and keeps the pair when s.y > 1e-12 sqrt(max(1e-30, s.s y.y)) (rho = 1 / s.y in its
+// slot), else clears the history.
+__global__ void __launch_bounds__(kThreads) k_accept(DevTopo t, const SolveCtl* __restrict__ ctl, LbfgsBufs v) {
+    __shared__ double sm[4][kWarps];
+    __shared__ double total[4];
+    const int H = v.H;
+    const int4 q = t.sblk[blockIdx.x];
+    const int inst = q.z;
+    const SolveCtl c = load_ctl(ctl, v.hist, inst);
     if (!(c.flags & (kOpTakeGrad | kOpAccept))) return;
-    const size_t b = 6 * size_t(mp.i);
     if (c.flags & kOpTakeGrad) {
-        if (mp.valid)
-#pragma unroll
-            for (int k = 0; k < 6; k++) g[b + k] = geval[b + k];
+        for (int i = threadIdx.x; i < 6 * q.y; i += kThreads) v.g[6 * size_t(q.x) + i] = v.geval[6 * size_t(q.x) + i];
         return;
     }
-    double acc[3] = {0, 0, 0};
-    if (mp.valid) {
-        double sv[6], yv[6];
-#pragma unroll
-        for (int k = 0; k < 6; k++) {
-            sv[k] = zeval[b + k] - z[b + k];
-            yv[k] = geval[b + k] - g[b + k];
-        }
+    const int target = c.m < H ? (c.head + c.m) % H : c.head;
+    double sy = 0, ss = 0, yy = 0;
+    for (int i = threadIdx.x; i < 2 * q.y; i += kThreads) {
+        const size_t o = 6 * size_t(q.x) + 3 * size_t(i);
+        const d3 ze = ld3(v.zeval + o), ge = ld3(v.geval + o);
+        const d3 a = ze - ld3(v.z + o), b = ge - ld3(v.g + o);
         if (c.flags & kOpPair) {
-            const int target = c.m < H ? (c.head + c.m) % H : c.head;
-            double* s = S + stride * target + b;
-            double* y = Y + stride * target + b;
-#pragma unroll
-            for (int k = 0; k < 6; k++) {
-                s[k] = sv[k];
-                y[k] = yv[k];
-            }
+            st3(v.S + v.stride * target + o, a);
+            st3(v.Y + v.stride * target + o, b);
         }
-        acc[0] = dot6(sv, yv);
-        acc[1] = dot6(sv, sv);
-        acc[2] = dot6(yv, yv);
-#pragma unroll
-        for (int k = 0; k < 6; k++) {
-            z[b + k] = zeval[b + k];
-            g[b + k] = geval[b + k];
-        }
-        if (c.flags & kOpKeepBestAfter)
-#pragma unroll
-            for (int k = 0; k < 6; k++) best[b + k] = zeval[b + k];
+        sy = fma(a.z, b.z, fma(a.y, b.y, fma(a.x, b.x, sy)));
+        ss = fma(a.z, a.z, fma(a.y, a.y, fma(a.x, a.x, ss)));
+        yy = fma(b.z, b.z, fma(b.y, b.y, fma(b.x, b.x, yy)));
+        st3(v.z + o, ze);
+        st3(v.g + o, ge);
+        if (c.flags & kOpKeepBestAfter) st3(v.best + o, ze);
     }
-    block_sum<3>(acc, sm);
-    if (threadIdx.x == 0) {
-        part[blockIdx.x] = acc[0];
-        part[size_t(t.n_nblk) + blockIdx.x] = acc[1];
-        part[2 * size_t(t.n_nblk) + blockIdx.x] = acc[2];
-    }
-}
-
-// ---- the whole direction in one CTA per instance ---------------------------------------------
-// For instances of at most kFuseChunks node blocks: the same steps as k_tl_start ...
-// k_finish + k_inst_final (each block partial here is one chunk of kBlock nodes reduced by the
-// same tree, each instance sum the same strided tree), so the result is bit for bit that of
-// the multi-launch path; one launch instead of 2 H + 4.
-constexpr int kFuseChunks = 64;
-
-// Partial of one chunk: thread t the node first + t (if valid), then the block tree.
-__device__ __forceinline__ double chunk_dot(const double* a, const double* b, int first, int count, double* sm) {
-    double acc[1] = {0};
-    if (int(threadIdx.x) < count) acc[0] = dot6(a + 6 * size_t(first + threadIdx.x), b + 6 * size_t(first + threadIdx.x));
-    block_sum<1>(acc, sm);
-    return acc[0];
-}
-
-// Sum of nchunk partials held in shared memory, strided as instance_sum.
-template <int K>
-__device__ __forceinline__ void chunk_sum(const double (*part)[kFuseChunks], int nchunk, double (&acc)[K], double* sm) {
-#pragma unroll
-    for (int k = 0; k < K; k++) acc[k] = 0;
-    for (int b = int(threadIdx.x); b < nchunk; b += blockDim.x)
-#pragma unroll
-        for (int k = 0; k < K; k++) acc[k] += part[k][b];
-    block_sum<K>(acc, sm);
-}
-
-__global__ void __launch_bounds__(kBlock) k_direction_fused(DevTopo t, const SolveCtl* __restrict__ ctl, const int2* __restrict__ hist, int H,
-                                                            double* __restrict__ p, const double* __restrict__ g,
-                                                            const double* __restrict__ S, const double* __restrict__ Y,
-                                                            long long stride, const double* __restrict__ rho,
-                                                            double* __restrict__ dg, double mt, double mr) {
-    __shared__ double sm[2 * (kBlock / 32)];
-    __shared__ double part[2][kFuseChunks];
-    __shared__ double alpha[64];
-    __shared__ double coef;
-    const int inst = blockIdx.x;
-    const SolveCtl c = load_ctl(ctl, hist, inst);
-    if (!(c.flags & kOpDirFused)) return;
-    const int4 r = t.irange[inst];
-    const int nchunk = r.y - r.x;
-    // p = g; partials of <s, y>, <y, y> of the newest pair
-    for (int b = 0; b < nchunk; b++) {
-        const int4 q = t.nblk[r.x + b];
-        if (int(threadIdx.x) < q.y)
-#pragma unroll
-            for (int d = 0; d < 6; d++) p[6 * size_t(q.x + threadIdx.x) + d] = g[6 * size_t(q.x + threadIdx.x) + d];
-        if (c.m > 0) {
-            const int slot = ring_slot(c, H, c.m - 1);
-            double acc[2] = {0, 0};
-            if (int(threadIdx.x) < q.y) {
-                const double* sv = hist_slot(S, stride, slot) + 6 * size_t(q.x + threadIdx.x);
-                const double* yv = hist_slot(Y, stride, slot) + 6 * size_t(q.x + threadIdx.x);
-                acc[0] = dot6(sv, yv);
-                acc[1] = dot6(yv, yv);
-            }
-            block_sum<2>(acc, sm);
-            if (threadIdx.x == 0) {
-                part[0][b] = acc[0];
-                part[1][b] = acc[1];
-            }
-        }
-    }
-    __syncthreads();
-    double h0acc[2] = {0, 0};
-    if (c.m > 0) chunk_sum<2>(part, nchunk, h0acc, sm);
-    __syncthreads();
-    // loop 1, newest first
-    for (int j = 0; j < c.m; j++) {
-        const int h = c.m - 1 - j, slot = ring_slot(c, H, h);
-        for (int b = 0; b < nchunk; b++) {
-            const int4 q = t.nblk[r.x + b];
-            const double v = chunk_dot(hist_slot(S, stride, slot), p, q.x, q.y, sm);
-            if (threadIdx.x == 0) part[0][b] = v;
-        }
-        __syncthreads();
-        double acc[1];
-        chunk_sum<1>(part, nchunk, acc, sm);
-        if (threadIdx.x == 0) {
-            coef = rho[size_t(inst) * H + slot] * acc[0];
-            alpha[h] = coef;
-        }
-        __syncthreads();
-        const double k = coef;
-        const double* yv = hist_slot(Y, stride, slot);
-        for (int b = 0; b < nchunk; b++) {
-            const int4 q = t.nblk[r.x + b];
-            if (int(threadIdx.x) < q.y)
-#pragma unroll
-                for (int d = 0; d < 6; d++) p[6 * size_t(q.x + threadIdx.x) + d] -= k * yv[6 * size_t(q.x + threadIdx.x) + d];
-        }
-        __syncthreads();
-    }
-    // H0 (sim.cpp:186); the block sums are complete in thread 0 only
-    if (threadIdx.x == 0) {
-        double v = .10;
-        if (c.m > 0 && h0acc[0] > 1e-20 && h0acc[1] > 1e-20) v = clampd(h0acc[0] / h0acc[1], 1e-7, 1e4);
-        coef = v;
-    }
-    __syncthreads();
-    {
-        const double v = coef;
-        for (int b = 0; b < nchunk; b++) {
-            const int4 q = t.nblk[r.x + b];
-            if (int(threadIdx.x) < q.y)
-#pragma unroll
-                for (int d = 0; d < 6; d++) p[6 * size_t(q.x + threadIdx.x) + d] *= v;
-        }
-        __syncthreads();
-    }
-    // loop 2, oldest first
-    for (int j = 0; j < c.m; j++) {
-        const int slot = ring_slot(c, H, j);
-        for (int b = 0; b < nchunk; b++) {
-            const int4 q = t.nblk[r.x + b];
-            const double v = chunk_dot(hist_slot(Y, stride, slot), p, q.x, q.y, sm);
-            if (threadIdx.x == 0) part[0][b] = v;
-        }
-        __syncthreads();
-        double acc[1];
-        chunk_sum<1>(part, nchunk, acc, sm);
-        if (threadIdx.x == 0) coef = alpha[j] - rho[size_t(inst) * H + slot] * acc[0];
-        __syncthreads();
-        const double k = coef;
-        const double* sv = hist_slot(S, stride, slot);
-        for (int b = 0; b < nchunk; b++) {
-            const int4 q = t.nblk[r.x + b];
-            if (int(threadIdx.x) < q.y)
-#pragma unroll
-                for (int d = 0; d < 6; d++) p[6 * size_t(q.x + threadIdx.x) + d] += sv[6 * size_t(q.x + threadIdx.x) + d] * k;
-        }
-        __syncthreads();
-    }
-    // finish: clamp (sim.cpp:188-190, 46) and <g, p>
-    for (int b = 0; b < nchunk; b++) {
-        const int4 q = t.nblk[r.x + b];
-        double acc[1] = {0};
-        if (int(threadIdx.x) < q.y) {
-            const size_t o = 6 * size_t(q.x + threadIdx.x);
-            const uint8_t* lk = t.locked + o;
-            double v[6];
-#pragma unroll
-            for (int k = 0; k < 6; k++) {
-                v[k] = -p[o + k];
-                if (lk[k]) v[k] = 0;
-            }
-            const double lt = sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
-            if (lt > mt) {
-                const double f = mt / lt;
-                v[0] *= f; v[1] *= f; v[2] *= f;
-            }
-            const double lr = sqrt(v[3] * v[3] + v[4] * v[4] + v[5] * v[5]);
-            if (lr > mr) {
-                const double f = mr / lr;
-                v[3] *= f; v[4] *= f; v[5] *= f;
-            }
-#pragma unroll
-            for (int k = 0; k < 6; k++) {
-                v[k] = lk[k] ? 0.0 : v[k];
-                p[o + k] = v[k];
-            }
-            acc[0] = dot6(g + o, v);
-        }
-        block_sum<1>(acc, sm);
-        if (threadIdx.x == 0) part[0][b] = acc[0];
-    }
-    __syncthreads();
-    double acc[1];
-    chunk_sum<1>(part, nchunk, acc, sm);
-    if (threadIdx.x == 0) dg[inst] = acc[0];
-}
-
-// ---- decisions the device takes itself ------------------------------------------------------
-// Not a descent direction (sim.cpp:191): steepest descent instead.  For the instances that
-// computed a direction and found dg >= 0: p = clamp(lock(-g)) and the partial of <g, p>.
-__global__ void __launch_bounds__(kBlock) k_descent_fix(DevTopo t, const SolveCtl* __restrict__ ctl,
-                                                        const double* __restrict__ dg, double* __restrict__ p,
-                                                        const double* __restrict__ g, double mt, double mr,
-                                                        double* __restrict__ part) {
-    __shared__ double sm[kBlock / 32];
-    const MapPos mp = map_pos(t.nblk);
-    if (!(ctl[mp.inst].flags & (kOpDirection | kOpDirFused)) || dg[mp.inst] < 0) return;  // block-uniform
-    double acc[1] = {0};
-    if (mp.valid) {
-        const size_t b = 6 * size_t(mp.i);
-        const uint8_t* lk = t.locked + b;
-        double v[6];
-#pragma unroll
-        for (int k = 0; k < 6; k++) v[k] = lk[k] ? 0.0 : -g[b + k];
-        const double lt = sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
-        if (lt > mt) {
-            const double f = mt / lt;
-            v[0] *= f; v[1] *= f; v[2] *= f;
-        }
-        const double lr = sqrt(v[3] * v[3] + v[4] * v[4] + v[5] * v[5]);
-        if (lr > mr) {
-            const double f = mr / lr;
-            v[3] *= f; v[4] *= f; v[5] *= f;
-        }
-#pragma unroll
-        for (int k = 0; k < 6; k++) {
-            v[k] = lk[k] ? 0.0 : v[k];
-            p[b + k] = v[k];
-        }
-        acc[0] = dot6(g + b, v);
-    }
-    block_sum<1>(acc, sm);
-    if (threadIdx.x == 0) part[blockIdx.x] = acc[0];
-}
-// ... and per instance: the new dg and the history cleared (m = 0).
-__global__ void __launch_bounds__(kBlock) k_descent_final(DevTopo t, const SolveCtl* __restrict__ ctl,
-                                                          const double* __restrict__ part, double* __restrict__ dg,
-                                                          int2* __restrict__ hist) {
-    __shared__ double sm[kBlock / 32];
-    const int inst = blockIdx.x;
-    if (!(ctl[inst].flags & (kOpDirection | kOpDirFused))) return;
-    if (dg[inst] < 0) return;
-    double acc[1];
-    instance_sum<1>(t, part, inst, acc, sm);
-    if (threadIdx.x == 0) {
-        dg[inst] = acc[0];
-        hist[inst].x = 0;
-    }
-}
-// The steepest-descent retry (sim.cpp:193-196) starts with an empty history.
-__global__ void k_clear_history(int I, const SolveCtl* __restrict__ ctl, int bits, int2* __restrict__ hist) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < I && (ctl[i].flags & bits)) hist[i] = make_int2(0, 0);
-}
-__global__ void k_clear_history_m(int I, const SolveCtl* __restrict__ ctl, int bits, int2* __restrict__ hist) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < I && (ctl[i].flags & bits)) hist[i].x = 0;
-}
-// History after an accepted step (sim.cpp:205-206): keep the pair when
-// s.y > 1e-12 sqrt(max(1e-30, s.s y.y)) (rho = 1 / s.y in its slot), else clear the history.
-__global__ void k_history_update(int I, int H, const SolveCtl* __restrict__ ctl, const double* __restrict__ dots3,
-                                 int2* __restrict__ hist, double* __restrict__ rho) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= I || !(ctl[i].flags & kOpAccept) || H <= 0) return;
-    const double sy = dots3[3 * i], ss = dots3[3 * i + 1], yy = dots3[3 * i + 2];
-    int2 h = hist[i];
-    if (sy > 1e-12 * sqrt(fmax(1e-30, ss * yy))) {
-        const int target = h.x < H ? (h.y + h.x) % H : h.y;
-        rho[size_t(i) * H + target] = 1 / sy;
+    block_part<3>(sy, ss, yy, 0, v.part + blockIdx.x, t.n_sblk, sm);
+    const int2 r = t.srange[inst];
+    if (!last_block(v.done + 4 * inst + 3, unsigned(r.y - r.x))) return;
+    part_totals(v.part, t.n_sblk, r.x, r.y - r.x, 3, total);
+    if (threadIdx.x == 32 && (c.flags & kOpPair))  // sim.cpp:186
+        v.h0[inst] = total[0] > 1e-20 && total[2] > 1e-20 ? clampd(total[0] / total[2], 1e-7, 1e4) : .10;
+    if (threadIdx.x != 0 || !(c.flags & kOpPair)) return;
+    int2 h = v.hist[inst];
+    if (total[0] > 1e-12 * sqrt(fmax(1e-30, total[1] * total[2]))) {
+        v.rho[size_t(inst) * H + target] = 1 / total[0];
         if (h.x == H) h.y = (h.y + 1) % H;
         else h.x++;
     } else {
         h.x = 0;
     }
-    hist[i] = h;
+    v.hist[inst] = h;
 }
 
 }  // namespace
 
-size_t lbfgs_part_doubles(int n_nblk) { return 4 * size_t(n_nblk) + 8; }
+size_t lbfgs_part_doubles(int n_sblk, int H) { return size_t(2 * H + 4) * size_t(n_sblk) + 8; }
 
-int fused_direction_limit() { return kFuseChunks; }
-
-void bl_direction_fused(const DevTopo& t, const SolveCtl* ctl, int2* hist, int H, double* p, const double* g,
-                        const double* S, const double* Y, long long stride, const double* rho, double* dg, double mt,
-                        double mr, cudaStream_t s) {
-    (k_direction_fused<<<t.I, kBlock, 0, s>>>(t, ctl, hist, H, p, g, S, Y, stride, rho, dg, mt, mr), note_launches(1));
+// Nodes per solver block of an instance of n nodes: one unit while that makes at most kSolveBlocks
+// blocks, else runs that keep every thread busy.
+int solve_block_nodes(int n) {
+    if (n <= kUnit * kSolveBlocks) return kUnit;
+    constexpr int step = kThreads / 2;
+    const int steps = (n + step - 1) / step;
+    return step * ((steps + kSolveBlocks - 1) / kSolveBlocks);
 }
 
-void bl_direction_multi(const DevTopo& t, const SolveCtl* ctl, int2* hist, int H, double* p, const double* g,
-                        const double* S, const double* Y, long long stride, const double* rho, double* alpha,
-                        double* part, double* dg, double mt, double mr, cudaStream_t s) {
-    const int nb = t.n_nblk;
-    // partials: step dot products ping-pong between part and part + nb; H0's in part + 2 nb
-    double* pp[2] = {part, part + size_t(nb)};
-    double* h0part = part + 2 * size_t(nb);
-    (k_tl_start<<<nb, kBlock, 0, s>>>(t, ctl, hist, H, p, g, S, Y, stride, h0part, pp[0]), note_launches(1));
-    for (int j = 0; j < H; j++)
-        (k_tl_step<1><<<nb, kBlock, 0, s>>>(t, ctl, hist, H, j, p, S, Y, stride, rho, alpha, pp[j & 1],
-                                            pp[(j + 1) & 1]),
-         note_launches(1));
-    (k_tl_scale<<<nb, kBlock, 0, s>>>(t, ctl, hist, H, p, Y, stride, h0part, pp[0]), note_launches(1));
-    for (int j = 0; j < H; j++)
-        (k_tl_step<2><<<nb, kBlock, 0, s>>>(t, ctl, hist, H, j, p, S, Y, stride, rho, alpha, pp[j & 1],
-                                            pp[(j + 1) & 1]),
-         note_launches(1));
-    (k_finish<<<nb, kBlock, 0, s>>>(t, ctl, kOpDirection, p, p, g, mt, mr, part), note_launches(1));
-    (k_inst_final<1><<<t.I, kBlock, 0, s>>>(t, ctl, kOpDirection, part, dg), note_launches(1));
+void bl_direction(const DevTopo& t, const SolveCtl* ctl, const LbfgsBufs& v, cudaStream_t s) {
+    (k_dir_dots<<<dim3(unsigned(t.n_sblk), unsigned((v.H + kDotPairs - 1) / kDotPairs)), kThreads, 0, s>>>(t, ctl, v), note_launches(1));
+    (k_dir_first<<<t.n_sblk, kThreads, 0, s>>>(t, ctl, v), note_launches(1));
+    (k_dir_second<<<t.n_sblk, kThreads, 0, s>>>(t, ctl, v), note_launches(1));
 }
 
-void bl_descent_fix(const DevTopo& t, const SolveCtl* ctl, int2* hist, double* p, const double* g, double* part,
-                    double* dg, double mt, double mr, cudaStream_t s) {
-    // not a descent direction: steepest descent, history cleared (sim.cpp:191)
-    (k_descent_fix<<<t.n_nblk, kBlock, 0, s>>>(t, ctl, dg, p, g, mt, mr, part), note_launches(1));
-    (k_descent_final<<<t.I, kBlock, 0, s>>>(t, ctl, part, dg, hist), note_launches(1));
+void bl_steepest(const DevTopo& t, const SolveCtl* ctl, const LbfgsBufs& v, cudaStream_t s) {
+    (k_steepest<<<t.n_sblk, kThreads, 0, s>>>(t, ctl, v), note_launches(1));
 }
 
-void bl_direction(const DevTopo& t, const SolveCtl* ctl, int2* hist, int H, bool multi, double* p, const double* g,
-                  const double* S, const double* Y, long long stride, const double* rho, double* alpha, double* part,
-                  double* dg, double mt, double mr, cudaStream_t s) {
-    bl_direction_fused(t, ctl, hist, H, p, g, S, Y, stride, rho, dg, mt, mr, s);
-    if (multi) bl_direction_multi(t, ctl, hist, H, p, g, S, Y, stride, rho, alpha, part, dg, mt, mr, s);
-    bl_descent_fix(t, ctl, hist, p, g, part, dg, mt, mr, s);
+void bl_prepare(const DevTopo& t, const SolveCtl* ctl, const LbfgsBufs& v, cudaStream_t s) {
+    (k_prepare<<<t.n_eblk, kEvalBlock, 0, s>>>(t, ctl, v), note_launches(1));
 }
 
-void bl_steepest(const DevTopo& t, const SolveCtl* ctl, int2* hist, double* p, const double* g, double* part,
-                 double* dg, double mt, double mr, cudaStream_t s) {
-    (k_clear_history_m<<<(t.I + kBlock - 1) / kBlock, kBlock, 0, s>>>(t.I, ctl, kOpSteepest, hist), note_launches(1));
-    (k_finish<<<t.n_nblk, kBlock, 0, s>>>(t, ctl, kOpSteepest, p, g, g, mt, mr, part), note_launches(1));
-    (k_inst_final<1><<<t.I, kBlock, 0, s>>>(t, ctl, kOpSteepest, part, dg), note_launches(1));
-}
-
-void bl_prepare(const DevTopo& t, const SolveCtl* ctl, int2* hist, double* z, double* best, double* zeval,
-                const double* p, double* zfinal, cudaStream_t s) {
-    (k_clear_history<<<(t.I + kBlock - 1) / kBlock, kBlock, 0, s>>>(t.I, ctl, kOpResetHistory, hist),
-     note_launches(1));
-    (k_prepare<<<t.n_nblk, kBlock, 0, s>>>(t, ctl, z, best, zeval, p, zfinal), note_launches(1));
-}
-
-void bl_accept(const DevTopo& t, const SolveCtl* ctl, int2* hist, int H, double* z, double* g, const double* zeval,
-               const double* geval, double* S, double* Y, long long stride, double* best, double* rho, double* part,
-               double* out3, cudaStream_t s) {
-    (k_accept<<<t.n_nblk, kBlock, 0, s>>>(t, ctl, hist, H, z, g, zeval, geval, S, Y, stride, best, part),
-     note_launches(1));
-    (k_inst_final<3><<<t.I, kBlock, 0, s>>>(t, ctl, kOpAccept, part, out3), note_launches(1));
-    (k_history_update<<<(t.I + kBlock - 1) / kBlock, kBlock, 0, s>>>(t.I, H, ctl, out3, hist, rho), note_launches(1));
+void bl_accept(const DevTopo& t, const SolveCtl* ctl, const LbfgsBufs& v, cudaStream_t s) {
+    (k_accept<<<t.n_sblk, kThreads, 0, s>>>(t, ctl, v), note_launches(1));
 }
 
 }  // namespace mcg
-

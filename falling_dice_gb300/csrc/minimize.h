@@ -87,10 +87,10 @@ MCG_HD inline void mz_iterate(const MzParams& p, Minimizer& s) {
 
 // Stage A: the operation of the instance's search direction, two-loop (sim.cpp:184-190) or
 // the steepest-descent retry (:193-196); 0 when the instance computes none this round.
-MCG_HD inline int mz_stage_direction(Minimizer& s, bool fused) {
+MCG_HD inline int mz_stage_direction(Minimizer& s) {
     using M = Minimizer;
     int flags;
-    if (s.phase == M::kDirection) flags = fused ? kOpDirFused : kOpDirection;
+    if (s.phase == M::kDirection) flags = kOpDirection;
     else if (s.phase == M::kSteepest) flags = kOpSteepest;
     else return 0;
     s.phase = M::kTrial;  // first trial of the new direction, step 1
@@ -204,7 +204,6 @@ struct MzStatus {
 struct MzDev {
     int I;
     Minimizer* mins;         // [I]
-    const uint8_t* fused;    // [I] the instance's direction is computed by one CTA
     SolveCtl* ctl;           // [I]
     uint8_t* active;         // [I] evaluated this round
     uint8_t* trial_inst;     // [I] writes trial states this round
@@ -216,9 +215,9 @@ struct MzDev {
     int round_cap;           // rounds a launch may run before it returns to the host
 };
 // Stage kernels of one round; each sets the conditional handles of the graph nodes that
-// follow it (directions of each kind; the accept step; the loop).
-void launch_mz_direction(const MzDev& d, cudaGraphConditionalHandle h_fused, cudaGraphConditionalHandle h_multi,
-                         cudaGraphConditionalHandle h_dir, cudaGraphConditionalHandle h_sd, cudaStream_t s);
+// follow it (directions, steepest-descent retries; the accept step; the loop).
+void launch_mz_direction(const MzDev& d, cudaGraphConditionalHandle h_dir, cudaGraphConditionalHandle h_sd,
+                         cudaStream_t s);
 void launch_mz_eval(const MzDev& d, cudaStream_t s);
 void launch_mz_decide(const MzDev& d, const MzParams& p, cudaGraphConditionalHandle h_post,
                       cudaGraphConditionalHandle h_loop, cudaStream_t s);

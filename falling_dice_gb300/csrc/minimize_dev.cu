@@ -29,28 +29,22 @@ __device__ __forceinline__ void stage_mark(MzStatus* st, unsigned long long* acc
     st->t_last = t;
 }
 
-__global__ void __launch_bounds__(kMzThreads) k_mz_direction(MzDev d, cudaGraphConditionalHandle h_fused,
-                                                             cudaGraphConditionalHandle h_multi,
-                                                             cudaGraphConditionalHandle h_dir,
+__global__ void __launch_bounds__(kMzThreads) k_mz_direction(MzDev d, cudaGraphConditionalHandle h_dir,
                                                              cudaGraphConditionalHandle h_sd) {
-    int fused = 0, multi = 0, sd = 0;
+    int dir = 0, sd = 0;
     for (int i = threadIdx.x; i < d.I; i += blockDim.x) {
         Minimizer s = d.mins[i];
-        const int f = mz_stage_direction(s, d.fused[i] != 0);
+        const int f = mz_stage_direction(s);
         if (f) d.mins[i] = s;
         d.ctl[i] = SolveCtl{0.0, f, 0, 0, 0};
-        fused |= f == kOpDirFused;
-        multi |= f == kOpDirection;
+        dir |= f == kOpDirection;
         sd |= f == kOpSteepest;
     }
-    fused = __syncthreads_or(fused);
-    multi = __syncthreads_or(multi);
+    dir = __syncthreads_or(dir);
     sd = __syncthreads_or(sd);
     if (threadIdx.x == 0) {
         stage_mark(d.status, &d.status->t_post);
-        cudaGraphSetConditional(h_fused, fused ? 1u : 0u);
-        cudaGraphSetConditional(h_multi, multi ? 1u : 0u);
-        cudaGraphSetConditional(h_dir, (fused | multi) ? 1u : 0u);
+        cudaGraphSetConditional(h_dir, dir ? 1u : 0u);
         cudaGraphSetConditional(h_sd, sd ? 1u : 0u);
     }
 }
@@ -117,9 +111,9 @@ __global__ void k_mz_reset(MzStatus* st) {
 
 }  // namespace
 
-void launch_mz_direction(const MzDev& d, cudaGraphConditionalHandle h_fused, cudaGraphConditionalHandle h_multi,
-                         cudaGraphConditionalHandle h_dir, cudaGraphConditionalHandle h_sd, cudaStream_t s) {
-    k_mz_direction<<<1, kMzThreads, 0, s>>>(d, h_fused, h_multi, h_dir, h_sd);
+void launch_mz_direction(const MzDev& d, cudaGraphConditionalHandle h_dir, cudaGraphConditionalHandle h_sd,
+                         cudaStream_t s) {
+    k_mz_direction<<<1, kMzThreads, 0, s>>>(d, h_dir, h_sd);
     note_launches(1);
 }
 

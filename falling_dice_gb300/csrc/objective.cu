@@ -17,7 +17,7 @@
 
 namespace mcg {
 
-static_assert(kMapBlock == kBlock, "mapped blocks are launched with kBlock threads");
+static_assert(kMapBlock == kBlock, "the mixed form's beam blocks are launched with kBlock threads");
 
 // ---- node state: MC/src/sim.cpp:136 -------------------------------------------------------
 // Bound by the FP64 pipe like the beam kernel: rotations up to one radian by polynomials
@@ -669,13 +669,13 @@ __global__ void __launch_bounds__(kBlock) k_finalize(DevTopo t, PhysParams p, Ev
         out->kernel_error = *e.err;
         if (flags) flags[0] = flags[1] = 0;  // for the next evaluation
     }
-    const int4 r = t.irange[inst];
+    const int2 r = t.brange[inst];
     const int2 er = t.erange[inst];
-    const int fan = (r.w - r.z) + (er.y - er.x) <= kFinSingle ? 1 : kFinFan;
+    const int fan = (r.y - r.x) + (er.y - er.x) <= kFinSingle ? 1 : kFinFan;
     if (!t.active[inst] || f >= fan) return;
     double all[9] = {};  // sums: beamE, elastic, plastic, gravityE, platenE, reaction, contactE, contacts, |g|^2
     long long m2[2] = {0, 0};  // max penetration, max |g| (bits of non-negative doubles)
-    for (int k = r.z + f + fan * int(threadIdx.x); k < r.w; k += fan * int(blockDim.x)) {
+    for (int k = r.x + f + fan * int(threadIdx.x); k < r.y; k += fan * int(blockDim.x)) {
         const double* q = e.part_beam + 3 * size_t(k);
         all[0] += q[0]; all[1] += q[1]; all[2] += q[2];
     }
@@ -765,11 +765,11 @@ __global__ void __launch_bounds__(kBlock) k_finalize(DevTopo t, PhysParams p, Ev
 }
 
 // ---- commit (MC/src/sim.cpp:212): base state <- current state, plastic <- trial ----------
-__global__ void __launch_bounds__(kBlock) k_commit_nodes(DevTopo t, const uint8_t* __restrict__ mask,
+__global__ void __launch_bounds__(kEvalBlock) k_commit_nodes(DevTopo t, const uint8_t* __restrict__ mask,
                                                          const double4_32a* __restrict__ x4,
                                                          const double4_32a* __restrict__ R4, double* __restrict__ bx,
                                                          double* __restrict__ br) {
-    const MapPos mp = map_pos(t.nblk);
+    const MapPos mp = map_pos(t.eblk);
     if (!mp.valid || (mask && !mask[mp.inst])) return;
     const int i = mp.i;
     const double4_32a x = x4[i], r = R4[i];
@@ -819,10 +819,10 @@ __global__ void __launch_bounds__(kBlock) k_plastic_final(DevTopo t, const doubl
                                                           double* __restrict__ out) {
     __shared__ double sm[4 * (kBlock / 32)];
     __shared__ double smx[kBlock / 32];
-    const int4 r = t.irange[blockIdx.x];
+    const int2 r = t.brange[blockIdx.x];
     double acc[4] = {0, 0, 0, 0};
     double m0 = 0, m1 = 0;
-    for (int k = r.z + int(threadIdx.x); k < r.w; k += blockDim.x) {
+    for (int k = r.x + int(threadIdx.x); k < r.y; k += blockDim.x) {
         const double* q = part + 6 * size_t(k);
         acc[0] += q[0]; acc[1] += q[2]; acc[2] += q[4]; acc[3] += q[5];
         m0 = fmax(m0, q[1]); m1 = fmax(m1, q[3]);
@@ -867,7 +867,7 @@ void launch_center(const DevTopo& t, const PhysParams& p, const BuildArgs& b, Ev
 
 void launch_commit(const DevTopo& t, const uint8_t* mask, const EvalBufs& e, double* base_x, double* base_r,
                    double* plastic, cudaStream_t s) {
-    k_commit_nodes<<<t.n_nblk, kBlock, 0, s>>>(t, mask, e.x, e.R, base_x, base_r);
+    k_commit_nodes<<<t.n_eblk, kEvalBlock, 0, s>>>(t, mask, e.x, e.R, base_x, base_r);
     note_launches(1);
     if (t.B > 0 && plastic) {
         k_commit_plastic<<<t.n_bblk, t.bdim, 0, s>>>(t, mask, e.trial_next, plastic);

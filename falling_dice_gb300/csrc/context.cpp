@@ -256,7 +256,6 @@ struct mcg_ctx {
         for (cudaEvent_t& e : fork_ev) ck(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
         ck(cudaStreamCreateWithPriority(&fork, cudaStreamNonBlocking, greatest), "cudaStreamCreate");
     }
-    cudaStream_t side = nullptr;  // captures the bodies of the loop's conditional nodes
     bool device_loop = true;
     std::string loop_error;
     static constexpr int kLoopRoundCap = 4096;
@@ -292,7 +291,6 @@ struct mcg_ctx {
         drop_graphs();
         for (auto& e : ev_t)
             if (e) cudaEventDestroy(e);
-        if (side) cudaStreamDestroy(side);
         if (fork) cudaStreamDestroy(fork);
         for (cudaEvent_t e : fork_ev)
             if (e) cudaEventDestroy(e);
@@ -643,21 +641,17 @@ struct mcg_ctx {
         const LbfgsBufs L = lbfgs();
         // A. search directions: two-loop (sim.cpp:184-190), or steepest descent for the retry
         //    after a failed line search (:193-196)
-        bool any_dir = false, any_sd = false;
+        bool any_dir = false;
         clear_ctl(0);
         SolveCtl* ca = ctl_stage(0);
         for (int i = 0; i < I; i++) {
-            const int f = mz_stage_direction(mins[size_t(i)]);
-            ca[i].flags = f;
-            any_dir |= f == kOpDirection;
-            any_sd |= f == kOpSteepest;
+            ca[i].flags = mz_stage_direction(mins[size_t(i)]);
+            any_dir |= ca[i].flags != 0;
+            mz_directed(mins[size_t(i)]);
         }
-        if (any_dir || any_sd) {
+        if (any_dir) {
             upload_ctl(0);
-            replay(1 | (any_dir ? 2 : 0) | (any_sd ? 4 : 0), [&] {
-                if (any_dir) bl_direction(topo, d_ctl, L, stream);
-                if (any_sd) bl_steepest(topo, d_ctl, L, stream);
-            });
+            replay(1, [&] { bl_direction(topo, d_ctl, L, stream); });
         }
         // B. one evaluation per instance: the start point, a line-search candidate
         //    (sim.cpp:179) or the final state with trials (sim.cpp:210)
@@ -701,33 +695,6 @@ struct mcg_ctx {
         return true;
     }
 
-    // Adds, to the graph being captured on `stream`, an IF node on handle h whose body is
-    // what inner(side) launches (captured on the side stream).
-    template <typename F>
-    void capture_if(cudaGraphConditionalHandle h, F&& inner) {
-        cudaStreamCaptureStatus st;
-        cudaGraph_t g = nullptr;
-        const cudaGraphNode_t* deps = nullptr;
-        const cudaGraphEdgeData* edges = nullptr;
-        size_t nd = 0;
-        ck(cudaStreamGetCaptureInfo(stream, &st, nullptr, &g, &deps, &edges, &nd), "cudaStreamGetCaptureInfo");
-        cudaGraphNodeParams prm{};
-        prm.type = cudaGraphNodeTypeConditional;
-        prm.conditional.handle = h;
-        prm.conditional.type = cudaGraphCondTypeIf;
-        prm.conditional.size = 1;
-        cudaGraphNode_t node;
-        ck(cudaGraphAddNode(&node, g, deps, edges, nd, &prm), "cudaGraphAddNode (IF)");
-        cudaGraph_t body = prm.conditional.phGraph_out[0];
-        ck(cudaStreamUpdateCaptureDependencies(stream, &node, nullptr, 1, cudaStreamSetCaptureDependencies),
-           "cudaStreamUpdateCaptureDependencies");
-        ck(cudaStreamBeginCaptureToGraph(side, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal),
-           "cudaStreamBeginCaptureToGraph");
-        inner(side);
-        cudaGraph_t out = nullptr;
-        ck(cudaStreamEndCapture(side, &out), "cudaStreamEndCapture (IF body)");
-    }
-
     MzDev mz_dev() {
         MzDev d{};
         d.I = I;
@@ -744,11 +711,10 @@ struct mcg_ctx {
         return d;
     }
 
-    // The round loop as one graph: WHILE(loop) { A; IF(any direction) directions; IF(steepest)
-    // retry; B; prepare; evaluation (trial states per instance); C; IF(accept) accept step }.
+    // The round loop as one graph: WHILE(loop) { directions; preparation; evaluation (trial states
+    // per instance); decisions; accept step }, after the directions' kind of the first round.
     void build_loop() {
         make_fork();
-        if (!side) ck(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking), "cudaStreamCreate");
         const LbfgsBufs L = lbfgs();
         const MzDev md = mz_dev();
         const MzParams P = mz_params();
@@ -765,21 +731,15 @@ struct mcg_ctx {
             cudaGraphNode_t wnode;
             ck(cudaGraphAddNode(&wnode, g, nullptr, nullptr, 0, &wp), "cudaGraphAddNode (WHILE)");
             cudaGraph_t body = wp.conditional.phGraph_out[0];
-            cudaGraphConditionalHandle hd, hs, hpost;
-            for (cudaGraphConditionalHandle* h : {&hd, &hs, &hpost})
-                ck(cudaGraphConditionalHandleCreate(h, body, 0, cudaGraphCondAssignDefault), "conditional handle");
             const long long before = g_launch_count.load();
             ck(cudaStreamBeginCaptureToGraph(stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal),
                "cudaStreamBeginCaptureToGraph");
             try {
-                launch_mz_direction(md, hd, hs, stream);
-                capture_if(hd, [&](cudaStream_t s2) { bl_direction(topo, d_ctl, L, s2); });
-                capture_if(hs, [&](cudaStream_t s2) { bl_steepest(topo, d_ctl, L, s2); });
-                launch_mz_eval(md, stream);
-                bl_prepare(topo, d_ctl, L, stream);
+                bl_direction(topo, d_ctl, L, stream, d_mz);
+                bl_prepare(topo, nullptr, L, stream, &md);
                 eval_launches(d_zeval, 2, d_geval, true);
-                launch_mz_decide(md, P, hpost, h_loop, stream);
-                capture_if(hpost, [&](cudaStream_t s2) { bl_accept(topo, d_ctl, L, s2); });
+                launch_mz_decide(md, P, h_loop, stream);
+                bl_accept(topo, d_ctl + I, L, stream);
             } catch (...) {
                 cudaGraph_t junk = nullptr;
                 cudaStreamEndCapture(stream, &junk);
@@ -808,7 +768,7 @@ struct mcg_ctx {
             if (!loop_exec) build_loop();
             std::copy(mins.begin(), mins.end(), hp.mins);
             h2d(d_mins, hp.mins, size_t(I), stream);
-            launch_mz_reset(mz_dev(), stream);
+            launch_mz_begin(mz_dev(), stream);
             const auto w0 = std::chrono::steady_clock::now();
             ck(cudaGraphLaunch(loop_exec, stream), "cudaGraphLaunch (loop)");
             d2h(hp.mins, d_mins, size_t(I), stream);
@@ -1560,7 +1520,7 @@ void upload_instances(mcg_ctx* c, const std::vector<InstIn>& ins) {
     c->d_dg = Q.get<double>(size_t(I));
     c->d_h0 = Q.get<double>(size_t(I));
     c->d_pstats = Q.get<double>(6 * size_t(I));
-    c->d_ctl = Q.get<SolveCtl>(size_t(I));
+    c->d_ctl = Q.get<SolveCtl>(2 * size_t(I));
     c->d_hist = Q.get<int2>(size_t(I));
     ck(cudaMemsetAsync(c->d_hist, 0, size_t(I) * sizeof(int2), s), "memset");
     ck(cudaMemsetAsync(c->d_rho, 0, size_t(I) * Hs * sizeof(double), s), "memset");

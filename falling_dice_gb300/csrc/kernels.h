@@ -359,18 +359,19 @@ struct LbfgsBufs {
     unsigned* done;      // [4 I] blocks that have arrived, per pass; zero between passes
     double mt, mr;       // largest translation (in units of the scale) and rotation of a step
 };
+struct MzStatus;  // minimize.h
+struct MzDev;
 size_t lbfgs_part_doubles(int n_sblk, int H);
 // Nodes per solver block of an instance of n nodes.
 int solve_block_nodes(int n);
-// Two-loop recursion (sim.cpp:184-187) into p for the kOpDirection instances; then
-// p = clamp(lock(-p)) and dg = <g, p>; where not dg < 0, steepest descent with the history
-// cleared (sim.cpp:191).
-void bl_direction(const DevTopo& t, const SolveCtl* ctl, const LbfgsBufs& v, cudaStream_t s);
-// The steepest-descent retry for the kOpSteepest instances: history cleared,
-// p = clamp(lock(-g)), dg = <g, p> (sim.cpp:193-196).
-void bl_steepest(const DevTopo& t, const SolveCtl* ctl, const LbfgsBufs& v, cudaStream_t s);
-// kOpResetHistory / kOpZero / kOpRestore / kOpKeepBest / kOpCandidate / kOpEvalAtZ / kOpFinal
-void bl_prepare(const DevTopo& t, const SolveCtl* ctl, const LbfgsBufs& v, cudaStream_t s);
+// Two-loop recursion (sim.cpp:184-187) into p for the kOpDirection instances, then
+// p = clamp(lock(-p)) and dg = <g, p>; where not dg < 0, and for the kOpSteepest instances (the
+// retry, sim.cpp:193-196), p = clamp(lock(-g)) with the history cleared (sim.cpp:191).
+// st: the loop's status, for its stage times.
+void bl_direction(const DevTopo& t, const SolveCtl* ctl, const LbfgsBufs& v, cudaStream_t s, MzStatus* st = nullptr);
+// kOpResetHistory / kOpZero / kOpRestore / kOpKeepBest / kOpCandidate / kOpEvalAtZ / kOpFinal as ctl
+// says, or as the device-resident minimizers of d say.
+void bl_prepare(const DevTopo& t, const SolveCtl* ctl, const LbfgsBufs& v, cudaStream_t s, const MzDev* d = nullptr);
 // kOpTakeGrad / kOpAccept (+kOpPair, kOpKeepBestAfter), h0 and the history
 // update of the accepted instances (sim.cpp:205-206).
 void bl_accept(const DevTopo& t, const SolveCtl* ctl, const LbfgsBufs& v, cudaStream_t s);

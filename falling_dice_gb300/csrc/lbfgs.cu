@@ -33,7 +33,7 @@
 // With 64 blocks an instance 32x32x16 takes 98 us a direction, with 152 51; with 304 55 (the last
 // block's totals).
 #include "common.cuh"
-#include "kernels.h"
+#include "minimize.h"
 
 namespace mcg {
 
@@ -128,7 +128,8 @@ __device__ __forceinline__ void part_totals(const double* part, size_t stride, i
 // Block (b, k): the partials of <s, g> and <s, y_new> for history pairs 4 k ... 4 k + 3; the last
 // block of the instance stores the newest column of the products and solves the first loop's
 // alphas, newest to oldest: alpha_i = rho_i (<s_i, g> - sum_{j > i} alpha_j <s_i, y_j>).
-__global__ void __launch_bounds__(kThreads) k_dir_dots(DevTopo t, const SolveCtl* __restrict__ ctl, LbfgsBufs v) {
+__global__ void __launch_bounds__(kThreads) k_dir_dots(DevTopo t, const SolveCtl* __restrict__ ctl, LbfgsBufs v, MzStatus* st) {
+    if (st && threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0) stage_mark(st, &st->t_post);
     __shared__ double sm[4][kWarps];
     __shared__ double val[2 * 64], R[kSmallHistory][kSmallHistory + 1];
     const int H = v.H;
@@ -335,7 +336,8 @@ __device__ __forceinline__ double steepest_part(const DevTopo& t, const double* 
 // ---- direction, third pass ------------------------------------------------------------------
 // p = clamp(lock(-(H0 q + sum c_i s_i))) and the partial of <g, p>; the last block of the instance
 // sums dg.  Not a descent direction (sim.cpp:191): that block takes steepest descent instead and
-// clears the history.
+// clears the history.  Instances of the steepest-descent retry (kOpSteepest, sim.cpp:193-196) take
+// p = clamp(lock(-g)) with the history cleared here as well.
 __global__ void __launch_bounds__(kThreads) k_dir_second(DevTopo t, const SolveCtl* __restrict__ ctl, LbfgsBufs v) {
     __shared__ double sm[4][kWarps];
     __shared__ double co[64], total[1];
@@ -343,13 +345,14 @@ __global__ void __launch_bounds__(kThreads) k_dir_second(DevTopo t, const SolveC
     const int4 q = t.sblk[blockIdx.x];
     const int inst = q.z;
     const SolveCtl c = load_ctl(ctl, v.hist, inst);
-    if (!(c.flags & kOpDirection)) return;
+    if (!(c.flags & (kOpDirection | kOpSteepest))) return;
+    const bool steepest = c.flags & kOpSteepest;
     const int m = c.m;
     for (int i = threadIdx.x; i < m; i += kThreads) co[i] = v.coef[size_t(inst) * H + i];
     const double h0 = initial_scale(v, inst, m);
     __syncthreads();
-    double d = 0;
-    for (int i = threadIdx.x; i < 2 * q.y; i += kThreads) {
+    double d = steepest ? steepest_part(t, v.g, v.p, q.x, 2 * q.y, v.mt, v.mr) : 0;
+    for (int i = steepest ? 2 * q.y : threadIdx.x; i < 2 * q.y; i += kThreads) {
         const size_t o = 6 * size_t(q.x) + 3 * size_t(i);
         d3 a = ld3(v.p + o);
         if (m <= kRegHistory) {  // every load in flight at once
@@ -376,30 +379,15 @@ __global__ void __launch_bounds__(kThreads) k_dir_second(DevTopo t, const SolveC
     if (!last_block(v.done + 4 * inst + 2, unsigned(nb))) return;
     part_totals(v.part, t.n_sblk, r.x, nb, 1, total);
     const double dg = total[0];
-    if (dg < 0) {
-        if (threadIdx.x == 0) v.dg[inst] = dg;
+    if (steepest || dg < 0) {
+        if (threadIdx.x == 0) {
+            v.dg[inst] = dg;
+            if (steepest) v.hist[inst].x = 0;
+        }
         return;
     }
     const double e = steepest_part(t, v.g, v.p, t.sblk[r.x].x, 2 * t.inst_n[inst], v.mt, v.mr);
     block_part<1>(e, 0, 0, 0, total, 1, sm);
-    if (threadIdx.x == 0) {
-        v.dg[inst] = total[0];
-        v.hist[inst].x = 0;
-    }
-}
-
-// The steepest-descent retry (sim.cpp:193-196): history cleared, p = clamp(lock(-g)), dg.
-__global__ void __launch_bounds__(kThreads) k_steepest(DevTopo t, const SolveCtl* __restrict__ ctl, LbfgsBufs v) {
-    __shared__ double sm[4][kWarps];
-    __shared__ double total[1];
-    const int4 q = t.sblk[blockIdx.x];
-    const int inst = q.z;
-    if (!(ctl[inst].flags & kOpSteepest)) return;
-    const double d = steepest_part(t, v.g, v.p, q.x, 2 * q.y, v.mt, v.mr);
-    block_part<1>(d, 0, 0, 0, v.part + blockIdx.x, t.n_sblk, sm);
-    const int2 r = t.srange[inst];
-    if (!last_block(v.done + 4 * inst + 2, unsigned(r.y - r.x))) return;
-    part_totals(v.part, t.n_sblk, r.x, r.y - r.x, 1, total);
     if (threadIdx.x == 0) {
         v.dg[inst] = total[0];
         v.hist[inst].x = 0;
@@ -411,11 +399,28 @@ __global__ void __launch_bounds__(kThreads) k_steepest(DevTopo t, const SolveCtl
 // best = z (kOpKeepBest), zeval = z + step p with locked entries 0 (kOpCandidate, sim.cpp:179)
 // or zeval = z (kOpEvalAtZ), zfinal = z (kOpFinal); a new minimization starts with an empty
 // history (kOpResetHistory).
-__global__ void __launch_bounds__(kEvalBlock) k_prepare(DevTopo t, const SolveCtl* __restrict__ ctl, LbfgsBufs v) {
+// In the device-resident loop (d.mins) the operations follow from the instance's minimizer, and
+// its first block writes what the evaluation reads: active and trial masks, platen height, and the
+// request for a new candidate list when the instance joins (its shapes have to be in it).
+__global__ void __launch_bounds__(kEvalBlock) k_prepare(DevTopo t, const SolveCtl* __restrict__ ctl, LbfgsBufs v, MzDev d) {
     const MapPos mp = map_pos(t.eblk);
-    const SolveCtl c = ctl[mp.inst];
-    if ((c.flags & kOpResetHistory) && threadIdx.x == 0 && int(blockIdx.x) == t.erange[mp.inst].x)
-        v.hist[mp.inst] = make_int2(0, 0);
+    const bool first = threadIdx.x == 0 && int(blockIdx.x) == t.erange[mp.inst].x;
+    SolveCtl c{};
+    if (d.mins) {
+        if (threadIdx.x == 0 && blockIdx.x == 0) stage_mark(d.status, &d.status->t_dir);
+        bool trials = false;
+        c.flags = mz_stage_eval(d.mins[mp.inst], c.step, trials);
+        if (first) {
+            const uint8_t a = c.flags ? 1 : 0;
+            if (a && !d.active[mp.inst] && d.contact_flags) d.contact_flags[2] = 1u;
+            d.active[mp.inst] = a;
+            d.trial_inst[mp.inst] = trials ? 1 : 0;
+            if (a) d.tops[mp.inst] = d.mins[mp.inst].top;
+        }
+    } else {
+        c = ctl[mp.inst];
+    }
+    if ((c.flags & kOpResetHistory) && first) v.hist[mp.inst] = make_int2(0, 0);
     if (!mp.valid || !(c.flags & (kOpZero | kOpRestore | kOpKeepBest | kOpCandidate | kOpEvalAtZ | kOpFinal))) return;
     const size_t o = 6 * size_t(mp.i);
     double a[6];
@@ -505,18 +510,15 @@ int solve_block_nodes(int n) {
     return step * ((steps + kSolveBlocks - 1) / kSolveBlocks);
 }
 
-void bl_direction(const DevTopo& t, const SolveCtl* ctl, const LbfgsBufs& v, cudaStream_t s) {
-    (k_dir_dots<<<dim3(unsigned(t.n_sblk), unsigned((v.H + kDotPairs - 1) / kDotPairs)), kThreads, 0, s>>>(t, ctl, v), note_launches(1));
+void bl_direction(const DevTopo& t, const SolveCtl* ctl, const LbfgsBufs& v, cudaStream_t s, MzStatus* st) {
+    (k_dir_dots<<<dim3(unsigned(t.n_sblk), unsigned((v.H + kDotPairs - 1) / kDotPairs)), kThreads, 0, s>>>(t, ctl, v, st),
+     note_launches(1));
     (k_dir_first<<<t.n_sblk, kThreads, 0, s>>>(t, ctl, v), note_launches(1));
     (k_dir_second<<<t.n_sblk, kThreads, 0, s>>>(t, ctl, v), note_launches(1));
 }
 
-void bl_steepest(const DevTopo& t, const SolveCtl* ctl, const LbfgsBufs& v, cudaStream_t s) {
-    (k_steepest<<<t.n_sblk, kThreads, 0, s>>>(t, ctl, v), note_launches(1));
-}
-
-void bl_prepare(const DevTopo& t, const SolveCtl* ctl, const LbfgsBufs& v, cudaStream_t s) {
-    (k_prepare<<<t.n_eblk, kEvalBlock, 0, s>>>(t, ctl, v), note_launches(1));
+void bl_prepare(const DevTopo& t, const SolveCtl* ctl, const LbfgsBufs& v, cudaStream_t s, const MzDev* d) {
+    (k_prepare<<<t.n_eblk, kEvalBlock, 0, s>>>(t, ctl, v, d ? *d : MzDev{}), note_launches(1));
 }
 
 void bl_accept(const DevTopo& t, const SolveCtl* ctl, const LbfgsBufs& v, cudaStream_t s) {

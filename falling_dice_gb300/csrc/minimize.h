@@ -87,17 +87,19 @@ MCG_HD inline void mz_iterate(const MzParams& p, Minimizer& s) {
 
 // Stage A: the operation of the instance's search direction, two-loop (sim.cpp:184-190) or
 // the steepest-descent retry (:193-196); 0 when the instance computes none this round.
-MCG_HD inline int mz_stage_direction(Minimizer& s) {
+MCG_HD inline int mz_stage_direction(const Minimizer& s) {
     using M = Minimizer;
-    int flags;
-    if (s.phase == M::kDirection) flags = kOpDirection;
-    else if (s.phase == M::kSteepest) flags = kOpSteepest;
-    else return 0;
-    s.phase = M::kTrial;  // first trial of the new direction, step 1
+    return s.phase == M::kDirection ? kOpDirection : s.phase == M::kSteepest ? kOpSteepest : 0;
+}
+
+// The instance's direction has been computed: its first trial, at step 1.
+MCG_HD inline void mz_directed(Minimizer& s) {
+    using M = Minimizer;
+    if (s.phase != M::kDirection && s.phase != M::kSteepest) return;
+    s.phase = M::kTrial;
     s.step = 1.0;
     s.bt = 0;
     s.fresh = true;
-    return flags;
 }
 
 // Stage B: what the instance evaluates this round; 0 when it evaluates nothing.
@@ -106,6 +108,10 @@ MCG_HD inline int mz_stage_eval(const Minimizer& s, double& step, bool& trials) 
     switch (s.phase) {
         case M::kStart:
             return kOpResetHistory | (s.zero_first ? kOpZero : 0) | kOpEvalAtZ | kOpKeepBest;
+        case M::kDirection:
+        case M::kSteepest:  // (directed, not yet recorded: mz_directed)
+            step = 1.0;
+            return kOpCandidate;
         case M::kTrial:
             step = s.step;
             return kOpCandidate;
@@ -124,6 +130,7 @@ MCG_HD inline int mz_stage_eval(const Minimizer& s, double& step, bool& trials) 
 MCG_HD inline int mz_stage_decide(const MzParams& p, Minimizer& s, const EvalOut& o, double dg) {
     using M = Minimizer;
     int flags = 0;
+    mz_directed(s);
     switch (s.phase) {
         case M::kStart:
             s.cur = o;
@@ -196,15 +203,14 @@ struct MzStatus {
     int overflow;   // the last evaluation overflowed a contact buffer (nothing was decided)
     int done;       // an instance finished its minimization
     int pad_;
-    // device time of the launch's rounds by stage (global timer, ns): directions (stage A
-    // to B), evaluations (B to C, with the vector preparation), decisions and accept steps
-    // (C to the next round's A); t_last is the last stage boundary
+    // device time of the launch's rounds by stage (global timer, ns): directions, evaluations (with
+    // the vector preparation), decisions and accept steps; t_last is the last stage boundary
     unsigned long long t_dir, t_eval, t_post, t_last;
 };
 struct MzDev {
     int I;
     Minimizer* mins;         // [I]
-    SolveCtl* ctl;           // [I]
+    SolveCtl* ctl;           // [2 I] directions; accept steps
     uint8_t* active;         // [I] evaluated this round
     uint8_t* trial_inst;     // [I] writes trial states this round
     double* tops;            // [I]
@@ -214,13 +220,19 @@ struct MzDev {
     MzStatus* status;
     int round_cap;           // rounds a launch may run before it returns to the host
 };
-// Stage kernels of one round; each sets the conditional handles of the graph nodes that
-// follow it (directions, steepest-descent retries; the accept step; the loop).
-void launch_mz_direction(const MzDev& d, cudaGraphConditionalHandle h_dir, cudaGraphConditionalHandle h_sd,
-                         cudaStream_t s);
-void launch_mz_eval(const MzDev& d, cudaStream_t s);
-void launch_mz_decide(const MzDev& d, const MzParams& p, cudaGraphConditionalHandle h_post,
-                      cudaGraphConditionalHandle h_loop, cudaStream_t s);
-void launch_mz_reset(const MzDev& d, cudaStream_t s);
+// Stage kernels: the directions of a launch's first round; the decisions of a round, which set the
+// accept steps, the next round's directions and the loop's condition.
+void launch_mz_begin(const MzDev& d, cudaStream_t s);
+void launch_mz_decide(const MzDev& d, const MzParams& p, cudaGraphConditionalHandle h_loop, cudaStream_t s);
+
+#ifdef __CUDACC__
+// Adds the time since the last stage boundary to *acc and moves the boundary (one thread).
+__device__ __forceinline__ void stage_mark(MzStatus* st, unsigned long long* acc) {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    if (st->t_last && acc) *acc += t - st->t_last;
+    st->t_last = t;
+}
+#endif
 
 }  // namespace mcg

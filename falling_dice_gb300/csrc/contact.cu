@@ -42,7 +42,10 @@ constexpr int kPairWarps = kPairThreads / 32;
 constexpr int kPairGroups = 4;           // groups of 32 shapes of a bin staged at a time
 constexpr int kChunk = 32 * kPairGroups;  // shapes of a unit of pair work (ContactBufs::units)
 constexpr int kLevelBits = 5;            // box levels inside a bin: 2^kLevelBits = 32 per axis
-constexpr int kStreamBlocks = 4 * 152;   // grid of the list kernels (256 threads, grid-stride)
+constexpr int kFilterBlocks = 4 * 152;   // 256 threads each, grid-stride
+constexpr int kListThreads = 128;        // the contact kernel: a warp per FP64 unit and block
+constexpr int kListWarps = kListThreads / 32;
+constexpr int kListBlocks = 5 * 152;
 
 __device__ __forceinline__ uint32_t spread3_10(uint32_t v) {  // 10 bits -> every third bit
     v &= 0x3ffu;
@@ -567,9 +570,9 @@ __global__ void __launch_bounds__(kPairThreads, 7) k_bin_pairs(DevTopo t, const 
     }
 }
 
-// Certified single-precision distance bounds of a candidate pair.  A pair certainly farther
-// apart than pad_a + pad_b (>= the reference's target ra + rb + margin) fails the reference's
-// test dist < target; a pair certainly closer than the target passes it.
+// Certified single-precision lower bound on the distance of a candidate pair.  A pair certainly
+// farther apart than pad_a + pad_b (>= the reference's target ra + rb + margin) fails the
+// reference's test dist < target; the others go to the exact test.
 //
 // For any unit vector n, the distance between segments p1 + s d1 and p2 + t d2 (s, t in
 // [0, 1]) is at least  L(n) = n.(p1 - p2) + min(0, n.d1) - max(0, n.d2):  n.(P - Q) <= |P - Q|
@@ -578,15 +581,12 @@ __global__ void __launch_bounds__(kPairThreads, 7) k_bin_pairs(DevTopo t, const 
 // sim.cpp:9-18), which makes the bound nearly tight.  L is evaluated from FP32 endpoints
 // rounded down (|error| <= 2^-23 X per coordinate, X the largest endpoint coordinate); the
 // rounding of the differences, the three dot products and the sums adds at most about
-// 4e-6 X in total, bounded here by 3e-5 X + 1e-9 m, and |n| = 1 up to 1e-6.  A pair that
-// cannot be certified (touching segments, non-finite data) goes to the exact test.
+// 4e-6 X in total, bounded here by 3e-5 X + 1e-9 m, and |n| = 1 up to 1e-6.  Nothing is certified
+// of touching segments and non-finite data.
 struct DistBounds {
     bool far_ok;      // far is a valid lower bound (the closest points are not within 1e-7 m)
     float far;        // certified lower bound on the distance, already less its error
-    float near;       // certified upper bound on the distance between points at (s, tt)
-    bool near_ok;     // near bounds the reference's distance too (below)
     float pad_sum;    // pad_a + pad_b >= the reference's target
-    float target_lo;  // <= the reference's target ra + rb + margin
 };
 __device__ __forceinline__ DistBounds dist_bounds(const DevTopo& t, const PhysParams& p, const float4* __restrict__ xf,
                                                   uint32_t sa, uint32_t sb) {
@@ -629,14 +629,6 @@ __device__ __forceinline__ DistBounds dist_bounds(const DevTopo& t, const PhysPa
     const float err = 3e-5f * X + 1e-9f;
     DistBounds r;
     r.pad_sum = (pa + pb) * 1.000001f;
-    // the pads less one margin exceed the target by at most two FP32 roundings
-    r.target_lo = (pa + pb - float(p.contact_margin)) * 0.999999f;
-    // The reference takes s = 0 where a e - b^2 <= 1e-20, whatever the angle (sim.cpp:14): its points
-    // then lie up to sqrt(1e-20 / min(a, e)) farther apart than the closest ones.  Struts of a
-    // millimetre stay far inside the allowance; for tiny ones only the exact test can tell.
-    const float shorter = fminf(a, e);
-    r.near_ok = shorter == 0.f || err * err * shorter >= 1e-20f;
-    r.near = isfinite(nn) ? sqrtf(nn) * 1.000001f + err : __int_as_float(0x7f800000);
     r.far_ok = nn > 1e-14f;  // false also when not finite
     r.far = 0.f;
     if (r.far_ok) {
@@ -647,15 +639,6 @@ __device__ __forceinline__ DistBounds dist_bounds(const DevTopo& t, const PhysPa
         r.far = L * 0.999999f - err;
     }
     return r;
-}
-
-// -1: certainly no contact; +1: certainly within the target (if not a local pair); 0: only
-// the exact test can tell.
-__device__ __forceinline__ int distance_class(const DevTopo& t, const PhysParams& p, const float4* __restrict__ xf,
-                                              uint32_t sa, uint32_t sb) {
-    const DistBounds d = dist_bounds(t, p, xf, sa, sb);
-    if (d.near_ok && d.near < d.target_lo) return 1;
-    return d.far_ok && d.far > d.pad_sum ? -1 : 0;
 }
 
 constexpr int kBatch = 4;  // candidates per lane behind one list atomic
@@ -724,39 +707,6 @@ __global__ void __launch_bounds__(kBlock) k_filter(DevTopo t, PhysParams p, cons
     }
 }
 
-// Narrow phase over the filtered list: the pairs in contact (of the evaluated instances) are
-// appended to the contact list; more than its capacity raises kOverContacts.
-__global__ void __launch_bounds__(kBlock) k_narrow(DevTopo t, PhysParams p, const double4_32a* __restrict__ x,
-                                                   const float4* __restrict__ xf, ContactBufs c) {
-    const long long thread = (long long)blockIdx.x * blockDim.x + threadIdx.x, threads = (long long)gridDim.x * blockDim.x;
-    const int lane = threadIdx.x & 31;
-    const uint32_t total = uint32_t(min((long long)c.counts[kKept], c.cand_cap));
-    for (long long g0 = thread / 32 * 32; g0 < total; g0 += threads) {
-        bool hit = false;
-        uint2 q = make_uint2(0, 0);
-        if (g0 + lane < total) {
-            q = c.cand2[g0 + lane];  // not a local pair (k_filter)
-            if (t.I == 1 || t.active[t.node_inst[shape_nodes(t, q.x).x]]) {
-                const int cls = distance_class(t, p, xf, q.x, q.y);
-                if (cls > 0) hit = true;  // certainly within the target
-                else if (cls == 0) hit = narrow_phase(t, p, x, q.x, q.y).hit;
-            }
-        }
-        const unsigned m = __ballot_sync(0xffffffffu, hit);
-        if (!m) continue;  // warp-uniform
-        uint32_t base = 0;
-        if (lane == 0) {
-            base = atomicAdd(c.counts + kContacts, uint32_t(__popc(m)));
-            if ((long long)base + __popc(m) > c.contact_cap) atomicOr(c.flags, uint32_t(kOverContacts));
-        }
-        const long long at = (long long)__shfl_sync(0xffffffffu, base, 0) + __popc(m & ((1u << lane) - 1u));
-        if (hit && at < c.contact_cap) {
-            c.c_a[at] = q.x;
-            c.c_b[at] = q.y;
-        }
-    }
-}
-
 // Adds v to a fixed-point sum of quantum 2^e0 (kSumLimbs signed counters of 32 bits each, which
 // hold 2^31 additions): the 53-bit mantissa lands in at most three limbs, added with v's sign.
 // Bits below the quantum are dropped; false when v is not finite or beyond the top limb.
@@ -789,47 +739,107 @@ __device__ __forceinline__ bool add_fixed(long long* __restrict__ sum, double v,
     return ok;
 }
 
-// The contacts, one per thread (dense: the FP64 closest points run with full warps): the forces
-// of the penalty (sim.cpp:163-164, addShapeGradient sim.cpp:23: capsule ends split the force
-// (1 - u, u)) onto the nodes' fixed-point sums, the contact's energy, count and penetration onto
-// the first node of its lower shape.
-__global__ void __launch_bounds__(64) k_contacts(DevTopo t, PhysParams p, const double4_32a* __restrict__ x,
-                                                 ContactBufs c) {
-    const long long nc = min((long long)c.counts[kContacts], c.contact_cap);
-    for (long long o = (long long)blockIdx.x * blockDim.x + threadIdx.x; o < nc; o += (long long)gridDim.x * blockDim.x) {
-        const uint32_t sa = c.c_a[o], sb = c.c_b[o];
-        const PairHit h = narrow_phase(t, p, x, sa, sb);
-        if (!h.hit) continue;
-        const double mag = p.contact_k * h.pen;
-        bool ok = true;
+// One contact (or pair too close to tell from FP32 bounds; valid: the lane has one): the exact FP64
+// test, a place in the contact list, the forces of the penalty (sim.cpp:163-164, addShapeGradient
+// sim.cpp:23: capsule ends split the force (1 - u, u)) onto the nodes' fixed-point sums, the
+// contact's energy, count and penetration onto the first node of its lower shape.  All lanes of a
+// warp call it.
+__device__ __forceinline__ void add_contact(const DevTopo& t, const PhysParams& p, const double4_32a* __restrict__ x,
+                                            const ContactBufs& c, bool valid, uint2 q) {
+    const int lane = threadIdx.x & 31;
+    const uint32_t sa = q.x, sb = q.y;
+    PairHit h;
+    h.hit = false;
+    if (valid) h = narrow_phase(t, p, x, sa, sb);
+    const unsigned m = __ballot_sync(0xffffffffu, h.hit);
+    if (!m) return;  // warp-uniform
+    uint32_t base = 0;
+    if (lane == 0) {
+        base = atomicAdd(c.counts + kContacts, uint32_t(__popc(m)));
+        if ((long long)base + __popc(m) > c.contact_cap) atomicOr(c.flags, uint32_t(kOverContacts));
+    }
+    const long long at = (long long)__shfl_sync(0xffffffffu, base, 0) + __popc(m & ((1u << lane) - 1u));
+    if (!h.hit) return;
+    if (at < c.contact_cap) {
+        c.c_a[at] = sa;
+        c.c_b[at] = sb;
+    }
+    const double mag = p.contact_k * h.pen;
+    bool ok = true;
 #pragma unroll
-        for (int side = 0; side < 2; side++) {
-            const uint32_t shape = side ? sb : sa;
-            const bool capsule = shape >= uint32_t(t.N);
-            const int2 nd = shape_nodes(t, shape);
-            const d3 v = h.n * (side ? -mag : mag);
-            const double u = side ? h.t : h.s;
+    for (int side = 0; side < 2; side++) {
+        const uint32_t shape = side ? sb : sa;
+        const bool capsule = shape >= uint32_t(t.N);
+        const int2 nd = shape_nodes(t, shape);
+        const d3 v = h.n * (side ? -mag : mag);
+        const double u = side ? h.t : h.s;
 #pragma unroll
-            for (int end = 0; end < 2; end++) {
-                if (end && !capsule) break;
-                const int node = end ? nd.y : nd.x;
-                const d3 f = !capsule ? v : end ? v * u : v * (1 - u);
-                NodeContact& r = c.n_sum[node];
-                ok &= add_fixed(r.f[0], f.x, c.force_e0);
-                ok &= add_fixed(r.f[1], f.y, c.force_e0);
-                ok &= add_fixed(r.f[2], f.z, c.force_e0);
-                if (side == 0 && end == 0) {
-                    ok &= add_fixed(r.energy, .5 * p.contact_k * h.pen * h.pen, c.energy_e0);
-                    atomicMax(&r.pen, (unsigned long long)__double_as_longlong(h.pen));  // pen > 0
-                    atomicAdd(c.n_count + node, 1ULL | (1ULL << 32));
-                } else {
-                    atomicAdd(c.n_count + node, 1ULL);
-                }
+        for (int end = 0; end < 2; end++) {
+            if (end && !capsule) break;
+            const int node = end ? nd.y : nd.x;
+            const d3 f = !capsule ? v : end ? v * u : v * (1 - u);
+            NodeContact& r = c.n_sum[node];
+            ok &= add_fixed(r.f[0], f.x, c.force_e0);
+            ok &= add_fixed(r.f[1], f.y, c.force_e0);
+            ok &= add_fixed(r.f[2], f.z, c.force_e0);
+            if (side == 0 && end == 0) {
+                ok &= add_fixed(r.energy, .5 * p.contact_k * h.pen * h.pen, c.energy_e0);
+                atomicMax(&r.pen, (unsigned long long)__double_as_longlong(h.pen));  // pen > 0
+                atomicAdd(c.n_count + node, 1ULL | (1ULL << 32));
+            } else {
+                atomicAdd(c.n_count + node, 1ULL);
             }
         }
-        // not finite: the evaluation's energy must be, too (the gather reads the flag)
-        if (!ok) atomicOr(c.n_count + shape_nodes(t, sa).x, kContactNotFinite);
     }
+    // not finite: the evaluation's energy must be, too (the gather reads the flag)
+    if (!ok) atomicOr(c.n_count + shape_nodes(t, sa).x, kContactNotFinite);
+}
+
+// The filtered list's pairs in contact and their forces, every evaluation.  A warp queues the pairs
+// of the evaluated instances that are not certainly apart and takes them to FP64 as soon as it has
+// one for every lane, a block's warps the rest together at the end: the closest points run with
+// full warps, and a short list spreads over the SMs.  The launch, the list between them and the
+// second kernel's start bounded the two kernels this was (narrow phase, then contacts).  A whole
+// evaluation of the 2x4x2 specimen 47.3 -> 43.0 us on the GPU, of the compressed 32x32x16 lattice in
+// mixed precision 59.6 -> 51.5.  Filtering in this kernel too took 20 us longer on the 64x64x32 lattice
+// (the closest points' registers halve the warps the filter has in flight).
+__global__ void __launch_bounds__(kListThreads) k_contacts(DevTopo t, PhysParams p, const double4_32a* __restrict__ x,
+                                                           const float4* __restrict__ xf, ContactBufs c) {
+    __shared__ uint2 queue[kListWarps][64];
+    __shared__ uint32_t left[kListWarps];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const long long thread = (long long)blockIdx.x * kListThreads + threadIdx.x, threads = (long long)gridDim.x * kListThreads;
+    const uint32_t total = uint32_t(min((long long)c.counts[kKept], c.cand_cap));
+    uint32_t n = 0;  // pairs in the warp's queue
+    for (long long b0 = thread / 32 * 32; b0 < total; b0 += threads) {  // warp-uniform
+        uint2 q = make_uint2(0, 0);
+        bool close = false;
+        if (b0 + lane < total) {
+            q = c.cand2[b0 + lane];  // not a local pair (k_filter)
+            if (t.I == 1 || t.active[t.node_inst[shape_nodes(t, q.x).x]]) {
+                const DistBounds d = dist_bounds(t, p, xf, q.x, q.y);
+                close = !(d.far_ok && d.far > d.pad_sum);
+            }
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, close);
+        if (close) queue[warp][n + __popc(m & ((1u << lane) - 1u))] = q;
+        n += __popc(m);
+        __syncwarp();
+        if (n >= 32) {
+            n -= 32;
+            add_contact(t, p, x, c, true, queue[warp][n + lane]);
+            __syncwarp();
+        }
+    }
+    if (lane == 0) left[warp] = n;
+    __syncthreads();
+    // the rest of all warps' queues, dense
+    int from = threadIdx.x, w = 0, all = 0;
+    for (int k = 0; k < kListWarps; k++) all += left[k];
+    if (int(threadIdx.x & ~31u) >= all) return;
+    const bool mine = from < all;
+    while (mine && from >= int(left[w])) from -= left[w++];
+    add_contact(t, p, x, c, mine, mine ? queue[w][from] : make_uint2(0, 0));
 }
 
 }  // namespace
@@ -855,11 +865,10 @@ void launch_contacts(const DevTopo& t, const PhysParams& p, const EvalBufs& e, C
                                                 c.cand_cap, c.cand, c.flags),
      note_launches(1));
     if (pairs_end) cudaEventRecord(pairs_end, s);
-    (k_filter<<<kStreamBlocks, kBlock, 0, s>>>(t, p, e.xf_lo, skin > 0.f ? 2.0001f * skin : 0.f, c),  // >= 2 skin
+    (k_filter<<<kFilterBlocks, kBlock, 0, s>>>(t, p, e.xf_lo, skin > 0.f ? 2.0001f * skin : 0.f, c),  // >= 2 skin
      note_launches(1));
-    // every evaluation: the pairs in contact, then their forces
-    (k_narrow<<<kStreamBlocks, kBlock, 0, s>>>(t, p, e.x, e.xf_lo, c), note_launches(1));
-    (k_contacts<<<2 * kStreamBlocks, 64, 0, s>>>(t, p, e.x, c), note_launches(1));
+    // every evaluation: the list's pairs in contact and their forces
+    (k_contacts<<<kListBlocks, kListThreads, 0, s>>>(t, p, e.x, e.xf_lo, c), note_launches(1));
 }
 
 }  // namespace mcg

@@ -246,7 +246,12 @@ struct mcg_ctx {
     cudaGraphExec_t loop_exec = nullptr;
     // Captured evaluations run the contact pipeline (integer work) beside the beam kernel (FP64
     // pipe or memory): its branch of the graph is captured on this stream, whose priority lets
-    // the pipeline's short kernels in between the beam kernel's blocks.
+    // the pipeline's kernels in between the beam kernel's blocks.  A graph keeps its nodes'
+    // priorities only when instantiated so: without it the first contact kernel started when the
+    // FP64 beam kernel's last block had, 78 us into the 98 us of a compressed 32x32x16 lattice
+    // (evaluation 251 -> 224 us).  The mixed beam kernel is short and better out of the way first
+    // (64x64x32: 667 us a call against 681).
+    unsigned long long graph_flags() const { return mixed ? 0 : cudaGraphInstantiateFlagUseNodePriority; }
     cudaStream_t fork = nullptr;
     cudaEvent_t fork_ev[2] = {};
     void make_fork() {
@@ -487,7 +492,7 @@ struct mcg_ctx {
                 ck(cudaStreamEndCapture(stream, &graph), "cudaStreamEndCapture");
                 const long long kernels = g_launch_count.load() - before;
                 g_launch_count -= kernels;  // counted when the graph runs
-                const cudaError_t e = cudaGraphInstantiate(&exec, graph, 0);
+                const cudaError_t e = cudaGraphInstantiate(&exec, graph, graph_flags());
                 cudaGraphDestroy(graph);
                 ck(e, "cudaGraphInstantiate");
                 graphs.push_back(EvalGraph{dz, d_gout, trials, exec, kernels});
@@ -750,7 +755,7 @@ struct mcg_ctx {
             ck(cudaStreamEndCapture(stream, &out), "cudaStreamEndCapture (loop body)");
             loop_round_kernels = g_launch_count.load() - before;
             g_launch_count -= loop_round_kernels;  // counted per round run (rounds_device)
-            ck(cudaGraphInstantiate(&loop_exec, g, 0), "cudaGraphInstantiate (loop)");
+            ck(cudaGraphInstantiate(&loop_exec, g, graph_flags()), "cudaGraphInstantiate (loop)");
         } catch (...) {
             cudaGraphDestroy(g);
             throw;

@@ -28,6 +28,8 @@
 // No host synchronisation: sizes that can overflow a buffer (a bin's slots, bins, candidates,
 // contacts, a shape spanning too many cells) raise a flag instead of writing out of bounds, and
 // the host repeats the evaluation with larger buffers (or coarser cells) when it sees one.
+#include <algorithm>
+
 #include "common.cuh"
 #include "kernels.h"
 
@@ -231,15 +233,12 @@ __device__ __noinline__ PairHit narrow_phase(const DevTopo& t, const PhysParams&
 // returning atomics in flight per thread; the entry that begins a chunk of its bin lists the
 // chunk as a unit of pair work.  A bin that fills up keeps counting (kOverEntries, and
 // the largest count in counts[kLargestBin] so the host can size bin_slots).
-__global__ void __launch_bounds__(kBlock) k_shapes(DevTopo t, PhysParams p, const float4* __restrict__ xf_lo,
-                                                   const float4* __restrict__ xf_hi, float skin, ContactBufs c) {
-    const int S = t.N + t.B;
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= S || !c.flags[1]) return;
-    const int* __restrict__ grid = c.grid;
+__device__ __forceinline__ void emit_shape(const DevTopo& t, const PhysParams& p, const float4* __restrict__ xf_lo,
+                                           const float4* __restrict__ xf_hi, float skin, const ContactBufs& c,
+                                           const int* __restrict__ grid, int s) {
     const int2 nd = shape_nodes(t, uint32_t(s));
     const int n1 = nd.y >= 0 ? nd.y : nd.x;
-    if (!grid[7] || !t.active[t.node_inst[nd.x]]) return;  // inactive instances take no part
+    if (!t.active[t.node_inst[nd.x]]) return;  // inactive instances take no part
     const float4 al = xf_lo[nd.x], ah = xf_hi[nd.x], bl = xf_lo[n1], bh = xf_hi[n1];
     const float pad = __fadd_ru(s < t.N ? p.joint_padf : t.padf[s - t.N], skin);
     const float lo[3] = {__fsub_rd(fminf(al.x, bl.x), pad), __fsub_rd(fminf(al.y, bl.y), pad),
@@ -301,6 +300,15 @@ __global__ void __launch_bounds__(kBlock) k_shapes(DevTopo t, PhysParams p, cons
             }
         }
     }
+}
+
+__global__ void __launch_bounds__(kBlock) k_shapes(DevTopo t, PhysParams p, const float4* __restrict__ xf_lo,
+                                                   const float4* __restrict__ xf_hi, float skin, ContactBufs c) {
+    const int S = t.N + t.B;
+    const int* __restrict__ grid = c.grid;
+    if (!c.flags[1] || !grid[7]) return;
+    for (unsigned s = blockIdx.x * blockDim.x + threadIdx.x; s < unsigned(S); s += gridDim.x * blockDim.x)
+        emit_shape(t, p, xf_lo, xf_hi, skin, c, grid, int(s));
 }
 
 // ---- pair enumeration inside a bin ---------------------------------------------------------
@@ -848,17 +856,22 @@ __global__ void __launch_bounds__(kListThreads) k_contacts(DevTopo t, PhysParams
 long long pair_units(long long bins, int slots) { return bins * ((slots + kChunk - 1) / kChunk); }
 
 // One unit of pair work per warp or so (a bin at the default cell holds about 100 shapes, each in
-// about three bins), and no more blocks than the GPU holds at a time.
-int contact_pair_blocks(long long shapes) {
-    const long long b = shapes / 128;
-    return int(b < 1 ? 1 : (b > 4 * 152 ? 4 * 152 : b));
+// about three bins), and no more blocks than the GPU holds at a time: all of it, or five of eight
+// per SM when it runs beside the FP64 beam kernel (shared).  That one lives on the FP64 pipe, this
+// on the integer pipe, but whichever fills the SMs' registers runs alone: an evaluation of
+// 44x44x22 cubic+BCC takes 391 us with all blocks, 376 with five an SM (and at most four of the
+// box kernel), 367 with four; compressed 32x32x16, where the contacts take longer than the beams,
+// 225, 217 and 221.
+int contact_pair_blocks(long long shapes, bool shared) {
+    const long long b = shapes / 128, most = shared ? 5 * 152 / (8 / kPairWarps) : 4 * 152;
+    return int(b < 1 ? 1 : (b > most ? most : b));
 }
 
 void launch_contacts(const DevTopo& t, const PhysParams& p, const EvalBufs& e, ContactBufs& c, float skin,
                      cudaStream_t s, cudaEvent_t pairs_begin, cudaEvent_t pairs_end) {
     const float grow = skin > 0.f ? skin : 0.f;
     // candidate list (only when rebuilding)
-    (k_shapes<<<grid_for((long long)t.N + t.B), kBlock, 0, s>>>(t, p, e.xf_lo, e.xf_hi, grow, c), note_launches(1));
+    (k_shapes<<<std::min(grid_for((long long)t.N + t.B), unsigned(c.shape_blocks)), kBlock, 0, s>>>(t, p, e.xf_lo, e.xf_hi, grow, c), note_launches(1));
     if (pairs_begin) cudaEventRecord(pairs_begin, s);
     (k_bin_pairs<<<8 / kPairWarps * c.pair_blocks, kPairThreads, 0, s>>>(t, c.grid, c.bin_count, c.bin_slots, c.counts, c.units, c.bin_items,
                                                            c.rec,

@@ -326,7 +326,7 @@ struct mcg_ctx {
     // 59 / 215 at 2.5 times; the densely compressed 32x32x16 lattice does not gain beyond that.
     double default_cell() const { return 2 * reference_cell(); }
     int pair_blocks_for(long long shapes) const {
-        return pair_blocks_set > 0 ? pair_blocks_set : contact_pair_blocks(shapes);
+        return pair_blocks_set > 0 ? pair_blocks_set : contact_pair_blocks(shapes, !mixed);
     }
     // bin_slots: entries a grid bin holds (rounded up to a power of two, at least 8)
     long long builds_before = 0;  // candidate-list builds counted by buffers since released
@@ -353,6 +353,7 @@ struct mcg_ctx {
         c.bin_items = contact_mem.get<uint32_t>(size_t(bin_cap) * size_t(slots));
         c.units = contact_mem.get<uint2>(size_t(pair_units(bin_cap, slots)));
         c.pair_blocks = pair_blocks_for(S);
+        c.shape_blocks = mixed ? 0x7fffffff : 4 * 152;  // in FP64 beside the beam kernel
         c.cand_cap = std::max<long long>(1024, (cand_cap + 31) / 32 * 32);
         c.cand = contact_mem.get<uint2>(size_t(c.cand_cap));
         c.cand2 = contact_mem.get<uint2>(size_t(c.cand_cap));
@@ -2050,7 +2051,7 @@ int mcg_autotune(mcg_ctx* c, const double* z, const double* tops, int32_t reps, 
         const long long S = (long long)c->N + c->B;
         std::vector<int> blocks{0};
         for (int b : {152, 304, 608, 1216})
-            if (b != contact_pair_blocks(S) && (long long)b * 8 * 32 <= std::max<long long>(S, 8 * 32)) blocks.push_back(b);
+            if (b != contact_pair_blocks(S, !c->mixed) && (long long)b * 8 * 32 <= std::max<long long>(S, 8 * 32)) blocks.push_back(b);
         const double cell0 = c->default_cell();
         std::vector<double> ref_e, e(size_t(c->I));
         std::vector<double> ref_g, g(n);

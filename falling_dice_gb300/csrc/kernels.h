@@ -172,6 +172,7 @@ struct ContactBufs {
     uint2* units;           // [pair_units()] (bin, chunk of the bin's shapes) with an entry
     // narrow-phase candidates: one flat list, appended by the pair grid's warps in chunks
     int pair_blocks;        // blocks of the pair grid (8 warps each)
+    int shape_blocks;       // most blocks of the box kernel
     long long cand_cap;     // candidate slots, a multiple of 32
     uint2* cand;            // [cand_cap] (lower shape, higher shape)
     uint2* cand2;           // [cand_cap] the ones that can reach contact before the next build
@@ -307,8 +308,8 @@ void launch_plastic_mixed_to_f64(const DevTopo& t, const uint8_t* mask, const Mi
 void launch_plastic_stats(const DevTopo& t, const double* plastic, double* part, double* out6, cudaStream_t s);
 
 // ---- contact pipeline (contact.cu) ------------------------------------------------------
-// Blocks of the pair / narrow-phase grid for a model of `shapes` shapes (8 warps each).
-int contact_pair_blocks(long long shapes);
+// Blocks of the pair grid for a model of `shapes` shapes (8 warps each); shared: beside the FP64 beam kernel.
+int contact_pair_blocks(long long shapes, bool shared);
 // Units of pair work that `bins` bins of `slots` entries can hold.
 long long pair_units(long long bins, int slots);
 // The whole broad/narrow phase after the state and center kernels: bins, pairs and filtered

@@ -94,7 +94,8 @@ bool carve(unsigned char* base, long long N, long long S, ContactBufs& c, size_t
     c.xref = reinterpret_cast<float4*>(take(size_t(N > 0 ? N : 1) * sizeof(float4)));
     c.bin_items = reinterpret_cast<uint32_t*>(take(size_t(kNoAllocBins) * kNoAllocBinSlots * 4));
     c.units = reinterpret_cast<uint2*>(take(size_t(pair_units(kNoAllocBins, kNoAllocBinSlots)) * sizeof(uint2)));
-    c.pair_blocks = contact_pair_blocks(S);
+    c.pair_blocks = contact_pair_blocks(S, false);
+    c.shape_blocks = 0x7fffffff;
     c.cand_cap = kNoAllocCandidates;
     c.cand = reinterpret_cast<uint2*>(take(size_t(kNoAllocCandidates) * sizeof(uint2)));
     c.cand2 = reinterpret_cast<uint2*>(take(size_t(kNoAllocCandidates) * sizeof(uint2)));

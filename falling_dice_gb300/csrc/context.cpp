@@ -413,8 +413,6 @@ struct mcg_ctx {
     }
 
     // ---- evaluation ----------------------------------------------------------------------
-    // Platen heights of all instances from hp.tops (the host changes them only after a sync).
-    void upload_tops() { h2d(ev.tops, hp.tops, size_t(I), stream); }
 
     // Captured evaluations: the launch sequence of eval_launches for one (z, gradient,
     // trials) combination, replayed as one graph.  Any change of what the launches bake in
@@ -511,6 +509,8 @@ struct mcg_ctx {
     // forked: captured launches, the contact pipeline on its own branch beside the beam kernel
     void eval_launches(const double* dz, int trials, double* d_gout, bool forked) {
         PhysParams p = phys;
+        EvalBufs ev = this->ev;
+        if (trials == 2) ev.tops_host = nullptr;  // the loop's platens are on the device
         p.broad_cell = broad_cell;
         p.inv_cell_f = float(1.0 / broad_cell);
         mark(0);
@@ -571,8 +571,7 @@ struct mcg_ctx {
         return hp.outs;
     }
     void read_outs() {
-        d2h(hp.outs, ev.out, size_t(I), stream);
-        sync();
+        sync();  // hp.outs is written by the finalize
         check_kernel_error();
     }
     // A kernel's bounded wait that gave up (ev.err, copied into the totals)
@@ -680,7 +679,6 @@ struct mcg_ctx {
         if (!any) return false;
         set_active(a);
         upload_ctl(1);
-        upload_tops();
         replay(16, [&] { bl_prepare(topo, d_ctl, L, stream); });
         d2h(hp.dg, d_dg, size_t(I), stream);  // read back with the evaluation's totals
         const EvalOut* out = eval_read(d_zeval, trials, d_geval);
@@ -779,7 +777,6 @@ struct mcg_ctx {
             ck(cudaGraphLaunch(loop_exec, stream), "cudaGraphLaunch (loop)");
             d2h(hp.mins, d_mins, size_t(I), stream);
             d2h(hp.mz, d_mz, 1, stream);
-            d2h(hp.outs, ev.out, size_t(I), stream);
             sync();
             check_launch();
             check_kernel_error();
@@ -790,6 +787,8 @@ struct mcg_ctx {
             loop_rounds += hp.mz->rounds;
             note_launches(int(hp.mz->rounds) * int(loop_kernels_per_round()));
             std::copy(hp.mins, hp.mins + I, mins.begin());
+            for (int i = 0; i < I; i++)  // what an evaluation outside the loop would read
+                if (mins[size_t(i)].phase != Minimizer::kIdle) hp.tops[i] = mins[size_t(i)].top;
             active.assign(size_t(I), 2);  // the loop wrote d_active: the host mirror is unknown
             last_z = d_zeval;
             last_trials = false;
@@ -840,7 +839,9 @@ struct mcg_ctx {
         DevTopo all = topo;  // the committed instances' states (others are recomputed before use)
         all.active = d_all;
         launch_state(all, p, d_zfinal, d_baseX, d_baseR, BuildArgs{}, ev, stream);
-        launch_center(all, p, BuildArgs{}, ev, stream);
+        EvalBufs at = ev;
+        at.tops_host = nullptr;
+        launch_center(all, p, BuildArgs{}, at, stream);
         if (mixed) {
             launch_commit(topo, d_mask, ev, d_baseX, d_baseR, nullptr, stream);
             launch_plastic_mixed(topo, d_mask, nullptr, ev.trial_nextf, mb, stream);
@@ -1436,6 +1437,8 @@ void upload_instances(mcg_ctx* c, const std::vector<InstIn>& ins) {
     e.cforce = V.get<double>(2 * size_t(I));
     e.tops = V.get<double>(size_t(I));
     e.out = V.get<EvalOut>(size_t(I));
+    e.tops_host = c->hp.tops;  // (the host changes them only after a sync)
+    e.out_host = c->hp.outs;
     e.trial_next = V.get<double>(7 * size_t(B));
     e.trial_aux = V.get<double>(7 * size_t(B));
     e.trial_flags = V.get<uint8_t>(3 * size_t(B));
@@ -1467,7 +1470,6 @@ void upload_instances(mcg_ctx* c, const std::vector<InstIn>& ins) {
     }
     c->ev = e;
     for (int k = 0; k < I; k++) c->hp.tops[k] = ih[size_t(k)].geom.top0;
-    c->upload_tops();
     c->d_zin = V.get<double>(6 * size_t(N));
     c->d_grad = V.get<double>(6 * size_t(N));
     ck(cudaMemsetAsync(c->d_zin, 0, 6 * size_t(N) * sizeof(double), s), "memset");
@@ -1698,7 +1700,6 @@ int mcg_objective(mcg_ctx* c, const double* z, double top, int trials, double* e
         const size_t n = 6 * size_t(c->N), B = size_t(c->B);
         h2d(c->d_zin, z, n, s);
         c->hp.tops[0] = top;
-        c->upload_tops();
         c->set_active(std::vector<uint8_t>(1, 1));
         const EvalOut o = c->eval_read(c->d_zin, trials != 0, c->d_grad, grad)[0];
         if (trials) c->have_final = false;
@@ -1733,7 +1734,6 @@ int mcg_batch_objective(mcg_ctx* c, const double* z, const double* tops, double*
         const size_t n = 6 * size_t(c->N);
         h2d(c->d_zin, z, n, c->stream);
         for (int i = 0; i < c->I; i++) c->hp.tops[i] = tops[i];
-        c->upload_tops();
         c->set_active(std::vector<uint8_t>(size_t(c->I), 1));
         const EvalOut* o = c->eval_read(c->d_zin, false, c->d_grad, grad);
         for (int i = 0; i < c->I; i++) {
@@ -1759,7 +1759,6 @@ int mcg_objective_resident(mcg_ctx* c, double top, int trials) {
         if (c->hp.tops[0] != top) {
             c->sync();
             c->hp.tops[0] = top;
-            c->upload_tops();
         }
         c->eval(c->d_zin, trials != 0, c->d_grad);
         if (trials) c->have_final = false;
@@ -1794,7 +1793,6 @@ int objective_with_fixed_contacts(mcg_ctx* c, ContactBufs& fixed, size_t zero_by
         const size_t n = 6 * size_t(c->N);
         h2d(c->d_zin, z, n, s);
         c->hp.tops[0] = top;
-        c->upload_tops();
         c->set_active(std::vector<uint8_t>(1, 1));
         PhysParams p = c->phys;
         // its bins are few and small: the reference's cell unless another was set
@@ -1821,7 +1819,6 @@ int objective_with_fixed_contacts(mcg_ctx* c, ContactBufs& fixed, size_t zero_by
         launch_finalize(c->topo, p, cptr, c->d_grad, c->ev, s);
         c->check_launch();
         c->contacts_stale = p.self_contact != 0;
-        d2h(c->hp.outs, c->ev.out, 1, s);
         c->sync();
         const EvalOut o = c->hp.outs[0];
         if (o.overflow) {
@@ -2044,7 +2041,6 @@ int mcg_autotune(mcg_ctx* c, const double* z, const double* tops, int32_t reps, 
         if (z) h2d(c->d_zin, z, n, s);
         else ck(cudaMemsetAsync(c->d_zin, 0, n * sizeof(double), s), "memset");
         for (int i = 0; i < c->I; i++) c->hp.tops[i] = tops ? tops[i] : c->inst[size_t(i)].geom.top0;
-        c->upload_tops();
         c->set_active(std::vector<uint8_t>(size_t(c->I), 1));
         const float skin = c->contact_skin;
         c->contact_skin = 0.f;  // time full builds

@@ -220,6 +220,10 @@ struct EvalBufs {
     double* cforce;         // [2 I] centering force of the instance on each node (x, z)
     double* tops;           // [I] platen height per instance
     EvalOut* out;           // [I]
+    // the host's page-locked side of both, which the kernels read and write themselves: an
+    // evaluation needs no copies for them (null: the device's only)
+    const double* tops_host;
+    EvalOut* out_host;
     double* trial_next;     // [7B] SoA
     double* trial_aux;      // [7B] SoA
     uint8_t* trial_flags;   // [3B] SoA

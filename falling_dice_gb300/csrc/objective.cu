@@ -126,6 +126,7 @@ __device__ void grid_params(const BuildArgs& b, const double* ext) {
 // list: every kernel of the build returns at once when it does not.
 __global__ void __launch_bounds__(kBlock) k_center(DevTopo t, double centering, const double* __restrict__ part,
                                                    double* __restrict__ cen, double* __restrict__ cforce,
+                                                   double* __restrict__ tops, const double* __restrict__ tops_host,
                                                    BuildArgs build) {
     __shared__ double sm[6 * kBlock];
     __shared__ double ext[6];
@@ -168,6 +169,7 @@ __global__ void __launch_bounds__(kBlock) k_center(DevTopo t, double centering, 
         c[3 + j] = ext[j];
     }
     if (inst < t.I) {
+        if (threadIdx.x == 32 && tops_host) tops[inst] = tops_host[inst];
         if (threadIdx.x == 0) {
             const double n = double(t.inst_n[inst]), inv = 1.0 / n;
             c[0] = acc[0] * inv; c[1] = acc[1] * inv; c[2] = acc[2] * inv;
@@ -662,11 +664,13 @@ __global__ void __launch_bounds__(kBlock) k_finalize(DevTopo t, PhysParams p, Ev
     __shared__ double tot[kFinVals];
     __shared__ int state;  // 0 done, 1 this block sums up, 2 the gradient is to be cleared
     const int inst = blockIdx.y, f = blockIdx.x;
-    EvalOut* out = e.out + inst;
     if (inst == 0 && f == 0 && threadIdx.x == 0) {  // of the whole evaluation, whether instance 0 is active or not
-        out->overflow = flags ? int(flags[0] & ~uint32_t(kNonFinite)) : 0;
-        out->pairs = counts ? counts[kContacts] : 0u;
-        out->kernel_error = *e.err;
+        for (EvalOut* out : {e.out, e.out_host}) {
+            if (!out) continue;
+            out->overflow = flags ? int(flags[0] & ~uint32_t(kNonFinite)) : 0;
+            out->pairs = counts ? counts[kContacts] : 0u;
+            out->kernel_error = *e.err;
+        }
         if (flags) flags[0] = flags[1] = 0;  // for the next evaluation
     }
     const int2 r = t.brange[inst];
@@ -738,23 +742,28 @@ __global__ void __launch_bounds__(kBlock) k_finalize(DevTopo t, PhysParams p, Ev
         energy += tot[6];
         energy += tot[4];
         const int nonfinite = isfinite(energy) ? 0 : 1;
-        out->energy = nonfinite ? __longlong_as_double(0x7ff0000000000000LL) : energy;
-        out->elastic = tot[1];
-        out->plastic = tot[2];
-        out->contact = tot[6] + tot[4];
-        out->reaction = tot[5];
-        out->max_pen = tot[9];
-        out->contacts = int(tot[7]);
-        out->nonfinite = nonfinite;
-        out->beam_energy = tot[0];
-        out->node_energy = tot[3];
-        out->center_energy = center;
-        out->contact_energy = tot[6];
-        out->platen_energy = tot[4];
         // a non-finite evaluation has a zero gradient
         const long long nf = t.inst_free[inst];
-        out->rms = nonfinite ? 0.0 : (nf ? sqrt(tot[8] / double(nf)) : 0.0);
-        out->gmax = nonfinite ? 0.0 : tot[10];
+        const double rms = nonfinite ? 0.0 : (nf ? sqrt(tot[8] / double(nf)) : 0.0);
+        for (EvalOut* o : {e.out, e.out_host}) {
+            if (!o) continue;
+            EvalOut* out = o + inst;
+            out->energy = nonfinite ? __longlong_as_double(0x7ff0000000000000LL) : energy;
+            out->elastic = tot[1];
+            out->plastic = tot[2];
+            out->contact = tot[6] + tot[4];
+            out->reaction = tot[5];
+            out->max_pen = tot[9];
+            out->contacts = int(tot[7]);
+            out->nonfinite = nonfinite;
+            out->beam_energy = tot[0];
+            out->node_energy = tot[3];
+            out->center_energy = center;
+            out->contact_energy = tot[6];
+            out->platen_energy = tot[4];
+            out->rms = rms;
+            out->gmax = nonfinite ? 0.0 : tot[10];
+        }
         state = nonfinite ? 2 : 0;
     }
     __syncthreads();
@@ -861,7 +870,7 @@ void launch_state(const DevTopo& t, const PhysParams& p, const double* z, const 
 }
 
 void launch_center(const DevTopo& t, const PhysParams& p, const BuildArgs& b, EvalBufs& e, cudaStream_t s) {
-    k_center<<<t.I + 1, kBlock, 0, s>>>(t, p.centering, e.part_state, e.cen, e.cforce, b);
+    k_center<<<t.I + 1, kBlock, 0, s>>>(t, p.centering, e.part_state, e.cen, e.cforce, e.tops, e.tops_host, b);
     note_launches(1);
 }
 

@@ -518,6 +518,21 @@ __device__ __forceinline__ void state_block_parts(const double (&acc)[3], const 
     }
 }
 
+// Whether this is the last of `total` blocks to arrive at a counter; then every
+// block's earlier writes are visible.  All threads call it.
+__device__ __forceinline__ bool last_block(unsigned* counter, unsigned total) {
+    __shared__ int last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        last = atomicAdd(counter, 1u) == total - 1u;
+        if (last) *counter = 0;  // for the next pass
+    }
+    __syncthreads();
+    if (last) __threadfence();
+    return last;
+}
+
 inline unsigned grid_for(long long n, int block = kBlock) {
     long long g = (n + block - 1) / block;
     return unsigned(g < 1 ? 1 : g);

@@ -543,7 +543,7 @@ struct mcg_ctx {
         if (mixed) launch_gather_mixed(topo, p, cptr, d_gout, ev, stream, gather_variant);
         else launch_gather(topo, p, cptr, d_gout, ev, stream, gather_variant);
         mark(6);
-        launch_finalize(topo, p, cptr, d_gout, ev, stream);
+        launch_finalize(topo, p, d_gout, ev, stream);
         mark(7);
         check_launch();
         collect();
@@ -1317,6 +1317,11 @@ void upload_instances(mcg_ctx* c, const std::vector<InstIn>& ins) {
     T.n_bblk = int(bblk.size());
     T.bdim = bdim;
     T.n_eblk = int(eblk.size());
+    T.large_totals = false;
+    for (int k = 0; k < I; k++) {
+        const int2 b = brange[size_t(k)], e = erange[size_t(k)];
+        T.large_totals |= (b.y - b.x) + 2 * (e.y - e.x) > kFinSingle;
+    }
     T.n_sblk = int(sblk.size());
     {
         auto up4 = [&](const std::vector<int4>& v) {
@@ -1430,9 +1435,10 @@ void upload_instances(mcg_ctx* c, const std::vector<InstIn>& ins) {
     e.part_beam = V.get<double>(3 * size_t(std::max(T.n_bblk, 1)));
     e.err = V.get<unsigned>(1);
     ck(cudaMemsetAsync(e.err, 0, sizeof(unsigned), s), "memset");
-    e.part_node = V.get<double>(kNodeParts * size_t(T.n_eblk));
+    e.part_node = V.get<double>(kNodeParts * 2 * size_t(T.n_eblk));
+    e.done = V.get<unsigned>(size_t(I));
+    ck(cudaMemsetAsync(e.done, 0, size_t(I) * sizeof(unsigned), s), "memset");
     e.part_fin = V.get<double>(size_t(kFinPartDoubles) * size_t(I));
-    ck(cudaMemsetAsync(e.part_fin, 0, size_t(kFinPartDoubles) * size_t(I) * sizeof(double), s), "memset");
     e.cen = V.get<double>(9 * size_t(I + 1));
     e.cforce = V.get<double>(2 * size_t(I));
     e.tops = V.get<double>(size_t(I));
@@ -1816,7 +1822,7 @@ int objective_with_fixed_contacts(mcg_ctx* c, ContactBufs& fixed, size_t zero_by
         }
         if (c->mixed) launch_gather_mixed(c->topo, p, cptr, c->d_grad, c->ev, s, c->gather_variant);
         else launch_gather(c->topo, p, cptr, c->d_grad, c->ev, s, c->gather_variant);
-        launch_finalize(c->topo, p, cptr, c->d_grad, c->ev, s);
+        launch_finalize(c->topo, p, c->d_grad, c->ev, s);
         c->check_launch();
         c->contacts_stale = p.self_contact != 0;
         c->sync();

@@ -56,6 +56,7 @@ struct DevTopo {
     int bdim;                 // beams per beam block: kBeamBlock (FP64) or kMapBlock (mixed)
     const int2* brange;       // [I] beam blocks [x, y) of the instance
     int n_eblk;               // evaluation node blocks
+    bool large_totals;        // an instance has more than kFinSingle beam and gather blocks
     const int4* eblk;         // [n_eblk] first node, node count, instance, 0
     const int2* erange;       // [I] evaluation node blocks [x, y) of the instance
     int n_sblk;               // solver blocks: at most kSolveBlocks runs of nodes per instance
@@ -200,7 +201,8 @@ struct BuildArgs {
 // per node block: gravity E, platen E, reaction, max penetration, contacts, self-contact E,
 // sum of squared free gradient entries, max |free gradient entry|
 constexpr int kNodeParts = 8;
-constexpr int kFinPartDoubles = 32 * 11 + 1;  // per instance: 32 first-stage blocks x 11 totals, a counter
+constexpr int kFinPartDoubles = 32 * 11;  // per instance: 32 first-stage blocks x 11 totals
+constexpr int kFinSingle = 768;  // block partials one block sums: six per thread
 
 struct EvalBufs {
     double4_32a* x;             // [N]
@@ -213,7 +215,8 @@ struct EvalBufs {
     double* part_state;     // [9 * n_eblk] sum, -min, max of x per block
     double* part_beam;      // [3 * nb_beams]
     unsigned* err;          // [1] a kernel's bounded wait gave up (the host reports it)
-    double* part_node;      // [kNodeParts * n_eblk]
+    double* part_node;      // [kNodeParts * 2 n_eblk] per gather block
+    unsigned* done;         // [I] blocks that have arrived; zero between kernels
     double* part_fin;       // [I * kFinPartDoubles] first-stage totals of the finalize
     double* cen;            // [9 (I + 1)] per instance mean, min, max of the node positions (min/max
                             //   in the contact grid's frame); then min/max over all instances
@@ -277,8 +280,7 @@ void launch_beams(const DevTopo& t, const Material& m, const double* plastic, in
                   EvalBufs& e, cudaStream_t s, int variant = 0);
 void launch_gather(const DevTopo& t, const PhysParams& p, const ContactBufs* c, double* grad,
                    EvalBufs& e, cudaStream_t s, int variant = 0);
-void launch_finalize(const DevTopo& t, const PhysParams& p, const ContactBufs* c, double* grad,
-                     EvalBufs& e, cudaStream_t s);
+void launch_finalize(const DevTopo& t, const PhysParams& p, double* grad, EvalBufs& e, cudaStream_t s);
 // base state <- current state, plastic <- trial (plastic == nullptr skips it) for the
 // instances with mask[i] != 0 (mask == nullptr: all)
 void launch_commit(const DevTopo& t, const uint8_t* mask, const EvalBufs& e, double* base_x, double* base_r,

@@ -68,21 +68,6 @@ __device__ __forceinline__ void st3(double* v, d3 a) {
     v[2] = a.z;
 }
 
-// Whether this is the last of `total` blocks to arrive at an instance's counter; then every
-// block's earlier writes are visible.  All threads call it.
-__device__ __forceinline__ bool last_block(unsigned* counter, unsigned total) {
-    __shared__ int last;
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        last = atomicAdd(counter, 1u) == total - 1u;
-        if (last) *counter = 0;  // for the next pass
-    }
-    __syncthreads();
-    if (last) __threadfence();
-    return last;
-}
-
 // Block partial of up to four values into q[k * stride] (thread k writes value k).
 template <int NV>
 __device__ __forceinline__ void block_part(double a, double b, double c, double d, double* q, size_t stride,

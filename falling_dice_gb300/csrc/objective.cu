@@ -488,250 +488,121 @@ __device__ __forceinline__ double fixed_value(const long long* l, int e0) {
 }
 
 // ---- per-node gather: the scatter of MC/src/sim.cpp:139-172, as a deterministic CSR sum ---
-// Sums the incident beams' end vectors of node i in ascending beam order: FP64 slots
-// directly, FP32 slots (mixed form) with compensated FP32 sums.
+// Sums one half (0 translations, 1 rotations) of the incident beams' end vectors of node i in
+// ascending beam order: FP64 slots directly, FP32 slots (mixed form) with compensated FP32 sums.
 template <bool F32>
-__device__ __forceinline__ void sum_slots(const DevTopo& t, const EvalBufs& e, int i, d3& gx, d3& gr) {
+__device__ __forceinline__ d3 sum_slots(const DevTopo& t, const EvalBufs& e, int i, int half) {
     const int k0 = t.inc_start[i], k1 = t.inc_start[i + 1];
     // unrolled so that the loads of several incident beams are in flight together; the
     // additions keep their order
     if (!F32) {
+        d3 g{0, 0, 0};
 #pragma unroll 4
         for (int k = k0; k < k1; k++) {
-            const double2* s = reinterpret_cast<const double2*>(e.slot) + 3 * size_t(t.inc[k]);
-            const double2 a = s[0], b = s[1], c = s[2];
-            gx.x += a.x; gx.y += a.y; gx.z += b.x;
-            gr.x += b.y; gr.y += c.x; gr.z += c.y;
+            const double* s = e.slot + 6 * size_t(t.inc[k]);  // 16-byte aligned, as are s + 2 and s + 4
+            const double2 u = *reinterpret_cast<const double2*>(s + 4 * half);
+            const double v = s[2 + half];
+            g.x += half ? v : u.x;
+            g.y += half ? u.x : u.y;
+            g.z += half ? u.y : v;
         }
-    } else {
-        float hi[6] = {0, 0, 0, 0, 0, 0}, lo[6] = {0, 0, 0, 0, 0, 0};
-#pragma unroll 4
-        for (int k = k0; k < k1; k++) {
-            const float2* s2 = reinterpret_cast<const float2*>(e.slotf) + 3 * size_t(t.inc[k]);
-            const float2 p = s2[0], q = s2[1], r = s2[2];
-            const float s[6] = {p.x, p.y, q.x, q.y, r.x, r.y};
-#pragma unroll
-            for (int j = 0; j < 6; j++) {  // two-sum
-                const float a = s[j], sum = hi[j] + a, bp = sum - hi[j];
-                lo[j] += (hi[j] - (sum - bp)) + (a - bp);
-                hi[j] = sum;
-            }
-        }
-        gx = d3{to_double(hi[0]) + to_double(lo[0]), to_double(hi[1]) + to_double(lo[1]), to_double(hi[2]) + to_double(lo[2])};
-        gr = d3{to_double(hi[3]) + to_double(lo[3]), to_double(hi[4]) + to_double(lo[4]), to_double(hi[5]) + to_double(lo[5])};
+        return g;
     }
+    float hi[3] = {0, 0, 0}, lo[3] = {0, 0, 0};
+#pragma unroll 4
+    for (int k = k0; k < k1; k++) {
+        const float* s = e.slotf + 6 * size_t(t.inc[k]);  // 8-byte aligned, as are s + 2 and s + 4
+        const float2 u = *reinterpret_cast<const float2*>(s + 4 * half);
+        const float v = s[2 + half];
+        const float x[3] = {half ? v : u.x, half ? u.x : u.y, half ? u.y : v};
+#pragma unroll
+        for (int j = 0; j < 3; j++) {  // two-sum
+            const float a = x[j], sum = hi[j] + a, bp = sum - hi[j];
+            lo[j] += (hi[j] - (sum - bp)) + (a - bp);
+            hi[j] = sum;
+        }
+    }
+    return d3{to_double(hi[0]) + to_double(lo[0]), to_double(hi[1]) + to_double(lo[1]), to_double(hi[2]) + to_double(lo[2])};
 }
 
-// Per-warp totals of the gather.
+// Per-warp totals of the gather; then the evaluation's totals.
+constexpr int kGatherNodes = kEvalBlock / 2;  // nodes of a gather block: two threads each
 struct GatherParts {
-    double sum[5][kEvalBlock / 32];  // gravity E, |g|^2, platen E, reaction, self-contact E
-    int count[kEvalBlock / 32];
-    long long m[2][kEvalBlock / 32];  // max penetration, max |g| (bits of non-negative doubles)
+    double g2[kGatherNodes];             // |g|^2 and max |g| of the rotations
+    long long gbits[kGatherNodes];
+    double sum[5][kGatherNodes / 32];    // gravity E, |g|^2, platen E, reaction, self-contact E
+    int count[kGatherNodes / 32];
+    long long m[2][kGatherNodes / 32];   // max penetration, max |g| (bits of non-negative doubles)
 };
 
-// Bound by the FP64 pipe (the incident vectors' additions) and the latency of their loads.
-// Only what nearly every node has is reduced always (gravity energy and |g|^2, in five FP64
-// additions a warp); platen and contact totals where a node of the warp touches something.
-// 34,897 nodes with 41,722 contacts: 39 -> 33 us.
-// kMinBlocks: units of 256 threads per SM the register allocation must allow.
-template <bool F32, int kMinBlocks>
-__global__ void __launch_bounds__(kEvalBlock, 2 * kMinBlocks) k_gather(DevTopo t, PhysParams p, ContactBufs c,
-                                                                       int use_contacts, EvalBufs e,
-                                                                       double* __restrict__ grad) {
-    __shared__ GatherParts sm;
-    const MapPos mp = map_pos(t.eblk);
-    if (!t.active[mp.inst]) return;  // block-uniform
-    const int i = mp.i;
-    const int N = t.N;
-    double egrav = 0, g2 = 0, eplat = 0, reac = 0, econt = 0, pen_max = 0;
-    int count = 0;
-    unsigned long long gbits = 0;  // max |g| as the bits of a non-negative double (integer max)
-    if (mp.valid) {
-        d3 gx{0, 0, 0}, gr{0, 0, 0};
-        sum_slots<F32>(t, e, i, gx, gr);
-        const d3 xi = ldx(e.x, i);
-        // gravity (sim.cpp:142)
-        const double mg = t.mass[i] * p.gravity;
-        egrav = mg * xi.y;
-        gx.y += mg;
-        // centering (sim.cpp:143), the same force for all nodes of the instance
-        gx.x += e.cforce[2 * mp.inst];
-        gx.z += e.cforce[2 * mp.inst + 1];
-        // self-contact: the node's fixed-point sums, cleared for the next evaluation
-        const unsigned long long items = use_contacts ? c.n_count[i] : 0ULL;
-        if (items) {
-            NodeContact& r = c.n_sum[i];
-            gx.x += fixed_value(r.f[0], c.force_e0);
-            gx.y += fixed_value(r.f[1], c.force_e0);
-            gx.z += fixed_value(r.f[2], c.force_e0);
-            if (items >> 32) {
-                econt = fixed_value(r.energy, c.energy_e0);
-                pen_max = __longlong_as_double((long long)r.pen);
-            }
-            if (items & kContactNotFinite) econt = __longlong_as_double(0x7ff8000000000000LL);
-            count = int(items >> 32);
-            r = NodeContact{};
-            c.n_count[i] = 0;
-        }
-        // platens (sim.cpp:168-171)
-        const double jr = p.joint_radius, kc = p.contact_k;
-        const double pb = jr - xi.y;
-        if (positive(pb)) {
-            const double mm = kc * pb;
-            eplat += .5 * kc * pb * pb;
-            pen_max = fmax(pen_max, pb);
-            count += 1;
-            gx.y -= mm;
-        }
-        const double pt = xi.y + jr - e.tops[mp.inst];
-        if (positive(pt)) {
-            const double mm = kc * pt;
-            eplat += .5 * kc * pt * pt;
-            reac += mm;
-            pen_max = fmax(pen_max, pt);
-            count += 1;
-            gx.y += mm;
-        }
-        // pack, scale and lock (sim.cpp:172)
-        const double ts = p.translation_scale;
-        const uint8_t* li = t.locked + 6 * size_t(i);
-        double gv[6] = {ts * gx.x, ts * gx.y, ts * gx.z, gr.x, gr.y, gr.z};
-#pragma unroll
-        for (int k = 0; k < 6; k++) {
-            if (li[k]) gv[k] = 0.0;
-            // residual over free DOFs for the solver's convergence test (sim.cpp:44-45)
-            g2 = fma(gv[k], gv[k], g2);
-            // fmax(gmax, |g|) on the bit patterns; a NaN (above the infinity pattern) is
-            // skipped as fmax skips it
-            const unsigned long long b = (unsigned long long)__double_as_longlong(gv[k]) & 0x7fffffffffffffffULL;
-            if (b <= 0x7ff0000000000000ULL && b > gbits) gbits = b;
-        }
-        double2* g = reinterpret_cast<double2*>(grad + 6 * size_t(i));
-        g[0] = make_double2(gv[0], gv[1]);
-        g[1] = make_double2(gv[2], gv[3]);
-        g[2] = make_double2(gv[4], gv[5]);
-    }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const double v = warp_sum2(egrav, g2);
-    const long long gm = warp_max_key((long long)gbits);
-    double w = 0;
-    long long pm = 0;
-    int cn = 0;
-    if (__any_sync(0xffffffffu, count != 0 || __double_as_longlong(econt) != 0)) {
-        w = warp_sum4(eplat, reac, econt, 0.0);
-        pm = warp_max_key(__double_as_longlong(pen_max));
-        cn = __reduce_add_sync(0xffffffffu, count);
-    }
-    if (lane == 0) {
-        sm.m[0][warp] = pm;
-        sm.m[1][warp] = gm;
-        sm.count[warp] = cn;
-    }
-    if ((lane & 15) == 0) sm.sum[lane >> 4][warp] = v;
-    if ((lane & 7) == 0 && lane < 24) sm.sum[2 + (lane >> 3)][warp] = w;
-    __syncthreads();
-    constexpr int nw = kEvalBlock / 32;
-    const int tid = threadIdx.x;
-    double* q = e.part_node + kNodeParts * size_t(blockIdx.x);
-    if (tid < 5) {
-        double s = sm.sum[tid][0];
-        for (int k = 1; k < nw; k++) s += sm.sum[tid][k];
-        q[tid == 0 ? 0 : tid == 1 ? 6 : tid == 2 ? 1 : tid == 3 ? 2 : 5] = s;
-    } else if (tid < 7) {
-        long long m = sm.m[tid - 5][0];
-        for (int k = 1; k < nw; k++) m = max(m, sm.m[tid - 5][k]);
-        q[tid == 5 ? 3 : 7] = __longlong_as_double(m);
-    } else if (tid == 7) {
-        int n = 0;
-        for (int k = 0; k < nw; k++) n += sm.count[k];
-        q[4] = double(n);
-    }
-}
-
 // ---- totals and the non-finite guard ---------------------------------------------------------
-// One launch: an instance of few block partials is summed by one block, a larger one by kFinFan
-// blocks (block f takes the partials first + f + kFinFan j), the last of which to finish sums
-// their results in order, so the FP64 additions spread over many SMs.  Which way an instance
-// goes depends on its own size only, so it sums alike alone and in a batch.
+// An instance of few block partials (kFinSingle; a block reads six per thread in about the time of a
+// launch) is summed by the last of its gather blocks to finish; a larger
+// one by kFinFan blocks of k_finalize (block f takes the partials first + f + kFinFan j), the last
+// of which to finish sums their results in order, so the FP64 additions spread over many SMs.
+// Which way an instance goes depends on its own size only, so it sums alike alone and in a batch.
 constexpr int kFinFan = 32;
 constexpr int kFinVals = 11;  // beamE, elastic, plastic, gravityE, platenE, reaction, contactE,
                               // contacts, |g|^2, max penetration, max |g|
-constexpr int kFinSingle = 512;  // block partials one block sums: two per thread
-static_assert(kFinPartDoubles == kFinFan * kFinVals + 1, "first-stage totals and their counter");
-__global__ void __launch_bounds__(kBlock) k_finalize(DevTopo t, PhysParams p, EvalBufs e, uint32_t* __restrict__ flags,
-                                                     const uint32_t* __restrict__ counts, double* __restrict__ grad) {
-    __shared__ double sm[9 * kBlock];
-    __shared__ double tot[kFinVals];
-    __shared__ int state;  // 0 done, 1 this block sums up, 2 the gradient is to be cleared
-    const int inst = blockIdx.y, f = blockIdx.x;
-    if (inst == 0 && f == 0 && threadIdx.x == 0) {  // of the whole evaluation, whether instance 0 is active or not
-        for (EvalOut* out : {e.out, e.out_host}) {
-            if (!out) continue;
-            out->overflow = flags ? int(flags[0] & ~uint32_t(kNonFinite)) : 0;
-            out->pairs = counts ? counts[kContacts] : 0u;
-            out->kernel_error = *e.err;
-        }
-        if (flags) flags[0] = flags[1] = 0;  // for the next evaluation
-    }
-    const int2 r = t.brange[inst];
-    const int2 er = t.erange[inst];
-    const int fan = (r.y - r.x) + (er.y - er.x) <= kFinSingle ? 1 : kFinFan;
-    if (!t.active[inst] || f >= fan) return;
-    double all[9] = {};  // sums: beamE, elastic, plastic, gravityE, platenE, reaction, contactE, contacts, |g|^2
+static_assert(kFinPartDoubles == kFinFan * kFinVals, "first-stage totals");
+
+struct TotalParts {
+    double sum[9][kEvalBlock / 32];
+    long long m[2][kEvalBlock / 32];
+    double tot[kFinVals];
+    int nonfinite;
+};
+// Totals of the beam blocks r and gather blocks er (every fan-th from f on) into sm.tot.
+__device__ __forceinline__ void sum_parts(const EvalBufs& e, int2 r, int2 er, int f, int fan, TotalParts& sm) {
+    double all[9] = {};        // sums: beamE, elastic, plastic, gravityE, platenE, reaction, contactE, contacts, |g|^2
     long long m2[2] = {0, 0};  // max penetration, max |g| (bits of non-negative doubles)
-    for (int k = r.x + f + fan * int(threadIdx.x); k < r.y; k += fan * int(blockDim.x)) {
+    for (int k = r.x + f + fan * int(threadIdx.x); k < r.y; k += fan * kEvalBlock) {
         const double* q = e.part_beam + 3 * size_t(k);
         all[0] += q[0]; all[1] += q[1]; all[2] += q[2];
     }
-    for (int k = er.x + f + fan * int(threadIdx.x); k < er.y; k += fan * int(blockDim.x)) {
+#pragma unroll 2
+    for (int k = er.x + f + fan * int(threadIdx.x); k < er.y; k += fan * kEvalBlock) {
         const double* q = e.part_node + kNodeParts * size_t(k);
-        all[3] += q[0]; all[4] += q[1]; all[5] += q[2];
-        m2[0] = max(m2[0], __double_as_longlong(q[3]));
-        all[7] += q[4];
-        all[6] += q[5];
-        all[8] += q[6];
-        m2[1] = max(m2[1], __double_as_longlong(q[7]));
+        all[3] += __ldcg(q); all[4] += __ldcg(q + 1); all[5] += __ldcg(q + 2);
+        m2[0] = max(m2[0], __double_as_longlong(__ldcg(q + 3)));
+        all[7] += __ldcg(q + 4);
+        all[6] += __ldcg(q + 5);
+        all[8] += __ldcg(q + 6);
+        m2[1] = max(m2[1], __double_as_longlong(__ldcg(q + 7)));
     }
-    block_sum_t<9>(all, sm);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    long long* smx = reinterpret_cast<long long*>(sm);
-#pragma unroll
-    for (int k = 0; k < 2; k++) {
-        const long long m = warp_max_key(m2[k]);
-        if (lane == 0) smx[k * (kBlock / 32) + warp] = m;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, j = lane >> 3;
+    const double a = warp_sum4(all[0], all[1], all[2], all[3]), b = warp_sum4(all[4], all[5], all[6], all[7]);
+    const double c = warp_sum(all[8]);
+    const long long pm = warp_max_key(m2[0]), gm = warp_max_key(m2[1]);
+    if ((lane & 7) == 0) {
+        sm.sum[j][warp] = a;
+        sm.sum[4 + j][warp] = b;
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int w = 1; w < kBlock / 32; w++) {
-            smx[0] = max(smx[0], smx[w]);
-            smx[kBlock / 32] = max(smx[kBlock / 32], smx[kBlock / 32 + w]);
-        }
-        for (int k = 0; k < 9; k++) tot[k] = all[k];
-        tot[9] = __longlong_as_double(smx[0]);
-        tot[10] = __longlong_as_double(smx[kBlock / 32]);
-        state = 1;
-        if (fan > 1) {
-            double* fp = e.part_fin + size_t(kFinPartDoubles) * inst;
-            for (int k = 0; k < kFinVals; k++) fp[kFinVals * f + k] = tot[k];
-            __threadfence();
-            unsigned* done = reinterpret_cast<unsigned*>(fp + kFinPartDoubles - 1);
-            state = atomicAdd(done, 1u) == unsigned(fan) - 1u;
-            if (state) *done = 0;
-            __threadfence();
-        }
+    if (lane == 0) {
+        sm.sum[8][warp] = c;
+        sm.m[0][warp] = pm;
+        sm.m[1][warp] = gm;
     }
     __syncthreads();
-    if (!state) return;
-    if (fan > 1) {
-        const double* fp = e.part_fin + size_t(kFinPartDoubles) * inst;
-        for (int k = warp; k < kFinVals; k += kBlock / 32) {
-            const double v = __ldcg(fp + kFinVals * lane + k);
-            const double s = k < 9 ? warp_sum(v) : warp_max(v);
-            if (lane == 0) tot[k] = s;
-        }
-        __syncthreads();
+    const int tid = threadIdx.x;
+    constexpr int nw = kEvalBlock / 32;
+    if (tid < 9) {
+        double s = sm.sum[tid][0];
+        for (int w = 1; w < nw; w++) s += sm.sum[tid][w];
+        sm.tot[tid] = s;
+    } else if (tid < kFinVals) {
+        long long m = sm.m[tid - 9][0];
+        for (int w = 1; w < nw; w++) m = max(m, sm.m[tid - 9][w]);
+        sm.tot[tid] = __longlong_as_double(m);
     }
-    if (threadIdx.x == 0) {
+    __syncthreads();
+}
+// The instance's results from its totals sm.tot, by a whole block; clears the gradient of a
+// non-finite evaluation (sim.cpp:172).
+__device__ __forceinline__ void write_out(const DevTopo& t, const PhysParams& p, const EvalBufs& e, int inst, TotalParts& sm,
+                                          double* __restrict__ grad) {
+    const double* tot = sm.tot;
+    if (threadIdx.x == 0 || threadIdx.x == 32) {  // one the energies, one the residual (a division and a root)
         const double* c = e.cen + 9 * size_t(inst);
         const double center = .5 * p.centering * (sqr(c[0]) + sqr(c[2]));
         // Group order of the reference's accumulation: beams, gravity, centering,
@@ -742,35 +613,201 @@ __global__ void __launch_bounds__(kBlock) k_finalize(DevTopo t, PhysParams p, Ev
         energy += tot[6];
         energy += tot[4];
         const int nonfinite = isfinite(energy) ? 0 : 1;
-        // a non-finite evaluation has a zero gradient
-        const long long nf = t.inst_free[inst];
-        const double rms = nonfinite ? 0.0 : (nf ? sqrt(tot[8] / double(nf)) : 0.0);
-        for (EvalOut* o : {e.out, e.out_host}) {
-            if (!o) continue;
-            EvalOut* out = o + inst;
-            out->energy = nonfinite ? __longlong_as_double(0x7ff0000000000000LL) : energy;
-            out->elastic = tot[1];
-            out->plastic = tot[2];
-            out->contact = tot[6] + tot[4];
-            out->reaction = tot[5];
-            out->max_pen = tot[9];
-            out->contacts = int(tot[7]);
-            out->nonfinite = nonfinite;
-            out->beam_energy = tot[0];
-            out->node_energy = tot[3];
-            out->center_energy = center;
-            out->contact_energy = tot[6];
-            out->platen_energy = tot[4];
-            out->rms = rms;
-            out->gmax = nonfinite ? 0.0 : tot[10];
+        if (threadIdx.x == 32) {
+            const long long nf = t.inst_free[inst];
+            const double rms = nonfinite ? 0.0 : (nf ? sqrt(tot[8] / double(nf)) : 0.0);
+            for (EvalOut* o : {e.out, e.out_host}) {
+                if (!o) continue;
+                o[inst].rms = rms;
+                o[inst].gmax = nonfinite ? 0.0 : tot[10];
+            }
+        } else {
+            for (EvalOut* o : {e.out, e.out_host}) {
+                if (!o) continue;
+                EvalOut* out = o + inst;
+                out->energy = nonfinite ? __longlong_as_double(0x7ff0000000000000LL) : energy;
+                out->elastic = tot[1];
+                out->plastic = tot[2];
+                out->contact = tot[6] + tot[4];
+                out->reaction = tot[5];
+                out->max_pen = tot[9];
+                out->contacts = int(tot[7]);
+                out->nonfinite = nonfinite;
+                out->beam_energy = tot[0];
+                out->node_energy = tot[3];
+                out->center_energy = center;
+                out->contact_energy = tot[6];
+                out->platen_energy = tot[4];
+            }
+            sm.nonfinite = nonfinite;
         }
-        state = nonfinite ? 2 : 0;
     }
     __syncthreads();
-    if (state == 2) {  // non-finite energy: the instance's whole gradient is zero (sim.cpp:172)
-        double* g = grad + 6 * size_t(t.eblk[er.x].x);
+    if (sm.nonfinite) {  // non-finite energy: the instance's whole gradient is zero
+        double* g = grad + 6 * size_t(t.eblk[t.erange[inst].x].x);
         for (long long k = threadIdx.x; k < 6LL * t.inst_n[inst]; k += blockDim.x) g[k] = 0;
     }
+}
+// Gather blocks of an instance: two per evaluation block.
+__device__ __forceinline__ int2 gather_range(const DevTopo& t, int inst) {
+    const int2 er = t.erange[inst];
+    return make_int2(2 * er.x, 2 * er.y);
+}
+
+// One half-node per thread (warps 0 and 1 the translations of 64 nodes, 2 and 3 their rotations).
+// Bound by the FP64 pipe (the incident vectors' additions) and, up to 10^4 nodes, the latency of
+// their loads: a whole node per thread takes twice the additions in a row.
+// Only what nearly every node has is reduced always (gravity energy and |g|^2, in five FP64
+// additions a warp); platen and contact totals where a node of the warp touches something.
+// 2x4x2 specimen 73.3 -> 66.5 us a call, 19x15x11 88.4 -> 82.4, a minimization of 6x6x6 1.04x, with
+// the totals summed here; 64x64x32 and larger as before with whole nodes per thread.
+// kMinBlocks: units of 256 threads per SM the register allocation must allow.
+template <bool F32, int kMinBlocks>
+__global__ void __launch_bounds__(kEvalBlock, 2 * kMinBlocks) k_gather(DevTopo t, PhysParams p, ContactBufs c,
+                                                                       int use_contacts, EvalBufs e,
+                                                                       double* __restrict__ grad) {
+    constexpr int kNodes = kGatherNodes;
+    static_assert(kNodes == 64, "two warps of translations, two of rotations");
+    __shared__ GatherParts sm;
+    __shared__ TotalParts ts;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {  // of the whole evaluation, whether instance 0 is active or not
+        for (EvalOut* out : {e.out, e.out_host}) {
+            if (!out) continue;
+            out->overflow = use_contacts ? int(c.flags[0] & ~uint32_t(kNonFinite)) : 0;
+            out->pairs = use_contacts ? c.counts[kContacts] : 0u;
+            out->kernel_error = *e.err;
+        }
+        if (use_contacts) c.flags[0] = c.flags[1] = 0;  // for the next evaluation
+    }
+    const int4 blk = t.eblk[blockIdx.x >> 1];
+    const int inst = blk.z;
+    if (!t.active[inst]) return;  // block-uniform
+    const int half = threadIdx.x / kNodes, at = kNodes * (blockIdx.x & 1) + threadIdx.x % kNodes;
+    const int i = blk.x + at;
+    double egrav = 0, g2 = 0, eplat = 0, reac = 0, econt = 0, pen_max = 0;
+    int count = 0;
+    unsigned long long gbits = 0;  // max |g| as the bits of a non-negative double (integer max)
+    if (at < blk.y) {
+        d3 g = sum_slots<F32>(t, e, i, half);
+        if (half == 0) {
+            const d3 xi = ldx(e.x, i);
+            // gravity (sim.cpp:142)
+            const double mg = t.mass[i] * p.gravity;
+            egrav = mg * xi.y;
+            g.y += mg;
+            // centering (sim.cpp:143), the same force for all nodes of the instance
+            g.x += e.cforce[2 * inst];
+            g.z += e.cforce[2 * inst + 1];
+            // self-contact: the node's fixed-point sums, cleared for the next evaluation
+            const unsigned long long items = use_contacts ? c.n_count[i] : 0ULL;
+            if (items) {
+                NodeContact& r = c.n_sum[i];
+                g.x += fixed_value(r.f[0], c.force_e0);
+                g.y += fixed_value(r.f[1], c.force_e0);
+                g.z += fixed_value(r.f[2], c.force_e0);
+                if (items >> 32) {
+                    econt = fixed_value(r.energy, c.energy_e0);
+                    pen_max = __longlong_as_double((long long)r.pen);
+                }
+                if (items & kContactNotFinite) econt = __longlong_as_double(0x7ff8000000000000LL);
+                count = int(items >> 32);
+                r = NodeContact{};
+                c.n_count[i] = 0;
+            }
+            // platens (sim.cpp:168-171)
+            const double jr = p.joint_radius, kc = p.contact_k;
+            const double pb = jr - xi.y;
+            if (positive(pb)) {
+                const double mm = kc * pb;
+                eplat += .5 * kc * pb * pb;
+                pen_max = fmax(pen_max, pb);
+                count += 1;
+                g.y -= mm;
+            }
+            const double pt = xi.y + jr - e.tops[inst];
+            if (positive(pt)) {
+                const double mm = kc * pt;
+                eplat += .5 * kc * pt * pt;
+                reac += mm;
+                pen_max = fmax(pen_max, pt);
+                count += 1;
+                g.y += mm;
+            }
+            g = g * p.translation_scale;
+        }
+        // pack and lock (sim.cpp:172)
+        const uint8_t* li = t.locked + 6 * size_t(i) + 3 * half;
+        double gv[3] = {g.x, g.y, g.z};
+        double* out = grad + 6 * size_t(i) + 3 * half;
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            if (li[k]) gv[k] = 0.0;
+            // residual over free DOFs for the solver's convergence test (sim.cpp:44-45)
+            g2 = fma(gv[k], gv[k], g2);
+            // fmax(gmax, |g|) on the bit patterns; a NaN (above the infinity pattern) is
+            // skipped as fmax skips it
+            const unsigned long long b = (unsigned long long)__double_as_longlong(gv[k]) & 0x7fffffffffffffffULL;
+            if (b <= 0x7ff0000000000000ULL && b > gbits) gbits = b;
+            out[k] = gv[k];
+        }
+    }
+    // the rotations' share of the residual goes to the translations' thread of the node
+    if (half == 1) {
+        sm.g2[threadIdx.x - kNodes] = g2;
+        sm.gbits[threadIdx.x - kNodes] = (long long)gbits;
+    }
+    __syncthreads();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (half == 0) {
+        const double v = warp_sum2(egrav, g2 + sm.g2[threadIdx.x]);
+        const long long gm = warp_max_key(max((long long)gbits, sm.gbits[threadIdx.x]));
+        double w = 0;
+        long long pm = 0;
+        int cn = 0;
+        if (__any_sync(0xffffffffu, count != 0 || __double_as_longlong(econt) != 0)) {
+            w = warp_sum4(eplat, reac, econt, 0.0);
+            pm = warp_max_key(__double_as_longlong(pen_max));
+            cn = __reduce_add_sync(0xffffffffu, count);
+        }
+        if (lane == 0) {
+            sm.m[0][warp] = pm;
+            sm.m[1][warp] = gm;
+            sm.count[warp] = cn;
+        }
+        if ((lane & 15) == 0) sm.sum[lane >> 4][warp] = v;
+        if ((lane & 7) == 0 && lane < 24) sm.sum[2 + (lane >> 3)][warp] = w;
+    }
+    __syncthreads();
+    const int tid = threadIdx.x;
+    double* q = e.part_node + kNodeParts * size_t(blockIdx.x);
+    if (tid < 5) q[tid == 0 ? 0 : tid == 1 ? 6 : tid == 2 ? 1 : tid == 3 ? 2 : 5] = sm.sum[tid][0] + sm.sum[tid][1];
+    else if (tid < 7) q[tid == 5 ? 3 : 7] = __longlong_as_double(max(sm.m[tid - 5][0], sm.m[tid - 5][1]));
+    else if (tid == 7) q[4] = double(sm.count[0] + sm.count[1]);
+    const int2 r = t.brange[inst], gr = gather_range(t, inst);
+    if ((r.y - r.x) + (gr.y - gr.x) > kFinSingle) return;  // k_finalize's
+    if (!last_block(e.done + inst, unsigned(gr.y - gr.x))) return;
+    sum_parts(e, r, gr, 0, 1, ts);
+    write_out(t, p, e, inst, ts, grad);
+}
+
+// Totals of the instances of more than kFinSingle block partials.
+__global__ void __launch_bounds__(kEvalBlock) k_finalize(DevTopo t, PhysParams p, EvalBufs e, double* __restrict__ grad) {
+    __shared__ TotalParts sm;
+    const int inst = blockIdx.y, f = blockIdx.x;
+    const int2 r = t.brange[inst], gr = gather_range(t, inst);
+    if (!t.active[inst] || (r.y - r.x) + (gr.y - gr.x) <= kFinSingle) return;
+    sum_parts(e, r, gr, f, kFinFan, sm);
+    double* fp = e.part_fin + size_t(kFinPartDoubles) * inst;
+    if (threadIdx.x < kFinVals) fp[kFinVals * f + threadIdx.x] = sm.tot[threadIdx.x];
+    if (!last_block(e.done + inst, kFinFan)) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int k = warp; k < kFinVals; k += kEvalBlock / 32) {
+        const double v = __ldcg(fp + kFinVals * lane + k);
+        const double s = k < 9 ? warp_sum(v) : warp_max(v);
+        if (lane == 0) sm.tot[k] = s;
+    }
+    __syncthreads();
+    write_out(t, p, e, inst, sm, grad);
 }
 
 // ---- commit (MC/src/sim.cpp:212): base state <- current state, plastic <- trial ----------
@@ -908,7 +945,7 @@ void launch_from_records7(long long B, const double* aos, double* soa, cudaStrea
 
 // Occupancy variants of the FP64 beam kernel (256-thread units per SM) and of the gather.
 constexpr int kBeamBlocks[] = {1, 2, 3};
-constexpr int kGatherBlocks[] = {1, 2, 4};
+constexpr int kGatherBlocks[] = {4, 2, 1};
 
 int shape_variants(ShapeKernel k) {
     switch (k) {
@@ -944,9 +981,9 @@ void gather_variant(const DevTopo& t, const PhysParams& p, const ContactBufs* c,
     if (c) cc = *c;
     const int uc = c ? 1 : 0;
     switch (variant) {
-        case 1: k_gather<F32, kGatherBlocks[1]><<<t.n_eblk, kEvalBlock, 0, s>>>(t, p, cc, uc, e, grad); break;
-        case 2: k_gather<F32, kGatherBlocks[2]><<<t.n_eblk, kEvalBlock, 0, s>>>(t, p, cc, uc, e, grad); break;
-        default: k_gather<F32, kGatherBlocks[0]><<<t.n_eblk, kEvalBlock, 0, s>>>(t, p, cc, uc, e, grad); break;
+        case 1: k_gather<F32, kGatherBlocks[1]><<<2 * t.n_eblk, kEvalBlock, 0, s>>>(t, p, cc, uc, e, grad); break;
+        case 2: k_gather<F32, kGatherBlocks[2]><<<2 * t.n_eblk, kEvalBlock, 0, s>>>(t, p, cc, uc, e, grad); break;
+        default: k_gather<F32, kGatherBlocks[0]><<<2 * t.n_eblk, kEvalBlock, 0, s>>>(t, p, cc, uc, e, grad); break;
     }
     note_launches(1);
 }
@@ -961,9 +998,9 @@ void launch_gather_mixed(const DevTopo& t, const PhysParams& p, const ContactBuf
     gather_variant<true>(t, p, c, grad, e, s, variant);
 }
 
-void launch_finalize(const DevTopo& t, const PhysParams& p, const ContactBufs* c, double* grad, EvalBufs& e,
-                     cudaStream_t s) {
-    k_finalize<<<dim3(kFinFan, t.I), kBlock, 0, s>>>(t, p, e, c ? c->flags : nullptr, c ? c->counts : nullptr, grad);
+void launch_finalize(const DevTopo& t, const PhysParams& p, double* grad, EvalBufs& e, cudaStream_t s) {
+    if (!t.large_totals) return;
+    k_finalize<<<dim3(kFinFan, t.I), kEvalBlock, 0, s>>>(t, p, e, grad);
     note_launches(1);
 }
 

@@ -1,0 +1,57 @@
+"""The node gather and the totals at the sizes where their blocks and paths end: fewer nodes than a
+64-node gather block, exactly one and two, one more; and lattices on either side of the number of
+block partials (768) up to which the last gather block sums the totals instead of a kernel of its
+own.  FP64 against the CPU restatement at the bars of the reference fixtures; both forms in a batch,
+bit for bit what each lattice gives alone."""
+import numpy as np
+import pytest
+
+from conftest import rel_err
+from falling_dice_gb300 import abi, workloads
+
+pytestmark = pytest.mark.gpu
+
+
+def specimen(mcg, cells, kind, precision=abi.MCG_FP64):
+    cfg, spec = workloads.bcc(cells)
+    spec.kind = kind
+    cfg.precision = precision
+    lat = mcg.generate_lattice(spec, cfg)
+    z, pl = mcg.random_state(lat, 0.05, 0.1, 0.02, 7)
+    return cfg, lat, z, pl, lat.geometry.top0 - 0.002
+
+
+# nodes: 8, 63, 64, 66, 126, 128, 130
+SMALL = [(1, 1, 1), (2, 2, 6), (3, 3, 3), (1, 2, 10), (2, 5, 6), (1, 7, 7), (1, 4, 12)]
+# block partials of the cubic+BCC lattices: 717 and 841
+CASES = [(c, abi.MCG_LATTICE_CUBIC) for c in SMALL] + [((n, n, n), abi.MCG_LATTICE_CUBIC_BCC) for n in (18, 19)]
+
+
+@pytest.mark.parametrize("cells,kind", CASES)
+def test_totals_and_gradient_against_the_restatement(mcg, mco, cells, kind):
+    cfg, lat, z, pl, top = specimen(mcg, cells, kind)
+    sol, orc = mcg.Solver(cfg, lat), mco.Model("mco", cfg, lattice=lat)
+    sol.set_state(plastic=pl)
+    orc.set_state(plastic=pl)
+    r, o = sol.objective(z, top), orc.objective(z, top)
+    assert abs(r["energy"] - o["energy"]) <= 1e-10 * abs(o["energy"])
+    assert rel_err(r["grad"], o["grad"]) <= 1e-10
+    for k in ("elastic", "plastic", "contact", "reaction"):
+        assert abs(r["diag"][k] - o["diag"][k]) <= 1e-10 * max(abs(o["diag"][k]), 1e-12), k
+    assert r["diag"]["max_pen"] == o["diag"]["max_pen"] and r["diag"]["contacts"] == int(o["diag"]["contacts"])
+
+
+@pytest.mark.parametrize("precision,sizes", [(abi.MCG_FP64, (19, 1, 18, 3)), (abi.MCG_MIXED, (22, 1, 21, 3))])
+def test_a_batch_across_the_paths_is_bitwise_the_single_lattices(mcg, precision, sizes):
+    parts = [specimen(mcg, (n, n, n), abi.MCG_LATTICE_CUBIC_BCC, precision) for n in sizes]
+    batch = mcg.BatchSolver(parts[0][0], [p[1] for p in parts])
+    batch.set_state(plastic=np.concatenate([p[3] for p in parts]))
+    got = batch.objective(np.concatenate([p[2] for p in parts]), [p[4] for p in parts])
+    off = batch.node_offsets
+    for k, (cfg, lat, z, pl, top) in enumerate(parts):
+        sol = mcg.Solver(cfg, lat)
+        sol.set_state(plastic=pl)
+        ref = sol.objective(z, top)
+        assert got["energy"][k] == ref["energy"], k
+        assert np.array_equal(got["grad"][6 * off[k]:6 * off[k + 1]], ref["grad"]), k
+        assert got["diag"][k] == ref["diag"], k

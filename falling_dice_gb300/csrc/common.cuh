@@ -220,15 +220,7 @@ __device__ __forceinline__ q4 qnorm_near(q4 q) {
     return {q.w * r, q.x * r, q.y * r, q.z * r};
 }
 
-// Rotation matrix of a unit quaternion, rows as 32-byte records (x, y, z, pad).
 struct m3 { d3 r0, r1, r2; };
-__device__ __forceinline__ m3 quat_matrix(q4 q) {
-    const double x2 = twice(q.x), y2 = twice(q.y), z2 = twice(q.z);
-    const double wx = q.w * x2, wy = q.w * y2, wz = q.w * z2;
-    return m3{d3{fma(-q.y, y2, fma(-q.z, z2, 1.0)), fma(q.x, y2, -wz), fma(q.x, z2, wy)},
-              d3{fma(q.x, y2, wz), fma(-q.x, x2, fma(-q.z, z2, 1.0)), fma(q.y, z2, -wx)},
-              d3{fma(q.x, z2, -wy), fma(q.y, z2, wx), fma(-q.x, x2, fma(-q.y, y2, 1.0))}};
-}
 __device__ __forceinline__ d3 fmrot(const m3& m, d3 v) { return d3{fdot(m.r0, v), fdot(m.r1, v), fdot(m.r2, v)}; }
 __device__ __forceinline__ d3 fmrot_t(const m3& m, d3 v) {
     return fmadd(m.r2, v.z, fmadd(m.r1, v.y, m.r0 * v.x));
@@ -237,6 +229,125 @@ __device__ __forceinline__ d3 mrot(const m3& m, d3 v) { return d3{dot(m.r0, v), 
 __device__ __forceinline__ d3 mrot_t(const m3& m, d3 v) {
     return d3{m.r0.x * v.x + m.r1.x * v.y + m.r2.x * v.z, m.r0.y * v.x + m.r1.y * v.y + m.r2.y * v.z,
               m.r0.z * v.x + m.r1.z * v.y + m.r2.z * v.z};
+}
+
+// ---- unit vectors in fixed point -----------------------------------------------------------
+// An FP64 instruction occupies a sub-partition for 64 cycles, a 32 x 32 -> 64-bit multiply-add for a
+// few: sums of products of numbers up to two in magnitude (rotation matrices, unit quaternions and
+// vectors) are cheaper on the integer pipe, which stands idle beside FP64, and no less exact.
+// A number is (h 2^30 + l) 2^-58, |l| <= 2^29: products of two upper halves, and of an upper and a
+// lower one, sum up in 64 bits each; the lower halves' products, below 2^-58, are left out.  A sum
+// of three products is off by at most 2^-56 = 1.4e-17 (FP64 additions near one: 1.1e-16 each).
+// "Units" are 64-bit integers of 2^-58.
+struct fx { int h, l; };
+struct fx3 { fx x, y, z; };
+struct fx4 { fx w, x, y, z; };
+constexpr long long kFxOne = 1LL << 58;
+__device__ __forceinline__ fx fx_of(long long n) {
+    const int h = int((n + (1 << 29)) >> 30);
+    return fx{h, int(unsigned(n) - (unsigned(h) << 30))};
+}
+__device__ __forceinline__ fx operator-(fx a) { return fx{-a.h, -a.l}; }
+// m 2^-s or m 2^s of a 53-bit mantissa; 0 from 2^-63 on.
+__device__ __forceinline__ unsigned long long shift_mantissa(unsigned long long m, int s) {
+    return s >= 0 ? m << min(s, 11) : m >> min(-s, 63);
+}
+// v in units of 2^(scale - 1075) ... for a double's mantissa m 2^(e - 1075): m 2^(e - scale).
+__device__ __forceinline__ unsigned long long fixed_magnitude(double v, int scale) {
+    const unsigned hi = unsigned(__double2hiint(v));
+    const unsigned long long m = (unsigned long long)(hi & 0xfffffu | 0x100000u) << 32 | unsigned(__double2loint(v));
+    return shift_mantissa(m, int(hi >> 20 & 0x7ffu) - scale);
+}
+// v (|v| < 2) in units, rounded toward zero; some integer when v is larger or not finite.
+__device__ __forceinline__ long long fx_units(double v) {
+    const long long n = (long long)fixed_magnitude(v, 1017);
+    return __double2hiint(v) < 0 ? -n : n;
+}
+// n 2^e2, rounded to nearest; 2^-900 < the magnitude < 2^900 or zero.
+__device__ __forceinline__ double fx_double(long long n, int e2 = -58) {
+    const unsigned long long a = n < 0 ? 0ULL - (unsigned long long)n : (unsigned long long)n;
+    const int z = __clzll((long long)a);
+    const unsigned long long m = a << z;
+    unsigned long long b = ((unsigned long long)(1023 + 62 - z + e2) << 52) + (m >> 11) + (m >> 10 & 1);
+    if (n == 0) b = 0;
+    return __longlong_as_double((long long)(n < 0 ? b | 0x8000000000000000ULL : b));
+}
+__device__ __forceinline__ double fx_double(fx a) { return fx_double((long long)a.h * (1 << 30) + a.l); }
+__device__ __forceinline__ long long fx_hh(fx a, fx b) { return (long long)a.h * b.h; }
+__device__ __forceinline__ long long fx_hl(fx a, fx b) { return (long long)a.h * b.l + (long long)a.l * b.h; }
+__device__ __forceinline__ long long fx_sum(long long hh, long long hl) { return hh * 4 + ((hl + (1 << 27)) >> 28); }
+__device__ __forceinline__ long long fx_dot(const fx3& a, const fx3& b) {
+    return fx_sum(fx_hh(a.x, b.x) + fx_hh(a.y, b.y) + fx_hh(a.z, b.z), fx_hl(a.x, b.x) + fx_hl(a.y, b.y) + fx_hl(a.z, b.z));
+}
+__device__ __forceinline__ long long fx_dot(const fx4& a, const fx4& b) {
+    return fx_sum(fx_hh(a.w, b.w) + fx_hh(a.x, b.x) + fx_hh(a.y, b.y) + fx_hh(a.z, b.z),
+                  fx_hl(a.w, b.w) + fx_hl(a.x, b.x) + fx_hl(a.y, b.y) + fx_hl(a.z, b.z));
+}
+// 2 (a b + c d)
+__device__ __forceinline__ long long fx_twice(fx a, fx b, fx c, fx d) {
+    return (fx_hh(a, b) + fx_hh(c, d)) * 8 + ((fx_hl(a, b) + fx_hl(c, d) + (1 << 26)) >> 27);
+}
+// n scaled by 1 - d / 2, d in units (the square of a length that is one but for rounding, less one).
+__device__ __forceinline__ long long fx_renorm(long long n, int d) { return n - (((n >> 30) * d) >> 29); }
+
+// A record of four numbers is stored as four doubles' bits.
+__device__ __forceinline__ double fx_bits(fx a) { return __hiloint2double(a.h, a.l); }
+__device__ __forceinline__ fx fx_load(double v) { return fx{__double2hiint(v), __double2loint(v)}; }
+
+// A node's rotation: the unit quaternion and its matrix, in fixed point.  A quaternion that is not
+// finite has w.h = kFxInvalid.
+constexpr int kFxInvalid = 0x7fffffff;
+struct FxRot { fx3 r0, r1, r2; };
+// Rows 0-2 of the matrix and the quaternion as the node's four records; q normalized to rounding
+// already, here to 2^-56.
+__device__ __forceinline__ void store_rotation(q4 q, double4_32a* __restrict__ rec) {
+    const long long u[4] = {fx_units(q.w), fx_units(q.x), fx_units(q.y), fx_units(q.z)};
+    fx4 f{fx_of(u[0]), fx_of(u[1]), fx_of(u[2]), fx_of(u[3])};
+    const int d = int(fx_dot(f, f) - kFxOne);
+    f = fx4{fx_of(fx_renorm(u[0], d)), fx_of(fx_renorm(u[1], d)), fx_of(fx_renorm(u[2], d)), fx_of(fx_renorm(u[3], d))};
+    const auto one_less = [](long long n) { return fx_bits(fx_of(kFxOne - n)); };
+    const auto entry = [](long long n) { return fx_bits(fx_of(n)); };
+    rec[0] = make_double4_32a(one_less(fx_twice(f.y, f.y, f.z, f.z)), entry(fx_twice(f.x, f.y, -f.w, f.z)),
+                              entry(fx_twice(f.x, f.z, f.w, f.y)), 0.0);
+    rec[1] = make_double4_32a(entry(fx_twice(f.x, f.y, f.w, f.z)), one_less(fx_twice(f.x, f.x, f.z, f.z)),
+                              entry(fx_twice(f.y, f.z, -f.w, f.x)), 0.0);
+    rec[2] = make_double4_32a(entry(fx_twice(f.x, f.z, -f.w, f.y)), entry(fx_twice(f.y, f.z, f.w, f.x)),
+                              one_less(fx_twice(f.x, f.x, f.y, f.y)), 0.0);
+    const bool ok = isfinite(q.w) && isfinite(q.x) && isfinite(q.y) && isfinite(q.z);
+    if (!ok) f.w.h = kFxInvalid;
+    rec[3] = make_double4_32a(fx_bits(f.w), fx_bits(f.x), fx_bits(f.y), fx_bits(f.z));
+}
+__device__ __forceinline__ fx3 load_fx3(const double4_32a* rec) {
+    const double4_32a v = *rec;
+    return fx3{fx_load(v.x), fx_load(v.y), fx_load(v.z)};
+}
+__device__ __forceinline__ fx4 load_fx4(const double4_32a* rec) {
+    const double4_32a v = *rec;
+    return fx4{fx_load(v.x), fx_load(v.y), fx_load(v.z), fx_load(v.w)};
+}
+__device__ __forceinline__ FxRot load_rotation(const double4_32a* rec) {
+    return FxRot{load_fx3(rec), load_fx3(rec + 1), load_fx3(rec + 2)};
+}
+__device__ __forceinline__ m3 fx_matrix(const FxRot& r) {
+    const auto row = [](const fx3& v) { return d3{fx_double(v.x), fx_double(v.y), fx_double(v.z)}; };
+    return m3{row(r.r0), row(r.r1), row(r.r2)};
+}
+// M v for any vector: its components to one exponent, 58 bits below the largest.
+__device__ __forceinline__ d3 fx_rotate(const FxRot& r, d3 v) {
+    const auto exponent = [](double a) { return int(unsigned(__double2hiint(a)) >> 20 & 0x7ffu); };
+    const int e = max(exponent(v.x), max(exponent(v.y), exponent(v.z)));
+    if (unsigned(e - 300) > 1400u) {  // tiny (zero, usually) or huge
+        const m3 m = fx_matrix(r);
+        return fmrot(m, v);
+    }
+    // the largest component in [1/2, 1): its exponent 1022
+    const auto units = [e](double a) {
+        const long long n = (long long)fixed_magnitude(a, e - 5);
+        return __double2hiint(a) < 0 ? -n : n;
+    };
+    const fx3 f{fx_of(units(v.x)), fx_of(units(v.y)), fx_of(units(v.z))};
+    return d3{fx_double(fx_dot(r.r0, f), e - 1022 - 58), fx_double(fx_dot(r.r1, f), e - 1022 - 58),
+              fx_double(fx_dot(r.r2, f), e - 1022 - 58)};
 }
 
 // ---- deterministic reductions ------------------------------------------------------------

@@ -253,7 +253,7 @@ struct mcg_ctx {
     // (64x64x32: 667 us a call against 681).
     unsigned long long graph_flags() const { return mixed ? 0 : cudaGraphInstantiateFlagUseNodePriority; }
     cudaStream_t fork = nullptr;
-    cudaEvent_t fork_ev[2] = {};
+    cudaEvent_t fork_ev[3] = {};
     void make_fork() {
         if (fork) return;
         int least = 0, greatest = 0;
@@ -515,17 +515,28 @@ struct mcg_ctx {
         p.inv_cell_f = float(1.0 / broad_cell);
         mark(0);
         const BuildArgs ba = build_args(cb, contact_skin, broad_cell);
-        if (mixed) launch_state_mixed(topo, p, dz, d_baseX, mn, ba, ev, stream);
-        else launch_state(topo, p, dz, d_baseX, d_baseR, ba, ev, stream);
         const ContactBufs* cptr = p.self_contact ? &cb : nullptr;
         const bool branch = forked && cptr;
         cudaStream_t cs = branch ? fork : stream;
+        // In the FP64 form the rotations run beside the contact branch; inside the solver's loop beside
+        // the positions too (a graph of its own is launched 2 us later when it begins with two kernels:
+        // 2x4x2 specimen 63.7 us a call this way, 66.2 the other; a minimization of the 6x6x6
+        // specimen 1346 us this way, 1239 the other).
+        const bool beside = branch && !mixed && trials == 2;
+        if (mixed) launch_state_mixed(topo, p, dz, d_baseX, mn, ba, ev, stream);
+        else if (!beside) launch_state(topo, p, dz, d_baseX, ba, ev, stream);
         if (branch) {
             ck(cudaEventRecord(fork_ev[0], stream), "cudaEventRecord");
             ck(cudaStreamWaitEvent(fork, fork_ev[0], 0), "cudaStreamWaitEvent");
         }
+        if (beside) {
+            launch_state(topo, p, dz, d_baseX, ba, ev, fork);
+            ck(cudaEventRecord(fork_ev[2], fork), "cudaEventRecord");
+        }
         launch_center(topo, p, ba, ev, cs);
+        if (!mixed) launch_rotations(topo, dz, d_baseR, ev, stream);
         if (branch) launch_contacts(topo, p, ev, cb, contact_skin, cs);
+        if (beside) ck(cudaStreamWaitEvent(stream, fork_ev[2], 0), "cudaStreamWaitEvent");
         mark(1);
         if (mixed) launch_beams_mixed(topo, mat, mb, mn, trials, ev, stream, beam_variant);
         else launch_beams(topo, mat, d_plastic, trials, ev, stream, beam_variant);
@@ -838,7 +849,8 @@ struct mcg_ctx {
         PhysParams p = phys;
         DevTopo all = topo;  // the committed instances' states (others are recomputed before use)
         all.active = d_all;
-        launch_state(all, p, d_zfinal, d_baseX, d_baseR, BuildArgs{}, ev, stream);
+        launch_state(all, p, d_zfinal, d_baseX, BuildArgs{}, ev, stream);
+        launch_rotations(all, d_zfinal, d_baseR, ev, stream);
         EvalBufs at = ev;
         at.tops_host = nullptr;
         launch_center(all, p, BuildArgs{}, at, stream);
@@ -1427,7 +1439,7 @@ void upload_instances(mcg_ctx* c, const std::vector<InstIn>& ins) {
     EvalBufs e{};
     e.x = V.get<double4_32a>(size_t(N));
     e.R = V.get<double4_32a>(size_t(N));
-    e.M = V.get<double4_32a>(3 * size_t(N));
+    e.M = V.get<double4_32a>(4 * size_t(N));
     e.xf_lo = V.get<float4>(size_t(N));
     e.xf_hi = V.get<float4>(size_t(N));
     e.slot = V.get<double>(12 * size_t(B));
@@ -1811,7 +1823,8 @@ int objective_with_fixed_contacts(mcg_ctx* c, ContactBufs& fixed, size_t zero_by
         }
         const BuildArgs ba = c->build_args(fixed, 0.f, p.broad_cell);  // always rebuilds
         if (c->mixed) launch_state_mixed(c->topo, p, c->d_zin, c->d_baseX, c->mn, ba, c->ev, s);
-        else launch_state(c->topo, p, c->d_zin, c->d_baseX, c->d_baseR, ba, c->ev, s);
+        else launch_state(c->topo, p, c->d_zin, c->d_baseX, ba, c->ev, s);
+        if (!c->mixed) launch_rotations(c->topo, c->d_zin, c->d_baseR, c->ev, s);
         launch_center(c->topo, p, ba, c->ev, s);
         if (c->mixed) launch_beams_mixed(c->topo, c->mat, c->mb, c->mn, false, c->ev, s, c->beam_variant);
         else launch_beams(c->topo, c->mat, c->d_plastic, false, c->ev, s, c->beam_variant);

@@ -207,7 +207,7 @@ constexpr int kFinSingle = 768;  // block partials one block sums: six per threa
 struct EvalBufs {
     double4_32a* x;             // [N]
     double4_32a* R;             // [N]
-    double4_32a* M;             // [3N] rotation matrix rows of R (x, y, z, pad)
+    double4_32a* M;             // [4N] R in fixed point: matrix rows (x, y, z, pad), quaternion (fx)
     float4* xf_lo;              // [N] position rounded down to single precision
     float4* xf_hi;              // [N] position rounded up
     double* slot;           // [12B] per beam: (-F, Ga), added to node a, then (+F, Gb), added to
@@ -264,8 +264,9 @@ extern std::atomic<long long> g_launch_count;
 inline void note_launches(int k) { g_launch_count += k; }
 
 // ---- launchers (objective.cu) ----------------------------------------------------------
-void launch_state(const DevTopo& t, const PhysParams& p, const double* z, const double* base_x,
-                  const double* base_r, const BuildArgs& b, EvalBufs& e, cudaStream_t s);
+void launch_state(const DevTopo& t, const PhysParams& p, const double* z, const double* base_x, const BuildArgs& b, EvalBufs& e,
+                  cudaStream_t s);
+void launch_rotations(const DevTopo& t, const double* z, const double* base_r, EvalBufs& e, cudaStream_t s);
 // Occupancy variants of the beam kernels and the gather (CTAs per SM the register allocation
 // allows; the arithmetic is the same in every variant).  Variant 0 is the default.
 enum class ShapeKernel { kBeams, kBeamsMixed, kGather };

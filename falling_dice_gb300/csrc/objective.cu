@@ -4,7 +4,8 @@
 // Compiled without contraction: fused multiply-adds are written out where they are meant, so
 // that a kernel's occupancy variants round identically.
 //
-//   k_state    per node: z -> current position/orientation; block partial sums of x
+//   k_state    per node: z -> current position; block partial sums of x
+//   k_rotations per node: z -> current orientation
 //   k_center   per instance: mean position for the centering term; the contact grid
 //   k_beams    per beam: axial/shear/bending/torsion energy with return mapping,
 //              the two end 6-vectors of its gradient, optional trial state
@@ -20,16 +21,12 @@ namespace mcg {
 static_assert(kMapBlock == kBlock, "the mixed form's beam blocks are launched with kBlock threads");
 
 // ---- node state: MC/src/sim.cpp:136 -------------------------------------------------------
-// Bound by the FP64 pipe like the beam kernel: rotations up to one radian by polynomials
-// (larger ones by the general exponential), the quaternion normalized by one step when its norm
-// is one but for rounding, conversions and maxima on the integer pipe; 128-node blocks.  222 ->
-// 72 FP64 instructions per 32 nodes; 34,897 nodes: 24.1 -> 11.5 us.
+// Positions, their FP32 bounds and block partial sums and extrema: what the contact branch of an
+// evaluation waits for.  Conversions and maxima on the integer pipe; 128-node blocks.
 __global__ void __launch_bounds__(kEvalBlock) k_state(DevTopo t, PhysParams p, const double* __restrict__ z,
-                                                      const double* __restrict__ bx, const double* __restrict__ br,
-                                                      double4_32a* __restrict__ x4, double4_32a* __restrict__ R4,
-                                                      double4_32a* __restrict__ M4, float4* __restrict__ xf_lo,
-                                                      float4* __restrict__ xf_hi, double* __restrict__ part,
-                                                      BuildArgs build) {
+                                                      const double* __restrict__ bx, double4_32a* __restrict__ x4,
+                                                      float4* __restrict__ xf_lo, float4* __restrict__ xf_hi,
+                                                      double* __restrict__ part, BuildArgs build) {
     __shared__ StateParts sm;
     const MapPos mp = map_pos(t.eblk);
     if (!t.active[mp.inst]) return;  // block-uniform
@@ -39,32 +36,16 @@ __global__ void __launch_bounds__(kEvalBlock) k_state(DevTopo t, PhysParams p, c
     bool moved = false;
     if (mp.valid) {
         const double2* z2 = reinterpret_cast<const double2*>(z + 6 * size_t(i));
-        const double2 za = z2[0], zb = z2[1], zc = z2[2];
-        const double zi[6] = {za.x, za.y, zb.x, zb.y, zc.x, zc.y};
+        const double2 za = z2[0], zb = z2[1];
         const uint8_t* li = t.locked + 6 * size_t(i);
-        double tr[3], r[3];
-#pragma unroll
-        for (int d = 0; d < 3; d++) {
-            tr[d] = li[d] ? 0.0 : zi[d];
-            r[d] = li[d + 3] ? 0.0 : zi[d + 3];
-        }
+        const double tr[3] = {li[0] ? 0.0 : za.x, li[1] ? 0.0 : za.y, li[2] ? 0.0 : zb.x};
         // x = base + s t, rounded exactly as the reference (no fused multiply-add), so that
         // positions -- and with them the contact pair set -- are bit-identical.
         const double ts = p.translation_scale;
         const double xx = __dadd_rn(bx[3 * size_t(i)], __dmul_rn(ts, tr[0]));
         const double xy = __dadd_rn(bx[3 * size_t(i) + 1], __dmul_rn(ts, tr[1]));
         const double xz = __dadd_rn(bx[3 * size_t(i) + 2], __dmul_rn(ts, tr[2]));
-        const double4_32a b4 = reinterpret_cast<const double4_32a*>(br)[i];
-        const d3 rv{r[0], r[1], r[2]};
-        const double r2 = fdot(rv, rv);
-        const q4 e = unsigned(__double2hiint(r2)) < 0x3ff00000u ? exp_map_small(rv, r2) : exp_map(rv);
-        const q4 R = qnorm_near(fqmul(e, q4{b4.x, b4.y, b4.z, b4.w}));
         x4[i] = make_double4_32a(xx, xy, xz, 0.0);
-        R4[i] = make_double4_32a(R.w, R.x, R.y, R.z);
-        const m3 M = quat_matrix(R);
-        M4[3 * size_t(i)] = make_double4_32a(M.r0.x, M.r0.y, M.r0.z, 0.0);
-        M4[3 * size_t(i) + 1] = make_double4_32a(M.r1.x, M.r1.y, M.r1.z, 0.0);
-        M4[3 * size_t(i) + 2] = make_double4_32a(M.r2.x, M.r2.y, M.r2.z, 0.0);
         float4 lo, hi;
         bounds.take(xx, xy, xz, t.off[mp.inst], lo, hi);
         xf_lo[i] = lo;
@@ -74,6 +55,28 @@ __global__ void __launch_bounds__(kEvalBlock) k_state(DevTopo t, PhysParams p, c
     }
     if (build.flags) ask_build(build, moved);
     state_block_parts(acc, bounds, sm, part + 9 * size_t(blockIdx.x));
+}
+
+// Orientations R = exp(r) R_base and their fixed-point records, beside the contact branch.  Bound
+// by the FP64 pipe like the beam kernel: rotations up to one radian by polynomials (larger ones by
+// the general exponential), the quaternion normalized by one step when its norm is one but for
+// rounding, the matrix on the integer pipe.  One kernel with the positions held the contact branch
+// of a small lattice back (2x4x2 specimen: 68.5 us a call, split 63.7).
+__global__ void __launch_bounds__(kEvalBlock) k_rotations(DevTopo t, const double* __restrict__ z, const double* __restrict__ br,
+                                                          double4_32a* __restrict__ R4, double4_32a* __restrict__ M4) {
+    const MapPos mp = map_pos(t.eblk);
+    if (!t.active[mp.inst] || !mp.valid) return;
+    const int i = mp.i;
+    const double2* z2 = reinterpret_cast<const double2*>(z + 6 * size_t(i));
+    const double2 zb = z2[1], zc = z2[2];
+    const uint8_t* li = t.locked + 6 * size_t(i);
+    const d3 rv{li[3] ? 0.0 : zb.y, li[4] ? 0.0 : zc.x, li[5] ? 0.0 : zc.y};
+    const double4_32a b4 = reinterpret_cast<const double4_32a*>(br)[i];
+    const double r2 = fdot(rv, rv);
+    const q4 e = unsigned(__double2hiint(r2)) < 0x3ff00000u ? exp_map_small(rv, r2) : exp_map(rv);
+    const q4 R = qnorm_near(fqmul(e, q4{b4.x, b4.y, b4.z, b4.w}));
+    R4[i] = make_double4_32a(R.w, R.x, R.y, R.z);
+    store_rotation(R, M4 + 4 * size_t(i));
 }
 
 // The grid of a rebuilt candidate list: origin, extent and bin numbering from the node bounding
@@ -193,19 +196,10 @@ __global__ void __launch_bounds__(kBlock) k_center(DevTopo t, double centering, 
     if (rebuild) grid_params(build, ext);
 }
 
-__device__ __forceinline__ q4 ldq(const double4_32a* R, int i) {
-    const double4_32a v = R[i];
-    return q4{v.x, v.y, v.z, v.w};
-}
 __device__ __forceinline__ d3 ldx(const double4_32a* x, int i) {
     const double4_32a v = x[i];
     return d3{v.x, v.y, v.z};
 }
-__device__ __forceinline__ m3 ldm(const double4_32a* M, int i) {
-    const double4_32a a = M[3 * size_t(i)], b = M[3 * size_t(i) + 1], c = M[3 * size_t(i) + 2];
-    return m3{d3{a.x, a.y, a.z}, d3{b.x, b.y, b.z}, d3{c.x, c.y, c.z}};
-}
-
 // ---- constitutive return maps: MC/src/sim.cpp:5-8 ------------------------------------------
 // e: the trial elastic part (total - plastic), updated to the elastic part after the return;
 // inv_kH = 1 / max(1e-20, k + H), precomputed per beam (the reference divides).  Elastic and
@@ -268,35 +262,50 @@ __device__ __forceinline__ void chord_length(double l2, double& L, double& invL)
     }
 }
 
+// Polynomials in fixed point, coefficients c of units 2^-kBits, the argument x < 2^(64 - kArg) in
+// units 2^-kArg: Horner's rule by the upper halves of 64 x 64-bit products.
+template <int kBits>
+__device__ constexpr unsigned long long poly_units(double c) {
+    return (unsigned long long)(c * double(1ULL << (kBits - 32)) * 0x1p32);
+}
+template <int kArg>
+__device__ __forceinline__ unsigned long long poly_step(unsigned long long acc, unsigned long long x, unsigned long long c) {
+    return c + (__umul64hi(acc, x) >> (kArg - 64));
+}
+
 // Rotation vector of the relative rotation Q = Ra^* Rb (MC/include/core.hpp:52 quatLog of the
 // normalized Q with w >= 0) and its squared length.  With s = |v| of the unit Q, the vector is
 // 2 asin(s) / s v: a polynomial in s^2 up to s^2 = 0.1 (angles up to 36.9 degrees; Chebyshev
 // interpolation, error 2e-18), so that the usual beam takes no square root, division or
-// arctangent; larger angles take atan2 as the reference does.  Q is a product of two unit
-// quaternions, so its norm differs from one by rounding only and one step corrects it.
-__device__ __forceinline__ d3 relative_rotation(q4 Ra, q4 Rb, double& phi2) {
-    q4 Q = fqmul(conj(Ra), Rb);
-    const d3 v{Q.x, Q.y, Q.z};
-    const double v2 = fdot(v, v), n2 = fma(Q.w, Q.w, v2);
-    const double r = fma(-.5, n2, 1.5);
-    const double s2 = v2 * (r * r);
-    if (near_one(n2) && unsigned(__double2hiint(s2)) < 0x3fb99999u) {  // s2 < 0.1
-        double g = 0x1.c42a558b8b15bp-6;
-        g = fma(g, s2, 0x1.11d08867c9adep-6);
-        g = fma(g, s2, 0x1.80fd1940cecf2p-6);
-        g = fma(g, s2, 0x1.c90c2f25d23e5p-6);
-        g = fma(g, s2, 0x1.1c529e3ddf7c6p-5);
-        g = fma(g, s2, 0x1.6e8b80a6ac006p-5);
-        g = fma(g, s2, 0x1.f1c71d2f31c2ep-5);
-        g = fma(g, s2, 0x1.6db6db6c86271p-4);
-        g = fma(g, s2, 0x1.33333333342e1p-3);
-        g = fma(g, s2, 0x1.5555555555550p-2);
-        g = fma(g, s2, 2.0);
-        phi2 = (g * g) * s2;
-        g = xor_sign(g * r, Q.w);
-        return d3{Q.x * g, Q.y * g, Q.z * g};
+// arctangent; larger angles take atan2 as the reference does.  Q is a product of two quaternions
+// of length one to 2^-56, in fixed point as the polynomial, which lies in [2, 2.04].
+__device__ __forceinline__ d3 relative_rotation(const fx4& a, const fx4& b, double& phi2) {
+    const long long x = fx_dot(a, fx4{b.x, -b.w, -b.z, b.y}), y = fx_dot(a, fx4{b.y, b.z, -b.w, -b.x}),
+                    z = fx_dot(a, fx4{b.z, -b.y, b.x, -b.w});
+    const d3 v{fx_double(x), fx_double(y), fx_double(z)};
+    const double s2 = fdot(v, v);
+    if (unsigned(__double2hiint(s2)) < 0x3fb99999u) {  // s2 < 0.1
+        constexpr int B = 62, X = 67;
+        const unsigned long long u = fixed_magnitude(s2, 1075 - X);
+        unsigned long long g = poly_units<B>(0x1.c42a558b8b15bp-6);
+        g = poly_step<X>(g, u, poly_units<B>(0x1.11d08867c9adep-6));
+        g = poly_step<X>(g, u, poly_units<B>(0x1.80fd1940cecf2p-6));
+        g = poly_step<X>(g, u, poly_units<B>(0x1.c90c2f25d23e5p-6));
+        g = poly_step<X>(g, u, poly_units<B>(0x1.1c529e3ddf7c6p-5));
+        g = poly_step<X>(g, u, poly_units<B>(0x1.6e8b80a6ac006p-5));
+        g = poly_step<X>(g, u, poly_units<B>(0x1.f1c71d2f31c2ep-5));
+        g = poly_step<X>(g, u, poly_units<B>(0x1.6db6db6c86271p-4));
+        g = poly_step<X>(g, u, poly_units<B>(0x1.33333333342e1p-3));
+        g = poly_step<X>(g, u, poly_units<B>(0x1.5555555555550p-2));
+        g = poly_step<X>(g, u, poly_units<B>(2.0));
+        double gd = __longlong_as_double((long long)((1023ULL << 52) + (g >> 11) + (g >> 10 & 1)));
+        phi2 = (gd * gd) * s2;
+        // the sign of Q's real part, which is close to one
+        const long long w = fx_hh(a.w, b.w) + fx_hh(a.x, b.x) + fx_hh(a.y, b.y) + fx_hh(a.z, b.z);
+        gd = __hiloint2double(__double2hiint(gd) | (w < 0 ? int(0x80000000u) : 0), __double2loint(gd));
+        return d3{v.x * gd, v.y * gd, v.z * gd};
     }
-    Q = qnorm(Q);
+    q4 Q = qnorm(q4{fx_double(fx_dot(a, b)), v.x, v.y, v.z});
     if (Q.w < 0) Q = q4{-Q.w, -Q.x, -Q.y, -Q.z};
     const double s = sqrt(Q.x * Q.x + Q.y * Q.y + Q.z * Q.z);
     d3 phi{2 * Q.x, 2 * Q.y, 2 * Q.z};
@@ -307,35 +316,47 @@ __device__ __forceinline__ d3 relative_rotation(q4 Ra, q4 Rb, double& phi2) {
 
 // J_l^{-T}(phi) v (jl_inv_t) with the coefficient as a polynomial in phi2 = |phi|^2 up to 0.42
 // (every angle of relative_rotation's polynomial; Chebyshev interpolation, error 4e-17 against
-// 1/12, which enters multiplied by phi2).
+// 1/12, which enters multiplied by phi2), in [1/12, 0.084] and in fixed point.
 __device__ __forceinline__ d3 transport(d3 phi, double phi2, d3 v) {
     if (unsigned(__double2hiint(phi2)) >= 0x3fdae000u) return jl_inv_t(phi, v);  // 0.4199
-    double A = 0x1.2bf59666dc69ep-31;
-    A = fma(A, phi2, 0x1.6684f73f8bd8ep-26);
-    A = fma(A, phi2, 0x1.bbd7b81461d47p-21);
-    A = fma(A, phi2, 0x1.1566aba745146p-15);
-    A = fma(A, phi2, 0x1.6c16c16c1de72p-10);
-    A = fma(A, phi2, 0x1.5555555555553p-4);
+    constexpr int B = 66, X = 65;
+    const unsigned long long u = fixed_magnitude(phi2, 1075 - X);
+    unsigned long long p = poly_units<B>(0x1.2bf59666dc69ep-31);
+    p = poly_step<X>(p, u, poly_units<B>(0x1.6684f73f8bd8ep-26));
+    p = poly_step<X>(p, u, poly_units<B>(0x1.bbd7b81461d47p-21));
+    p = poly_step<X>(p, u, poly_units<B>(0x1.1566aba745146p-15));
+    p = poly_step<X>(p, u, poly_units<B>(0x1.6c16c16c1de72p-10));
+    p = poly_step<X>(p, u, poly_units<B>(0x1.5555555555553p-4));
+    const double A = __longlong_as_double((long long)((1018ULL << 52) + (p >> 10) + (p >> 9 & 1)));
     const d3 c1 = fcross(phi, v), c2 = fcross(phi, c1);
     return d3{fma(A, c2.x, fma(.5, c1.x, v.x)), fma(A, c2.y, fma(.5, c1.y, v.y)), fma(A, c2.z, fma(.5, c1.z, v.z))};
 }
 
-// The beam's axis in the material frame: unit(Ra^T t), t a unit vector.
-__device__ __forceinline__ d3 material_axis(const m3& Ma, d3 t) {
-    const d3 a = fmrot_t(Ma, t);
-    const double l2 = fdot(a, a);
-    if (near_one(l2)) return a * fma(-.5, l2, 1.5);
-    return unit(a);
+// The beam's axis in the material frame: unit(Ra^T t), t of length one but for rounding.
+__device__ __forceinline__ d3 material_axis(const FxRot& m, const fx3& t) {
+    const int d = int(fx_dot(t, t) - kFxOne);
+    const auto part = [&](fx a, fx b, fx c) { return fx_double(fx_renorm(fx_dot(fx3{a, b, c}, t), d)); };
+    return d3{part(m.r0.x, m.r1.x, m.r2.x), part(m.r0.y, m.r1.y, m.r2.y), part(m.r0.z, m.r1.z, m.r2.z)};
+}
+// R e0 - t: a director's deviation from the chord, in fixed point (e0 of components below two;
+// others, which are no directions, in FP64).
+__device__ __forceinline__ d3 deviation(const FxRot& r, const fx3& e0, const long long (&t)[3], bool unit, d3 e0d, d3 td) {
+    if (unit) return d3{fx_double(fx_dot(r.r0, e0) - t[0]), fx_double(fx_dot(r.r1, e0) - t[1]), fx_double(fx_dot(r.r2, e0) - t[2])};
+    return fmrot(fx_matrix(r), e0d) - td;
 }
 
 // ---- beam kernel: MC/src/sim.cpp:139-141 ---------------------------------------------------
-// Bound by the FP64 pipe (one warp instruction per 19 cycles and SM, beside which loads and the
+// Bound by the FP64 pipe (one warp instruction per 16 cycles and SM, beside which loads and the
 // other pipes are idle), so the formulas are written for few FP64 instructions: energies summed
 // as twice their value, shear from the director-chord differences (2 t - da - db = -(ma + mb)),
-// polynomials for the rotation vector and its transport, square roots from the FP32 estimate,
-// comparisons on bit patterns.
-// Measured at 184,400 beams (32x32x16): 391 -> 265 FP64 instructions per 32 beams, 0.159 ->
-// 0.109 ms (84 % of the FP64 pipe's instruction rate).
+// square roots from the FP32 estimate, comparisons on bit patterns, and everything that is a sum of
+// products of unit vectors (directors, relative rotation, material axis, the moment's rotation) or
+// a polynomial of one's coordinates in fixed point on the integer pipe.  The error against 64 bits
+// is no larger for it (1.2e-16 against 1.3e-16 on the largest lattice, 5.4e-17 / 5.6e-17 on
+// 19x15x11): a fixed-point sum rounds once.
+// FP64 instructions per 32 beams: 391 at first, 265 with all of it in FP64, about 160 now; a call
+// at 2.95 million beams 2474 -> 2100 us, a batch of 762,000 beams 603 -> 509, 184,400 beams
+// compressed 274 -> 258.
 // Blocks of kBeamBlock = 128 beams: one warp on each of an SM's four FP64 units, so that a
 // lattice of a few hundred beams spreads over several SMs.
 // kMinBlocks: units of 256 threads per SM the register allocation must allow (an occupancy
@@ -382,11 +403,14 @@ __global__ void __launch_bounds__(kBeamBlock, 2 * kMinBlocks) k_beams(DevTopo t,
             const double uax2 = t.aL[b] * ax.energy2;
             if (ax.yielded) diss = t.aLsy[b] * ax.dg;
             // shear: the end directors against the chord (rotations by the nodes' matrices)
-            const m3 Ma = ldm(e.M, ab.x), Mb = ldm(e.M, ab.y);
+            const FxRot Ma = load_rotation(e.M + 4 * size_t(ab.x)), Mb = load_rotation(e.M + 4 * size_t(ab.y));
             const d3 e0{t.e0x[b], t.e0y[b], t.e0z[b]};
-            const d3 da = fmrot(Ma, e0), db = fmrot(Mb, e0);
+            const long long tu[3] = {fx_units(tt.x), fx_units(tt.y), fx_units(tt.z)};
+            const fx3 e0f{fx_of(fx_units(e0.x)), fx_of(fx_units(e0.y)), fx_of(fx_units(e0.z))};
+            const auto below_two = [](double v) { return (unsigned(__double2hiint(v)) & 0x7fffffffu) < 0x40000000u; };
+            const bool unit_e0 = below_two(e0.x) && below_two(e0.y) && below_two(e0.z);
+            const d3 ma = deviation(Ma, e0f, tu, unit_e0, e0, tt), mb = deviation(Mb, e0f, tu, unit_e0, e0, tt);
             const double cs = t.cs[b];
-            const d3 ma = da - tt, mb = db - tt;
             const double us2 = fma(mb.z, mb.z, fma(mb.y, mb.y, fma(mb.x, mb.x, fdot(ma, ma))));  // times cs
             const d3 gm = ma + mb;
             const double kt_ = cs * invL;
@@ -394,12 +418,13 @@ __global__ void __launch_bounds__(kBeamBlock, 2 * kMinBlocks) k_beams(DevTopo t,
             // F = t N + ((I - t t^T) g) / L with g = -cs (ma + mb)
             const d3 F{fma(tt.x, kf, -(kt_ * gm.x)), fma(tt.y, kf, -(kt_ * gm.y)), fma(tt.z, kf, -(kt_ * gm.z))};
             const d3 tc = tt * cs;
-            d3 Ga = fcross(tc, da);
-            d3 Gb = fcross(tc, db);
+            d3 Ga = fcross(tc, ma);  // t x (R e0), as t x t = 0
+            d3 Gb = fcross(tc, mb);
             // bending and torsion from the relative rotation Q = Ra^* Rb
             double phi2;
-            const d3 phi = relative_rotation(ldq(e.R, ab.x), ldq(e.R, ab.y), phi2);
-            const d3 axis = material_axis(Ma, tt);
+            const fx4 qa = load_fx4(e.M + 4 * size_t(ab.x) + 3), qb = load_fx4(e.M + 4 * size_t(ab.y) + 3);
+            const d3 phi = relative_rotation(qa, qb, phi2);
+            const d3 axis = material_axis(Ma, fx3{fx_of(tu[0]), fx_of(tu[1]), fx_of(tu[2])});
             const double tw = fdot(phi, axis), ptw = fdot(rotp, axis);
             const d3 bend = fmadd(axis, -tw, phi), pb = fmadd(axis, -ptw, rotp);
             const double kb = t.kb[b], kt = t.kt[b];
@@ -409,10 +434,11 @@ __global__ void __launch_bounds__(kBeamBlock, 2 * kMinBlocks) k_beams(DevTopo t,
             double dr = 0;
             if (br.yielded) dr = t.my[b] * br.dg;
             if (tor.yielded) dr = fma(t.ty[b], tor.dg, dr);
-            const d3 world = fmrot(Ma, transport(phi, phi2, moment));
+            const d3 world = fx_rotate(Ma, transport(phi, phi2, moment));
             Ga = Ga - world;
             Gb = Gb + world;
             elastic2 = fma(cs, us2, uax2) + (br.energy2 + tor.energy2);
+            if (qa.w.h == kFxInvalid || qb.w.h == kFxInvalid) elastic2 = __longlong_as_double(0x7ff8000000000000LL);
             slot[0] = make_double2(-F.x, -F.y);
             slot[1] = make_double2(-F.z, Ga.x);
             slot[2] = make_double2(Ga.y, Ga.z);
@@ -900,9 +926,14 @@ __global__ void __launch_bounds__(kBlock) k_from_records7(long long B, const dou
 }
 
 // ---- launchers ------------------------------------------------------------------------------
-void launch_state(const DevTopo& t, const PhysParams& p, const double* z, const double* base_x,
-                  const double* base_r, const BuildArgs& b, EvalBufs& e, cudaStream_t s) {
-    k_state<<<t.n_eblk, kEvalBlock, 0, s>>>(t, p, z, base_x, base_r, e.x, e.R, e.M, e.xf_lo, e.xf_hi, e.part_state, b);
+void launch_state(const DevTopo& t, const PhysParams& p, const double* z, const double* base_x, const BuildArgs& b, EvalBufs& e,
+                  cudaStream_t s) {
+    k_state<<<t.n_eblk, kEvalBlock, 0, s>>>(t, p, z, base_x, e.x, e.xf_lo, e.xf_hi, e.part_state, b);
+    note_launches(1);
+}
+
+void launch_rotations(const DevTopo& t, const double* z, const double* base_r, EvalBufs& e, cudaStream_t s) {
+    k_rotations<<<t.n_eblk, kEvalBlock, 0, s>>>(t, z, base_r, e.R, e.M);
     note_launches(1);
 }
 

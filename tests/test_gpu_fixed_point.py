@@ -1,0 +1,62 @@
+"""The FP64 beam kernel's fixed-point parts (rotation matrices, relative rotations, directors, the
+moment's rotation) where they take their general forms: quaternions of either sign and any base
+orientation, directors that are no unit vectors, moments beyond the exponents a common scale covers,
+rotations that are not finite; against the CPU restatement at the bars of the reference fixtures."""
+import numpy as np
+import pytest
+
+from conftest import rel_err
+from test_gpu_fp64_paths import model
+from test_gpu_objective import TOL
+
+pytestmark = pytest.mark.gpu
+
+
+def agree(sol, orc, z, top, scale=1.0):
+    r, o = sol.objective(z, top, True), orc.objective(z, top, True)
+    assert np.isfinite(o["energy"])
+    assert abs(r["energy"] - o["energy"]) <= TOL * abs(o["energy"])
+    assert rel_err(r["grad"] * scale, o["grad"] * scale) <= TOL
+    assert rel_err(r["trial_next"] * scale, o["trial_next"] * scale) <= TOL
+    assert np.array_equal(r["trial_flags"], o["trial_flags"])
+
+
+@pytest.mark.parametrize("sigma_b,sigma_r", [(0.0, 0.1), (0.2, 0.0), (0.5, 0.3), (3.0, 0.5)])
+def test_base_orientations_of_either_sign(mcg, mco, sigma_b, sigma_r):
+    cfg, lat, sol, orc = model(mcg, mco, "bcc", (3, 2, 2))
+    rng = np.random.default_rng(4)
+    v = sigma_b * rng.standard_normal((lat.n_nodes, 3))
+    a = np.maximum(np.linalg.norm(v, axis=1, keepdims=True), 1e-300)
+    q = np.hstack([np.cos(a / 2), np.sin(a / 2) * v / a]) * rng.choice([-1.0, 1.0], (lat.n_nodes, 1))
+    z, _ = mcg.random_state(lat, 0.02, sigma_r, 0.0, 5)
+    for m in (sol, orc):
+        m.set_state(base_r=q.ravel())
+    agree(sol, orc, z, lat.geometry.top0 + 0.01)
+
+
+@pytest.mark.parametrize("length", [1.0, 1.5, 40.0, 1e-3])
+def test_directors_that_are_no_unit_vectors(mcg, mco, length):
+    cfg, lat, _, _ = model(mcg, mco, "bcc", (2, 2, 2))
+    lat.e0[:] = (lat.e0.reshape(-1, 3) * np.where(np.arange(lat.n_beams) % 2, length, 1.0)[:, None]).reshape(lat.e0.shape)
+    z, _ = mcg.random_state(lat, 0.02, 0.1, 0.0, 5)
+    agree(mcg.Solver(cfg, lat), mco.Model("mco", cfg, lattice=lat), z, lat.geometry.top0 + 0.01)
+
+
+@pytest.mark.parametrize("young", [2.0e-230, 2.0e-3, 2.0e120])
+def test_moments_of_any_exponent(mcg, mco, young):
+    cfg, lat, _, _ = model(mcg, mco, "bcc", (2, 2, 2), young=young)
+    cfg.material.hardening = 0.05 * young
+    cfg.material.yield_ = 1e3 * young  # elastic
+    cfg.gravity = cfg.centering_stiffness = cfg.contact_stiffness = 0.0
+    z, _ = mcg.random_state(lat, 0.02, 0.1, 0.0, 5)
+    agree(mcg.Solver(cfg, lat), mco.Model("mco", cfg, lattice=lat), z, lat.geometry.top0 + 0.01, 1.0 / young)
+
+
+@pytest.mark.parametrize("value", [np.nan, np.inf, -np.inf])
+def test_a_rotation_that_is_not_finite(mcg, mco, value):
+    cfg, lat, sol, _ = model(mcg, mco, "bcc", (2, 2, 2))
+    z, _ = mcg.random_state(lat, 0.02, 0.1, 0.0, 5)
+    free = np.flatnonzero(~lat.locked.astype(bool))
+    z[free[free % 6 >= 3][7]] = value
+    r = sol.objective(z, lat.geometry.top0 + 0.01)
+    assert r["energy"] == np.inf and not np.any(r["grad"])

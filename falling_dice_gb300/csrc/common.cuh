@@ -233,13 +233,14 @@ __device__ __forceinline__ d3 mrot_t(const m3& m, d3 v) {
 
 // ---- unit vectors in fixed point -----------------------------------------------------------
 // An FP64 instruction occupies a sub-partition for 64 cycles, a 32 x 32 -> 64-bit multiply-add for a
-// few: sums of products of numbers up to two in magnitude (rotation matrices, unit quaternions and
-// vectors) are cheaper on the integer pipe, which stands idle beside FP64, and no less exact.
+// few: sums of products of numbers of a few units (rotation matrices, unit quaternions and vectors,
+// rotation vectors; sums up to 32, numbers below 8) are cheaper on the integer pipe, which stands idle beside FP64, and no less exact.
 // A number is (h 2^30 + l) 2^-58, |l| <= 2^29: products of two upper halves, and of an upper and a
 // lower one, sum up in 64 bits each; the lower halves' products, below 2^-58, are left out.  A sum
 // of three products is off by at most 2^-56 = 1.4e-17 (FP64 additions near one: 1.1e-16 each).
 // "Units" are 64-bit integers of 2^-58.
 struct fx { int h, l; };
+struct u3 { long long x, y, z; };  // units
 struct fx3 { fx x, y, z; };
 struct fx4 { fx w, x, y, z; };
 constexpr long long kFxOne = 1LL << 58;
@@ -258,11 +259,14 @@ __device__ __forceinline__ unsigned long long fixed_magnitude(double v, int scal
     const unsigned long long m = (unsigned long long)(hi & 0xfffffu | 0x100000u) << 32 | unsigned(__double2loint(v));
     return shift_mantissa(m, int(hi >> 20 & 0x7ffu) - scale);
 }
-// v (|v| < 2) in units, rounded toward zero; some integer when v is larger or not finite.
+// v (|v| < 8) in units, rounded toward zero; some integer when v is larger or not finite.
 __device__ __forceinline__ long long fx_units(double v) {
     const long long n = (long long)fixed_magnitude(v, 1017);
     return __double2hiint(v) < 0 ? -n : n;
 }
+// |v| < 2^n, v finite.
+__device__ __forceinline__ bool below_power(double v, int n) { return (unsigned(__double2hiint(v)) & 0x7fffffffu) < unsigned(0x3ff + n) << 20; }
+__device__ __forceinline__ bool below_power(d3 v, int n) { return below_power(v.x, n) && below_power(v.y, n) && below_power(v.z, n); }
 // n 2^e2, rounded to nearest; 2^-900 < the magnitude < 2^900 or zero.
 __device__ __forceinline__ double fx_double(long long n, int e2 = -58) {
     const unsigned long long a = n < 0 ? 0ULL - (unsigned long long)n : (unsigned long long)n;
@@ -273,6 +277,8 @@ __device__ __forceinline__ double fx_double(long long n, int e2 = -58) {
     return __longlong_as_double((long long)(n < 0 ? b | 0x8000000000000000ULL : b));
 }
 __device__ __forceinline__ double fx_double(fx a) { return fx_double((long long)a.h * (1 << 30) + a.l); }
+__device__ __forceinline__ d3 fx_double(u3 n) { return d3{fx_double(n.x), fx_double(n.y), fx_double(n.z)}; }
+__device__ __forceinline__ u3 fx_units(d3 v) { return u3{fx_units(v.x), fx_units(v.y), fx_units(v.z)}; }
 __device__ __forceinline__ long long fx_hh(fx a, fx b) { return (long long)a.h * b.h; }
 __device__ __forceinline__ long long fx_hl(fx a, fx b) { return (long long)a.h * b.l + (long long)a.l * b.h; }
 __device__ __forceinline__ long long fx_sum(long long hh, long long hl) { return hh * 4 + ((hl + (1 << 27)) >> 28); }
@@ -282,6 +288,12 @@ __device__ __forceinline__ long long fx_dot(const fx3& a, const fx3& b) {
 __device__ __forceinline__ long long fx_dot(const fx4& a, const fx4& b) {
     return fx_sum(fx_hh(a.w, b.w) + fx_hh(a.x, b.x) + fx_hh(a.y, b.y) + fx_hh(a.z, b.z),
                   fx_hl(a.w, b.w) + fx_hl(a.x, b.x) + fx_hl(a.y, b.y) + fx_hl(a.z, b.z));
+}
+__device__ __forceinline__ fx3 fx_of(u3 n) { return fx3{fx_of(n.x), fx_of(n.y), fx_of(n.z)}; }
+__device__ __forceinline__ long long fx_mul(fx a, fx b) { return fx_sum(fx_hh(a, b), fx_hl(a, b)); }
+__device__ __forceinline__ u3 fx_cross(const fx3& a, const fx3& b) {
+    const auto minor = [](fx p, fx q, fx r, fx s) { return fx_sum(fx_hh(p, q) - fx_hh(r, s), fx_hl(p, q) - fx_hl(r, s)); };
+    return u3{minor(a.y, b.z, a.z, b.y), minor(a.z, b.x, a.x, b.z), minor(a.x, b.y, a.y, b.x)};
 }
 // 2 (a b + c d)
 __device__ __forceinline__ long long fx_twice(fx a, fx b, fx c, fx d) {
@@ -296,7 +308,6 @@ __device__ __forceinline__ fx fx_load(double v) { return fx{__double2hiint(v), _
 
 // A node's rotation: the unit quaternion and its matrix, in fixed point.  A quaternion that is not
 // finite has w.h = kFxInvalid.
-constexpr int kFxInvalid = 0x7fffffff;
 struct FxRot { fx3 r0, r1, r2; };
 // Rows 0-2 of the matrix and the quaternion as the node's four records; q normalized to rounding
 // already, here to 2^-56.
@@ -332,20 +343,22 @@ __device__ __forceinline__ m3 fx_matrix(const FxRot& r) {
     const auto row = [](const fx3& v) { return d3{fx_double(v.x), fx_double(v.y), fx_double(v.z)}; };
     return m3{row(r.r0), row(r.r1), row(r.r2)};
 }
-// M v for any vector: its components to one exponent, 58 bits below the largest.
-__device__ __forceinline__ d3 fx_rotate(const FxRot& r, d3 v) {
+// Any vector as fixed point times 2^(e - 1022): its components to one exponent, 58 bits below the
+// largest; false when that is tiny (zero, usually) or huge.
+__device__ __forceinline__ bool block_units(d3 v, u3& n, int& e) {
     const auto exponent = [](double a) { return int(unsigned(__double2hiint(a)) >> 20 & 0x7ffu); };
-    const int e = max(exponent(v.x), max(exponent(v.y), exponent(v.z)));
-    if (unsigned(e - 300) > 1400u) {  // tiny (zero, usually) or huge
-        const m3 m = fx_matrix(r);
-        return fmrot(m, v);
-    }
+    e = max(exponent(v.x), max(exponent(v.y), exponent(v.z)));
     // the largest component in [1/2, 1): its exponent 1022
     const auto units = [e](double a) {
-        const long long n = (long long)fixed_magnitude(a, e - 5);
-        return __double2hiint(a) < 0 ? -n : n;
+        const long long m = (long long)fixed_magnitude(a, e - 5);
+        return __double2hiint(a) < 0 ? -m : m;
     };
-    const fx3 f{fx_of(units(v.x)), fx_of(units(v.y)), fx_of(units(v.z))};
+    n = u3{units(v.x), units(v.y), units(v.z)};
+    return unsigned(e - 300) <= 1400u;
+}
+// M v, v in units times 2^(e - 1022).
+__device__ __forceinline__ d3 fx_rotate(const FxRot& r, u3 v, int e) {
+    const fx3 f = fx_of(v);
     return d3{fx_double(fx_dot(r.r0, f), e - 1022 - 58), fx_double(fx_dot(r.r1, f), e - 1022 - 58),
               fx_double(fx_dot(r.r2, f), e - 1022 - 58)};
 }

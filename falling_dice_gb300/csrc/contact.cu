@@ -856,14 +856,13 @@ __global__ void __launch_bounds__(kListThreads) k_contacts(DevTopo t, PhysParams
 long long pair_units(long long bins, int slots) { return bins * ((slots + kChunk - 1) / kChunk); }
 
 // One unit of pair work per warp or so (a bin at the default cell holds about 100 shapes, each in
-// about three bins), and no more blocks than the GPU holds at a time: all of it, or five of eight
+// about three bins), and no more blocks than the GPU holds at a time: all of it, or four of eight
 // per SM when it runs beside the FP64 beam kernel (shared).  That one lives on the FP64 pipe, this
-// on the integer pipe, but whichever fills the SMs' registers runs alone: an evaluation of
-// 44x44x22 cubic+BCC takes 391 us with all blocks, 376 with five an SM (and at most four of the
-// box kernel), 367 with four; compressed 32x32x16, where the contacts take longer than the beams,
-// 225, 217 and 221.
+// on the integer pipe, but whichever fills the SMs' registers runs alone.  A call of the largest
+// lattice (2.95 million beams): 1980 us with eight blocks an SM, 1934 with five, 1915 with four, 1927
+// with three; compressed 32x32x16, where the contacts take longer than the beams: 259, 247, 243, 260.
 int contact_pair_blocks(long long shapes, bool shared) {
-    const long long b = shapes / 128, most = shared ? 5 * 152 / (8 / kPairWarps) : 4 * 152;
+    const long long b = shapes / 128, most = shared ? 4 * 152 / (8 / kPairWarps) : 4 * 152;
     return int(b < 1 ? 1 : (b > most ? most : b));
 }
 

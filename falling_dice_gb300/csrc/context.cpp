@@ -1292,6 +1292,11 @@ void upload_instances(mcg_ctx* c, const std::vector<InstIn>& ins) {
         h2d(d, v.data(), v.size(), s);
         return static_cast<const double*>(d);
     };
+    auto up2 = [&](const std::vector<int2>& v) {
+        int2* d = M.get<int2>(v.size());
+        h2d(d, v.data(), v.size(), s);
+        return static_cast<const int2*>(d);
+    };
     int2* dab = M.get<int2>(size_t(B));
     h2d(dab, ab.data(), size_t(B), s);
     T.ab = dab;
@@ -1299,6 +1304,20 @@ void upload_instances(mcg_ctx* c, const std::vector<InstIn>& ins) {
     T.area = upd(areav);
     T.radius = upd(radv);
     T.e0x = upd(e0x); T.e0y = upd(e0y); T.e0z = upd(e0z);
+    {  // directors in units of 2^-58, (h 2^30 + l), where every component is below two
+        std::vector<int2> f[3];
+        const std::vector<double>* e0[3] = {&e0x, &e0y, &e0z};
+        for (int d = 0; d < 3; d++) {
+            f[d].resize(size_t(B));
+            for (int b = 0; b < B; b++) {
+                const bool ok = std::abs(e0x[size_t(b)]) < 2 && std::abs(e0y[size_t(b)]) < 2 && std::abs(e0z[size_t(b)]) < 2;
+                const long long n = ok ? (long long)std::ldexp((*e0[d])[size_t(b)], 58) : 0;
+                const long long h = (n + (1LL << 29)) >> 30;
+                f[d][size_t(b)] = make_int2(int(n - h * (1LL << 30)), ok ? int(h) : kFxInvalid);
+            }
+        }
+        T.e0fx = up2(f[0]); T.e0fy = up2(f[1]); T.e0fz = up2(f[2]);
+    }
     T.kb = upd(kb); T.kt = upd(kt); T.my = upd(my); T.ty = upd(ty); T.hb = upd(hb); T.ht = upd(ht);
     T.cs = upd(cs); T.aL = upd(aL); T.aLsy = upd(aLsy);
     T.invL0 = upd(invL0); T.inv_kbh = upd(inv_kbh); T.inv_kth = upd(inv_kth);
@@ -1340,11 +1359,6 @@ void upload_instances(mcg_ctx* c, const std::vector<InstIn>& ins) {
             int4* d = M.get<int4>(v.size());
             h2d(d, v.data(), v.size(), s);
             return static_cast<const int4*>(d);
-        };
-        auto up2 = [&](const std::vector<int2>& v) {
-            int2* d = M.get<int2>(v.size());
-            h2d(d, v.data(), v.size(), s);
-            return static_cast<const int2*>(d);
         };
         T.bblk = up4(bblk);
         T.eblk = up4(eblk);

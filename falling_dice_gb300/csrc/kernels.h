@@ -33,6 +33,7 @@ struct DevTopo {
     const int2* ab;
     const double *L0, *area, *radius;
     const double *e0x, *e0y, *e0z;
+    const int2 *e0fx, *e0fy, *e0fz;  // the same in fixed point (fx: l, h); e0fx.y = kFxInvalid: no direction
     const double *kb, *kt, *my, *ty, *hb, *ht, *cs, *aL, *aLsy;
     const double *invL0, *inv_kbh, *inv_kth;  // 1/L0, 1/max(1e-20, kb+hb), 1/max(1e-20, kt+ht)
     const double* mass;
@@ -77,6 +78,7 @@ constexpr int kBeamBlock = 128;
 // Nodes per evaluation node block (state and gather).
 constexpr int kEvalBlock = 128;
 // Solver blocks an instance's vectors are divided into at most: one per SM.
+constexpr int kFxInvalid = 0x7fffffff;  // the upper half of a fixed-point number that is none
 constexpr int kSolveBlocks = 152;
 
 #if defined(__CUDACC__)

@@ -274,19 +274,19 @@ __device__ __forceinline__ unsigned long long poly_step(unsigned long long acc, 
 }
 
 // Rotation vector of the relative rotation Q = Ra^* Rb (MC/include/core.hpp:52 quatLog of the
-// normalized Q with w >= 0) and its squared length.  With s = |v| of the unit Q, the vector is
+// normalized Q with w >= 0) in units.  With s = |v| of the unit Q, the vector is
 // 2 asin(s) / s v: a polynomial in s^2 up to s^2 = 0.1 (angles up to 36.9 degrees; Chebyshev
 // interpolation, error 2e-18), so that the usual beam takes no square root, division or
 // arctangent; larger angles take atan2 as the reference does.  Q is a product of two quaternions
-// of length one to 2^-56, in fixed point as the polynomial, which lies in [2, 2.04].
-__device__ __forceinline__ d3 relative_rotation(const fx4& a, const fx4& b, double& phi2) {
-    const long long x = fx_dot(a, fx4{b.x, -b.w, -b.z, b.y}), y = fx_dot(a, fx4{b.y, b.z, -b.w, -b.x}),
-                    z = fx_dot(a, fx4{b.z, -b.y, b.x, -b.w});
-    const d3 v{fx_double(x), fx_double(y), fx_double(z)};
-    const double s2 = fdot(v, v);
-    if (unsigned(__double2hiint(s2)) < 0x3fb99999u) {  // s2 < 0.1
+// of length one to 2^-56.
+constexpr long long fx_limit(double v) { return (long long)(v * 0x1p58); }
+__device__ __forceinline__ u3 relative_rotation(const fx4& a, const fx4& b) {
+    const u3 v{fx_dot(a, fx4{b.x, -b.w, -b.z, b.y}), fx_dot(a, fx4{b.y, b.z, -b.w, -b.x}), fx_dot(a, fx4{b.z, -b.y, b.x, -b.w})};
+    const fx3 vf = fx_of(v);
+    const long long s2 = fx_dot(vf, vf);
+    if (s2 < fx_limit(0.1)) {
         constexpr int B = 62, X = 67;
-        const unsigned long long u = fixed_magnitude(s2, 1075 - X);
+        const unsigned long long u = (unsigned long long)s2 << (X - 58);
         unsigned long long g = poly_units<B>(0x1.c42a558b8b15bp-6);
         g = poly_step<X>(g, u, poly_units<B>(0x1.11d08867c9adep-6));
         g = poly_step<X>(g, u, poly_units<B>(0x1.80fd1940cecf2p-6));
@@ -298,51 +298,58 @@ __device__ __forceinline__ d3 relative_rotation(const fx4& a, const fx4& b, doub
         g = poly_step<X>(g, u, poly_units<B>(0x1.33333333342e1p-3));
         g = poly_step<X>(g, u, poly_units<B>(0x1.5555555555550p-2));
         g = poly_step<X>(g, u, poly_units<B>(2.0));
-        double gd = __longlong_as_double((long long)((1023ULL << 52) + (g >> 11) + (g >> 10 & 1)));
-        phi2 = (gd * gd) * s2;
         // the sign of Q's real part, which is close to one
         const long long w = fx_hh(a.w, b.w) + fx_hh(a.x, b.x) + fx_hh(a.y, b.y) + fx_hh(a.z, b.z);
-        gd = __hiloint2double(__double2hiint(gd) | (w < 0 ? int(0x80000000u) : 0), __double2loint(gd));
-        return d3{v.x * gd, v.y * gd, v.z * gd};
+        const long long gu = (long long)(g >> (B - 58));
+        const fx gf = fx_of(w < 0 ? -gu : gu);
+        return u3{fx_mul(vf.x, gf), fx_mul(vf.y, gf), fx_mul(vf.z, gf)};
     }
-    q4 Q = qnorm(q4{fx_double(fx_dot(a, b)), v.x, v.y, v.z});
+    const d3 vd = fx_double(v);
+    q4 Q = qnorm(q4{fx_double(fx_dot(a, b)), vd.x, vd.y, vd.z});
     if (Q.w < 0) Q = q4{-Q.w, -Q.x, -Q.y, -Q.z};
     const double s = sqrt(Q.x * Q.x + Q.y * Q.y + Q.z * Q.z);
     d3 phi{2 * Q.x, 2 * Q.y, 2 * Q.z};
     if (!(s < 1e-12)) phi = d3{Q.x, Q.y, Q.z} * (2 * atan2(s, clampd(Q.w, -1, 1)) / s);
-    phi2 = len2(phi);
-    return phi;
+    return fx_units(phi);
 }
 
-// J_l^{-T}(phi) v (jl_inv_t) with the coefficient as a polynomial in phi2 = |phi|^2 up to 0.42
-// (every angle of relative_rotation's polynomial; Chebyshev interpolation, error 4e-17 against
-// 1/12, which enters multiplied by phi2), in [1/12, 0.084] and in fixed point.
-__device__ __forceinline__ d3 transport(d3 phi, double phi2, d3 v) {
-    if (unsigned(__double2hiint(phi2)) >= 0x3fdae000u) return jl_inv_t(phi, v);  // 0.4199
-    constexpr int B = 66, X = 65;
-    const unsigned long long u = fixed_magnitude(phi2, 1075 - X);
-    unsigned long long p = poly_units<B>(0x1.2bf59666dc69ep-31);
-    p = poly_step<X>(p, u, poly_units<B>(0x1.6684f73f8bd8ep-26));
-    p = poly_step<X>(p, u, poly_units<B>(0x1.bbd7b81461d47p-21));
-    p = poly_step<X>(p, u, poly_units<B>(0x1.1566aba745146p-15));
-    p = poly_step<X>(p, u, poly_units<B>(0x1.6c16c16c1de72p-10));
-    p = poly_step<X>(p, u, poly_units<B>(0x1.5555555555553p-4));
-    const double A = __longlong_as_double((long long)((1018ULL << 52) + (p >> 10) + (p >> 9 & 1)));
-    const d3 c1 = fcross(phi, v), c2 = fcross(phi, c1);
-    return d3{fma(A, c2.x, fma(.5, c1.x, v.x)), fma(A, c2.y, fma(.5, c1.y, v.y)), fma(A, c2.z, fma(.5, c1.z, v.z))};
+// R J_l^{-T}(phi) v (jl_inv_t): J^{-T} v = v + phi x v / 2 + A phi x (phi x v), the coefficient A a
+// polynomial in |phi|^2 up to 0.42 (every angle of relative_rotation's polynomial; Chebyshev
+// interpolation, error 4e-17 against 1/12, which enters multiplied by |phi|^2), in [1/12, 0.084].
+__device__ __forceinline__ d3 transport_rotated(const FxRot& r, u3 phi, d3 v) {
+    const fx3 pf = fx_of(phi);
+    const long long phi2 = fx_dot(pf, pf);
+    u3 n;
+    int e;
+    if (!block_units(v, n, e)) return fmrot(fx_matrix(r), jl_inv_t(fx_double(phi), v));
+    if (phi2 < fx_limit(0.4199)) {
+        constexpr int B = 66, X = 65;
+        const unsigned long long u = (unsigned long long)phi2 << (X - 58);
+        unsigned long long p = poly_units<B>(0x1.2bf59666dc69ep-31);
+        p = poly_step<X>(p, u, poly_units<B>(0x1.6684f73f8bd8ep-26));
+        p = poly_step<X>(p, u, poly_units<B>(0x1.bbd7b81461d47p-21));
+        p = poly_step<X>(p, u, poly_units<B>(0x1.1566aba745146p-15));
+        p = poly_step<X>(p, u, poly_units<B>(0x1.6c16c16c1de72p-10));
+        p = poly_step<X>(p, u, poly_units<B>(0x1.5555555555553p-4));
+        const fx A = fx_of((long long)(p >> (B - 58)));
+        const u3 c1 = fx_cross(pf, fx_of(n));
+        const fx3 c2 = fx_of(fx_cross(pf, fx_of(c1)));
+        n = u3{n.x + (c1.x >> 1) + fx_mul(A, c2.x), n.y + (c1.y >> 1) + fx_mul(A, c2.y), n.z + (c1.z >> 1) + fx_mul(A, c2.z)};
+    } else {
+        if (!block_units(jl_inv_t(fx_double(phi), v), n, e)) return d3{0, 0, 0};  // v is in range, so this is a zero
+    }
+    return fx_rotate(r, n, e);
 }
 
-// The beam's axis in the material frame: unit(Ra^T t), t of length one but for rounding.
-__device__ __forceinline__ d3 material_axis(const FxRot& m, const fx3& t) {
+// The beam's axis in the material frame in units: unit(Ra^T t), t of length one but for rounding.
+__device__ __forceinline__ u3 material_axis(const FxRot& m, const fx3& t) {
     const int d = int(fx_dot(t, t) - kFxOne);
-    const auto part = [&](fx a, fx b, fx c) { return fx_double(fx_renorm(fx_dot(fx3{a, b, c}, t), d)); };
-    return d3{part(m.r0.x, m.r1.x, m.r2.x), part(m.r0.y, m.r1.y, m.r2.y), part(m.r0.z, m.r1.z, m.r2.z)};
+    const auto part = [&](fx a, fx b, fx c) { return fx_renorm(fx_dot(fx3{a, b, c}, t), d); };
+    return u3{part(m.r0.x, m.r1.x, m.r2.x), part(m.r0.y, m.r1.y, m.r2.y), part(m.r0.z, m.r1.z, m.r2.z)};
 }
-// R e0 - t: a director's deviation from the chord, in fixed point (e0 of components below two;
-// others, which are no directions, in FP64).
-__device__ __forceinline__ d3 deviation(const FxRot& r, const fx3& e0, const long long (&t)[3], bool unit, d3 e0d, d3 td) {
-    if (unit) return d3{fx_double(fx_dot(r.r0, e0) - t[0]), fx_double(fx_dot(r.r1, e0) - t[1]), fx_double(fx_dot(r.r2, e0) - t[2])};
-    return fmrot(fx_matrix(r), e0d) - td;
+// R e0 - t: a director's deviation from the chord, in units.
+__device__ __forceinline__ u3 deviation(const FxRot& r, const fx3& e0, u3 t) {
+    return u3{fx_dot(r.r0, e0) - t.x, fx_dot(r.r1, e0) - t.y, fx_dot(r.r2, e0) - t.z};
 }
 
 // ---- beam kernel: MC/src/sim.cpp:139-141 ---------------------------------------------------
@@ -350,13 +357,13 @@ __device__ __forceinline__ d3 deviation(const FxRot& r, const fx3& e0, const lon
 // other pipes are idle), so the formulas are written for few FP64 instructions: energies summed
 // as twice their value, shear from the director-chord differences (2 t - da - db = -(ma + mb)),
 // square roots from the FP32 estimate, comparisons on bit patterns, and everything that is a sum of
-// products of unit vectors (directors, relative rotation, material axis, the moment's rotation) or
-// a polynomial of one's coordinates in fixed point on the integer pipe.  The error against 64 bits
-// is no larger for it (1.2e-16 against 1.3e-16 on the largest lattice, 5.4e-17 / 5.6e-17 on
-// 19x15x11): a fixed-point sum rounds once.
-// FP64 instructions per 32 beams: 391 at first, 265 with all of it in FP64, about 160 now; a call
-// at 2.95 million beams 2474 -> 2100 us, a batch of 762,000 beams 603 -> 509, 184,400 beams
-// compressed 274 -> 258.
+// products of unit vectors and rotation vectors (directors, relative rotation, material axis, trial
+// twist and bending, the moment's transport and rotation) or a polynomial of one's coordinates in
+// fixed point on the integer pipe.  The error against 64 bits is no larger for it (1.2e-16 against
+// 1.3e-16 on the largest lattice, 1.1e-16 / 1.2e-16 in a batch of 48): a fixed-point sum rounds once.
+// FP64 instructions per 32 beams: 391 at first, 265 with all of it in FP64, 130 now (3500 in all).
+// The kernel alone: 184,400 beams 159 -> 98 -> 66 us, 2.95 million 1372 -> 818 us (80 % of the FP64
+// pipe's rate); a call at 2.95 million beams 2474 -> 1914 us, a batch of 762,000 beams 603 -> 450.
 // Blocks of kBeamBlock = 128 beams: one warp on each of an SM's four FP64 units, so that a
 // lattice of a few hundred beams spreads over several SMs.
 // kMinBlocks: units of 256 threads per SM the register allocation must allow (an occupancy
@@ -404,37 +411,65 @@ __global__ void __launch_bounds__(kBeamBlock, 2 * kMinBlocks) k_beams(DevTopo t,
             if (ax.yielded) diss = t.aLsy[b] * ax.dg;
             // shear: the end directors against the chord (rotations by the nodes' matrices)
             const FxRot Ma = load_rotation(e.M + 4 * size_t(ab.x)), Mb = load_rotation(e.M + 4 * size_t(ab.y));
-            const d3 e0{t.e0x[b], t.e0y[b], t.e0z[b]};
-            const long long tu[3] = {fx_units(tt.x), fx_units(tt.y), fx_units(tt.z)};
-            const fx3 e0f{fx_of(fx_units(e0.x)), fx_of(fx_units(e0.y)), fx_of(fx_units(e0.z))};
-            const auto below_two = [](double v) { return (unsigned(__double2hiint(v)) & 0x7fffffffu) < 0x40000000u; };
-            const bool unit_e0 = below_two(e0.x) && below_two(e0.y) && below_two(e0.z);
-            const d3 ma = deviation(Ma, e0f, tu, unit_e0, e0, tt), mb = deviation(Mb, e0f, tu, unit_e0, e0, tt);
+            const int2 e0x = t.e0fx[b], e0y = t.e0fy[b], e0z = t.e0fz[b];
             const double cs = t.cs[b];
+            const u3 tu = fx_units(tt);
+            const fx3 tf = fx_of(tu);
+            d3 ma, mb, gm, Ga, Gb;  // deviations, their sum, and cs t x (R e0) = cs t x m
+            if (e0x.y != kFxInvalid) {
+                const fx3 e0f{fx{e0x.y, e0x.x}, fx{e0y.y, e0y.x}, fx{e0z.y, e0z.x}};
+                const u3 ua = deviation(Ma, e0f, tu), ub = deviation(Mb, e0f, tu);
+                ma = fx_double(ua);
+                mb = fx_double(ub);
+                gm = ma + mb;
+                Ga = fx_double(fx_cross(tf, fx_of(ua))) * cs;
+                Gb = fx_double(fx_cross(tf, fx_of(ub))) * cs;
+            } else {  // no direction
+                const d3 e0{t.e0x[b], t.e0y[b], t.e0z[b]};
+                ma = fmrot(fx_matrix(Ma), e0) - tt;
+                mb = fmrot(fx_matrix(Mb), e0) - tt;
+                gm = ma + mb;
+                Ga = fcross(tt, ma) * cs;
+                Gb = fcross(tt, mb) * cs;
+            }
             const double us2 = fma(mb.z, mb.z, fma(mb.y, mb.y, fma(mb.x, mb.x, fdot(ma, ma))));  // times cs
-            const d3 gm = ma + mb;
             const double kt_ = cs * invL;
             const double kf = fma(kt_, fdot(gm, tt), t.area[b] * ax.force);
             // F = t N + ((I - t t^T) g) / L with g = -cs (ma + mb)
             const d3 F{fma(tt.x, kf, -(kt_ * gm.x)), fma(tt.y, kf, -(kt_ * gm.y)), fma(tt.z, kf, -(kt_ * gm.z))};
-            const d3 tc = tt * cs;
-            d3 Ga = fcross(tc, ma);  // t x (R e0), as t x t = 0
-            d3 Gb = fcross(tc, mb);
             // bending and torsion from the relative rotation Q = Ra^* Rb
-            double phi2;
             const fx4 qa = load_fx4(e.M + 4 * size_t(ab.x) + 3), qb = load_fx4(e.M + 4 * size_t(ab.y) + 3);
-            const d3 phi = relative_rotation(qa, qb, phi2);
-            const d3 axis = material_axis(Ma, fx3{fx_of(tu[0]), fx_of(tu[1]), fx_of(tu[2])});
-            const double tw = fdot(phi, axis), ptw = fdot(rotp, axis);
-            const d3 bend = fmadd(axis, -tw, phi), pb = fmadd(axis, -ptw, rotp);
+            const u3 phi = relative_rotation(qa, qb), axis_u = material_axis(Ma, tf);
+            const d3 axis = fx_double(axis_u);
+            // trial elastic parts: the twist and the bending of d = phi - rotp
+            double dtw;
+            d3 dbend;
+            if (below_power(rotp, 2)) {
+                const u3 rp = fx_units(rotp), d{phi.x - rp.x, phi.y - rp.y, phi.z - rp.z};
+                const fx3 af = fx_of(axis_u);
+                const long long w = fx_dot(fx_of(d), af);
+                const fx wf = fx_of(w);
+                dtw = fx_double(w);
+                dbend = fx_double(u3{d.x - fx_mul(af.x, wf), d.y - fx_mul(af.y, wf), d.z - fx_mul(af.z, wf)});
+            } else {
+                const d3 d = fx_double(phi) - rotp;
+                dtw = fdot(d, axis);
+                dbend = fmadd(axis, -dtw, d);
+            }
+            double ptw = 0;  // the plastic parts enter the trial state only
+            d3 pb{0, 0, 0};
+            if (trials) {
+                ptw = fdot(rotp, axis);
+                pb = fmadd(axis, -ptw, rotp);
+            }
             const double kb = t.kb[b], kt = t.kt[b];
-            const Ret3 br = return3(bend - pb, pb, pl_alphaB, kb, t.my[b], t.hb[b], t.inv_kbh[b]);
-            const Ret1 tor = return1(tw - ptw, ptw, pl_alphaT, kt, t.ty[b], t.ht[b], t.inv_kth[b]);
+            const Ret3 br = return3(dbend, pb, pl_alphaB, kb, t.my[b], t.hb[b], t.inv_kbh[b]);
+            const Ret1 tor = return1(dtw, ptw, pl_alphaT, kt, t.ty[b], t.ht[b], t.inv_kth[b]);
             const d3 moment = fmadd(axis, tor.force, br.force);
             double dr = 0;
             if (br.yielded) dr = t.my[b] * br.dg;
             if (tor.yielded) dr = fma(t.ty[b], tor.dg, dr);
-            const d3 world = fx_rotate(Ma, transport(phi, phi2, moment));
+            const d3 world = transport_rotated(Ma, phi, moment);
             Ga = Ga - world;
             Gb = Gb + world;
             elastic2 = fma(cs, us2, uax2) + (br.energy2 + tor.energy2);
@@ -974,8 +1009,11 @@ void launch_from_records7(long long B, const double* aos, double* soa, cudaStrea
     if (B) (k_from_records7<<<record_grid(7 * B), kBlock, 0, s>>>(B, aos, soa), note_launches(1));
 }
 
-// Occupancy variants of the FP64 beam kernel (256-thread units per SM) and of the gather.
-constexpr int kBeamBlocks[] = {1, 2, 3};
+// Occupancy variants of the FP64 beam kernel (256-thread units per SM) and of the gather.  The
+// defaults first: four beam blocks of 128 threads an SM (two leave the integer pipe's latency
+// uncovered: largest lattice 2165 us a call against 1930; six spill and gain nothing), eight of the
+// gather's (64x64x32 480 us on the GPU against 499 with two).
+constexpr int kBeamBlocks[] = {2, 1, 3};
 constexpr int kGatherBlocks[] = {4, 2, 1};
 
 int shape_variants(ShapeKernel k) {

@@ -91,35 +91,6 @@ __device__ __forceinline__ double sat(double x) { return clampd(x, 0.0, 1.0); }
 
 struct Closest { double s, t; d3 pa, pb; };
 
-__device__ Closest seg_seg(d3 p1, d3 q1, d3 p2, d3 q2) {
-    const d3 d1 = q1 - p1, d2 = q2 - p2, r = p1 - p2;
-    const double a = dot(d1, d1), e = dot(d2, d2), f = dot(d2, r);
-    double s = 0, t = 0;
-    if (a <= 1e-20 && e <= 1e-20) return {0, 0, p1, p2};
-    if (a <= 1e-20) {
-        s = 0;
-        t = sat(f / e);
-    } else {
-        const double c = dot(d1, r);
-        if (e <= 1e-20) {
-            t = 0;
-            s = sat(-c / a);
-        } else {
-            const double b = dot(d1, d2), den = a * e - b * b;
-            s = fabs(den) > 1e-20 ? sat((b * f - c * e) / den) : 0;
-            t = (b * s + f) / e;
-            if (t < 0) {
-                t = 0;
-                s = sat(-c / a);
-            } else if (t > 1) {
-                t = 1;
-                s = sat((b - c) / a);
-            }
-        }
-    }
-    return {s, t, p1 + d1 * s, p2 + d2 * t};
-}
-
 struct ShapeRef {
     d3 a, b;
     double r;
@@ -150,19 +121,25 @@ __device__ __forceinline__ ShapeRef load_shape(const DevTopo& t, const double4_3
     return sh;
 }
 
-__device__ Closest shape_closest(const ShapeRef& a, const ShapeRef& b) {
-    if (a.capsule && b.capsule) return seg_seg(a.a, a.b, b.a, b.b);
-    if (a.capsule && !b.capsule) {
-        const d3 d = a.b - a.a;
-        const double s = sat(dot(b.a - a.a, d) / fmax(1e-30, len2(d)));
-        return {s, 0, a.a + d * s, b.a};
+// Closest points of two shapes (sim.cpp:9-22: sphere or segment against sphere or segment), a the
+// lower one, so never a segment against a sphere.  The lanes of a warp hold all three cases; they
+// take one path, each case's quotients and clamps selected, as the reference rounds them.  Two
+// divisions, and a third where a lane's t is clamped; comparisons on bit patterns.
+__device__ __forceinline__ Closest shape_closest(const ShapeRef& A, const ShapeRef& B) {
+    const d3 d1 = A.b - A.a, d2 = B.b - B.a, r = A.a - B.a;
+    const double a = dot(d1, d1), e = dot(d2, d2), f = dot(d2, r), c = dot(d1, r), b = dot(d1, d2);
+    // does the shape have a direction (a sphere against a segment has no threshold for the segment)
+    const bool ga = A.capsule && less_bits(1e-20, a), gb = A.capsule ? less_bits(1e-20, e) : B.capsule;
+    double s = 0, t = 0;
+    if (ga && gb) {
+        const double den = a * e - b * b;
+        if (less_bits(1e-20, fabs(den))) s = sat((b * f - c * e) / den);
     }
-    if (!a.capsule && b.capsule) {
-        const d3 d = b.b - b.a;
-        const double t = sat(dot(a.a - b.a, d) / fmax(1e-30, len2(d)));
-        return {0, t, a.a, b.a + d * t};
-    }
-    return {0, 0, a.a, b.a};
+    if (gb) t = (ga ? b * s + f : f) / (A.capsule ? e : fmax(1e-30, e));
+    const bool low = ga && (!gb || t < 0), high = ga && gb && t > 1;
+    if (low || high) s = sat((low ? -c : b - c) / a);
+    t = low ? 0 : high ? 1 : ga ? t : sat(t);
+    return {s, t, A.a + d1 * s, B.a + d2 * t};
 }
 
 // Membership of the node pair (u, v) in the connected set (sim.cpp:24-39 reads

@@ -566,20 +566,28 @@ struct mcg_ctx {
     // Evaluation whose totals are read back (hp.outs); repeats it with larger contact
     // buffers when a capacity was exceeded.
     // host_grad: the gradient is also copied there, in the same synchronisation.
-    const EvalOut* eval_read(const double* dz, bool trials, double* d_gout, double* host_grad = nullptr) {
-        eval(dz, trials, d_gout);
-        if (host_grad) d2h(host_grad, d_gout, 6 * size_t(N), stream);
-        read_outs();
+    // behind: what else the caller enqueues before it (launches first, then copies to the host).
+    template <typename F>
+    const EvalOut* eval_read(const double* dz, bool trials, double* d_gout, double* host_grad, F&& behind) {
+        const auto run = [&] {
+            eval(dz, trials, d_gout);
+            behind(host_grad);
+            read_outs();
+        };
+        run();
         for (int tries = 0; hp.outs[0].overflow && tries < 16; tries++) {
             if (!grow_contacts(hp.outs[0].overflow)) break;
-            eval(dz, trials, d_gout);
-            if (host_grad) d2h(host_grad, d_gout, 6 * size_t(N), stream);
-            read_outs();
+            run();
         }
         if (hp.outs[0].overflow) throw Fail(MCG_ERR_CAPACITY, "contact buffers could not be sized");
         last_contacts = hp.outs[0].pairs;
         contacts_stale = false;
         return hp.outs;
+    }
+    const EvalOut* eval_read(const double* dz, bool trials, double* d_gout, double* host_grad = nullptr) {
+        return eval_read(dz, trials, d_gout, host_grad, [&](double* g) {
+            if (g) d2h(g, d_gout, 6 * size_t(N), stream);
+        });
     }
     void read_outs() {
         sync();  // hp.outs is written by the finalize
@@ -1456,7 +1464,7 @@ void upload_instances(mcg_ctx* c, const std::vector<InstIn>& ins) {
     e.M = V.get<double4_32a>(4 * size_t(N));
     e.xf_lo = V.get<float4>(size_t(N));
     e.xf_hi = V.get<float4>(size_t(N));
-    e.slot = V.get<double>(12 * size_t(B));
+    e.slot = V.get<double>(15 * size_t(B));  // (TrialRecords)
     e.part_state = V.get<double>(9 * size_t(T.n_eblk));
     e.part_beam = V.get<double>(3 * size_t(std::max(T.n_bblk, 1)));
     e.err = V.get<unsigned>(1);
@@ -1733,27 +1741,19 @@ int mcg_objective(mcg_ctx* c, const double* z, double top, int trials, double* e
         h2d(c->d_zin, z, n, s);
         c->hp.tops[0] = top;
         c->set_active(std::vector<uint8_t>(1, 1));
-        const EvalOut o = c->eval_read(c->d_zin, trials != 0, c->d_grad, grad)[0];
+        const EvalOut o = c->eval_read(c->d_zin, trials != 0, c->d_grad, grad, [&](double* g) {
+            const TrialRecords r(c->ev, (long long)B);
+            const bool records = trials && (trial_next || trial_aux || trial_flags);
+            if (records) launch_trial_records((long long)B, c->ev, c->mixed, r, s);
+            if (g) d2h(g, c->d_grad, n, s);
+            if (!records) return;
+            if (trial_next) d2h(trial_next, r.next, 7 * B, s);
+            if (trial_aux) d2h(trial_aux, r.aux, 7 * B, s);
+            if (trial_flags) d2h(trial_flags, r.flags, 3 * B, s);
+        })[0];
         if (trials) c->have_final = false;
         if (energy) *energy = o.energy;
         fill_diag(diag, o);
-        if (trials) {  // in the ABI's layout, through the beams' slots (the gather has read them)
-            double* rec = c->ev.slot;
-            if (trial_next) {
-                if (c->mixed) launch_records7(c->B, c->ev.trial_nextf, rec, s);
-                else launch_records7(c->B, c->ev.trial_next, rec, s);
-                d2h(trial_next, rec, 7 * B, s);
-            }
-            if (trial_aux) {
-                if (c->mixed) launch_records7(c->B, c->ev.trial_auxf, rec, s);
-                else launch_records7(c->B, c->ev.trial_aux, rec, s);
-                d2h(trial_aux, rec, 7 * B, s);
-            }
-            if (trial_flags) {
-                launch_records3(c->B, c->ev.trial_flags, reinterpret_cast<uint8_t*>(rec), s);
-                d2h(trial_flags, reinterpret_cast<const uint8_t*>(rec), 3 * B, s);
-            }
-        }
         c->sync();
     });
 }

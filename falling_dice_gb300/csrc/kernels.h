@@ -212,7 +212,7 @@ struct EvalBufs {
     double4_32a* M;             // [4N] R in fixed point: matrix rows (x, y, z, pad), quaternion (fx)
     float4* xf_lo;              // [N] position rounded down to single precision
     float4* xf_hi;              // [N] position rounded up
-    double* slot;           // [12B] per beam: (-F, Ga), added to node a, then (+F, Gb), added to
+    double* slot;           // [15B] per beam 12: (-F, Ga), added to node a, then (+F, Gb), added to
                             //   node b: entry 2 beam + role, the incidence list's numbering
     double* part_state;     // [9 * n_eblk] sum, -min, max of x per block
     double* part_beam;      // [3 * nb_beams]
@@ -291,8 +291,14 @@ void launch_commit(const DevTopo& t, const uint8_t* mask, const EvalBufs& e, dou
 void launch_center(const DevTopo& t, const PhysParams& p, const BuildArgs& b, EvalBufs& e, cudaStream_t s);
 // Per-beam arrays (7 values, 3 flags; structure of arrays) to and from consecutive values per beam.
 void launch_records7(long long B, const double* soa, double* aos, cudaStream_t s);
-void launch_records7(long long B, const float* soa, double* aos, cudaStream_t s);
-void launch_records3(long long B, const uint8_t* soa, uint8_t* aos, cudaStream_t s);
+// Trial states as records, in the slots (which the gather has read by then).
+struct TrialRecords {
+    double *next, *aux;  // [7 B]
+    uint8_t* flags;      // [3 B]
+    TrialRecords(const EvalBufs& e, long long B)
+        : next(e.slot), aux(e.slot + 7 * B), flags(reinterpret_cast<uint8_t*>(e.slot + 14 * B)) {}
+};
+void launch_trial_records(long long B, const EvalBufs& e, bool mixed, const TrialRecords& r, cudaStream_t s);
 void launch_from_records7(long long B, const double* aos, double* soa, cudaStream_t s);
 void launch_gather_mixed(const DevTopo& t, const PhysParams& p, const ContactBufs* c, double* grad, EvalBufs& e,
                          cudaStream_t s, int variant = 0);

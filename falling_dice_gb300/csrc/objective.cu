@@ -943,6 +943,18 @@ __global__ void __launch_bounds__(kBlock) k_plastic_final(DevTopo t, const doubl
     }
 }
 
+// The trial states of an evaluation (next, aux and flags) in one launch.
+template <typename In>
+__global__ void __launch_bounds__(kBlock) k_trial_records(long long B, const In* __restrict__ next, const In* __restrict__ aux,
+                                                          const uint8_t* __restrict__ flags, double* __restrict__ rnext,
+                                                          double* __restrict__ raux, uint8_t* __restrict__ rflags) {
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < 7 * B; i += (long long)gridDim.x * blockDim.x) {
+        const long long b = i / 7, from = (i - 7 * b) * B + b;
+        rnext[i] = double(next[from]);
+        raux[i] = double(aux[from]);
+        if (i < 3 * B) rflags[i] = flags[(i - i / 3 * 3) * B + i / 3];
+    }
+}
 // ---- per-beam records in the ABI's layout ----------------------------------------------------
 // K values per beam: structure of arrays (device) <-> K consecutive values per beam (host), so
 // that a host array is one copy.  Thread i handles the i-th value of the written layout.
@@ -999,11 +1011,11 @@ static unsigned record_grid(long long n) { return grid_for(n < 16 * 152 * kBlock
 void launch_records7(long long B, const double* soa, double* aos, cudaStream_t s) {
     if (B) (k_to_records<7><<<record_grid(7 * B), kBlock, 0, s>>>(B, soa, aos), note_launches(1));
 }
-void launch_records7(long long B, const float* soa, double* aos, cudaStream_t s) {
-    if (B) (k_to_records<7><<<record_grid(7 * B), kBlock, 0, s>>>(B, soa, aos), note_launches(1));
-}
-void launch_records3(long long B, const uint8_t* soa, uint8_t* aos, cudaStream_t s) {
-    if (B) (k_to_records<3><<<record_grid(3 * B), kBlock, 0, s>>>(B, soa, aos), note_launches(1));
+void launch_trial_records(long long B, const EvalBufs& e, bool mixed, const TrialRecords& r, cudaStream_t s) {
+    if (!B) return;
+    if (mixed) k_trial_records<<<record_grid(7 * B), kBlock, 0, s>>>(B, e.trial_nextf, e.trial_auxf, e.trial_flags, r.next, r.aux, r.flags);
+    else k_trial_records<<<record_grid(7 * B), kBlock, 0, s>>>(B, e.trial_next, e.trial_aux, e.trial_flags, r.next, r.aux, r.flags);
+    note_launches(1);
 }
 void launch_from_records7(long long B, const double* aos, double* soa, cudaStream_t s) {
     if (B) (k_from_records7<<<record_grid(7 * B), kBlock, 0, s>>>(B, aos, soa), note_launches(1));

@@ -94,11 +94,15 @@ struct Pinned {
     uint32_t* u32 = nullptr;   // [8]
     Minimizer* mins = nullptr; // [I] the device-resident solver's minimizers, in and out
     MzStatus* mz = nullptr;    // its status word
-    void alloc(int I) {
+    double* grad = nullptr;    // [6 N] gradient and
+    double* trials = nullptr;  // [15 B] trial records of small contexts, else null
+    void alloc(int I, int N, int B) {
         release();
+        const size_t grad_doubles = N <= kHostGradNodes ? 6 * size_t(N) : 0;
+        const size_t trial_doubles = B <= kHostTrialBeams ? 15 * size_t(B) : 0;
         const size_t bytes = I * sizeof(EvalOut) + 3 * I * sizeof(SolveCtl) +
                              sizeof(double) * (I + I + 6 * I + 9 * (I + 1)) + 8 * 4 + I * sizeof(Minimizer) +
-                             sizeof(MzStatus) + 1024;
+                             sizeof(MzStatus) + 1024 + sizeof(double) * (grad_doubles + trial_doubles);
         ck(cudaMallocHost(&base, bytes), "cudaMallocHost");
         std::memset(base, 0, bytes);
         char* p = static_cast<char*>(base);
@@ -116,6 +120,8 @@ struct Pinned {
         u32 = reinterpret_cast<uint32_t*>(take(8 * sizeof(uint32_t)));
         mins = reinterpret_cast<Minimizer*>(take(I * sizeof(Minimizer)));
         mz = reinterpret_cast<MzStatus*>(take(sizeof(MzStatus)));
+        grad = grad_doubles ? reinterpret_cast<double*>(take(sizeof(double) * grad_doubles)) : nullptr;
+        trials = trial_doubles ? reinterpret_cast<double*>(take(sizeof(double) * trial_doubles)) : nullptr;
     }
     void release() {
         if (base) cudaFreeHost(base);
@@ -511,6 +517,7 @@ struct mcg_ctx {
         PhysParams p = phys;
         EvalBufs ev = this->ev;
         if (trials == 2) ev.tops_host = nullptr;  // the loop's platens are on the device
+        if (d_gout != d_grad) ev.grad_host = nullptr;  // the solver's own gradients
         p.broad_cell = broad_cell;
         p.inv_cell_f = float(1.0 / broad_cell);
         mark(0);
@@ -570,9 +577,11 @@ struct mcg_ctx {
     template <typename F>
     const EvalOut* eval_read(const double* dz, bool trials, double* d_gout, double* host_grad, F&& behind) {
         const auto run = [&] {
+            const bool written = host_grad && hp.grad && d_gout == d_grad;  // by the gather
             eval(dz, trials, d_gout);
-            behind(host_grad);
+            behind(written ? nullptr : host_grad);
             read_outs();
+            if (written) std::memcpy(host_grad, hp.grad, 6 * sizeof(double) * size_t(N));
         };
         run();
         for (int tries = 0; hp.outs[0].overflow && tries < 16; tries++) {
@@ -1289,7 +1298,7 @@ void upload_instances(mcg_ctx* c, const std::vector<InstIn>& ins) {
     c->jr = cf.joint_scale * cf.max_radius;
     c->rmax = rmax;
     c->H = std::max(cf.history, 0);
-    c->hp.alloc(I);
+    c->hp.alloc(I, c->N, c->B);
     cudaStream_t s = c->stream;
     DevArena& M = c->topo_mem;
     DevTopo T{};
@@ -1479,6 +1488,7 @@ void upload_instances(mcg_ctx* c, const std::vector<InstIn>& ins) {
     e.out = V.get<EvalOut>(size_t(I));
     e.tops_host = c->hp.tops;  // (the host changes them only after a sync)
     e.out_host = c->hp.outs;
+    e.grad_host = c->hp.grad;
     e.trial_next = V.get<double>(7 * size_t(B));
     e.trial_aux = V.get<double>(7 * size_t(B));
     e.trial_flags = V.get<uint8_t>(3 * size_t(B));
@@ -1650,7 +1660,7 @@ int mcg_create(const mcg_config* cfg, int device, mcg_ctx** out) {
     try {
         c->set_device();
         ck(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking), "cudaStreamCreate");
-        c->hp.alloc(1);
+        c->hp.alloc(1, 0, 0);
     } catch (const Fail&) {
         delete c;
         return MCG_ERR_CUDA;
@@ -1741,16 +1751,21 @@ int mcg_objective(mcg_ctx* c, const double* z, double top, int trials, double* e
         h2d(c->d_zin, z, n, s);
         c->hp.tops[0] = top;
         c->set_active(std::vector<uint8_t>(1, 1));
+        const bool records = trials && (trial_next || trial_aux || trial_flags);
+        const TrialRecords r(c->hp.trials ? c->hp.trials : c->ev.slot, (long long)B);
         const EvalOut o = c->eval_read(c->d_zin, trials != 0, c->d_grad, grad, [&](double* g) {
-            const TrialRecords r(c->ev, (long long)B);
-            const bool records = trials && (trial_next || trial_aux || trial_flags);
             if (records) launch_trial_records((long long)B, c->ev, c->mixed, r, s);
             if (g) d2h(g, c->d_grad, n, s);
-            if (!records) return;
+            if (!records || c->hp.trials) return;
             if (trial_next) d2h(trial_next, r.next, 7 * B, s);
             if (trial_aux) d2h(trial_aux, r.aux, 7 * B, s);
             if (trial_flags) d2h(trial_flags, r.flags, 3 * B, s);
         })[0];
+        if (records && c->hp.trials) {
+            if (trial_next) std::memcpy(trial_next, r.next, 7 * B * sizeof(double));
+            if (trial_aux) std::memcpy(trial_aux, r.aux, 7 * B * sizeof(double));
+            if (trial_flags) std::memcpy(trial_flags, r.flags, 3 * B);
+        }
         if (trials) c->have_final = false;
         if (energy) *energy = o.energy;
         fill_diag(diag, o);
@@ -1864,7 +1879,8 @@ int objective_with_fixed_contacts(mcg_ctx* c, ContactBufs& fixed, size_t zero_by
             throw Fail(MCG_ERR_CAPACITY, "this state needs more" + what +
                                              " than the fixed scratch of mcg_objective_noalloc holds");
         }
-        if (grad) d2h(grad, c->d_grad, n, s);
+        if (grad && c->hp.grad) std::memcpy(grad, c->hp.grad, n * sizeof(double));  // (the gather's)
+        else if (grad) d2h(grad, c->d_grad, n, s);
         c->sync();
         if (energy) *energy = o.energy;
         fill_diag(diag, o);

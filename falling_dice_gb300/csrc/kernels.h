@@ -204,6 +204,13 @@ struct BuildArgs {
 // sum of squared free gradient entries, max |free gradient entry|
 constexpr int kNodeParts = 8;
 constexpr int kFinPartDoubles = 32 * 11;  // per instance: 32 first-stage blocks x 11 totals
+// Nodes up to which the gather writes the gradient to page-locked memory as well: a copy to the
+// caller's array takes 8 us whatever its size, the stores and the host's copying 3 us at 1024 nodes
+// (cubic+BCC 855 nodes 63 -> 58 us a call, 1241 65 -> 61, 1729 69 -> 66, 3059 even, 4941 73 -> 80).
+constexpr int kHostGradNodes = 2048;
+// Beams up to which trial states go the same way (three copies of 8 us): 6x6x6 cubic, 882 beams,
+// 102 -> 75 us a call with both.
+constexpr int kHostTrialBeams = 2048;
 constexpr int kFinSingle = 768;  // block partials one block sums: six per thread
 
 struct EvalBufs {
@@ -229,6 +236,7 @@ struct EvalBufs {
     // evaluation needs no copies for them (null: the device's only)
     const double* tops_host;
     EvalOut* out_host;
+    double* grad_host;      // [6 N] the gradient too, for lattices of up to kHostGradNodes
     double* trial_next;     // [7B] SoA
     double* trial_aux;      // [7B] SoA
     uint8_t* trial_flags;   // [3B] SoA
@@ -291,12 +299,12 @@ void launch_commit(const DevTopo& t, const uint8_t* mask, const EvalBufs& e, dou
 void launch_center(const DevTopo& t, const PhysParams& p, const BuildArgs& b, EvalBufs& e, cudaStream_t s);
 // Per-beam arrays (7 values, 3 flags; structure of arrays) to and from consecutive values per beam.
 void launch_records7(long long B, const double* soa, double* aos, cudaStream_t s);
-// Trial states as records, in the slots (which the gather has read by then).
+// Trial states as records in 15 B doubles: the slots (which the gather has read by then) or
+// page-locked memory.
 struct TrialRecords {
     double *next, *aux;  // [7 B]
     uint8_t* flags;      // [3 B]
-    TrialRecords(const EvalBufs& e, long long B)
-        : next(e.slot), aux(e.slot + 7 * B), flags(reinterpret_cast<uint8_t*>(e.slot + 14 * B)) {}
+    TrialRecords(double* mem, long long B) : next(mem), aux(mem + 7 * B), flags(reinterpret_cast<uint8_t*>(mem + 14 * B)) {}
 };
 void launch_trial_records(long long B, const EvalBufs& e, bool mixed, const TrialRecords& r, cudaStream_t s);
 void launch_from_records7(long long B, const double* aos, double* soa, cudaStream_t s);

@@ -705,8 +705,11 @@ __device__ __forceinline__ void write_out(const DevTopo& t, const PhysParams& p,
     }
     __syncthreads();
     if (sm.nonfinite) {  // non-finite energy: the instance's whole gradient is zero
-        double* g = grad + 6 * size_t(t.eblk[t.erange[inst].x].x);
-        for (long long k = threadIdx.x; k < 6LL * t.inst_n[inst]; k += blockDim.x) g[k] = 0;
+        const size_t o = 6 * size_t(t.eblk[t.erange[inst].x].x);
+        for (long long k = threadIdx.x; k < 6LL * t.inst_n[inst]; k += blockDim.x) {
+            grad[o + k] = 0;
+            if (e.grad_host) e.grad_host[o + k] = 0;
+        }
     }
 }
 // Gather blocks of an instance: two per evaluation block.
@@ -800,6 +803,7 @@ __global__ void __launch_bounds__(kEvalBlock, 2 * kMinBlocks) k_gather(DevTopo t
         const uint8_t* li = t.locked + 6 * size_t(i) + 3 * half;
         double gv[3] = {g.x, g.y, g.z};
         double* out = grad + 6 * size_t(i) + 3 * half;
+        double* host = e.grad_host ? e.grad_host + 6 * size_t(i) + 3 * half : nullptr;
 #pragma unroll
         for (int k = 0; k < 3; k++) {
             if (li[k]) gv[k] = 0.0;
@@ -810,6 +814,7 @@ __global__ void __launch_bounds__(kEvalBlock, 2 * kMinBlocks) k_gather(DevTopo t
             const unsigned long long b = (unsigned long long)__double_as_longlong(gv[k]) & 0x7fffffffffffffffULL;
             if (b <= 0x7ff0000000000000ULL && b > gbits) gbits = b;
             out[k] = gv[k];
+            if (host) host[k] = gv[k];
         }
     }
     // the rotations' share of the residual goes to the translations' thread of the node

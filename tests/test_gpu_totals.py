@@ -21,8 +21,8 @@ def specimen(mcg, cells, kind, precision=abi.MCG_FP64):
     return cfg, lat, z, pl, lat.geometry.top0 - 0.002
 
 
-# nodes: 8, 63, 64, 66, 126, 128, 130
-SMALL = [(1, 1, 1), (2, 2, 6), (3, 3, 3), (1, 2, 10), (2, 5, 6), (1, 7, 7), (1, 4, 12)]
+# nodes: 8, 63, 64, 66, 126, 128, 130; 2048 and 2057 (the gradient's two ways to the host)
+SMALL = [(1, 1, 1), (2, 2, 6), (3, 3, 3), (1, 2, 10), (2, 5, 6), (1, 7, 7), (1, 4, 12), (15, 15, 7), (10, 10, 16)]
 # block partials of the cubic+BCC lattices: 717 and 841
 CASES = [(c, abi.MCG_LATTICE_CUBIC) for c in SMALL] + [((n, n, n), abi.MCG_LATTICE_CUBIC_BCC) for n in (18, 19)]
 
@@ -39,6 +39,31 @@ def test_totals_and_gradient_against_the_restatement(mcg, mco, cells, kind):
     for k in ("elastic", "plastic", "contact", "reaction"):
         assert abs(r["diag"][k] - o["diag"][k]) <= 1e-10 * max(abs(o["diag"][k]), 1e-12), k
     assert r["diag"]["max_pen"] == o["diag"]["max_pen"] and r["diag"]["contacts"] == int(o["diag"]["contacts"])
+
+
+# beams: 2048 and 2049 (the trial states' two ways to the host); cubic (a, b, c)
+@pytest.mark.parametrize("cells", [(7, 7, 11), (2, 9, 26)])
+@pytest.mark.parametrize("precision", [abi.MCG_FP64, abi.MCG_MIXED])
+def test_what_the_host_receives_is_what_the_device_holds(mcg, precision, cells):
+    cfg, lat, z, pl, top = specimen(mcg, cells, abi.MCG_LATTICE_CUBIC, precision)
+    sol = mcg.Solver(cfg, lat)
+    sol.set_state(plastic=pl)
+    a = sol.objective(z, top, True)
+    b = sol.objective(z, top)
+    c = sol.read_result()
+    assert a["energy"] == b["energy"] == c["energy"]
+    assert np.array_equal(a["grad"], b["grad"]) and np.array_equal(a["grad"], c["grad"])
+    for k in ("trial_next", "trial_aux"):
+        assert np.all(np.isfinite(a[k])) and np.any(a[k])
+    # a state that is not finite: no gradient anywhere; then the same state again
+    bad = z.copy()
+    bad[np.flatnonzero(~lat.locked.astype(bool))[5]] = np.nan
+    r = sol.objective(bad, top, True)
+    assert r["energy"] == np.inf and not np.any(r["grad"]) and not np.any(sol.read_result()["grad"])
+    d = sol.objective(z, top, True)
+    assert np.array_equal(a["grad"], d["grad"])
+    for k in ("trial_next", "trial_aux", "trial_flags"):
+        assert np.array_equal(a[k], d[k])
 
 
 @pytest.mark.parametrize("precision,sizes", [(abi.MCG_FP64, (19, 1, 18, 3)), (abi.MCG_MIXED, (22, 1, 21, 3))])

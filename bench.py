@@ -42,13 +42,13 @@ BEAM_BYTES = 128    # per beam, FP64: a, b (2 x 4 B) + 15 reals
 NODE_BYTES = 166    # per node, FP64: z[6] + baseX[3] + baseR[4] + mass + grad[6], locked[6]
 # DRAM bytes (read + write, ncu dram__bytes_read.sum + dram__bytes_write.sum) of one launch,
 # captured with ncu on GB300 and scaled to the workload:
-#   k_beams (FP64), 32x32x16 cubic+BCC: 40.35 MB for 184,400 beams, scaled by beam count;
+#   k_beams (FP64), 32x32x16 cubic+BCC: 41.74 MB for 184,400 beams, scaled by beam count;
 #   k_beams_mixed, 64x64x32 cubic+BCC: 212.75 MB for 1,458,336 beams, scaled by beam count;
-#   k_bin_pairs, 64x64x32 cubic+BCC at the tuned shapes (4.5 mm cell, 1216 blocks): 107.87 MB
-#   where the algorithmic bytes below come to 123.55 MB, scaled by the algorithmic bytes.
-BEAM_TRAFFIC_PER_BEAM = 40.348160e6 / 184400
+#   k_bin_pairs, 64x64x32 cubic+BCC at the tuned shapes (9 mm cell, 1216 blocks): 83.96 MB
+#   where the algorithmic bytes below come to 106.69 MB, scaled by the algorithmic bytes.
+BEAM_TRAFFIC_PER_BEAM = 41.743360e6 / 184400
 BEAM_TRAFFIC_PER_BEAM_MIXED = 212.748800e6 / 1458336
-PAIR_TRAFFIC_PER_ALGORITHMIC_BYTE = 107.870720e6 / 123.545196e6
+PAIR_TRAFFIC_PER_ALGORITHMIC_BYTE = 83.956736e6 / 106.691384e6
 BEAM_BYTES_MIXED = 68    # per beam, mixed: a, b (2 x 4 B) + 15 reals as FP32
 NODE_BYTES_MIXED = 98    # per node, mixed: baseX (3 x 8 B) + 17 reals as FP32 + locked[6]
 # Pair enumeration (k_bin_pairs), algorithmic bytes: every cell entry's shape id (4 B), each
@@ -59,8 +59,9 @@ PAIR_ENTRY_BYTES, PAIR_SHAPE_BYTES, PAIR_BIN_BYTES, PAIR_CAND_BYTES = 4, 24, 12,
 # warp instructions per second against the issue peak of one warp instruction per clock on
 # each of the 4 x 152 SM sub-partitions.  Instructions per launch from ncu
 # (smsp__inst_executed.sum, profiles/k_bin_pairs_bcc64.md) at the benchmark state of the
-# 64x64x32 specimen with the 4.5 mm cell and 1216 pair blocks; other shapes have no figure.
-PAIR_WARP_INSTRUCTIONS = {("bcc64", 0.0045, 1216): 304137669}
+# 64x64x32 specimen with 1216 pair blocks and the 9 mm cell the tuner picks or a 4.5 mm one; other
+# shapes have no figure.
+PAIR_WARP_INSTRUCTIONS = {("bcc64", 0.009, 1216): 176060155, ("bcc64", 0.0045, 1216): 266694941}
 SM_SUBPARTITIONS = 4 * 152
 
 

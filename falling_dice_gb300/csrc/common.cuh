@@ -18,7 +18,6 @@ constexpr double kPiD = 3.1415926535897932384626433832795;
 struct d3 { double x, y, z; };
 struct q4 { double w, x, y, z; };
 
-__device__ __forceinline__ d3 mk3(double x, double y, double z) { return d3{x, y, z}; }
 __device__ __forceinline__ d3 operator+(d3 a, d3 b) { return {a.x + b.x, a.y + b.y, a.z + b.z}; }
 __device__ __forceinline__ d3 operator-(d3 a, d3 b) { return {a.x - b.x, a.y - b.y, a.z - b.z}; }
 __device__ __forceinline__ d3 operator-(d3 a) { return {-a.x, -a.y, -a.z}; }
@@ -53,7 +52,6 @@ __device__ __forceinline__ d3 qrot(q4 q, d3 v) {
     const d3 t = cross(u, v) * 2.0;
     return (v + t * q.w) + cross(u, t);
 }
-__device__ __forceinline__ d3 qrot_inv(q4 q, d3 v) { return qrot(conj(q), v); }
 
 // Unit quaternion of the rotation vector v (MC/include/core.hpp:51 quatExp, :42 quatAxisAngle).
 __device__ __forceinline__ q4 exp_map(d3 v) {
@@ -63,15 +61,6 @@ __device__ __forceinline__ q4 exp_map(d3 v) {
     double s, c;
     sincos(.5 * a, &s, &c);
     return qnorm(q4{c, axis.x * s, axis.y * s, axis.z * s});
-}
-// Rotation vector of a unit quaternion (MC/include/core.hpp:52 quatLog).
-__device__ __forceinline__ d3 log_map(q4 q) {
-    q = qnorm(q);
-    if (q.w < 0) q = q4{-q.w, -q.x, -q.y, -q.z};
-    const double s = sqrt(q.x * q.x + q.y * q.y + q.z * q.z);
-    if (s < 1e-12) return {2 * q.x, 2 * q.y, 2 * q.z};
-    const double a = 2 * atan2(s, clampd(q.w, -1, 1));
-    return d3{q.x, q.y, q.z} * (a / s);
 }
 // J_l^{-T}(p) v, the SO(3) left-Jacobian inverse transpose applied to v
 // (MC/include/core.hpp:53): v + p x v / 2 + A p x (p x v) with
@@ -127,11 +116,6 @@ __device__ __forceinline__ double xor_sign(double v, double s) {
 // v / 2 for a normal v above the smallest exponent.
 __device__ __forceinline__ double half_of(double v) {
     return __hiloint2double(__double2hiint(v) - 0x00100000, __double2loint(v));
-}
-// 2 v for a normal v below the largest exponent, or zero.
-__device__ __forceinline__ double twice(double v) {
-    const int hi = __double2hiint(v);
-    return __hiloint2double((hi & 0x7ff00000) ? hi + 0x00100000 : hi, __double2loint(v));
 }
 // |v - 1| < 2^-20: a squared norm whose square root is 1 + (v - 1) / 2 to FP64 precision when
 // it differs from one by rounding only.
@@ -222,14 +206,6 @@ __device__ __forceinline__ q4 qnorm_near(q4 q) {
 
 struct m3 { d3 r0, r1, r2; };
 __device__ __forceinline__ d3 fmrot(const m3& m, d3 v) { return d3{fdot(m.r0, v), fdot(m.r1, v), fdot(m.r2, v)}; }
-__device__ __forceinline__ d3 fmrot_t(const m3& m, d3 v) {
-    return fmadd(m.r2, v.z, fmadd(m.r1, v.y, m.r0 * v.x));
-}
-__device__ __forceinline__ d3 mrot(const m3& m, d3 v) { return d3{dot(m.r0, v), dot(m.r1, v), dot(m.r2, v)}; }
-__device__ __forceinline__ d3 mrot_t(const m3& m, d3 v) {
-    return d3{m.r0.x * v.x + m.r1.x * v.y + m.r2.x * v.z, m.r0.y * v.x + m.r1.y * v.y + m.r2.y * v.z,
-              m.r0.z * v.x + m.r1.z * v.y + m.r2.z * v.z};
-}
 
 // ---- unit vectors in fixed point -----------------------------------------------------------
 // An FP64 instruction occupies a sub-partition for 64 cycles, a 32 x 32 -> 64-bit multiply-add for a
@@ -407,16 +383,6 @@ __device__ __forceinline__ double warp_max(double v) {
     }
     return v;
 }
-__device__ __forceinline__ float warp_max_f(float v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_down_sync(0xffffffffu, v, o));
-    return v;
-}
-__device__ __forceinline__ long long warp_sum_ll(long long v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    return v;
-}
 
 // Sums NV values per thread over the block; thread 0 receives the totals.  `smem` needs
 // NV * (blockDim.x / 32) doubles.  blockDim.x must be a multiple of 32.
@@ -464,69 +430,8 @@ __device__ __forceinline__ void block_sum_t(double (&v)[NV], double* smem) {
     __syncthreads();
 }
 
-// The same for maxima (fmax skips NaN); `smem` needs NV * blockDim.x doubles.
-template <int NV>
-__device__ __forceinline__ void block_max_t(double (&v)[NV], double* smem) {
-    const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
-#pragma unroll
-    for (int k = 0; k < NV; k++) smem[k * nt + tid] = v[k];
-    __syncthreads();
-    for (int k = warp; k < NV; k += nw) {
-        const double* a = smem + k * nt;
-        double m = a[lane];
-        for (int j = lane + 32; j < nt; j += 32) m = fmax(m, a[j]);
-        m = warp_max(m);
-        __syncwarp();
-        if (lane == 0) smem[k * nt] = m;
-    }
-    __syncthreads();
-    if (tid == 0)
-#pragma unroll
-        for (int k = 0; k < NV; k++) v[k] = smem[k * nt];
-    __syncthreads();
-}
 
-// NV maxima over the block into thread 0, one barrier pair for all of them; smem holds
-// NV * (blockDim.x / 32) doubles.
-template <int NV>
-__device__ __forceinline__ void block_max_n(double (&v)[NV], double* smem) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-#pragma unroll
-    for (int k = 0; k < NV; k++) v[k] = warp_max(v[k]);
-    if (lane == 0)
-#pragma unroll
-        for (int k = 0; k < NV; k++) smem[k * nw + warp] = v[k];
-    __syncthreads();
-    if (threadIdx.x == 0)
-#pragma unroll
-        for (int k = 0; k < NV; k++) {
-            double m = smem[k * nw];
-            for (int w = 1; w < nw; w++) m = fmax(m, smem[k * nw + w]);
-            v[k] = m;
-        }
-    __syncthreads();
-}
 
-// The same in single precision (fmaxf skips NaN like fmax); smem holds NV * (blockDim.x / 32)
-// floats.
-template <int NV>
-__device__ __forceinline__ void block_max_nf(float (&v)[NV], float* smem) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-#pragma unroll
-    for (int k = 0; k < NV; k++) v[k] = warp_max_f(v[k]);
-    if (lane == 0)
-#pragma unroll
-        for (int k = 0; k < NV; k++) smem[k * nw + warp] = v[k];
-    __syncthreads();
-    if (threadIdx.x == 0)
-#pragma unroll
-        for (int k = 0; k < NV; k++) {
-            float m = smem[k * nw];
-            for (int w = 1; w < nw; w++) m = fmaxf(m, smem[k * nw + w]);
-            v[k] = m;
-        }
-    __syncthreads();
-}
 
 __device__ __forceinline__ double block_max(double v, double* smem) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;

@@ -724,65 +724,78 @@ __device__ __forceinline__ bool add_fixed(long long* __restrict__ sum, double v,
     return ok;
 }
 
-// One contact (or pair too close to tell from FP32 bounds; valid: the lane has one): the exact FP64
-// test, a place in the contact list, the forces of the penalty (sim.cpp:163-164, addShapeGradient
-// sim.cpp:23: capsule ends split the force (1 - u, u)) onto the nodes' fixed-point sums, the
-// contact's energy, count and penetration onto the first node of its lower shape.  All lanes of a
-// warp call it.
-__device__ __forceinline__ void add_contact(const DevTopo& t, const PhysParams& p, const double4_32a* __restrict__ x,
-                                            const ContactBufs& c, bool valid, uint2 q) {
+// A pair too close to tell from FP32 bounds (valid: the lane has one): the exact FP64 test and a place
+// in the contact list.  All lanes of a warp call it.
+__device__ __forceinline__ PairHit find_contact(const DevTopo& t, const PhysParams& p, const double4_32a* __restrict__ x,
+                                                const ContactBufs& c, bool valid, uint2 q) {
     const int lane = threadIdx.x & 31;
-    const uint32_t sa = q.x, sb = q.y;
     PairHit h;
     h.hit = false;
-    if (valid) h = narrow_phase(t, p, x, sa, sb);
+    if (valid) h = narrow_phase(t, p, x, q.x, q.y);
     const unsigned m = __ballot_sync(0xffffffffu, h.hit);
-    if (!m) return;  // warp-uniform
+    if (!m) return h;  // warp-uniform
     uint32_t base = 0;
     if (lane == 0) {
         base = atomicAdd(c.counts + kContacts, uint32_t(__popc(m)));
         if ((long long)base + __popc(m) > c.contact_cap) atomicOr(c.flags, uint32_t(kOverContacts));
     }
     const long long at = (long long)__shfl_sync(0xffffffffu, base, 0) + __popc(m & ((1u << lane) - 1u));
-    if (!h.hit) return;
-    if (at < c.contact_cap) {
-        c.c_a[at] = sa;
-        c.c_b[at] = sb;
+    if (h.hit && at < c.contact_cap) {
+        c.c_a[at] = q.x;
+        c.c_b[at] = q.y;
     }
-    const double mag = p.contact_k * h.pen;
-    bool ok = true;
-#pragma unroll
-    for (int side = 0; side < 2; side++) {
-        const uint32_t shape = side ? sb : sa;
-        const bool capsule = shape >= uint32_t(t.N);
-        const int2 nd = shape_nodes(t, shape);
-        const d3 v = h.n * (side ? -mag : mag);
-        const double u = side ? h.t : h.s;
-#pragma unroll
-        for (int end = 0; end < 2; end++) {
-            if (end && !capsule) break;
-            const int node = end ? nd.y : nd.x;
-            const d3 f = !capsule ? v : end ? v * u : v * (1 - u);
-            NodeContact& r = c.n_sum[node];
-            ok &= add_fixed(r.f[0], f.x, c.force_e0);
-            ok &= add_fixed(r.f[1], f.y, c.force_e0);
-            ok &= add_fixed(r.f[2], f.z, c.force_e0);
-            if (side == 0 && end == 0) {
-                ok &= add_fixed(r.energy, .5 * p.contact_k * h.pen * h.pen, c.energy_e0);
-                atomicMax(&r.pen, (unsigned long long)__double_as_longlong(h.pen));  // pen > 0
-                atomicAdd(c.n_count + node, 1ULL | (1ULL << 32));
-            } else {
-                atomicAdd(c.n_count + node, 1ULL);
-            }
-        }
-    }
-    // not finite: the evaluation's energy must be, too (the gather reads the flag)
-    if (!ok) atomicOr(c.n_count + shape_nodes(t, sa).x, kContactNotFinite);
+    return h;
 }
 
+// One end of one side of a contact: the force of the penalty (sim.cpp:163-164, addShapeGradient
+// sim.cpp:23: capsule ends split the force (1 - u, u); v the side's force, u its end's share) onto the
+// node's fixed-point sums; with the first end of the lower shape go the contact's energy, count and
+// penetration.
+__device__ __forceinline__ void add_end(const DevTopo& t, const PhysParams& p, const ContactBufs& c, uint2 q, d3 v, double u,
+                                        double pen, int side, int end) {
+    const uint32_t shape = side ? q.y : q.x;
+    const bool capsule = shape >= uint32_t(t.N);
+    if (end && !capsule) return;
+    const int2 nd = shape_nodes(t, shape);
+    const int node = end ? nd.y : nd.x;
+    const d3 f = !capsule ? v : end ? v * u : v * (1 - u);
+    NodeContact& r = c.n_sum[node];
+    bool ok = add_fixed(r.f[0], f.x, c.force_e0);
+    ok &= add_fixed(r.f[1], f.y, c.force_e0);
+    ok &= add_fixed(r.f[2], f.z, c.force_e0);
+    if (side == 0 && end == 0) {
+        ok &= add_fixed(r.energy, .5 * p.contact_k * pen * pen, c.energy_e0);
+        atomicMax(&r.pen, (unsigned long long)__double_as_longlong(pen));  // pen > 0
+        atomicAdd(c.n_count + node, 1ULL | (1ULL << 32));
+    } else {
+        atomicAdd(c.n_count + node, 1ULL);
+    }
+    // not finite: the evaluation's energy must be, too (the gather reads the flag)
+    if (!ok) atomicOr(c.n_count + node, kContactNotFinite);
+}
+
+// The whole contact by one lane.
+__device__ __forceinline__ void add_contact(const DevTopo& t, const PhysParams& p, const double4_32a* __restrict__ x,
+                                            const ContactBufs& c, bool valid, uint2 q) {
+    const PairHit h = find_contact(t, p, x, c, valid, q);
+    if (!h.hit) return;
+    const double mag = p.contact_k * h.pen;
+#pragma unroll
+    for (int side = 0; side < 2; side++)
+#pragma unroll
+        for (int end = 0; end < 2; end++) add_end(t, p, c, q, h.n * (side ? -mag : mag), side ? h.t : h.s, h.pen, side, end);
+}
+
+struct FoundContact {
+    d3 force;  // on the lower shape
+    double s, t, pen;
+    uint2 q;
+};
 // The filtered list's pairs in contact and their forces, every evaluation.  A warp queues the pairs
 // of the evaluated instances that are not certainly apart and takes them to FP64 as soon as it has
-// one for every lane, a block's warps the rest together at the end: the closest points run with
+// one for every lane, a block's warps the rest together at the end, where the ends of the contacts
+// found go over all threads (the sums of one contact by one lane are a chain of 13 additions: the
+// compressed 32x32x16 lattice, mixed, 118 -> 112 us a call): the closest points run with
 // full warps, and a short list spreads over the SMs.  The launch, the list between them and the
 // second kernel's start bounded the two kernels this was (narrow phase, then contacts).  A whole
 // evaluation of the 2x4x2 specimen 47.3 -> 43.0 us on the GPU, of the compressed 32x32x16 lattice in
@@ -792,6 +805,8 @@ __global__ void __launch_bounds__(kListThreads) k_contacts(DevTopo t, PhysParams
                                                            const float4* __restrict__ xf, ContactBufs c) {
     __shared__ uint2 queue[kListWarps][64];
     __shared__ uint32_t left[kListWarps];
+    __shared__ FoundContact found[kListThreads];
+    __shared__ int hits;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const long long thread = (long long)blockIdx.x * kListThreads + threadIdx.x, threads = (long long)gridDim.x * kListThreads;
     const uint32_t total = uint32_t(min((long long)c.counts[kKept], c.cand_cap));
@@ -817,14 +832,29 @@ __global__ void __launch_bounds__(kListThreads) k_contacts(DevTopo t, PhysParams
         }
     }
     if (lane == 0) left[warp] = n;
+    if (threadIdx.x == 0) hits = 0;
     __syncthreads();
-    // the rest of all warps' queues, dense
+    // the rest of all warps' queues, dense; the ends of its contacts over all threads
     int from = threadIdx.x, w = 0, all = 0;
     for (int k = 0; k < kListWarps; k++) all += left[k];
-    if (int(threadIdx.x & ~31u) >= all) return;
-    const bool mine = from < all;
-    while (mine && from >= int(left[w])) from -= left[w++];
-    add_contact(t, p, x, c, mine, mine ? queue[w][from] : make_uint2(0, 0));
+    if (all == 0) return;  // block-uniform
+    if (int(threadIdx.x & ~31u) < all) {
+        const bool mine = from < all;
+        while (mine && from >= int(left[w])) from -= left[w++];
+        const uint2 q = mine ? queue[w][from] : make_uint2(0, 0);
+        const PairHit h = find_contact(t, p, x, c, mine, q);
+        if (h.hit) {
+            const int k = atomicAdd(&hits, 1);
+            const double mag = p.contact_k * h.pen;
+            found[k] = FoundContact{h.n * mag, h.s, h.t, h.pen, q};
+        }
+    }
+    __syncthreads();
+    for (int k = threadIdx.x; k < 4 * hits; k += kListThreads) {
+        const FoundContact& f = found[k >> 2];
+        const int side = k >> 1 & 1;
+        add_end(t, p, c, f.q, side ? -f.force : f.force, side ? f.t : f.s, f.pen, side, k & 1);
+    }
 }
 
 }  // namespace

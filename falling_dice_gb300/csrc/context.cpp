@@ -260,12 +260,32 @@ struct mcg_ctx {
     unsigned long long graph_flags() const { return mixed ? 0 : cudaGraphInstantiateFlagUseNodePriority; }
     cudaStream_t fork = nullptr;
     cudaEvent_t fork_ev[3] = {};
+    // Where the caller wants a large gradient on the host, its graph gathers in kGradPieces launches and
+    // each piece is copied, on a stream of its own, while the next is gathered and the totals are
+    // summed: 270,497 nodes 659 -> 638 us a call, 544,644 1908 -> 1856; 149,940 no gain (a copy takes 8 us
+    // to begin).
+    static constexpr int kGradPieces = 3, kGradPiecesFrom = 200000;  // nodes
+    cudaStream_t copies = nullptr;
+    cudaEvent_t piece_ev[kGradPieces] = {};
+    int piece_block[kGradPieces + 1] = {}, piece_node[kGradPieces + 1] = {};
+    bool in_pieces(double* d_gout, const double* host_grad) const {
+        return host_grad && d_gout == d_grad && N >= kGradPiecesFrom && use_graphs && !timing;
+    }
+    void copy_pieces(double* host_grad) {
+        for (int k = 0; k < kGradPieces; k++) {
+            ck(cudaStreamWaitEvent(copies, piece_ev[k], 0), "cudaStreamWaitEvent");
+            const size_t from = 6 * size_t(piece_node[k]);
+            d2h(host_grad + from, d_grad + from, 6 * size_t(piece_node[k + 1]) - from, copies);
+        }
+    }
     void make_fork() {
         if (fork) return;
         int least = 0, greatest = 0;
         ck(cudaDeviceGetStreamPriorityRange(&least, &greatest), "cudaDeviceGetStreamPriorityRange");
         for (cudaEvent_t& e : fork_ev) ck(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
         ck(cudaStreamCreateWithPriority(&fork, cudaStreamNonBlocking, greatest), "cudaStreamCreate");
+        for (cudaEvent_t& e : piece_ev) ck(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
+        ck(cudaStreamCreateWithFlags(&copies, cudaStreamNonBlocking), "cudaStreamCreate");
     }
     bool device_loop = true;
     std::string loop_error;
@@ -304,6 +324,9 @@ struct mcg_ctx {
             if (e) cudaEventDestroy(e);
         if (fork) cudaStreamDestroy(fork);
         for (cudaEvent_t e : fork_ev)
+            if (e) cudaEventDestroy(e);
+        if (copies) cudaStreamDestroy(copies);
+        for (cudaEvent_t e : piece_ev)
             if (e) cudaEventDestroy(e);
         if (stream) cudaStreamDestroy(stream);
     }
@@ -426,7 +449,7 @@ struct mcg_ctx {
     struct EvalGraph {
         const double* dz;
         double* d_gout;
-        bool trials;
+        bool trials, pieces;
         cudaGraphExec_t exec;
         long long kernels;  // kernel launches a replay performs
     };
@@ -480,27 +503,28 @@ struct mcg_ctx {
 
     // One evaluation of every instance at device z; grad written to d_gout; totals in
     // ev.out[0..I).  Enqueues only: no host synchronisation.
-    void eval(const double* dz, bool trials, double* d_gout) {
+    // pieces: the gather in pieces, each marked by its event.
+    void eval(const double* dz, bool trials, double* d_gout, bool pieces = false) {
         if (!use_graphs || timing) {
             eval_launches(dz, trials, d_gout, false);
         } else {
             const EvalGraph* found = nullptr;
             for (const EvalGraph& g : graphs)
-                if (g.dz == dz && g.d_gout == d_gout && g.trials == trials) found = &g;
+                if (g.dz == dz && g.d_gout == d_gout && g.trials == trials && g.pieces == pieces) found = &g;
             if (!found) {
                 cudaGraph_t graph = nullptr;
                 cudaGraphExec_t exec = nullptr;
                 const long long before = g_launch_count.load();
                 make_fork();
                 ck(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal), "cudaStreamBeginCapture");
-                eval_launches(dz, trials, d_gout, true);
+                eval_launches(dz, trials, d_gout, true, pieces);
                 ck(cudaStreamEndCapture(stream, &graph), "cudaStreamEndCapture");
                 const long long kernels = g_launch_count.load() - before;
                 g_launch_count -= kernels;  // counted when the graph runs
                 const cudaError_t e = cudaGraphInstantiate(&exec, graph, graph_flags());
                 cudaGraphDestroy(graph);
                 ck(e, "cudaGraphInstantiate");
-                graphs.push_back(EvalGraph{dz, d_gout, trials, exec, kernels});
+                graphs.push_back(EvalGraph{dz, d_gout, trials, pieces, exec, kernels});
                 found = &graphs.back();
             }
             ck(cudaGraphLaunch(found->exec, stream), "cudaGraphLaunch");
@@ -513,7 +537,7 @@ struct mcg_ctx {
 
     // trials: 0 none, 1 every instance, 2 the instances of d_trial (device-resident loop)
     // forked: captured launches, the contact pipeline on its own branch beside the beam kernel
-    void eval_launches(const double* dz, int trials, double* d_gout, bool forked) {
+    void eval_launches(const double* dz, int trials, double* d_gout, bool forked, bool pieces = false) {
         PhysParams p = phys;
         EvalBufs ev = this->ev;
         if (trials == 2) ev.tops_host = nullptr;  // the loop's platens are on the device
@@ -558,8 +582,12 @@ struct mcg_ctx {
             mark(4);
         }
         mark(5);
-        if (mixed) launch_gather_mixed(topo, p, cptr, d_gout, ev, stream, gather_variant);
-        else launch_gather(topo, p, cptr, d_gout, ev, stream, gather_variant);
+        for (int k = 0; k < (pieces ? kGradPieces : 1); k++) {
+            const int first = pieces ? piece_block[k] : 0, n = pieces ? piece_block[k + 1] - first : -1;
+            if (mixed) launch_gather_mixed(topo, p, cptr, d_gout, ev, stream, gather_variant, first, n);
+            else launch_gather(topo, p, cptr, d_gout, ev, stream, gather_variant, first, n);
+            if (pieces) ck(cudaEventRecordWithFlags(piece_ev[k], stream, cudaEventRecordExternal), "cudaEventRecord");
+        }
         mark(6);
         launch_finalize(topo, p, d_gout, ev, stream);
         mark(7);
@@ -578,10 +606,17 @@ struct mcg_ctx {
     const EvalOut* eval_read(const double* dz, bool trials, double* d_gout, double* host_grad, F&& behind) {
         const auto run = [&] {
             const bool written = host_grad && hp.grad && d_gout == d_grad;  // by the gather
-            eval(dz, trials, d_gout);
-            behind(written ? nullptr : host_grad);
+            const bool pieces = in_pieces(d_gout, host_grad);
+            eval(dz, trials, d_gout, pieces);
+            if (pieces) copy_pieces(host_grad);
+            behind(written || pieces ? nullptr : host_grad);
             read_outs();
             if (written) std::memcpy(host_grad, hp.grad, 6 * sizeof(double) * size_t(N));
+            if (!pieces) return;
+            ck(cudaStreamSynchronize(copies), "stream sync");
+            for (int i = 0; i < I; i++)  // cleared on the device after its piece was copied
+                if (hp.outs[i].nonfinite)
+                    std::fill_n(host_grad + 6 * size_t(inst[size_t(i)].node0), 6 * size_t(inst[size_t(i)].N), 0.0);
         };
         run();
         for (int tries = 0; hp.outs[0].overflow && tries < 16; tries++) {
@@ -1365,6 +1400,11 @@ void upload_instances(mcg_ctx* c, const std::vector<InstIn>& ins) {
     T.n_bblk = int(bblk.size());
     T.bdim = bdim;
     T.n_eblk = int(eblk.size());
+    for (int k = 0; k <= mcg_ctx::kGradPieces; k++) {
+        const int b = int((long long)T.n_eblk * k / mcg_ctx::kGradPieces);
+        c->piece_block[k] = 2 * b;
+        c->piece_node[k] = b < T.n_eblk ? eblk[size_t(b)].x : N;
+    }
     T.large_totals = false;
     for (int k = 0; k < I; k++) {
         const int2 b = brange[size_t(k)], e = erange[size_t(k)];

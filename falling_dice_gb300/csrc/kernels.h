@@ -289,8 +289,9 @@ void prepare_beams_mixed(int device);
 int beams_mixed_blocks(int variant);
 void launch_beams(const DevTopo& t, const Material& m, const double* plastic, int trials,
                   EvalBufs& e, cudaStream_t s, int variant = 0);
+// Gather blocks [first, first + blocks) of the 2 n_eblk (all by default).
 void launch_gather(const DevTopo& t, const PhysParams& p, const ContactBufs* c, double* grad,
-                   EvalBufs& e, cudaStream_t s, int variant = 0);
+                   EvalBufs& e, cudaStream_t s, int variant = 0, int first = 0, int blocks = -1);
 void launch_finalize(const DevTopo& t, const PhysParams& p, double* grad, EvalBufs& e, cudaStream_t s);
 // base state <- current state, plastic <- trial (plastic == nullptr skips it) for the
 // instances with mask[i] != 0 (mask == nullptr: all)
@@ -309,7 +310,7 @@ struct TrialRecords {
 void launch_trial_records(long long B, const EvalBufs& e, bool mixed, const TrialRecords& r, cudaStream_t s);
 void launch_from_records7(long long B, const double* aos, double* soa, cudaStream_t s);
 void launch_gather_mixed(const DevTopo& t, const PhysParams& p, const ContactBufs* c, double* grad, EvalBufs& e,
-                         cudaStream_t s, int variant = 0);
+                         cudaStream_t s, int variant = 0, int first = 0, int blocks = -1);
 
 // ---- mixed-precision form (objective_mixed.cu) ------------------------------------------
 void launch_state_mixed(const DevTopo& t, const PhysParams& p, const double* z, const double* base_x,

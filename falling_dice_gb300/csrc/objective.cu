@@ -729,12 +729,13 @@ __device__ __forceinline__ int2 gather_range(const DevTopo& t, int inst) {
 template <bool F32, int kMinBlocks>
 __global__ void __launch_bounds__(kEvalBlock, 2 * kMinBlocks) k_gather(DevTopo t, PhysParams p, ContactBufs c,
                                                                        int use_contacts, EvalBufs e,
-                                                                       double* __restrict__ grad) {
+                                                                       double* __restrict__ grad, int first) {
     constexpr int kNodes = kGatherNodes;
     static_assert(kNodes == 64, "two warps of translations, two of rotations");
     __shared__ GatherParts sm;
     __shared__ TotalParts ts;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {  // of the whole evaluation, whether instance 0 is active or not
+    const int block = int(blockIdx.x) + first;
+    if (block == 0 && threadIdx.x == 0) {  // of the whole evaluation, whether instance 0 is active or not
         for (EvalOut* out : {e.out, e.out_host}) {
             if (!out) continue;
             out->overflow = use_contacts ? int(c.flags[0] & ~uint32_t(kNonFinite)) : 0;
@@ -743,10 +744,10 @@ __global__ void __launch_bounds__(kEvalBlock, 2 * kMinBlocks) k_gather(DevTopo t
         }
         if (use_contacts) c.flags[0] = c.flags[1] = 0;  // for the next evaluation
     }
-    const int4 blk = t.eblk[blockIdx.x >> 1];
+    const int4 blk = t.eblk[block >> 1];
     const int inst = blk.z;
     if (!t.active[inst]) return;  // block-uniform
-    const int half = threadIdx.x / kNodes, at = kNodes * (blockIdx.x & 1) + threadIdx.x % kNodes;
+    const int half = threadIdx.x / kNodes, at = kNodes * (block & 1) + threadIdx.x % kNodes;
     const int i = blk.x + at;
     double egrav = 0, g2 = 0, eplat = 0, reac = 0, econt = 0, pen_max = 0;
     int count = 0;
@@ -845,7 +846,7 @@ __global__ void __launch_bounds__(kEvalBlock, 2 * kMinBlocks) k_gather(DevTopo t
     }
     __syncthreads();
     const int tid = threadIdx.x;
-    double* q = e.part_node + kNodeParts * size_t(blockIdx.x);
+    double* q = e.part_node + kNodeParts * size_t(block);
     if (tid < 5) q[tid == 0 ? 0 : tid == 1 ? 6 : tid == 2 ? 1 : tid == 3 ? 2 : 5] = sm.sum[tid][0] + sm.sum[tid][1];
     else if (tid < 7) q[tid == 5 ? 3 : 7] = __longlong_as_double(max(sm.m[tid - 5][0], sm.m[tid - 5][1]));
     else if (tid == 7) q[4] = double(sm.count[0] + sm.count[1]);
@@ -1062,26 +1063,26 @@ void launch_beams(const DevTopo& t, const Material& m, const double* plastic, in
 
 template <bool F32>
 void gather_variant(const DevTopo& t, const PhysParams& p, const ContactBufs* c, double* grad, EvalBufs& e,
-                    cudaStream_t s, int variant) {
+                    cudaStream_t s, int variant, int first, int blocks) {
     ContactBufs cc{};
     if (c) cc = *c;
-    const int uc = c ? 1 : 0;
+    const int uc = c ? 1 : 0, n = blocks < 0 ? 2 * t.n_eblk : blocks;
     switch (variant) {
-        case 1: k_gather<F32, kGatherBlocks[1]><<<2 * t.n_eblk, kEvalBlock, 0, s>>>(t, p, cc, uc, e, grad); break;
-        case 2: k_gather<F32, kGatherBlocks[2]><<<2 * t.n_eblk, kEvalBlock, 0, s>>>(t, p, cc, uc, e, grad); break;
-        default: k_gather<F32, kGatherBlocks[0]><<<2 * t.n_eblk, kEvalBlock, 0, s>>>(t, p, cc, uc, e, grad); break;
+        case 1: k_gather<F32, kGatherBlocks[1]><<<n, kEvalBlock, 0, s>>>(t, p, cc, uc, e, grad, first); break;
+        case 2: k_gather<F32, kGatherBlocks[2]><<<n, kEvalBlock, 0, s>>>(t, p, cc, uc, e, grad, first); break;
+        default: k_gather<F32, kGatherBlocks[0]><<<n, kEvalBlock, 0, s>>>(t, p, cc, uc, e, grad, first); break;
     }
     note_launches(1);
 }
 
 void launch_gather(const DevTopo& t, const PhysParams& p, const ContactBufs* c, double* grad, EvalBufs& e,
-                   cudaStream_t s, int variant) {
-    gather_variant<false>(t, p, c, grad, e, s, variant);
+                   cudaStream_t s, int variant, int first, int blocks) {
+    gather_variant<false>(t, p, c, grad, e, s, variant, first, blocks);
 }
 
 void launch_gather_mixed(const DevTopo& t, const PhysParams& p, const ContactBufs* c, double* grad, EvalBufs& e,
-                         cudaStream_t s, int variant) {
-    gather_variant<true>(t, p, c, grad, e, s, variant);
+                         cudaStream_t s, int variant, int first, int blocks) {
+    gather_variant<true>(t, p, c, grad, e, s, variant, first, blocks);
 }
 
 void launch_finalize(const DevTopo& t, const PhysParams& p, double* grad, EvalBufs& e, cudaStream_t s) {

@@ -80,3 +80,34 @@ def test_a_batch_across_the_paths_is_bitwise_the_single_lattices(mcg, precision,
         assert got["energy"][k] == ref["energy"], k
         assert np.array_equal(got["grad"][6 * off[k]:6 * off[k + 1]], ref["grad"]), k
         assert got["diag"][k] == ref["diag"], k
+
+
+@pytest.mark.parametrize("precision", [abi.MCG_FP64, abi.MCG_MIXED])
+def test_a_gradient_copied_in_pieces_is_the_device_s(mcg, precision):
+    """205,379 nodes (copied while it is gathered), alone and behind a small lattice in a batch whose
+    large or small lattice is not finite: every call returns its own state's gradient."""
+    cfg, lat, z, pl, top = specimen(mcg, (58, 58, 58), abi.MCG_LATTICE_CUBIC, precision)
+    sol = mcg.Solver(cfg, lat)
+    sol.set_state(plastic=pl)
+    want = {}
+    for s in (1.0, 0.5):
+        sol.upload_z(s * z)
+        sol.objective_resident(top)
+        want[s] = sol.read_result()
+    for k in range(12):
+        s = 1.0 if k % 3 else 0.5
+        r = sol.objective(s * z, top)
+        assert r["energy"] == want[s]["energy"] and np.array_equal(r["grad"], want[s]["grad"]), k
+    _, small, zs, ps, _ = specimen(mcg, (3, 3, 3), abi.MCG_LATTICE_CUBIC, precision)
+    batch = mcg.BatchSolver(cfg, [small, lat])
+    batch.set_state(plastic=np.concatenate([ps, pl]))
+    tops = [small.geometry.top0, top]
+    for bad in (None, 0, 1):
+        zz = [zs.copy(), z.copy()]
+        if bad is not None:
+            one = (small, lat)[bad]
+            zz[bad][np.flatnonzero(~one.locked.astype(bool))[4]] = np.nan
+        r = batch.objective(np.concatenate(zz), tops)
+        g = np.split(r["grad"], [6 * small.n_nodes])
+        assert np.array_equal(g[1], want[1.0]["grad"]) if bad != 1 else not np.any(g[1])
+        assert np.any(g[0]) == (bad != 0)

@@ -277,6 +277,7 @@ struct mcg_ctx {
             const size_t from = 6 * size_t(piece_node[k]);
             d2h(host_grad + from, d_grad + from, 6 * size_t(piece_node[k + 1]) - from, copies);
         }
+        ck(cudaStreamSynchronize(copies), "stream sync");  // whatever the evaluation turns out to be
     }
     void make_fork() {
         if (fork) return;
@@ -612,9 +613,7 @@ struct mcg_ctx {
             behind(written || pieces ? nullptr : host_grad);
             read_outs();
             if (written) std::memcpy(host_grad, hp.grad, 6 * sizeof(double) * size_t(N));
-            if (!pieces) return;
-            ck(cudaStreamSynchronize(copies), "stream sync");
-            for (int i = 0; i < I; i++)  // cleared on the device after its piece was copied
+            for (int i = 0; pieces && i < I; i++)  // cleared on the device after its piece was copied
                 if (hp.outs[i].nonfinite)
                     std::fill_n(host_grad + 6 * size_t(inst[size_t(i)].node0), 6 * size_t(inst[size_t(i)].N), 0.0);
         };

@@ -6,14 +6,14 @@
 // reference's set bit for bit (positions are bit-identical, see k_state).
 //
 // Broad phase.  Every shape (N joint spheres, then B beam capsules, as sim.cpp:148-150)
-// enters every grid cell its margin-inflated AABB touches (sim.cpp:153-157; same cell size
-// and the same floor() cell coordinates).  Cells are numbered by the Morton code of their
+// enters every grid cell its margin-inflated AABB touches (sim.cpp:153-157; the same floor() cell
+// coordinates, the cell twice the reference's by default).  Cells are numbered by the Morton code of their
 // coordinates relative to the grid origin (row-major when the Morton range does not fit),
 // and each entry goes straight into a slot of its bin (bins of fixed capacity, the slot
-// handed out by the bin's atomic counter).  The pair pass gives each occupied bin to one
-// warp, which enumerates the bin's pairs in the order the atomics handed out: the candidate
-// list's order can vary from run to run, its content cannot, and nothing computed from it
-// depends on the order (pair sets are reported sorted).  A pair is examined only in the cell that is the
+// handed out by the bin's atomic counter).  The pair pass gives 128 shapes of a bin at
+// a time to a warp, which meets them with those before them in the order the atomics handed out:
+// the candidate list's order can vary from run to run, its content cannot, and nothing computed
+// from it depends on the order (pair sets are reported sorted).  A pair is examined only in the cell that is the
 // minimum corner of the intersection of the two shapes' cell ranges: every pair that
 // shares a cell is examined exactly once -- the reference's `tested` set without a set.
 // A conservative FP32 AABB test and the local-shape exclusion (sim.cpp:24-39) run before

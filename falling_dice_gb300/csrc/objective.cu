@@ -441,10 +441,11 @@ __global__ void __launch_bounds__(kBeamBlock, 2 * kMinBlocks) k_beams(DevTopo t,
             const fx4 qa = load_fx4(e.M + 4 * size_t(ab.x) + 3), qb = load_fx4(e.M + 4 * size_t(ab.y) + 3);
             const u3 phi = relative_rotation(qa, qb), axis_u = material_axis(Ma, tf);
             const d3 axis = fx_double(axis_u);
-            // trial elastic parts: the twist and the bending of d = phi - rotp
+            // trial elastic parts: the twist and the bending of d = phi - rotp (in fixed point below eight:
+            // |phi| <= pi, components of rotp below two, so |d| < pi + 2 sqrt(3) = 6.6)
             double dtw;
             d3 dbend;
-            if (below_power(rotp, 2)) {
+            if (below_power(rotp, 1)) {
                 const u3 rp = fx_units(rotp), d{phi.x - rp.x, phi.y - rp.y, phi.z - rp.z};
                 const fx3 af = fx_of(axis_u);
                 const long long w = fx_dot(fx_of(d), af);

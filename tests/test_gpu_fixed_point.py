@@ -4,6 +4,7 @@ orientation, directors that are no unit vectors, moments beyond the exponents a 
 rotations that are not finite; against the CPU restatement at the bars of the reference fixtures."""
 import numpy as np
 import pytest
+from scipy.spatial.transform import Rotation
 
 from conftest import rel_err
 from test_gpu_fp64_paths import model
@@ -60,3 +61,29 @@ def test_a_rotation_that_is_not_finite(mcg, mco, value):
     z[free[free % 6 >= 3][7]] = value
     r = sol.objective(z, lat.geometry.top0 + 0.01)
     assert r["energy"] == np.inf and not np.any(r["grad"])
+
+
+@pytest.mark.parametrize("size", [0.5, 1.9, 2.1, 3.5, 3.9, 4.1, 12.0, 1e6])
+def test_plastic_rotations_of_any_size(mcg, mco, size):
+    """Plastic rotations along the beams' axes, their largest component of the given size, against
+    relative rotations of either direction: the trial twist is larger than any of their components (up to
+    sqrt(3) sizes, and pi more or less)."""
+    cfg, lat, _, _ = model(mcg, mco, "bcc", (5, 4, 3))
+    cfg.material.yield_ = 1e12 * cfg.material.young  # elastic at any of these strains
+    sol, orc = mcg.Solver(cfg, lat), mco.Model("mco", cfg, lattice=lat)
+    z, _ = mcg.random_state(lat, 0.02, 1.5, 0.0, 5)
+    zn = z.reshape(-1, 6)
+    x = lat.x0.reshape(-1, 3) + cfg.translation_scale * zn[:, :3]
+    R = Rotation.from_rotvec(zn[:, 3:])
+    chord = x[lat.beam_b] - x[lat.beam_a]
+    axis = R[lat.beam_a].inv().apply(chord / np.linalg.norm(chord, axis=1, keepdims=True))
+    sign = np.where(np.arange(lat.n_beams) % 2, 1.0, -1.0)[:, None]
+    pl = np.zeros((lat.n_beams, 7))
+    pl[:, 2:5] = size * sign * axis / np.max(np.abs(axis), axis=1, keepdims=True)
+    twist = np.sum(((R[lat.beam_a].inv() * R[lat.beam_b]).as_rotvec() - pl[:, 2:5]) * axis, axis=1)
+    assert np.max(np.abs(twist)) > 1.5 * size
+    for m in (sol, orc):
+        m.set_state(plastic=pl.ravel())
+    agree(sol, orc, z, lat.geometry.top0 + 0.01)
+    a, b = (m.objective(z, lat.geometry.top0 + 0.01, True)["trial_aux"].reshape(-1, 7)[:, 2:5] for m in (sol, orc))
+    assert rel_err(a, b) <= TOL

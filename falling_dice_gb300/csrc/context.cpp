@@ -190,9 +190,9 @@ struct mcg_ctx {
     PhysParams phys{};
     EvalBufs ev{};
     ContactBufs cb{};
-    long long last_contacts = 0;
     // The last evaluation was mcg_objective_noalloc's: its contacts lived in the shared
-    // fixed scratch, so the pair and statistics queries have nothing current to report.
+    // fixed scratch, so the pair and statistics queries have nothing current to report, until an
+    // evaluation in the context's own buffers (eval, the device loop) is enqueued.
     bool contacts_stale = false;
     // Device address of mcg_objective_noalloc's fixed scratch on this context's device,
     // looked up by that entry point's first call on this context (noalloc.cu).
@@ -531,6 +531,7 @@ struct mcg_ctx {
             ck(cudaGraphLaunch(found->exec, stream), "cudaGraphLaunch");
             note_launches(int(found->kernels));
         }
+        contacts_stale = false;
         last_z = dz;
         last_trials = trials;
         last_grad = d_gout;
@@ -623,8 +624,6 @@ struct mcg_ctx {
             run();
         }
         if (hp.outs[0].overflow) throw Fail(MCG_ERR_CAPACITY, "contact buffers could not be sized");
-        last_contacts = hp.outs[0].pairs;
-        contacts_stale = false;
         return hp.outs;
     }
     const EvalOut* eval_read(const double* dz, bool trials, double* d_gout, double* host_grad = nullptr) {
@@ -649,8 +648,6 @@ struct mcg_ctx {
     EvalOut read_out() {
         read_outs();
         if (hp.outs[0].overflow) eval_read(last_z, last_trials, last_grad);
-        else last_contacts = hp.outs[0].pairs;
-        contacts_stale = false;
         return hp.outs[0];
     }
 
@@ -864,7 +861,6 @@ struct mcg_ctx {
                 throw Fail(MCG_ERR_CUDA, "the device-resident round loop ran no round");
             break;
         }
-        last_contacts = hp.outs[0].pairs;
         contacts_stale = false;
         return true;
     }
@@ -1950,7 +1946,13 @@ int mcg_contact_pairs(mcg_ctx* c, uint64_t* keys, int64_t capacity, int64_t* cou
         need_topo(c);
         if (c->contacts_stale)
             throw Fail(MCG_ERR_STATE, "the last evaluation was mcg_objective_noalloc's, whose contact pairs are not kept");
-        const long long nc = c->phys.self_contact ? c->last_contacts : 0;
+        // the list's own counter: whatever evaluation was read last, count and list belong together
+        long long nc = 0;
+        if (c->phys.self_contact) {
+            d2h(c->hp.u32, c->cb.counts + kContacts, 1, c->stream);
+            c->sync();
+            nc = std::min<long long>(c->hp.u32[0], c->cb.contact_cap);  // (more: an overflow not yet repeated)
+        }
         *count = nc;
         if (nc > capacity) throw Fail(MCG_ERR_CAPACITY, "pair buffer too small");
         std::vector<uint32_t> a(static_cast<size_t>(nc)), b(static_cast<size_t>(nc));

@@ -109,7 +109,6 @@ struct EvalOut {
     double beam_energy, node_energy, center_energy, contact_energy, platen_energy;
     int overflow;                    // ContactFlag bits that invalidate this evaluation
     unsigned kernel_error;           // a kernel's bounded wait gave up (EvalBufs::err)
-    unsigned pairs, pad_;            // self-contacts of all instances (ContactCount kContacts)
     double rms, gmax;                // residual over free DOFs: sqrt(mean g^2), max |g| (sim.cpp:44-45)
 };
 

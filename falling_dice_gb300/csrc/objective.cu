@@ -740,7 +740,6 @@ __global__ void __launch_bounds__(kEvalBlock, 2 * kMinBlocks) k_gather(DevTopo t
         for (EvalOut* out : {e.out, e.out_host}) {
             if (!out) continue;
             out->overflow = use_contacts ? int(c.flags[0] & ~uint32_t(kNonFinite)) : 0;
-            out->pairs = use_contacts ? c.counts[kContacts] : 0u;
             out->kernel_error = *e.err;
         }
         if (use_contacts) c.flags[0] = c.flags[1] = 0;  // for the next evaluation

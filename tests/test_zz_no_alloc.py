@@ -137,6 +137,27 @@ def test_contact_queries_refuse_after_a_noalloc_evaluation(mcg):
     assert np.array_equal(sol.contact_pairs(), s["pairs"])
 
 
+def test_reading_the_result_leaves_a_noalloc_evaluations_contacts_refused(mcg):
+    """mcg_read_result after the no-allocation call reads that call's totals; the context's own contact
+    list is still not theirs, so the queries refuse until the next allocating evaluation."""
+    g = golden("ref242")
+    s = g.state(3)
+    sol = mcg.Solver(g.cfg, g.lattice)
+    sol.set_state(plastic=s["plastic"])
+    quiet = np.zeros_like(s["z"])
+    ref = sol.objective(quiet, g.lattice.geometry.top0 + 0.01)  # another list than the next call's
+    rc, energy, _, diag = noalloc(sol, s["z"], s["top"])
+    assert rc == abi.MCG_OK and diag["contacts"] != ref["diag"]["contacts"]
+    assert sol.read_result()["energy"] == energy
+    for query in (sol.contact_pairs, sol.contact_stats):
+        with pytest.raises(mcg.MCGError) as e:
+            query()
+        assert e.value.status == abi.MCG_ERR_STATE
+    sol.objective(s["z"], s["top"])
+    sol.read_result()
+    assert np.array_equal(sol.contact_pairs(), s["pairs"])
+
+
 def test_noalloc_runs_beside_a_graph_capture_and_adds_nothing_to_it(mcg):
     """A caller may evaluate while one of its streams captures a CUDA graph: in relaxed
     capture mode on the capturing thread, and in thread-local mode from another thread.  The

@@ -346,7 +346,8 @@ struct mcg_ctx {
     }
 
     // ---- contact buffers ---------------------------------------------------------------
-    double broad_cell = 0;   // current grid cell (the reference's size unless coarsened)
+    double broad_cell = 0;   // current grid cell
+    bool cell_chosen = false;  // by the caller, a tuning or a growth; otherwise it is default_cell()
     float contact_skin = 0;  // candidate-list reuse distance (m); 0 rebuilds every evaluation
     int pair_blocks_set = 0; // blocks of the pair enumeration; 0: contact_pair_blocks(shapes)
     double reference_cell() const { return std::max(2.8 * jr, .72 * cfg.cell_size); }
@@ -430,13 +431,20 @@ struct mcg_ctx {
         sync();
         long long slots = cb.bin_slots, ccap = cb.contact_cap, bcap = cb.bin_cap, kcap = cb.cand_cap;
         if (flags & kOverCandidates) kcap = std::max(kcap, (long long)need[kCand] + need[kCand] / 4 + 1024);
-        if (flags & kOverSpan) broad_cell *= 2;
+        if (flags & kOverSpan) {
+            broad_cell *= 2;
+            cell_chosen = true;
+        }
         if (flags & kOverEntries) slots = std::max(slots, (long long)need[kLargestBin] + need[kLargestBin] / 4);
         if (flags & kOverContacts) ccap = std::max(ccap, (long long)need[kContacts] + need[kContacts] / 4 + 1024);
         if (flags & kOverBins) {
             const long long want = (long long)grid[9] + grid[9] / 4 + 1024;
-            if (want <= (1LL << 28)) bcap = std::max(bcap, want);
-            else broad_cell *= 2;  // a huge extent: coarser cells instead of more bins
+            if (want <= (1LL << 28)) {
+                bcap = std::max(bcap, want);
+            } else {
+                broad_cell *= 2;  // a huge extent: coarser cells instead of more bins
+                cell_chosen = true;
+            }
         }
         alloc_contacts(slots, ccap, bcap, kcap);
         return true;
@@ -1561,6 +1569,7 @@ void upload_instances(mcg_ctx* c, const std::vector<InstIn>& ins) {
     // contact buffers: a first guess, grown on demand
     const long long S = (long long)N + B;
     c->broad_cell = P.broad_cell;
+    c->cell_chosen = false;
     c->contact_skin = float(cf.cell_size / 32);
     {
         // bins: the Morton range of the rest-state extent (in the grid's frame) with room to
@@ -1876,34 +1885,43 @@ int objective_with_fixed_contacts(mcg_ctx* c, ContactBufs& fixed, size_t zero_by
         h2d(c->d_zin, z, n, s);
         c->hp.tops[0] = top;
         c->set_active(std::vector<uint8_t>(1, 1));
-        PhysParams p = c->phys;
-        // its bins are few and small: the reference's cell unless another was set
-        p.broad_cell = c->broad_cell == c->default_cell() ? c->reference_cell() : c->broad_cell;
-        p.inv_cell_f = float(1.0 / p.broad_cell);
-        if (p.self_contact) {
-            // the scratch holds whatever its last user left: the state between evaluations
-            c->set_sum_quanta(fixed);
-            ck(cudaMemsetAsync(fixed.flags, 0, zero_bytes, s), "memset");
-        }
-        const BuildArgs ba = c->build_args(fixed, 0.f, p.broad_cell);  // always rebuilds
-        if (c->mixed) launch_state_mixed(c->topo, p, c->d_zin, c->d_baseX, c->mn, ba, c->ev, s);
-        else launch_state(c->topo, p, c->d_zin, c->d_baseX, ba, c->ev, s);
-        if (!c->mixed) launch_rotations(c->topo, c->d_zin, c->d_baseR, c->ev, s);
-        launch_center(c->topo, p, ba, c->ev, s);
-        if (c->mixed) launch_beams_mixed(c->topo, c->mat, c->mb, c->mn, false, c->ev, s, c->beam_variant);
-        else launch_beams(c->topo, c->mat, c->d_plastic, false, c->ev, s, c->beam_variant);
-        const ContactBufs* cptr = nullptr;
-        if (p.self_contact) {
-            launch_contacts(c->topo, p, c->ev, fixed, 0.f, s);
-            cptr = &fixed;
-        }
-        if (c->mixed) launch_gather_mixed(c->topo, p, cptr, c->d_grad, c->ev, s, c->gather_variant);
-        else launch_gather(c->topo, p, cptr, c->d_grad, c->ev, s, c->gather_variant);
-        launch_finalize(c->topo, p, c->d_grad, c->ev, s);
-        c->check_launch();
-        c->contacts_stale = p.self_contact != 0;
-        c->sync();
-        const EvalOut o = c->hp.outs[0];
+        const auto evaluate = [&](double cell) {
+            PhysParams p = c->phys;
+            p.broad_cell = cell;
+            p.inv_cell_f = float(1.0 / cell);
+            if (p.self_contact) {
+                // the scratch holds whatever its last user left: the state between evaluations
+                c->set_sum_quanta(fixed);
+                ck(cudaMemsetAsync(fixed.flags, 0, zero_bytes, s), "memset");
+            }
+            const BuildArgs ba = c->build_args(fixed, 0.f, cell);  // always rebuilds
+            if (c->mixed) launch_state_mixed(c->topo, p, c->d_zin, c->d_baseX, c->mn, ba, c->ev, s);
+            else launch_state(c->topo, p, c->d_zin, c->d_baseX, ba, c->ev, s);
+            if (!c->mixed) launch_rotations(c->topo, c->d_zin, c->d_baseR, c->ev, s);
+            launch_center(c->topo, p, ba, c->ev, s);
+            if (c->mixed) launch_beams_mixed(c->topo, c->mat, c->mb, c->mn, false, c->ev, s, c->beam_variant);
+            else launch_beams(c->topo, c->mat, c->d_plastic, false, c->ev, s, c->beam_variant);
+            const ContactBufs* cptr = nullptr;
+            if (p.self_contact) {
+                launch_contacts(c->topo, p, c->ev, fixed, 0.f, s);
+                cptr = &fixed;
+            }
+            if (c->mixed) launch_gather_mixed(c->topo, p, cptr, c->d_grad, c->ev, s, c->gather_variant);
+            else launch_gather(c->topo, p, cptr, c->d_grad, c->ev, s, c->gather_variant);
+            launch_finalize(c->topo, p, c->d_grad, c->ev, s);
+            c->check_launch();
+            c->contacts_stale = p.self_contact != 0;
+            c->sync();
+            return c->hp.outs[0];
+        };
+        // The scratch's bins hold 128 entries: a cubic+BCC lattice at rest has about 25 in a bin of the
+        // reference's cell, 100 in one of the default, twice as wide, and too many at 1.25 times that
+        // (a tuner's choice).  So the reference's cell, or a finer one chosen for the context's own
+        // buffers; a coarser one that was chosen where that does not fit (large extents: fewer bins).
+        const double cell = std::min(c->reference_cell(), c->broad_cell);
+        EvalOut o = evaluate(cell);
+        if ((o.overflow & (kOverEntries | kOverBins | kOverSpan)) && c->cell_chosen && c->broad_cell > cell)
+            o = evaluate(c->broad_cell);
         if (o.overflow) {
             std::string what;
             if (o.overflow & kOverEntries) what += " entries in one grid bin";
@@ -2087,6 +2105,7 @@ int mcg_set_contact_cell(mcg_ctx* c, double cell) {
         need_topo(c);
         if (!(cell >= 0) || cell > 1e3) throw Fail(MCG_ERR_INVALID, "cell must be a length >= 0 (m)");
         c->broad_cell = cell > 0 ? cell : c->default_cell();
+        c->cell_chosen = cell > 0;
         c->sync();
         c->alloc_contacts(c->cb.bin_slots, c->cb.contact_cap, c->cb.bin_cap, c->cb.cand_cap);
     });
@@ -2098,6 +2117,7 @@ int mcg_set_contact_shapes(mcg_ctx* c, double cell, int32_t pair_blocks) {
         if (!(cell >= 0) || cell > 1e3) throw Fail(MCG_ERR_INVALID, "cell must be a length >= 0 (m)");
         if (pair_blocks < 0 || pair_blocks > (1 << 20)) throw Fail(MCG_ERR_INVALID, "pair_blocks must be in 0 .. 2^20");
         c->broad_cell = cell > 0 ? cell : c->default_cell();
+        c->cell_chosen = cell > 0;
         c->pair_blocks_set = pair_blocks;
         c->sync();
         c->alloc_contacts(c->cb.bin_slots, c->cb.contact_cap, c->cb.bin_cap, c->cb.cand_cap);
@@ -2206,6 +2226,7 @@ int mcg_autotune(mcg_ctx* c, const double* z, const double* tops, int32_t reps, 
                 (best.ms > 1e299 || q.blocks > best.blocks || (q.blocks == best.blocks && q.cell < best.cell)))
                 best = q;
         c->broad_cell = best.cell;
+        c->cell_chosen = true;
         c->pair_blocks_set = best.blocks;
         c->alloc_contacts(c->cb.bin_slots, c->cb.contact_cap, c->cb.bin_cap, c->cb.cand_cap);
         // then the occupancy variants of the beam kernel and of the gather, one after the

@@ -17,8 +17,9 @@
 // kNoAllocMaxNodes nodes and kNoAllocMaxShapes nodes + beams, and per evaluation at most
 // the entry/bin/candidate/contact counts below; a larger lattice or state is rejected with
 // MCG_ERR_CAPACITY and a message naming what overflowed.  The bins cover the grid box of the
-// deformed specimen at the grid cell (the reference's max(2.8 joint radius, 0.72 cell)):
-// about 9 cells per axis of a cube-shaped specimen.
+// deformed specimen at the reference's grid cell, max(2.8 joint radius, 0.72 cell): about 9
+// cells per axis of a cube-shaped specimen.  A finer cell that was chosen for the context
+// (mcg_set_contact_cell, a tuning) is used instead, a coarser one where that does not fit.
 //
 // Host code cannot use the array's name as an address: the first call on each context
 // looks the device address up with cudaGetSymbolAddress, with the context's device current,

@@ -158,6 +158,44 @@ def test_reading_the_result_leaves_a_noalloc_evaluations_contacts_refused(mcg):
     assert np.array_equal(sol.contact_pairs(), s["pairs"])
 
 
+@pytest.mark.parametrize("cell", [5.4e-3, 7.2e-3, 9e-3, 14e-3, 30e-3])
+def test_noalloc_after_a_contact_cell_was_chosen(mcg, cell):
+    """The fixed scratch has few and small bins: a grid cell that suits the context's own buffers (a
+    tuned one, 0.9 to 1.4 times twice the reference's, or the caller's) may fill them.  The evaluation
+    does not depend on the cell, and a state that fits at the reference's is not refused for it."""
+    cfg, spec = workloads.bcc((5, 4, 6))
+    lat = mcg.generate_lattice(spec, cfg)
+    sol = mcg.Solver(cfg, lat)
+    for squeeze in (0.0, 0.05):
+        z, pl, top = squeezed(mcg, lat, cfg, squeeze, 0.02)
+        sol.set_state(plastic=pl)
+        sol.set_contact_cell(0.0)
+        ref = sol.objective(z, top)
+        rc, energy, _, _ = noalloc(sol, z, top)
+        assert rc == abi.MCG_OK, sol.lib.mcg_last_error(sol.h)
+        sol.set_contact_shapes(cell, 0)
+        rc, e1, grad, diag = noalloc(sol, z, top)
+        assert rc == abi.MCG_OK, (squeeze, sol.lib.mcg_last_error(sol.h))
+        assert e1 == energy
+        assert abs(e1 - ref["energy"]) <= TOL * abs(ref["energy"]) and rel_err(grad, ref["grad"]) <= TOL
+        assert diag["contacts"] == ref["diag"]["contacts"]
+
+
+def test_noalloc_takes_a_coarser_cell_that_was_chosen_where_the_references_needs_too_many_bins(mcg):
+    cfg, spec = workloads.bcc((11, 11, 11))
+    spec.kind = abi.MCG_LATTICE_CUBIC
+    lat = mcg.generate_lattice(spec, cfg)
+    sol = mcg.Solver(cfg, lat)
+    z, top = np.zeros(6 * lat.n_nodes), lat.geometry.top0
+    ref = sol.objective(z, top)
+    for cell, status in ((7.2e-3, abi.MCG_OK), (0.0, abi.MCG_ERR_CAPACITY), (9e-3, abi.MCG_OK)):
+        sol.set_contact_cell(cell)
+        rc, energy, grad, _ = noalloc(sol, z, top)
+        assert rc == status, (cell, sol.lib.mcg_last_error(sol.h))
+        if rc == abi.MCG_OK:
+            assert abs(energy - ref["energy"]) <= TOL * abs(ref["energy"]) and rel_err(grad, ref["grad"]) <= TOL
+
+
 def test_noalloc_runs_beside_a_graph_capture_and_adds_nothing_to_it(mcg):
     """A caller may evaluate while one of its streams captures a CUDA graph: in relaxed
     capture mode on the capturing thread, and in thread-local mode from another thread.  The

@@ -117,10 +117,11 @@ __device__ __forceinline__ double xor_sign(double v, double s) {
 __device__ __forceinline__ double half_of(double v) {
     return __hiloint2double(__double2hiint(v) - 0x00100000, __double2loint(v));
 }
-// |v - 1| < 2^-20: a squared norm whose square root is 1 + (v - 1) / 2 to FP64 precision when
-// it differs from one by rounding only.
+// |v - 1| <= 2^-28 (2^25 numbers below one, 2^24 above it): a squared norm whose inverse square root
+// is 1 - (v - 1) / 2 to FP64 precision (what is left out, 3 (v - 1)^2 / 8, is below 2^-57).
 __device__ __forceinline__ bool near_one(double v) {
-    return unsigned(__double2hiint(v)) - 0x3feffffeu < 4u;
+    constexpr long long one = 0x3ff0000000000000LL;
+    return (unsigned long long)(__double_as_longlong(v) - (one - (1LL << 25))) <= (1ULL << 25) + (1ULL << 24);
 }
 // a in [2^-111, 2^98): its FP32 estimate below neither overflows nor loses bits.
 __device__ __forceinline__ bool rsqrt_range(double a) {
@@ -196,7 +197,8 @@ __device__ __forceinline__ q4 fqmul(q4 a, q4 b) {
             fma(a.z, b.x, fma(a.y, b.w, fma(-a.x, b.z, a.w * b.y))),
             fma(a.z, b.w, fma(-a.y, b.x, fma(a.x, b.y, a.w * b.z)))};
 }
-// Unit quaternion of q when |q| differs from one by rounding only, else qnorm.
+// Unit quaternion of q: by one step when |q| differs from one by little (rounding, usually; near_one),
+// else qnorm.
 __device__ __forceinline__ q4 qnorm_near(q4 q) {
     const double n2 = fma(q.z, q.z, fma(q.y, q.y, fma(q.x, q.x, q.w * q.w)));
     if (!near_one(n2)) return qnorm(q);

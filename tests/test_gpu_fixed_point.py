@@ -87,3 +87,20 @@ def test_plastic_rotations_of_any_size(mcg, mco, size):
     agree(sol, orc, z, lat.geometry.top0 + 0.01)
     a, b = (m.objective(z, lat.geometry.top0 + 0.01, True)["trial_aux"].reshape(-1, 7)[:, 2:5] for m in (sol, orc))
     assert rel_err(a, b) <= TOL
+
+@pytest.mark.parametrize("off", [0.0, 1e-12, -1e-9, 1e-8, -1e-7, 5e-7, -5e-7, 9e-7, 1e-3, -0.5])
+def test_base_orientations_given_to_few_digits_are_normalized(mcg, mco, off):
+    """Base quaternions of length 1 + off: the evaluation's orientations, which a commit keeps, have
+    length one to rounding (bar: a squared length by four products and three sums, a square root and a
+    quotient, each to half an ulp, 2^-53 relative: 4 of them on a length)."""
+    cfg, lat, _, _ = model(mcg, mco, "bcc", (2, 2, 2))
+    cfg.max_iterations = 1
+    sol = mcg.Solver(cfg, lat)
+    rng = np.random.default_rng(8)
+    q = rng.standard_normal((lat.n_nodes, 4))
+    q /= np.linalg.norm(q, axis=1, keepdims=True)
+    sol.set_state(base_r=((1.0 + off) * q).ravel())
+    sol.minimize(lat.geometry.top0 + 0.01, np.zeros(6 * lat.n_nodes))
+    sol.commit()
+    r = sol.get_state()[1].reshape(-1, 4).astype(np.longdouble)
+    assert np.max(np.abs(np.sqrt(np.sum(r * r, axis=1)) - 1)) <= 4 * 2.0 ** -53

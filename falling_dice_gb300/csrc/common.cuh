@@ -217,6 +217,13 @@ __device__ __forceinline__ d3 fmrot(const m3& m, d3 v) { return d3{fdot(m.r0, v)
 // lower one, sum up in 64 bits each; the lower halves' products, below 2^-58, are left out.  A sum
 // of three products is off by at most 2^-56 = 1.4e-17 (FP64 additions near one: 1.1e-16 each).
 // "Units" are 64-bit integers of 2^-58.
+// A number far below one has few bits above 2^-58, where FP64 keeps 53 of them whatever its size.  So
+// vectors of free magnitude (a rotation's vector part and its matrix less the identity, deviations
+// of directors from chords, rotation vectors, strains) have an exponent e for their components
+// together: units times 2^e, the largest component in [1/4, 1/2) where e was made for the vector.
+// Sums align their terms to the larger exponent, so that a result is off by 2^-55 of its largest
+// term, where FP64's rounding is 2^-53 of it.  With e = 0 throughout the moment of two rotations of
+// 1e-3 was off by 6e-15 of itself, of 1e-6 by 6e-12; with exponents 1e-16 (FP64: 2e-16).
 struct fx { int h, l; };
 struct u3 { long long x, y, z; };  // units
 struct fx3 { fx x, y, z; };
@@ -237,26 +244,33 @@ __device__ __forceinline__ unsigned long long fixed_magnitude(double v, int scal
     const unsigned long long m = (unsigned long long)(hi & 0xfffffu | 0x100000u) << 32 | unsigned(__double2loint(v));
     return shift_mantissa(m, int(hi >> 20 & 0x7ffu) - scale);
 }
-// v (|v| < 8) in units, rounded toward zero; some integer when v is larger or not finite.
-__device__ __forceinline__ long long fx_units(double v) {
-    const long long n = (long long)fixed_magnitude(v, 1017);
+// v (|v| < 8 2^e) in units times 2^e, rounded toward zero; some integer when v is larger or not finite.
+__device__ __forceinline__ long long fx_units(double v, int e = 0) {
+    const long long n = (long long)fixed_magnitude(v, 1017 + e);
     return __double2hiint(v) < 0 ? -n : n;
 }
-// |v| < 2^n, v finite.
-__device__ __forceinline__ bool below_power(double v, int n) { return (unsigned(__double2hiint(v)) & 0x7fffffffu) < unsigned(0x3ff + n) << 20; }
-__device__ __forceinline__ bool below_power(d3 v, int n) { return below_power(v.x, n) && below_power(v.y, n) && below_power(v.z, n); }
+// The exponent of a vector: its largest component is in [1/4, 1/2) 2^e; kFxLeast for a smaller one
+// (or zero), above kFxMost for one that is larger or not finite.
+constexpr int kFxLeast = -700, kFxMost = 700;
+__device__ __forceinline__ int fx_exponent(d3 v) {
+    const auto exponent = [](double a) { return int(unsigned(__double2hiint(a)) >> 20 & 0x7ffu); };
+    return max(max(exponent(v.x), max(exponent(v.y), exponent(v.z))) - 1021, kFxLeast);
+}
 // n 2^e2, rounded to nearest; 2^-900 < the magnitude < 2^900 or zero.
 __device__ __forceinline__ double fx_double(long long n, int e2 = -58) {
     const unsigned long long a = n < 0 ? 0ULL - (unsigned long long)n : (unsigned long long)n;
-    const int z = __clzll((long long)a);
+    const int z = __clzll((long long)(a | 1));
     const unsigned long long m = a << z;
     unsigned long long b = ((unsigned long long)(1023 + 62 - z + e2) << 52) + (m >> 11) + (m >> 10 & 1);
     if (n == 0) b = 0;
     return __longlong_as_double((long long)(n < 0 ? b | 0x8000000000000000ULL : b));
 }
-__device__ __forceinline__ double fx_double(fx a) { return fx_double((long long)a.h * (1 << 30) + a.l); }
-__device__ __forceinline__ d3 fx_double(u3 n) { return d3{fx_double(n.x), fx_double(n.y), fx_double(n.z)}; }
-__device__ __forceinline__ u3 fx_units(d3 v) { return u3{fx_units(v.x), fx_units(v.y), fx_units(v.z)}; }
+__device__ __forceinline__ double fx_double(fx a, int e2 = -58) { return fx_double((long long)a.h * (1 << 30) + a.l, e2); }
+__device__ __forceinline__ d3 fx_double(u3 n, int e2 = -58) { return d3{fx_double(n.x, e2), fx_double(n.y, e2), fx_double(n.z, e2)}; }
+__device__ __forceinline__ u3 fx_units(d3 v, int e = 0) { return u3{fx_units(v.x, e), fx_units(v.y, e), fx_units(v.z, e)}; }
+// n 2^-s, rounded down; s >= 0.
+__device__ __forceinline__ long long fx_shr(long long n, int s) { return n >> min(s, 63); }
+__device__ __forceinline__ u3 fx_shr(u3 n, int s) { return u3{fx_shr(n.x, s), fx_shr(n.y, s), fx_shr(n.z, s)}; }
 __device__ __forceinline__ long long fx_hh(fx a, fx b) { return (long long)a.h * b.h; }
 __device__ __forceinline__ long long fx_hl(fx a, fx b) { return (long long)a.h * b.l + (long long)a.l * b.h; }
 __device__ __forceinline__ long long fx_sum(long long hh, long long hl) { return hh * 4 + ((hl + (1 << 27)) >> 28); }
@@ -284,27 +298,37 @@ __device__ __forceinline__ long long fx_renorm(long long n, int d) { return n - 
 __device__ __forceinline__ double fx_bits(fx a) { return __hiloint2double(a.h, a.l); }
 __device__ __forceinline__ fx fx_load(double v) { return fx{__double2hiint(v), __double2loint(v)}; }
 
-// A node's rotation: the unit quaternion and its matrix, in fixed point.  A quaternion that is not
-// finite has w.h = kFxInvalid.
-struct FxRot { fx3 r0, r1, r2; };
-// Rows 0-2 of the matrix and the quaternion as the node's four records; q normalized to rounding
-// already, here to 2^-56.
+// A node's rotation in fixed point: the unit quaternion, its vector part with an exponent e <= 0, and
+// the matrix less the identity (2 (w [v] + [v]^2), of the vector part's size) with the same.  A
+// quaternion that is not finite has w.h = kFxInvalid.
+struct FxRot {
+    fx3 r0, r1, r2;  // rows of R - I, times 2^e
+    int e;
+};
+// The matrix rows with e beside the first, and the quaternion, as the node's four records; q
+// normalized to rounding already, here to 2^-56.
 __device__ __forceinline__ void store_rotation(q4 q, double4_32a* __restrict__ rec) {
-    const long long u[4] = {fx_units(q.w), fx_units(q.x), fx_units(q.y), fx_units(q.z)};
-    fx4 f{fx_of(u[0]), fx_of(u[1]), fx_of(u[2]), fx_of(u[3])};
-    const int d = int(fx_dot(f, f) - kFxOne);
-    f = fx4{fx_of(fx_renorm(u[0], d)), fx_of(fx_renorm(u[1], d)), fx_of(fx_renorm(u[2], d)), fx_of(fx_renorm(u[3], d))};
-    const auto one_less = [](long long n) { return fx_bits(fx_of(kFxOne - n)); };
+    const d3 qv{q.x, q.y, q.z};
+    const int e = min(fx_exponent(qv), 0);
+    const long long uw = fx_units(q.w);
+    u3 uv = fx_units(qv, e);
+    fx w = fx_of(uw);
+    fx3 v = fx_of(uv);  // times 2^e
+    const int d = int(fx_mul(w, w) + fx_shr(fx_dot(v, v), -2 * e) - kFxOne);
+    w = fx_of(fx_renorm(uw, d));
+    uv = u3{fx_renorm(uv.x, d), fx_renorm(uv.y, d), fx_renorm(uv.z, d)};
+    v = fx_of(uv);
+    const fx3 a = fx_of(fx_shr(uv, -e));  // the vector part itself
     const auto entry = [](long long n) { return fx_bits(fx_of(n)); };
-    rec[0] = make_double4_32a(one_less(fx_twice(f.y, f.y, f.z, f.z)), entry(fx_twice(f.x, f.y, -f.w, f.z)),
-                              entry(fx_twice(f.x, f.z, f.w, f.y)), 0.0);
-    rec[1] = make_double4_32a(entry(fx_twice(f.x, f.y, f.w, f.z)), one_less(fx_twice(f.x, f.x, f.z, f.z)),
-                              entry(fx_twice(f.y, f.z, -f.w, f.x)), 0.0);
-    rec[2] = make_double4_32a(entry(fx_twice(f.x, f.z, -f.w, f.y)), entry(fx_twice(f.y, f.z, f.w, f.x)),
-                              one_less(fx_twice(f.x, f.x, f.y, f.y)), 0.0);
+    rec[0] = make_double4_32a(entry(-fx_twice(a.y, v.y, a.z, v.z)), entry(fx_twice(a.x, v.y, -w, v.z)),
+                              entry(fx_twice(a.x, v.z, w, v.y)), fx_bits(fx{e, 0}));
+    rec[1] = make_double4_32a(entry(fx_twice(a.x, v.y, w, v.z)), entry(-fx_twice(a.x, v.x, a.z, v.z)),
+                              entry(fx_twice(a.y, v.z, -w, v.x)), 0.0);
+    rec[2] = make_double4_32a(entry(fx_twice(a.x, v.z, -w, v.y)), entry(fx_twice(a.y, v.z, w, v.x)),
+                              entry(-fx_twice(a.x, v.x, a.y, v.y)), 0.0);
     const bool ok = isfinite(q.w) && isfinite(q.x) && isfinite(q.y) && isfinite(q.z);
-    if (!ok) f.w.h = kFxInvalid;
-    rec[3] = make_double4_32a(fx_bits(f.w), fx_bits(f.x), fx_bits(f.y), fx_bits(f.z));
+    if (!ok) w.h = kFxInvalid;
+    rec[3] = make_double4_32a(fx_bits(w), fx_bits(v.x), fx_bits(v.y), fx_bits(v.z));
 }
 __device__ __forceinline__ fx3 load_fx3(const double4_32a* rec) {
     const double4_32a v = *rec;
@@ -315,11 +339,12 @@ __device__ __forceinline__ fx4 load_fx4(const double4_32a* rec) {
     return fx4{fx_load(v.x), fx_load(v.y), fx_load(v.z), fx_load(v.w)};
 }
 __device__ __forceinline__ FxRot load_rotation(const double4_32a* rec) {
-    return FxRot{load_fx3(rec), load_fx3(rec + 1), load_fx3(rec + 2)};
+    const double4_32a v = *rec;
+    return FxRot{fx3{fx_load(v.x), fx_load(v.y), fx_load(v.z)}, load_fx3(rec + 1), load_fx3(rec + 2), fx_load(v.w).h};
 }
 __device__ __forceinline__ m3 fx_matrix(const FxRot& r) {
-    const auto row = [](const fx3& v) { return d3{fx_double(v.x), fx_double(v.y), fx_double(v.z)}; };
-    return m3{row(r.r0), row(r.r1), row(r.r2)};
+    const auto row = [&](const fx3& v) { return d3{fx_double(v.x, r.e - 58), fx_double(v.y, r.e - 58), fx_double(v.z, r.e - 58)}; };
+    return m3{row(r.r0) + d3{1, 0, 0}, row(r.r1) + d3{0, 1, 0}, row(r.r2) + d3{0, 0, 1}};
 }
 // Any vector as fixed point times 2^(e - 1022): its components to one exponent, 58 bits below the
 // largest; false when that is tiny (zero, usually) or huge.
@@ -334,11 +359,11 @@ __device__ __forceinline__ bool block_units(d3 v, u3& n, int& e) {
     n = u3{units(v.x), units(v.y), units(v.z)};
     return unsigned(e - 300) <= 1400u;
 }
-// M v, v in units times 2^(e - 1022).
+// R v, v in units times 2^(e - 1022): v and (R - I) v.
 __device__ __forceinline__ d3 fx_rotate(const FxRot& r, u3 v, int e) {
     const fx3 f = fx_of(v);
-    return d3{fx_double(fx_dot(r.r0, f), e - 1022 - 58), fx_double(fx_dot(r.r1, f), e - 1022 - 58),
-              fx_double(fx_dot(r.r2, f), e - 1022 - 58)};
+    const u3 n{v.x + fx_shr(fx_dot(r.r0, f), -r.e), v.y + fx_shr(fx_dot(r.r1, f), -r.e), v.z + fx_shr(fx_dot(r.r2, f), -r.e)};
+    return fx_double(n, e - 1022 - 58);
 }
 
 // ---- deterministic reductions ------------------------------------------------------------

@@ -215,7 +215,7 @@ constexpr int kFinSingle = 768;  // block partials one block sums: six per threa
 struct EvalBufs {
     double4_32a* x;             // [N]
     double4_32a* R;             // [N]
-    double4_32a* M;             // [4N] R in fixed point: matrix rows (x, y, z, pad), quaternion (fx)
+    double4_32a* M;             // [4N] R in fixed point: rows of R - I with their exponent, quaternion (FxRot)
     float4* xf_lo;              // [N] position rounded down to single precision
     float4* xf_hi;              // [N] position rounded up
     double* slot;           // [15B] per beam 12: (-F, Ga), added to node a, then (+F, Gb), added to

@@ -274,16 +274,23 @@ __device__ __forceinline__ unsigned long long poly_step(unsigned long long acc, 
 }
 
 // Rotation vector of the relative rotation Q = Ra^* Rb (MC/include/core.hpp:52 quatLog of the
-// normalized Q with w >= 0) in units.  With s = |v| of the unit Q, the vector is
-// 2 asin(s) / s v: a polynomial in s^2 up to s^2 = 0.1 (angles up to 36.9 degrees; Chebyshev
-// interpolation, error 2e-18), so that the usual beam takes no square root, division or
-// arctangent; larger angles take atan2 as the reference does.  Q is a product of two quaternions
-// of length one to 2^-56.
+// normalized Q with w >= 0) in units times 2^e, Ra's and Rb's vector parts with exponents ea and eb.
+// With s = |v| of the unit Q, the vector is 2 asin(s) / s v: a polynomial in s^2 up to s^2 = 0.1
+// (angles up to 36.9 degrees; Chebyshev interpolation, error 2e-18), so that the usual beam takes no
+// square root, division or arctangent; larger angles take atan2 as the reference does.  Q is a
+// product of two quaternions of length one to 2^-56.  Its vector part a.w b - b.w a - a x b is summed
+// at the larger exponent (it is below 2 there, the rotation vector below 4).
 constexpr long long fx_limit(double v) { return (long long)(v * 0x1p58); }
-__device__ __forceinline__ u3 relative_rotation(const fx4& a, const fx4& b) {
-    const u3 v{fx_dot(a, fx4{b.x, -b.w, -b.z, b.y}), fx_dot(a, fx4{b.y, b.z, -b.w, -b.x}), fx_dot(a, fx4{b.z, -b.y, b.x, -b.w})};
+__device__ __forceinline__ u3 relative_rotation(const fx4& a, int ea, const fx4& b, int eb, int& e) {
+    e = max(ea, eb);
+    const fx3 av{a.x, a.y, a.z}, bv{b.x, b.y, b.z};
+    const u3 c = fx_cross(av, bv);
+    const auto part = [&](fx p, fx q, long long r) {
+        return fx_shr(fx_mul(a.w, q), e - eb) - fx_shr(fx_mul(b.w, p), e - ea) - fx_shr(r, e - ea - eb);
+    };
+    const u3 v{part(a.x, b.x, c.x), part(a.y, b.y, c.y), part(a.z, b.z, c.z)};
     const fx3 vf = fx_of(v);
-    const long long s2 = fx_dot(vf, vf);
+    const long long s2 = fx_shr(fx_dot(vf, vf), -2 * e);
     if (s2 < fx_limit(0.1)) {
         constexpr int B = 62, X = 67;
         const unsigned long long u = (unsigned long long)s2 << (X - 58);
@@ -299,17 +306,18 @@ __device__ __forceinline__ u3 relative_rotation(const fx4& a, const fx4& b) {
         g = poly_step<X>(g, u, poly_units<B>(0x1.5555555555550p-2));
         g = poly_step<X>(g, u, poly_units<B>(2.0));
         // the sign of Q's real part, which is close to one
-        const long long w = fx_hh(a.w, b.w) + fx_hh(a.x, b.x) + fx_hh(a.y, b.y) + fx_hh(a.z, b.z);
+        const long long w = fx_hh(a.w, b.w) + fx_shr(fx_hh(a.x, b.x) + fx_hh(a.y, b.y) + fx_hh(a.z, b.z), -(ea + eb));
         const long long gu = (long long)(g >> (B - 58));
         const fx gf = fx_of(w < 0 ? -gu : gu);
         return u3{fx_mul(vf.x, gf), fx_mul(vf.y, gf), fx_mul(vf.z, gf)};
     }
-    const d3 vd = fx_double(v);
-    q4 Q = qnorm(q4{fx_double(fx_dot(a, b)), vd.x, vd.y, vd.z});
+    const d3 vd = fx_double(v, e - 58);
+    q4 Q = qnorm(q4{fx_double(fx_mul(a.w, b.w) + fx_shr(fx_dot(av, bv), -(ea + eb))), vd.x, vd.y, vd.z});
     if (Q.w < 0) Q = q4{-Q.w, -Q.x, -Q.y, -Q.z};
     const double s = sqrt(Q.x * Q.x + Q.y * Q.y + Q.z * Q.z);
     d3 phi{2 * Q.x, 2 * Q.y, 2 * Q.z};
     if (!(s < 1e-12)) phi = d3{Q.x, Q.y, Q.z} * (2 * atan2(s, clampd(Q.w, -1, 1)) / s);
+    e = 0;
     return fx_units(phi);
 }
 
@@ -341,15 +349,18 @@ __device__ __forceinline__ d3 transport_rotated(const FxRot& r, u3 phi, d3 v) {
     return fx_rotate(r, n, e);
 }
 
-// The beam's axis in the material frame in units: unit(Ra^T t), t of length one but for rounding.
-__device__ __forceinline__ u3 material_axis(const FxRot& m, const fx3& t) {
+// The beam's axis in the material frame in units: unit(Ra^T t), t (units n) of length one but for
+// rounding.
+__device__ __forceinline__ u3 material_axis(const FxRot& m, u3 n, const fx3& t) {
     const int d = int(fx_dot(t, t) - kFxOne);
-    const auto part = [&](fx a, fx b, fx c) { return fx_renorm(fx_dot(fx3{a, b, c}, t), d); };
-    return u3{part(m.r0.x, m.r1.x, m.r2.x), part(m.r0.y, m.r1.y, m.r2.y), part(m.r0.z, m.r1.z, m.r2.z)};
+    const auto part = [&](long long k, fx a, fx b, fx c) { return fx_renorm(k + fx_shr(fx_dot(fx3{a, b, c}, t), -m.e), d); };
+    return u3{part(n.x, m.r0.x, m.r1.x, m.r2.x), part(n.y, m.r0.y, m.r1.y, m.r2.y), part(n.z, m.r0.z, m.r1.z, m.r2.z)};
 }
-// R e0 - t: a director's deviation from the chord, in units.
-__device__ __forceinline__ u3 deviation(const FxRot& r, const fx3& e0, u3 t) {
-    return u3{fx_dot(r.r0, e0) - t.x, fx_dot(r.r1, e0) - t.y, fx_dot(r.r2, e0) - t.z};
+// R e0 - t = (R - I) e0 - (t - e0): a director's deviation from the chord, in units times 2^e, as te is
+// of t - e0 (both small where the deviation is; below 8 with |e0| < 2 sqrt(3)).
+__device__ __forceinline__ u3 deviation(const FxRot& r, const fx3& e0, u3 te, int e) {
+    const int s = e - r.e;
+    return u3{fx_shr(fx_dot(r.r0, e0), s) - te.x, fx_shr(fx_dot(r.r1, e0), s) - te.y, fx_shr(fx_dot(r.r2, e0), s) - te.z};
 }
 
 // ---- beam kernel: MC/src/sim.cpp:139-141 ---------------------------------------------------
@@ -415,17 +426,19 @@ __global__ void __launch_bounds__(kBeamBlock, 2 * kMinBlocks) k_beams(DevTopo t,
             const double cs = t.cs[b];
             const u3 tu = fx_units(tt);
             const fx3 tf = fx_of(tu);
+            const d3 e0{t.e0x[b], t.e0y[b], t.e0z[b]};
             d3 ma, mb, gm, Ga, Gb;  // deviations, their sum, and cs t x (R e0) = cs t x m
             if (e0x.y != kFxInvalid) {
                 const fx3 e0f{fx{e0x.y, e0x.x}, fx{e0y.y, e0y.x}, fx{e0z.y, e0z.x}};
-                const u3 ua = deviation(Ma, e0f, tu), ub = deviation(Mb, e0f, tu);
-                ma = fx_double(ua);
-                mb = fx_double(ub);
+                const d3 te = tt - e0;
+                const int e = max(fx_exponent(te), max(Ma.e, Mb.e));
+                const u3 teu = fx_units(te, e), ua = deviation(Ma, e0f, teu, e), ub = deviation(Mb, e0f, teu, e);
+                ma = fx_double(ua, e - 58);
+                mb = fx_double(ub, e - 58);
                 gm = ma + mb;
-                Ga = fx_double(fx_cross(tf, fx_of(ua))) * cs;
-                Gb = fx_double(fx_cross(tf, fx_of(ub))) * cs;
+                Ga = fx_double(fx_cross(tf, fx_of(ua)), e - 58) * cs;
+                Gb = fx_double(fx_cross(tf, fx_of(ub)), e - 58) * cs;
             } else {  // no direction
-                const d3 e0{t.e0x[b], t.e0y[b], t.e0z[b]};
                 ma = fmrot(fx_matrix(Ma), e0) - tt;
                 mb = fmrot(fx_matrix(Mb), e0) - tt;
                 gm = ma + mb;
@@ -439,21 +452,23 @@ __global__ void __launch_bounds__(kBeamBlock, 2 * kMinBlocks) k_beams(DevTopo t,
             const d3 F{fma(tt.x, kf, -(kt_ * gm.x)), fma(tt.y, kf, -(kt_ * gm.y)), fma(tt.z, kf, -(kt_ * gm.z))};
             // bending and torsion from the relative rotation Q = Ra^* Rb
             const fx4 qa = load_fx4(e.M + 4 * size_t(ab.x) + 3), qb = load_fx4(e.M + 4 * size_t(ab.y) + 3);
-            const u3 phi = relative_rotation(qa, qb), axis_u = material_axis(Ma, tf);
+            int ep;  // exponent of phi
+            const u3 phi = relative_rotation(qa, Ma.e, qb, Mb.e, ep), axis_u = material_axis(Ma, tu, tf);
             const d3 axis = fx_double(axis_u);
-            // trial elastic parts: the twist and the bending of d = phi - rotp (in fixed point below eight:
-            // |phi| <= pi, components of rotp below two, so |d| < pi + 2 sqrt(3) = 6.6)
+            // trial elastic parts: the twist and the bending of d = phi - rotp, at the larger exponent
+            // (|phi| < 4 and |rotp| < sqrt(3)/2 there, so |d| < 5)
             double dtw;
             d3 dbend;
-            if (below_power(rotp, 1)) {
-                const u3 rp = fx_units(rotp), d{phi.x - rp.x, phi.y - rp.y, phi.z - rp.z};
+            const int ed = max(fx_exponent(rotp), ep);
+            if (ed <= kFxMost) {
+                const u3 rp = fx_units(rotp, ed), ph = fx_shr(phi, ed - ep), d{ph.x - rp.x, ph.y - rp.y, ph.z - rp.z};
                 const fx3 af = fx_of(axis_u);
                 const long long w = fx_dot(fx_of(d), af);
                 const fx wf = fx_of(w);
-                dtw = fx_double(w);
-                dbend = fx_double(u3{d.x - fx_mul(af.x, wf), d.y - fx_mul(af.y, wf), d.z - fx_mul(af.z, wf)});
+                dtw = fx_double(w, ed - 58);
+                dbend = fx_double(u3{d.x - fx_mul(af.x, wf), d.y - fx_mul(af.y, wf), d.z - fx_mul(af.z, wf)}, ed - 58);
             } else {
-                const d3 d = fx_double(phi) - rotp;
+                const d3 d = fx_double(phi, ep - 58) - rotp;
                 dtw = fdot(d, axis);
                 dbend = fmadd(axis, -dtw, d);
             }
@@ -470,7 +485,7 @@ __global__ void __launch_bounds__(kBeamBlock, 2 * kMinBlocks) k_beams(DevTopo t,
             double dr = 0;
             if (br.yielded) dr = t.my[b] * br.dg;
             if (tor.yielded) dr = fma(t.ty[b], tor.dg, dr);
-            const d3 world = transport_rotated(Ma, phi, moment);
+            const d3 world = transport_rotated(Ma, fx_shr(phi, -ep), moment);
             Ga = Ga - world;
             Gb = Gb + world;
             elastic2 = fma(cs, us2, uax2) + (br.energy2 + tor.energy2);

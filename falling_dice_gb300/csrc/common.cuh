@@ -97,10 +97,11 @@ __device__ __forceinline__ d3 jl_inv_t(d3 p, d3 v) {
 }
 
 // ---- FP64 arithmetic for a narrow FP64 pipe -----------------------------------------------
-// GB300 issues one FP64 warp instruction per 19 cycles and SM (measured: 64 cycles on each of
-// the four sub-partitions alone, adds, multiplies, compares and conversions alike), while the
-// integer and FP32 pipes idle beside it.  So comparisons, sign changes, halvings and
-// conversions are done on the bit patterns, and square roots start from the FP32 estimate.
+// A sub-partition issues one FP64 warp instruction per 64 cycles when one or two of an SM's four do,
+// per 76 when all do: one per 19 cycles and SM (measured: adds, multiplies and fused multiply-adds
+// alike, compares too; conversions from FP64 keep the 64), while the integer and FP32 pipes idle
+// beside it.  So comparisons, sign changes, halvings and conversions are done on the bit patterns,
+// and square roots start from the FP32 estimate.
 
 // v > 0 (false for NaN, as the comparison).
 __device__ __forceinline__ bool positive(double v) {
@@ -209,10 +210,11 @@ __device__ __forceinline__ q4 qnorm_near(q4 q) {
 struct m3 { d3 r0, r1, r2; };
 __device__ __forceinline__ d3 fmrot(const m3& m, d3 v) { return d3{fdot(m.r0, v), fdot(m.r1, v), fdot(m.r2, v)}; }
 
-// ---- unit vectors in fixed point -----------------------------------------------------------
-// An FP64 instruction occupies a sub-partition for 64 cycles, a 32 x 32 -> 64-bit multiply-add for a
+// ---- vectors in fixed point ----------------------------------------------------------------
+// An FP64 instruction occupies a sub-partition for 76 cycles, a 32 x 32 -> 64-bit multiply-add for a
 // few: sums of products of numbers of a few units (rotation matrices, unit quaternions and vectors,
-// rotation vectors; sums up to 32, numbers below 8) are cheaper on the integer pipe, which stands idle beside FP64, and no less exact.
+// rotation vectors; sums up to 32, numbers below 8) are cheaper on the integer pipe, which stands
+// idle beside FP64.
 // A number is (h 2^30 + l) 2^-58, |l| <= 2^29: products of two upper halves, and of an upper and a
 // lower one, sum up in 64 bits each; the lower halves' products, below 2^-58, are left out.  A sum
 // of three products is off by at most 2^-56 = 1.4e-17 (FP64 additions near one: 1.1e-16 each).
@@ -344,7 +346,11 @@ __device__ __forceinline__ FxRot load_rotation(const double4_32a* rec) {
 }
 __device__ __forceinline__ m3 fx_matrix(const FxRot& r) {
     const auto row = [&](const fx3& v) { return d3{fx_double(v.x, r.e - 58), fx_double(v.y, r.e - 58), fx_double(v.z, r.e - 58)}; };
-    return m3{row(r.r0) + d3{1, 0, 0}, row(r.r1) + d3{0, 1, 0}, row(r.r2) + d3{0, 0, 1}};
+    m3 m{row(r.r0), row(r.r1), row(r.r2)};
+    m.r0.x += 1;
+    m.r1.y += 1;
+    m.r2.z += 1;
+    return m;
 }
 // Any vector as fixed point times 2^(e - 1022): its components to one exponent, 58 bits below the
 // largest; false when that is tiny (zero, usually) or huge.
@@ -456,9 +462,6 @@ __device__ __forceinline__ void block_sum_t(double (&v)[NV], double* smem) {
         for (int k = 0; k < NV; k++) v[k] = smem[k * nt];
     __syncthreads();
 }
-
-
-
 
 __device__ __forceinline__ double block_max(double v, double* smem) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;

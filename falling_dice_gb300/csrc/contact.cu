@@ -16,8 +16,8 @@
 // from it depends on the order (pair sets are reported sorted).  A pair is examined only in the cell that is the
 // minimum corner of the intersection of the two shapes' cell ranges: every pair that
 // shares a cell is examined exactly once -- the reference's `tested` set without a set.
-// A conservative FP32 AABB test and the local-shape exclusion (sim.cpp:24-39) run before
-// the FP64 narrow phase.
+// A conservative box test (32 levels per axis inside the bin), the local-shape exclusion
+// (sim.cpp:24-39) and certified FP32 distance bounds run before the FP64 narrow phase.
 //
 // Sums without an order.  Candidates, kept candidates and contacts are appended to flat lists in
 // whatever order the warps arrive; a contact's forces and energy are added to its nodes' records
@@ -159,7 +159,7 @@ __device__ __forceinline__ bool is_connected(const DevTopo& t, int u, int v) {
 
 // Local shapes (sim.cpp:24-39): a shared node, or a connected node pair.  Shapes are
 // distinct here, so "same beam" cannot occur.  The shared-node half is cheap and decides
-// most broad-phase candidates in a lattice; the connected half scans adjacency lists.
+// most broad-phase candidates in a lattice; the connected half probes the hash set.
 __device__ __forceinline__ bool any_connected(const DevTopo& t, int2 a, int2 b) {
     const int an[2] = {a.x, a.y}, bn[2] = {b.x, b.y};
     const int na = a.y >= 0 ? 2 : 1, nb = b.y >= 0 ? 2 : 1;
@@ -363,6 +363,10 @@ struct PairShared {
 // node (three quarters of them share one in a cubic+BCC lattice) 32 at a time.  Candidates go on
 // to the flat list with one atomic and coalesced stores per flush; past cand_cap they are counted
 // but not stored and kOverCandidates is raised.
+// Every loop ends and every lane reaches every warp operation: nq, n and the claimed units are the
+// same in all lanes; a pass of add takes at least one bit from each lane that has one, at most
+// 32 kPairRound into a queue that holds less than 32 before; check takes min(32, nq) from it; a claim
+// moves the cursor on, so a warp claims until the units are gone.  No warp waits for another.
 struct PairQueue {
     PairShared& s;
     int nq, n;  // pairs queued, candidates held: the same in all lanes
@@ -867,7 +871,9 @@ long long pair_units(long long bins, int slots) { return bins * ((slots + kChunk
 // per SM when it runs beside the FP64 beam kernel (shared).  That one lives on the FP64 pipe, this
 // on the integer pipe, but whichever fills the SMs' registers runs alone.  A call of the largest
 // lattice (2.95 million beams): 1980 us with eight blocks an SM, 1934 with five, 1915 with four, 1927
-// with three; compressed 32x32x16, where the contacts take longer than the beams: 259, 247, 243, 260.
+// with three; compressed 32x32x16, where the contacts take longer than the beams: 259, 247, 243, 260;
+// where no list is built or the lattice is small, no difference (eight / four: 19x15x11 81.3 / 81.3, a
+// batch of 48 lattices 455 / 456).
 int contact_pair_blocks(long long shapes, bool shared) {
     const long long b = shapes / 128, most = shared ? 4 * 152 / (8 / kPairWarps) : 4 * 152;
     return int(b < 1 ? 1 : (b > most ? most : b));

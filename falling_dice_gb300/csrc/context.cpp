@@ -37,7 +37,6 @@ using namespace mcg;
 
 namespace {
 
-constexpr double kInf = std::numeric_limits<double>::infinity();
 
 struct Fail : std::runtime_error {
     int code;
@@ -254,9 +253,11 @@ struct mcg_ctx {
     // pipe or memory): its branch of the graph is captured on this stream, whose priority lets
     // the pipeline's kernels in between the beam kernel's blocks.  A graph keeps its nodes'
     // priorities only when instantiated so: without it the first contact kernel started when the
-    // FP64 beam kernel's last block had, 78 us into the 98 us of a compressed 32x32x16 lattice
-    // (evaluation 251 -> 224 us).  The mixed beam kernel is short and better out of the way first
-    // (64x64x32: 667 us a call against 681).
+    // FP64 beam kernel's last block had, 78 us into the 98 us of a compressed 32x32x16 lattice.  FP64
+    // calls with priorities / without: 2x4x2 specimen 56.6 / 56.5 us, 19x15x11 82.8 / 81.6, compressed
+    // 32x32x16 249 / 276, batch of 48 lattices 455 / 455, 80x81x41 1910 / 2304.  The mixed beam kernel is
+    // short and better out of the way first; with / without: compressed 32x32x16 114.5 / 114.4, a
+    // minimization of 32x32x16 2371 / 2372, 64x64x32 659 / 646.
     unsigned long long graph_flags() const { return mixed ? 0 : cudaGraphInstantiateFlagUseNodePriority; }
     cudaStream_t fork = nullptr;
     cudaEvent_t fork_ev[3] = {};
@@ -640,7 +641,7 @@ struct mcg_ctx {
         });
     }
     void read_outs() {
-        sync();  // hp.outs is written by the finalize
+        sync();  // the evaluation's kernels write hp.outs
         check_kernel_error();
     }
     // A kernel's bounded wait that gave up (ev.err, copied into the totals)

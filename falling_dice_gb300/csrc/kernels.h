@@ -78,8 +78,8 @@ constexpr int kBeamBlock = 128;
 // Nodes per evaluation node block (state and gather).
 constexpr int kEvalBlock = 128;
 // Solver blocks an instance's vectors are divided into at most: one per SM.
-constexpr int kFxInvalid = 0x7fffffff;  // the upper half of a fixed-point number that is none
 constexpr int kSolveBlocks = 152;
+constexpr int kFxInvalid = 0x7fffffff;  // the upper half of a fixed-point number that is none
 
 #if defined(__CUDACC__)
 // Position of a thread of a mapped block: element index, instance; valid == false past the
@@ -102,7 +102,8 @@ struct PhysParams {
     int self_contact;
 };
 
-// Totals of one evaluation, written by the finalize kernel.
+// Totals of one evaluation: of an instance, by the last of its gather blocks or by k_finalize; the
+// evaluation's flags (overflow, kernel_error), in the first instance's, by the first gather block.
 struct EvalOut {
     double energy, elastic, plastic, contact, reaction, max_pen;
     int contacts, nonfinite;
@@ -162,7 +163,7 @@ struct ContactBufs {
                             //      rebuilt by this evaluation, [2] rebuild forced (by the host,
                             //      or by a build that overflowed), [3] the pair pass's
                             //      cursor, [4] builds since allocation.  [0] and
-                            //      [1] are zero between evaluations (cleared by the finalize)
+                            //      [1] are zero between evaluations (cleared by the gather)
     uint32_t* counts;       // [kContactCounts]
     float4* xref;           // [N] node positions (FP32, rounded down) when the list was built
     // bins of fixed capacity: the shapes of bin b at bin_items[b * bin_slots ...]

@@ -364,17 +364,20 @@ __device__ __forceinline__ u3 deviation(const FxRot& r, const fx3& e0, u3 te, in
 }
 
 // ---- beam kernel: MC/src/sim.cpp:139-141 ---------------------------------------------------
-// Bound by the FP64 pipe (one warp instruction per 16 cycles and SM, beside which loads and the
+// Bound by the FP64 pipe (one warp instruction per 19 cycles and SM, beside which loads and the
 // other pipes are idle), so the formulas are written for few FP64 instructions: energies summed
 // as twice their value, shear from the director-chord differences (2 t - da - db = -(ma + mb)),
 // square roots from the FP32 estimate, comparisons on bit patterns, and everything that is a sum of
 // products of unit vectors and rotation vectors (directors, relative rotation, material axis, trial
 // twist and bending, the moment's transport and rotation) or a polynomial of one's coordinates in
-// fixed point on the integer pipe.  The error against 64 bits is no larger for it (1.2e-16 against
-// 1.3e-16 on the largest lattice, 1.1e-16 / 1.2e-16 in a batch of 48): a fixed-point sum rounds once.
-// FP64 instructions per 32 beams: 391 at first, 265 with all of it in FP64, 130 now (3500 in all).
-// The kernel alone: 184,400 beams 159 -> 98 -> 66 us, 2.95 million 1372 -> 818 us (80 % of the FP64
-// pipe's rate); a call at 2.95 million beams 2474 -> 1914 us, a batch of 762,000 beams 603 -> 450.
+// fixed point on the integer pipe.  A fixed-point sum rounds once: per beam against quadruple
+// precision, rotations from 1e-15 to 1, the moment's median error is 0.7e-16 to 1.8e-16 (all in FP64:
+// 0.9e-16 to 2.2e-16).
+// FP64 instructions per 32 beams: 391 at first, 265 with all of it in FP64, 135 now (3430 in all;
+// 132 and 3170 without the vectors' exponents, which cost 4 % of the kernel's time).
+// The kernel alone: 184,400 beams 159 -> 98 -> 66 us, 2.95 million 1372 -> 835 us (one FP64
+// instruction per 21 cycles and SM; nothing but FP64 reaches 19); a call at 2.95 million beams 2474 ->
+// 1895 us, a batch of 762,000 beams 603 -> 455.
 // Blocks of kBeamBlock = 128 beams: one warp on each of an SM's four FP64 units, so that a
 // lattice of a few hundred beams spreads over several SMs.
 // kMinBlocks: units of 256 threads per SM the register allocation must allow (an occupancy
@@ -457,8 +460,8 @@ __global__ void __launch_bounds__(kBeamBlock, 2 * kMinBlocks) k_beams(DevTopo t,
             const d3 axis = fx_double(axis_u);
             // trial elastic parts: the twist and the bending of d = phi - rotp, at the larger exponent
             // (|phi| < 4 and |rotp| < sqrt(3)/2 there, so |d| < 5)
-            double dtw;
-            d3 dbend;
+            double dtw = __longlong_as_double(0x7ff8000000000000LL);  // rotp not finite, or so large that
+            d3 dbend{dtw, dtw, dtw};                                  // its square, an energy, is not
             const int ed = max(fx_exponent(rotp), ep);
             if (ed <= kFxMost) {
                 const u3 rp = fx_units(rotp, ed), ph = fx_shr(phi, ed - ep), d{ph.x - rp.x, ph.y - rp.y, ph.z - rp.z};
@@ -467,10 +470,6 @@ __global__ void __launch_bounds__(kBeamBlock, 2 * kMinBlocks) k_beams(DevTopo t,
                 const fx wf = fx_of(w);
                 dtw = fx_double(w, ed - 58);
                 dbend = fx_double(u3{d.x - fx_mul(af.x, wf), d.y - fx_mul(af.y, wf), d.z - fx_mul(af.z, wf)}, ed - 58);
-            } else {
-                const d3 d = fx_double(phi, ep - 58) - rotp;
-                dtw = fdot(d, axis);
-                dbend = fmadd(axis, -dtw, d);
             }
             double ptw = 0;  // the plastic parts enter the trial state only
             d3 pb{0, 0, 0};

@@ -104,3 +104,15 @@ def test_base_orientations_given_to_few_digits_are_normalized(mcg, mco, off):
     sol.commit()
     r = sol.get_state()[1].reshape(-1, 4).astype(np.longdouble)
     assert np.max(np.abs(np.sqrt(np.sum(r * r, axis=1)) - 1)) <= 4 * 2.0 ** -53
+
+
+@pytest.mark.parametrize("value", [np.nan, np.inf, -1e250])
+def test_a_plastic_rotation_that_is_not_finite_or_whose_square_is_not(mcg, mco, value):
+    cfg, lat, sol, orc = model(mcg, mco, "bcc", (2, 2, 2))
+    z, _ = mcg.random_state(lat, 0.02, 0.1, 0.0, 5)
+    pl = np.zeros((lat.n_beams, 7))
+    pl[17, 3] = value
+    for m in (sol, orc):
+        m.set_state(plastic=pl.ravel())
+    r, o = (m.objective(z, lat.geometry.top0 + 0.01) for m in (sol, orc))
+    assert r["energy"] == o["energy"] == np.inf and not np.any(r["grad"]) and not np.any(o["grad"])

@@ -189,7 +189,8 @@ int mcg_objective(mcg_ctx* ctx, const double* z, double top, int trials, double*
  * beams, and per evaluation 4096 grid bins (the grid box of the deformed specimen at the
  * reference's grid cell: about 9 cells per axis of a cube) of at most 128 entries each,
  * 32768 candidate pairs and 8192 contacts; beyond them it returns MCG_ERR_CAPACITY, naming
- * what overflowed.  The first call on a context sets up: it looks up the array's device
+ * what overflowed.  It uses the reference's cell, or a finer one that was set (mcg_set_contact_cell,
+ * mcg_autotune), and a coarser one that was set where that does not fit.  The first call on a context sets up: it looks up the array's device
  * address on the context's device (cudaGetSymbolAddress) and keeps it in the context.  All
  * calls on a device share the array, which keeps the last call's contents: calls that
  * overlap on the GPU race.  After such a call mcg_contact_pairs and mcg_contact_stats

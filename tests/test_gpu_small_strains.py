@@ -65,3 +65,36 @@ def test_moments_of_small_rotations(mcg, mco, sigma, plastic, base):
     assert np.any(moments(o))
     assert rel_err(moments(r), moments(o)) <= 32 * U
     assert rel_err(r["trial_next"].reshape(-1, 7)[:, 2:5], o["trial_next"].reshape(-1, 7)[:, 2:5]) <= 32 * U
+
+
+# The chord's length is the correctly rounded square root the reference takes: the residual
+# correction leaves an error of the order of 2^-104 before the last rounding.  Strains (L - L0) / L0
+# then differ by the quotient's form alone: 1 / L0, a product and a quotient, each to half an ulp.
+@pytest.mark.parametrize("scale", [1.0, 1.0 + 1e-12, 1.0 + 1e-7, 0.9, 3.7, 1e-6, 1e9])
+def test_chord_lengths_are_the_references(mcg, mco, scale):
+    cfg, lat, sol, orc = model(mcg, mco, "bcc", (9, 8, 7), 0.02)
+    for m in (sol, orc):
+        m.set_state(base_x=lat.x0 * scale)
+    z = np.zeros(6 * lat.n_nodes)
+    top = 2.0 * scale
+    a, b = (m.objective(z, top, True)["trial_aux"].reshape(-1, 7)[:, 0] for m in (sol, orc))
+    assert np.all(np.abs(a - b) <= 3 * U * np.abs(b))
+
+
+# Orientations exp(z) from an identity base, as a commit stores them, against the exponential in
+# extended precision: its polynomials' last steps and products, and the normalization, 4 roundings on
+# a component (the angles of both the polynomials and the general form, limit one radian).
+@pytest.mark.parametrize("sigma", [1e-9, 1e-3, 0.3, 0.6, 1.0, 3.0])
+def test_orientations_are_the_exponentials_to_rounding(mcg, mco, sigma):
+    cfg, lat, _, _ = model(mcg, mco, "bcc", (4, 3, 3), 0.02)
+    cfg.max_iterations = 1
+    sol = mcg.Solver(cfg, lat)
+    z, _ = mcg.random_state(lat, 0.0, sigma, 0.0, 14)
+    z = sol.minimize(lat.geometry.top0 + 0.01, z)[0]
+    sol.commit()
+    q = sol.get_state()[1].reshape(-1, 4)
+    v = z.reshape(-1, 6)[:, 3:].astype(np.longdouble)
+    a = np.sqrt(np.sum(v * v, axis=1, keepdims=True))
+    s = np.where(a > 0, np.sin(a / 2) / np.where(a > 0, a, 1), np.longdouble(0.5))
+    want = np.hstack([np.cos(a / 2), s * v])
+    assert np.max(np.abs(q - want)) <= 4 * U
